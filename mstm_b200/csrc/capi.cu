@@ -140,14 +140,23 @@ static void find_hosts(mstmg_ctx* c, const std::vector<double>& ri)
 // Upload the tiles of this context's shard (all tiles when nshards == 1).
 int apply_shard(mstmg_ctx* c)
 {
+    c->tgroups = c->tgroups_host;
     std::vector<int4> sub;
-    sub.reserve(c->tiles_host.size() / (size_t)c->nshards + 1);
-    for (size_t t = 0; t < c->tiles_host.size(); t++)
-        if ((int)(t % (size_t)c->nshards) == c->shard) sub.push_back(c->tiles_host[t]);
-    c->ntiles = (int)sub.size();
-    if (!sub.empty()) {
-        CK(c->tiles.alloc(sub.size()));
-        CK(cudaMemcpyAsync(c->tiles.p, sub.data(), sizeof(int4) * sub.size(), cudaMemcpyHostToDevice, c->st));
+    const std::vector<int4>* use = &c->tiles_host;
+    if (c->nshards > 1) {
+        sub.reserve(c->tiles_host.size() / (size_t)c->nshards + 1);
+        for (auto& g : c->tgroups) g.count = 0;
+        for (size_t t = 0; t < c->tiles_host.size(); t++)
+            if ((int)(t % (size_t)c->nshards) == c->shard) {
+                auto& g = c->tgroups[c->tiles_host[t].w];
+                if (g.count++ == 0) g.first = (int)sub.size();   // the tiles are in group order
+                sub.push_back(c->tiles_host[t]);
+            }
+        use = &sub;
+    }
+    if (!use->empty()) {
+        CK(c->tiles.alloc(use->size()));
+        CK(cudaMemcpyAsync(c->tiles.p, use->data(), sizeof(int4) * use->size(), cudaMemcpyHostToDevice, c->st));
         CK(cudaStreamSynchronize(c->st));
     }
     c->layout_gen++;
@@ -169,43 +178,114 @@ int check_kernel_err(mstmg_ctx* c)
     return MSTMG_OK;
 }
 
-// Install a pair list (i < j) and, for the tiled kernel, its tiles: operator
-// record offsets, the device copies, and invalidated operators.
-int upload_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np, const std::vector<int4>& tl)
+// Spheres a tile group takes: 4 when the tiles fill many waves of two CTAs
+// per SM, fewer for smaller clusters (finer work) and larger orders (shared
+// memory holds the outputs of two groups).
+int tile_group_size(const mstmg_ctx* c, long long npairs, int L)
 {
-    std::vector<long long> off(np > 0 ? np : 1);
+    int B = L <= 4 ? 4 : L <= 8 ? 2 : 1;
+    while (B > 1 && npairs < 12LL * B * B * c->nsm) B /= 2;
+    return B;
+}
+
+// Install a pair list (i < j): operator record offsets, and with `ts` its
+// tiles (the pairs then in tile order).  Tiles are sorted by the largest
+// order among their pairs into launch groups of at least a few waves of
+// CTAs, whose work buffers have the strides of the group's largest order.
+int upload_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np, const TileSet* ts)
+{
+    // record lengths by order pair
+    std::vector<int> rec((MSTMG_LMAX + 1) * (MSTMG_LMAX + 1), 0);
+    for (int a = 1; a <= MSTMG_LMAX; a++)
+        for (int b = 1; b <= MSTMG_LMAX; b++) rec[a * (MSTMG_LMAX + 1) + b] = op_record_units(a, b);
+    auto rec_of = [&](const int2& q) { return rec[c->order[q.x] * (MSTMG_LMAX + 1) + c->order[q.y]]; };
+    const int omin = *std::min_element(c->order.begin(), c->order.end()), omax = *std::max_element(c->order.begin(), c->order.end());
+    const bool same = omin == omax;   // one order: offsets are multiples of one length
+    std::vector<long long> off(np > 0 && !same ? np : 1);
     long long u = 0;
     int maxrec = 4, pl = 1, lo = 1 << 30;
-    for (int t = 0; t < np; t++) {
+    if (same && np > 0) {
+        maxrec = rec_of(pr[0]);
+        pl = lo = omax;
+        u = (long long)np * maxrec;
+    }
+    for (int t = 0; t < np && !same; t++) {
         off[t] = u;
-        int rec = op_record_units(c->order[pr[t].x], c->order[pr[t].y]);
-        maxrec = std::max(maxrec, rec);
-        pl = std::max(pl, std::max(c->order[pr[t].x], c->order[pr[t].y]));
-        lo = std::min(lo, std::min(c->order[pr[t].x], c->order[pr[t].y]));
-        u += rec;
+        const int r = rec_of(pr[t]), li = c->order[pr[t].x], lj = c->order[pr[t].y];
+        maxrec = std::max(maxrec, r);
+        pl = std::max(pl, std::max(li, lj));
+        lo = std::min(lo, std::min(li, lj));
+        u += r;
     }
     c->npairs = np;
     c->pair_lmax = pl;
     c->pair_uniform = np > 0 && lo == pl;
-    c->tiles_host = tl;
-    if (!c->tiled) {   // shards need tiles; a re-layout without them drops the shard
-        c->shard = 0;
-        c->nshards = 1;
-    }
-    if (int rs = apply_shard(c)) return rs;
-    c->op_units = u;
-    c->maxrec = maxrec;
-    // FP32 passes of the tiled path run the row kernel on row records unless
-    // the rotation-tiled kernel is asked for (tile_pairs 1 or 2)
-    c->row32 = (c->tiled && c->opts.tile_pairs == 0 && rows_supported(c->tile_L, 1)) ? row_record_units(c->tile_L) : 0;
-    c->layout_gen++;
+    c->tiles_host.clear();
+    c->tgroups_host.clear();
+    c->tslots = 0;
+    if (ts && u / 4 > 0xffffffffLL) ts = nullptr;   // past the tiles' record range: the order-generic kernel
+    if (!ts) c->tiled = false;
     if (np > 0) {
         CK(c->pairs.alloc(np));
         CK(c->opoff.alloc(np));
         CK(cudaMemcpyAsync(c->pairs.p, pr.data(), sizeof(int2) * np, cudaMemcpyHostToDevice, c->st));
-        CK(cudaMemcpyAsync(c->opoff.p, off.data(), sizeof(long long) * np, cudaMemcpyHostToDevice, c->st));
-        CK(cudaStreamSynchronize(c->st));   // host vectors are freed on return
+        if (same) launch_pair_offsets(np, maxrec, c->opoff.p, c->nsm, c->st);
+        else CK(cudaMemcpyAsync(c->opoff.p, off.data(), sizeof(long long) * np, cudaMemcpyHostToDevice, c->st));
     }
+    DevBuf<uchar2> ps;
+    if (ts && np > 0) {
+        c->tslots = ts->slots;
+        CK(c->tsph.alloc(ts->ts.size()));
+        CK(c->tpairs.alloc(np));
+        CK(ps.alloc(np));
+        CK(cudaMemcpyAsync(c->tsph.p, ts->ts.data(), sizeof(int) * ts->ts.size(), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(ps.p, ts->ps.data(), sizeof(uchar2) * np, cudaMemcpyHostToDevice, c->st));
+        launch_mma_pairs(np, c->pairs.p, ps.p, c->d_order.p, c->d_offset.p, c->opoff.p, c->tpairs.p, c->nsm, c->st);
+        CK(cudaGetLastError());
+        auto& gs = c->tgroups_host;
+        const size_t nt = ts->tl.size();
+        if (lo == pl) {
+            c->tiles_host = ts->tl;
+            gs.push_back({0, (int)nt, pl, 1, maxrec});
+        } else {
+            struct TileInfo { int L, lo, rec; };
+            std::vector<TileInfo> ti(nt, TileInfo{0, 1 << 30, 0});
+            std::vector<int> idx(nt);
+            for (size_t k = 0; k < nt; k++) {
+                idx[k] = (int)k;
+                for (int q = ts->tl[k].x; q < ts->tl[k].x + ts->tl[k].y; q++) {
+                    const int li = c->order[pr[q].x], lj = c->order[pr[q].y];
+                    ti[k].L = std::max(ti[k].L, std::max(li, lj));
+                    ti[k].lo = std::min(ti[k].lo, std::min(li, lj));
+                    ti[k].rec = std::max(ti[k].rec, rec_of(pr[q]));
+                }
+            }
+            std::stable_sort(idx.begin(), idx.end(), [&](int x, int y) { return ti[x].L > ti[y].L; });
+            const int least = 4 * c->nsm;
+            c->tiles_host.reserve(nt);
+            for (size_t k = 0; k < nt; k++) {
+                const TileInfo& w = ti[idx[k]];
+                if (gs.empty() || (w.L < ti[idx[k - 1]].L && gs.back().count >= least && (int)(nt - k) >= least))
+                    gs.push_back({(int)k, 0, w.L, 1, 4});
+                auto& g = gs.back();
+                g.count++;
+                g.maxrec = std::max(g.maxrec, w.rec);
+                if (w.lo != g.L || w.L != g.L) g.uniform = 0;
+                int4 tile = ts->tl[idx[k]];
+                tile.w = (int)gs.size() - 1;
+                c->tiles_host.push_back(tile);
+            }
+        }
+    }
+    if (!c->tiled) {   // shards need tiles of one order; a re-layout without them drops the shard
+        c->shard = 0;
+        c->nshards = 1;
+    }
+    if (int rs = apply_shard(c)) return rs;   // synchronises: the host vectors and slots are done with
+    CK(cudaStreamSynchronize(c->st));
+    c->op_units = u;
+    c->maxrec = maxrec;
+    c->layout_gen++;
     c->ops64_ready = c->ops32_ready = false;
     if (c->tc_state == 1) c->tc_state = 0;
     return MSTMG_OK;
@@ -294,7 +374,7 @@ static int setup_host_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np)
     h.hunits = u;
     h.hmaxrec = maxrec;
     h.hlmax = hl;
-    h.hops_ready = h.hops32_ready = false;
+    h.hops_ready = false;
     if (h.nhp > 0) {
         CK(h.hpairs.alloc(h.nhp));
         CK(h.hopoff.alloc(h.nhp));
@@ -474,27 +554,16 @@ int setup_layout(mstmg_ctx* c)
         return MSTMG_ERR_UNSUPPORTED;
     }
     c->npairs = (int)np;
-    // Pair order.  Monodisperse clusters of a supported order use tiles of
-    // TILE_B x TILE_B sphere blocks (translate_tiled.cu); the block pairs are
-    // visited in round-robin tournament order (circle method), so tiles that
-    // run at the same time write mostly disjoint spheres.  Otherwise the pairs
-    // themselves follow the tournament order: each round holds floor(N/2)
-    // pairs with no sphere in common, so concurrent CTAs' atomic adds do not
-    // collide.  Pairs keep i < j, the reference's orientation of the operator.
-    std::vector<int2> pr(np > 0 ? np : 1);
-    std::vector<long long> off(np > 0 ? np : 1);
-    long long u = 0;
-    int maxrec = 4;
-    long long t = 0;
-    auto add_pair = [&](int i, int j) {
-        pr[t] = make_int2(i, j);
-        off[t] = u;
-        int rec = op_record_units(c->order[i], c->order[j]);
-        maxrec = std::max(maxrec, rec);
-        u += rec;
-        t++;
-    };
-    auto tournament = [](int n, std::vector<std::pair<int, int>>& out) {
+    // Pair order.  The spheres, sorted by host and order, form groups; a tile
+    // (translate_mma.cu) holds the pairs between two groups or inside one, and
+    // the group pairs are visited in round-robin tournament order (circle
+    // method), so tiles that run at the same time write mostly disjoint
+    // spheres.  For the order-generic kernel the pairs themselves follow the
+    // tournament order: each round holds floor(N/2) pairs with no sphere in
+    // common, so concurrent CTAs' atomic adds do not collide.  Pairs keep
+    // i < j, the reference's orientation of the operator.
+    std::vector<int2> pr;
+    auto tournament = [](int n, auto&& visit) {
         int M = (n % 2 == 0) ? n : n + 1;
         for (int r = 0; r < M - 1 && n > 1; r++)
             for (int k = 0; k < M / 2; k++) {
@@ -502,74 +571,69 @@ int setup_layout(mstmg_ctx* c)
                 if (k == 0) { a_ = M - 1; b_ = r; }
                 else { a_ = (r + k) % (M - 1); b_ = (r - k + (M - 1)) % (M - 1); }
                 if (a_ >= n || b_ >= n) continue;
-                out.push_back({std::min(a_, b_), std::max(a_, b_)});
+                visit(std::min(a_, b_), std::max(a_, b_));
             }
     };
-    c->tiled = !c->opts.generic_kernel && !hs.on() && (lm == lmin) && lmin >= tso && tiled_supported(lm, 1) && n > 1 && n < 65536;
-    std::vector<int4> tl;
-    if (c->tiled) {
-        const int B = TILE_B;
-        int nb = (n + B - 1) / B;
-        std::vector<std::pair<int, int>> bp;
-        tournament(nb, bp);
-        for (int I = 0; I < nb; I++) bp.push_back({I, I});
-        for (auto& IJ : bp) {
-            int I = IJ.first, J = IJ.second;
-            int i0 = I * B, j0 = J * B;
-            int start = (int)t;
-            // inside a tile, consecutive pairs (0,1), (2,3), ... share no
-            // sphere wherever the tile is whole: an off-diagonal tile runs the
-            // diagonals (a, a+s mod B) of its block pair, a diagonal tile the
-            // matchings {01, 23}, {02, 13}, {03, 12}; the row kernel takes two
-            // such pairs a step
-            static_assert(TILE_B == 4, "the diagonal-tile order below is for blocks of 4 spheres");
-            static const int dg[6][2] = {{0, 1}, {2, 3}, {0, 2}, {1, 3}, {0, 3}, {1, 2}};
-            auto try_add = [&](int i, int j) {
-                if (i < n && j < n && i < j && same_cfg(i, j)) add_pair(i, j);
-            };
-            if (I == J) {
-                for (const auto& d : dg) try_add(i0 + d[0], i0 + d[1]);
-            } else {
-                for (int sft = 0; sft < B; sft++)
-                    for (int a_ = 0; a_ < B; a_++) try_add(i0 + a_, j0 + (a_ + sft) % B);
-            }
-            int cnt = (int)t - start;
-            if (cnt > 0) tl.push_back(make_int4(start, cnt, (i0 << 16) | j0, I == J ? 1 : 0));
+    c->tiled = !c->opts.generic_kernel && !hs.on() && (lm == lmin) && lmin >= tso && tiled_order(lm) && n > 1 && n < 65536;
+    TileSet ts;
+    if (!c->opts.generic_kernel) {
+        std::vector<int> ord(n);
+        for (int i = 0; i < n; i++) ord[i] = i;
+        std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) {
+            const int hx = hs.on() ? hs.host[x] : 0, hy = hs.on() ? hs.host[y] : 0, cx = c->cfg_of.empty() ? 0 : c->cfg_of[x],
+                      cy = c->cfg_of.empty() ? 0 : c->cfg_of[y];
+            if (hx != hy) return hx < hy;
+            if (cx != cy) return cx < cy;
+            return c->order[x] > c->order[y];
+        });
+        int pl = 1;   // the largest order that has pairs on the tiles
+        for (int u = 0, v = 0; u < n; u = v) {
+            int many = 0, top = 1;
+            for (v = u; v < n && same_cfg(ord[u], ord[v]); v++)
+                if (c->order[ord[v]] >= tso) {
+                    many++;
+                    top = std::max(top, c->order[ord[v]]);
+                }
+            if (many > 1) pl = std::max(pl, top);
         }
+        const int B = tile_group_size(c, np, pl), nb = (n + B - 1) / B;
+        ts.slots = 2 * B;
+        ts.pr.reserve(np > 0 ? np : 1);
+        ts.ps.reserve(np > 0 ? np : 1);
+        auto add_tile = [&](int I, int J) {
+            const int start = (int)ts.pr.size();
+            for (int sft = 0; sft < B; sft++)
+                for (int a_ = 0; a_ < B; a_++) {
+                    const int b_ = (a_ + sft) % B, u = I * B + a_, v = J * B + b_;
+                    if (u >= n || v >= n || (I == J && a_ >= b_)) continue;
+                    const int i = std::min(ord[u], ord[v]), j = std::max(ord[u], ord[v]);
+                    if (!same_cfg(i, j) || dense_pair(i, j)) continue;
+                    const unsigned char su = (unsigned char)a_, sv = (unsigned char)(I == J ? b_ : B + b_);
+                    ts.pr.push_back(make_int2(i, j));
+                    ts.ps.push_back(i == ord[u] ? make_uchar2(su, sv) : make_uchar2(sv, su));
+                }
+            if ((int)ts.pr.size() == start) return;
+            ts.tl.push_back(make_int4(start, (int)ts.pr.size() - start, (int)ts.tl.size(), 0));
+            const size_t row = ts.ts.size();
+            ts.ts.resize(row + ts.slots, -1);
+            for (int q = start; q < (int)ts.pr.size(); q++) {   // only the spheres the tile's pairs write
+                ts.ts[row + ts.ps[q].x] = ts.pr[q].x;
+                ts.ts[row + ts.ps[q].y] = ts.pr[q].y;
+            }
+        };
+        tournament(nb, add_tile);
+        for (int I = 0; I < nb; I++) add_tile(I, I);
+        pr.swap(ts.pr);
     } else {
-        std::vector<std::pair<int, int>> pp;
-        tournament(n, pp);
-        for (auto& ij : pp)
-            if (same_cfg(ij.first, ij.second) && !dense_pair(ij.first, ij.second)) add_pair(ij.first, ij.second);
+        tournament(n, [&](int i, int j) {
+            if (same_cfg(i, j) && !dense_pair(i, j)) pr.push_back(make_int2(i, j));
+        });
     }
-    if (t != np) {
+    if ((long long)pr.size() != np) {
         set_err("internal error: pair schedule incomplete");
         return MSTMG_ERR_ARG;
     }
-    c->tile_L = lm;
-    c->tsph.release();   // block tiles
-    c->pslot.release();
-    if (hs.on() && !c->opts.generic_kernel && np > 0) {
-        // host spheres: when the pairs inside the hosts all have one order
-        // the tiled kernels take them on grouped tiles (the spheres of each
-        // host in groups, each sphere's block at its own offset)
-        const int L0 = c->order[pr[0].x];
-        bool uni = true;
-        for (long long q = 0; q < np && uni; q++) uni = c->order[pr[q].x] == L0 && c->order[pr[q].y] == L0;
-        if (uni && L0 >= tso && tiled_supported(L0, 1)) {
-            std::vector<char> inp(n, 0);
-            for (long long q = 0; q < np; q++) inp[pr[q].x] = inp[pr[q].y] = 1;
-            std::vector<std::vector<int>> members(n + 1);   // by host, the spheres outside every other first
-            for (int i = 0; i < n; i++)
-                if (inp[i]) members[hs.host[i] + 1].push_back(i);
-            if (int rg = group_tiles(c, members, pr, tl)) return rg;
-            c->tiled = true;
-            c->tile_L = L0;
-        }
-    }
-    (void)off;
-    (void)maxrec;
-    int rc_ = upload_pairs(c, pr, (int)np, tl);
+    int rc_ = upload_pairs(c, pr, (int)np, c->opts.generic_kernel ? nullptr : &ts);
     if (rc_) return rc_;
     if (hs.on()) {
         rc_ = setup_host_pairs(c, pr, (int)np);
@@ -805,7 +869,6 @@ extern "C" void mstmg_ctx_destroy(mstmg_ctx* c)
     DevBuf<zf>* fb[] = {&c->X32, &c->Y32, &c->vec32, &c->rvec32};
     for (auto* b : fb) b->release();
     c->an32.release();
-    c->op32.release();
     c->pairs.release();
     c->tiles.release();
     c->opoff.release();

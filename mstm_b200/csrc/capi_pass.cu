@@ -1,5 +1,5 @@
 // capi_pass.cu -- the pair operators and the translation passes behind the C
-// ABI: operator generation, the rotation kernels (tiled / order-generic), the
+// ABI: operator generation, the rotation kernels (tiles / order-generic), the
 // tensor-core pass of many columns, the FFT path (node_selection, the kernel
 // spectra and fft_external_to_external_expansion), sphereinteraction and the
 // translation-pass entry points.
@@ -58,13 +58,15 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
         if (need32) c->ops32_ready = true;
         return MSTMG_OK;
     }
+    // the rotation records serve the passes of either precision
+    if (!force && c->ops64_ready) {
+        c->ops32_ready = true;
+        return MSTMG_OK;
+    }
     {
-        const void* was[2] = {c->op64.p, c->op32.p};
-        if (need64) CK(c->op64.alloc(c->op_units));
-        if (need32) CK(c->op32.alloc(c->row32 ? (long long)c->npairs * c->row32 : c->op_units));
-        if (was[0] != c->op64.p || was[1] != c->op32.p) c->layout_gen++;
-        // row records: the padding of every row reads as zero
-        if (need32 && c->row32) CK(cudaMemsetAsync(c->op32.p, 0, sizeof(float) * (size_t)c->npairs * c->row32, c->st));
+        const void* was = c->op64.p;
+        CK(c->op64.alloc(c->op_units));
+        if (was != c->op64.p) c->layout_gen++;
     }
     NvtxRange nvtx_("pair operator generation");
     OpGenArgs a;
@@ -73,9 +75,7 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
     a.pos = c->pos.p;
     a.order = c->d_order.p;
     a.opoff = c->opoff.p;
-    a.op64 = need64 ? c->op64.p : nullptr;
-    a.op32 = need32 ? c->op32.p : nullptr;
-    a.row32 = c->row32;
+    a.op64 = c->op64.p;
     a.vcc = c->vcc.p;
     a.vnmax = c->vn;
     a.fnr = c->fnr.p;
@@ -89,28 +89,24 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
     a.xi = c->opgen_xi.p;
     launch_opgen(a, c->nsm, c->st);
     CK(cudaGetLastError());
-    if ((need64 || need32) && c->hs.nhp > 0) {
+    if (c->hs.nhp > 0) {
         // regular translations between hosts and the spheres they hold, in
         // the host's index (external_to_internal_expansion, modules:6579-6592)
         HostSpheres& h = c->hs;
-        if (need64) CK(h.hop64.alloc(h.hunits));
-        if (need32) CK(h.hop32.alloc(h.hunits));
+        CK(h.hop64.alloc(h.hunits));
         OpGenArgs b = a;
         b.npairs = h.nhp;
         b.pairs = h.hpairs.p;
         b.pos = h.xpos.p;
         b.opoff = h.hopoff.p;
-        b.op64 = need64 ? h.hop64.p : nullptr;
-        b.op32 = need32 ? h.hop32.p : nullptr;
-        b.row32 = 0;
+        b.op64 = h.hop64.p;
         b.pmed = h.hmed.p;
         b.regular = 1;
         launch_opgen(b, c->nsm, c->st);
         CK(cudaGetLastError());
-        if (need64) h.hops_ready = true;
-        if (need32) h.hops32_ready = true;
+        h.hops_ready = true;
     }
-    if (need64) c->ops64_ready = true;
+    c->ops64_ready = true;
     if (need32) c->ops32_ready = true;
     return MSTMG_OK;
 }
@@ -121,7 +117,7 @@ template <typename T> int translate_hosts(mstmg_ctx* c, const cpx<T>* x, cpx<T>*
     HostSpheres& h = c->hs;
     if (!h.on()) return MSTMG_OK;
     if (h.nhp > 0) {
-        if (sizeof(T) == 8 ? !h.hops_ready : !h.hops32_ready) {
+        if (!h.hops_ready) {
             set_err("internal error: host-sphere operators not generated");
             return MSTMG_ERR_ARG;
         }
@@ -130,7 +126,7 @@ template <typename T> int translate_hosts(mstmg_ctx* c, const cpx<T>* x, cpx<T>*
         a.pairs = h.hpairs.p;
         a.order = c->d_order.p;
         a.offset = c->d_offset.p;
-        a.ops = sizeof(T) == 8 ? (const T*)h.hop64.p : (const T*)h.hop32.p;
+        a.ops = h.hop64.p;
         a.opoff = h.hopoff.p;
         a.x = x;
         a.y = y;
@@ -168,92 +164,54 @@ template void mie_all<float>(mstmg_ctx*, int, int, const zf*, zf*);
 
 int ensure_ops(mstmg_ctx* c, int prec, bool force) { return ensure_ops_both(c, prec == 0, prec == 1, force); }
 
-template <typename T> static const T* ops_ptr(mstmg_ctx* c);
-template <> const double* ops_ptr<double>(mstmg_ctx* c) { return c->op64.p; }
-template <> const float* ops_ptr<float>(mstmg_ctx* c) { return c->op32.p; }
-
-// FP32 passes on row records: the row kernel, in groups of 4, 2 or 1 columns
-// when the pass has another column count (the records fit no other kernel)
-template <typename T> static int rows_pass(mstmg_ctx*, const TiledArgs<T>&, int, int, unsigned) { return -1; }
-template <> int rows_pass<float>(mstmg_ctx* c, const TiledArgs<float>& tf, int nrhs, int nchunk, unsigned contran)
+// FP64 copies of up to ncols FP32 columns for translate<float>; called ahead
+// of a stream capture, which cannot allocate
+int ensure_wide(mstmg_ctx* c, int ncols)
 {
-    if (rows_supported(c->tile_L, nrhs)) return launch_translate_rows(tf, c->tile_L, c->nsm, c->st);
-    if (nchunk != 1) return -1;
-    int rc = 0;
-    for (int c0 = 0; c0 < nrhs && rc == 0;) {
-        const int w = nrhs - c0 >= 4 ? 4 : (nrhs - c0 >= 2 ? 2 : 1);
-        TiledArgs<float> tw = tf;
-        tw.x = tf.x + (size_t)c0 * c->neqns;
-        tw.y = tf.y + (size_t)c0 * c->neqns;
-        tw.nrhs = w;
-        tw.contran = (contran >> c0) & ((1u << w) - 1u);
-        rc = launch_translate_rows(tw, c->tile_L, c->nsm, c->st);
-        c0 += w;
-    }
-    return rc;
+    const size_t need = 2 * (size_t)c->neqns * ncols;
+    if (c->tgroups_host.empty() || c->wide.n >= need) return MSTMG_OK;
+    c->layout_gen++;
+    CK(c->wide.alloc(need));
+    return MSTMG_OK;
 }
 
-// y[:, 0:nrhs*nchunk] = H x[:, 0:nrhs*nchunk]  (y zeroed here).  nchunk > 1
-// only on the tiled path: contran then applies to column r of every chunk.
-template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int nrhs, unsigned contran, int nchunk)
+// y[:, 0:ncols] = H x[:, 0:ncols]  (y zeroed here); column k is a
+// conjugate-transpose product when bit (k mod period) of contran is set
+// (period 32, one bit a column, or 1, 2 or 4).
+template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period)
 {
     NvtxRange nvtx_(sizeof(T) == 8 ? "translation pass FP64" : "translation pass FP32");
-    CK(cudaMemsetAsync(y, 0, sizeof(cpx<T>) * (size_t)c->neqns * nrhs * nchunk, c->st));
-    if (c->hs.on()) {
-        if (nchunk > 1) return MSTMG_ERR_UNSUPPORTED;
-        int rh = translate_hosts<T>(c, x, y, nrhs, contran);
-        if (rh) return rh;
-    }
+    const size_t ld = (size_t)c->neqns;
+    const bool wide = sizeof(T) == 4 && !c->tgroups_host.empty();   // FP32 columns through the FP64 tiles
+    const bool parts = c->hs.on() || c->ndense > 0;                 // contributions before the tiles'
+    if (!wide || parts) CK(cudaMemsetAsync(y, 0, sizeof(cpx<T>) * ld * ncols, c->st));
+    // the parts that take up to four columns a launch
+    auto groups = [&](auto&& part) -> int {
+        for (int k = 0; k < ncols; k += 4) {
+            const int w = std::min(4, ncols - k);
+            unsigned m = 0;
+            for (int r = 0; r < w; r++) m |= ((contran >> ((k + r) % period)) & 1u) << r;
+            if (int rc = part(x + k * ld, y + k * ld, w, m)) return rc;
+        }
+        return MSTMG_OK;
+    };
+    if (c->hs.on())
+        if (int rh = groups([&](const cpx<T>* xk, cpx<T>* yk, int w, unsigned m) { return translate_hosts<T>(c, xk, yk, w, m); })) return rh;
     if (c->ndense > 0) {
-        if (nchunk > 1) return MSTMG_ERR_UNSUPPORTED;
         const T* drec = sizeof(T) == 8 ? (const T*)c->dop64.p : (const T*)c->dop32.p;
-        launch_dense_apply<T>(dense_args(c), drec, x, y, c->neqns, nrhs, contran, c->st);
+        groups([&](const cpx<T>* xk, cpx<T>* yk, int w, unsigned m) {
+            launch_dense_apply<T>(dense_args(c), drec, xk, yk, c->neqns, w, m, c->st);
+            return MSTMG_OK;
+        });
         CK(cudaGetLastError());
     }
     // a sharded context: shard 0 adds the FFT path's far field, every shard its near-pair tiles
     const bool far = c->fft && c->fft->on && c->shard == 0;
-    if (c->npairs == 0) return far ? fft_far<T>(c, x, y, nrhs * nchunk, contran) : MSTMG_OK;
-    TransArgs<T> a;
-    a.npairs = c->npairs;
-    a.pairs = c->pairs.p;
-    a.order = c->d_order.p;
-    a.offset = c->d_offset.p;
-    a.ops = ops_ptr<T>(c);
-    a.opoff = c->opoff.p;
-    a.x = x;
-    a.y = y;
-    a.ld = c->neqns;
-    a.nrhs = nrhs;
-    a.contran = contran;
-    a.lmax = c->pair_lmax;
-    a.uniform = c->pair_uniform ? 1 : 0;
-    a.maxrec = c->maxrec;
-    a.err = c->err.p;
-    TiledArgs<T> ta;
-    // FP64 passes of orders 3 and 4 run the order-generic kernel on the tile
-    // ordered pairs (faster there than the rotation-tiled kernel); FP32 passes
-    // take the row kernel from order 3
-    bool use_tiled = c->tiled && (sizeof(T) == 4 || c->tile_L >= 5) && (tiled_supported(c->tile_L, nrhs) || (sizeof(T) == 4 && c->row32));
-    if (use_tiled) {
-        ta.ntiles = c->ntiles;
-        ta.tiles = c->tiles.p;
-        ta.pairs = c->pairs.p;
-        ta.ops = ops_ptr<T>(c);
-        ta.x = x;
-        ta.y = y;
-        ta.ld = c->neqns;
-        ta.nrhs = nrhs;
-        ta.nchunk = nchunk;
-        ta.nsph = c->n;
-        ta.contran = contran;
-        ta.err = c->err.p;
-        ta.ctas_per_sm = c->opts.tile_ctas_per_sm;
-        ta.tsph = c->tsph.p;
-        ta.pslot = c->pslot.p;
-        ta.pairs_per_step = c->opts.tile_pairs;
-        ta.soff = c->hs.on() ? c->d_offset.p : nullptr;
-    }
-    if (nchunk > 1 && !use_tiled) return MSTMG_ERR_UNSUPPORTED;
+    auto far_field = [&]() -> int {
+        if (!far) return MSTMG_OK;
+        return groups([&](const cpx<T>* xk, cpx<T>* yk, int w, unsigned m) { return fft_far<T>(c, xk, yk, w, m); });
+    };
+    if (c->npairs == 0) return far_field();
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     if (c->timing) {
         for (cudaEvent_t* ev : {&e0, &e1}) {
@@ -262,21 +220,68 @@ template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, in
         }
         CK(cudaEventRecord(e0, c->st));
     }
-    if (use_tiled && sizeof(T) == 4 && c->row32) {
-        const int rc = rows_pass(c, ta, nrhs, nchunk, contran);
-        if (rc != 0) {
-            if (e0) c->ev_pool.push_back(e0);
-            if (e1) c->ev_pool.push_back(e1);
-            set_err("FP32 translation pass: no row-kernel configuration for this order and column count");
-            return MSTMG_ERR_UNSUPPORTED;
+    int rt = 0;
+    if (!c->tgroups_host.empty()) {
+        MmaArgs a;
+        a.pairs = c->tpairs.p;
+        a.tsph = c->tsph.p;
+        a.order = c->d_order.p;
+        a.offset = c->d_offset.p;
+        a.ops = c->op64.p;
+        if constexpr (sizeof(T) == 8) {
+            a.x = x;
+            a.y = y;
+        } else {
+            const size_t vals = ld * ncols;
+            if (int rw = ensure_wide(c, ncols)) return rw;
+            a.x = c->wide.p;
+            a.y = c->wide.p + vals;
+            launch_mma_widen(vals, x, c->wide.p, c->wide.p + vals, c->nsm, c->st);
         }
-    } else if (!use_tiled || launch_translate_tiled<T>(ta, c->tile_L, c->nsm, c->st) != 0) {
-        if (nchunk > 1) {
-            if (e0) c->ev_pool.push_back(e0);
-            if (e1) c->ev_pool.push_back(e1);
-            return MSTMG_ERR_UNSUPPORTED;
+        a.ld = c->neqns;
+        a.ncols = ncols;
+        a.contran = contran;
+        a.period = period;
+        a.slots = c->tslots;
+        a.err = c->err.p;
+        a.ctas_per_sm = c->opts.tile_ctas_per_sm;
+        for (const auto& g : c->tgroups) {
+            if (g.count == 0) continue;
+            a.ntiles = g.count;
+            a.tiles = c->tiles.p + g.first;
+            a.L = g.L;
+            a.uniform = g.uniform;
+            a.maxrec = g.maxrec;
+            if ((rt = launch_translate_mma(a, c->nsm, c->st)) != 0) break;
         }
-        launch_translate<T>(a, c->nsm, c->st);
+        if constexpr (sizeof(T) == 4) launch_mma_narrow(ld * ncols, a.y, y, parts, c->nsm, c->st);
+    } else {
+        TransArgs<T> a;
+        a.npairs = c->npairs;
+        a.pairs = c->pairs.p;
+        a.order = c->d_order.p;
+        a.offset = c->d_offset.p;
+        a.ops = c->op64.p;
+        a.opoff = c->opoff.p;
+        a.ld = c->neqns;
+        a.lmax = c->pair_lmax;
+        a.uniform = c->pair_uniform ? 1 : 0;
+        a.maxrec = c->maxrec;
+        a.err = c->err.p;
+        groups([&](const cpx<T>* xk, cpx<T>* yk, int w, unsigned m) {
+            a.x = xk;
+            a.y = yk;
+            a.nrhs = w;
+            a.contran = m;
+            launch_translate<T>(a, c->nsm, c->st);
+            return MSTMG_OK;
+        });
+    }
+    if (rt != 0) {
+        if (e0) c->ev_pool.push_back(e0);
+        if (e1) c->ev_pool.push_back(e1);
+        set_err("translation pass: no kernel configuration for this order");
+        return MSTMG_ERR_UNSUPPORTED;
     }
     CK(cudaGetLastError());
     if (c->timing) {
@@ -285,61 +290,12 @@ template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, in
     }
     if (sizeof(T) == 8) c->passes64++;
     else c->passes32++;
-    if (far) return fft_far<T>(c, x, y, nrhs * nchunk, contran);
-    return MSTMG_OK;
-}
-
-// Columns per chunk of FP32 tiled passes: opts.fp32_chunk when set (2 or 4),
-// otherwise chosen once per context by timing one pass over the caller's
-// columns in chunks of 4 and of 2 (each run twice, the second timed), which
-// depends on the order and the cluster size (4 wins at L = 9, 2 at L = 8 and
-// for small column counts).  The timing passes write y, which the caller's
-// own pass then overwrites.
-int fp32_chunk(mstmg_ctx* c, const zf* x, zf* y, int ncols, unsigned pattern2)
-{
-    if (c->opts.fp32_chunk == 2 || c->opts.fp32_chunk == 4) return c->opts.fp32_chunk;
-    if (c->chunk32 > 0) return c->chunk32;
-    if (!c->tiled || ncols < 4 || ncols % 4 != 0 || !tiled_supported(c->tile_L, 2) || !tiled_supported(c->tile_L, 4)) return 4;
-    auto expand = [&](int w) {
-        unsigned m = 0;
-        for (int r = 0; r < w; r++)
-            if ((pattern2 >> (r & 1)) & 1u) m |= 1u << r;
-        return m;
-    };
-    cudaEvent_t e[3] = {nullptr, nullptr, nullptr};
-    for (auto& ev : e)
-        if (cudaEventCreate(&ev) != cudaSuccess) {
-            for (auto& f : e)
-                if (f) cudaEventDestroy(f);
-            return 4;
-        }
-    float ms[2] = {0.f, 0.f};
-    const int nr[2] = {4, 2};
-    const bool timing = c->timing;
-    c->timing = false;
-    bool ok = true;
-    for (int v = 0; v < 2 && ok; v++) {
-        ok = translate<float>(c, x, y, nr[v], expand(nr[v]), ncols / nr[v]) == MSTMG_OK;
-        cudaEventRecord(e[0], c->st);
-        ok = ok && translate<float>(c, x, y, nr[v], expand(nr[v]), ncols / nr[v]) == MSTMG_OK;
-        cudaEventRecord(e[1], c->st);
-        ok = ok && cudaEventSynchronize(e[1]) == cudaSuccess && cudaEventElapsedTime(&ms[v], e[0], e[1]) == cudaSuccess;
-    }
-    c->timing = timing;
-    for (auto& f : e) cudaEventDestroy(f);
-    if (!ok) return 4;
-    c->passes32 -= 4;   // the timing passes are not the caller's
-    c->chunk32 = ms[1] < ms[0] ? 2 : 4;
-    return c->chunk32;
+    return far_field();
 }
 
 // ---------------------------------------------------------------------------
 // the tensor-core pass of many FP32 columns (tcpass.cu)
 // ---------------------------------------------------------------------------
-// Columns from which a plain (no conjugate-transpose column) FP32 pass goes to
-// the tensor cores: one M tile costs the same for 1 or 128 columns, and at 12
-// columns it already beats the rotation kernel.
-#define TC_MIN_COLS 12
 
 // One sphere order (5..10), pairs translated directly (no FFT, no dense
 // pairs): the cases the dense TF32 images serve.
@@ -473,18 +429,9 @@ int tc_translate(mstmg_ctx* c, const zf* x, zf* y, int ncols)
 
 // Many columns: y[:, 0:ncols] = H x[:, 0:ncols], where column k is a
 // conjugate-transpose product when bit (k & 1) of pattern2 is set (BiCG packs
-// [p_1, w_1, p_2, w_2, ...]: pattern2 = 2).  On the tiled path the columns go
-// in chunks of 4 or 2 (FP32, fp32_chunk) or 2 (FP64) through one launch;
-// otherwise in groups of up to 4 columns, one launch each.
+// [p_1, w_1, p_2, w_2, ...]: pattern2 = 2).
 template <typename T> int translate_many(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned pattern2)
 {
-    auto expand = [&](int w) {
-        unsigned m = 0;
-        for (int r = 0; r < w; r++)
-            if ((pattern2 >> (r & 1)) & 1u) m |= 1u << r;
-        return m;
-    };
-    int NR = 2;
     if constexpr (sizeof(T) == 4) {
         // many plain columns: the tensor-core pass when the context has (or can
         // build) its dense operator images
@@ -492,20 +439,8 @@ template <typename T> int translate_many(mstmg_ctx* c, const cpx<T>* x, cpx<T>* 
             int rc = tc_translate(c, x, y, ncols);
             if (rc != MSTMG_ERR_UNSUPPORTED) return rc;
         }
-        NR = fp32_chunk(c, x, y, ncols, pattern2);
     }
-    if (c->tiled && (sizeof(T) == 4 || c->tile_L >= 5) && ncols > NR && ncols % NR == 0 && tiled_supported(c->tile_L, NR)) {
-        int rc = translate<T>(c, x, y, NR, expand(NR), ncols / NR);
-        if (rc != MSTMG_ERR_UNSUPPORTED) return rc;
-    }
-    if (ncols <= 4) return translate<T>(c, x, y, ncols, expand(ncols));
-    const size_t ld = (size_t)c->neqns;
-    for (int k = 0; k < ncols; k += 4) {
-        int w = std::min(4, ncols - k);
-        int rc = translate<T>(c, x + (size_t)k * ld, y + (size_t)k * ld, w, expand(w));
-        if (rc) return rc;
-    }
-    return MSTMG_OK;
+    return translate<T>(c, x, y, ncols, pattern2, 2);
 }
 
 int interaction_impl(mstmg_ctx* c, int nrhs, const double* ain, double* aout, const int* con_tran, const int* mie_mult,
@@ -667,32 +602,20 @@ template <typename T> int fft_far(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int 
     return MSTMG_OK;
 }
 
-// node_selection (fft:654-825) with target box = the sphere-centre extents,
-// the near-pair list, the node translations and the kernel spectra.
-// Grouped tiles (the tiled kernels' tiles over listed spheres): the spheres
-// of `members`, taken list by list, form groups of TILE_B; a tile holds the pairs
-// of pr between two groups (or inside one), its spheres listed by slot
-// (c->tsph) and each pair's slots (c->pslot).  pr is reordered tile by tile,
-// the pairs of a tile in slot-disjoint couples where it has them (the row
-// kernel runs such a couple as one step); tl gets the tiles.
-int group_tiles(mstmg_ctx* c, const std::vector<std::vector<int>>& members, std::vector<int2>& pr, std::vector<int4>& tl)
+// Tiles of a given pair list: the spheres of `members`, in that order, form
+// groups; a tile holds the pairs of pr between two groups or inside one.
+int group_tiles(mstmg_ctx* c, const std::vector<int>& members, const std::vector<int2>& pr, TileSet& t)
 {
-    const int B = TILE_B, n = c->n;
-    c->tsph.release();
-    c->pslot.release();
-    tl.clear();
+    const int n = c->n;
+    int pl = 1;
+    for (const int2& q : pr) pl = std::max(pl, std::max(c->order[q.x], c->order[q.y]));
+    const int B = tile_group_size(c, (long long)pr.size(), pl);
     std::vector<int> grp(n, -1), gs(n, 0);
-    int k = 0;
-    for (const auto& cm : members)
-        for (int i : cm) {
-            grp[i] = k / B;
-            gs[i] = k % B;
-            k++;
-        }
-    const long long ng = (k + B - 1) / B;
-    std::vector<int> gmem((size_t)std::max(ng, 1LL) * B, -1);
-    for (int i = 0; i < n; i++)
-        if (grp[i] >= 0) gmem[(size_t)grp[i] * B + gs[i]] = i;
+    for (size_t k = 0; k < members.size(); k++) {
+        grp[members[k]] = (int)(k / B);
+        gs[members[k]] = (int)(k % B);
+    }
+    const long long ng = ((long long)members.size() + B - 1) / B;
     std::vector<long long> key(pr.size());
     std::vector<int> idx(pr.size());
     for (size_t q = 0; q < pr.size(); q++) {
@@ -705,49 +628,31 @@ int group_tiles(mstmg_ctx* c, const std::vector<std::vector<int>>& members, std:
         idx[q] = (int)q;
     }
     std::stable_sort(idx.begin(), idx.end(), [&](int u, int v) { return key[u] < key[v]; });
-    std::vector<int2> pr2(pr.size());
-    std::vector<int> ts;
-    std::vector<short2> ps(pr.size());
-    size_t q = 0;
-    while (q < idx.size()) {
+    t = TileSet();
+    t.slots = 2 * B;
+    t.pr.resize(pr.size());
+    t.ps.resize(pr.size());
+    for (size_t q = 0; q < idx.size();) {
         const long long kk = key[idx[q]];
-        const int ga = (int)(kk / ng), gb = (int)(kk % ng);
-        const size_t start = q;
-        for (int s = 0; s < B; s++) ts.push_back(gmem[(size_t)ga * B + s]);
-        for (int s = 0; s < B; s++) ts.push_back(ga == gb ? -1 : gmem[(size_t)gb * B + s]);
+        const int ga = (int)(kk / ng);
+        const size_t start = q, row = t.ts.size();
+        t.ts.resize(row + t.slots, -1);
         for (; q < idx.size() && key[idx[q]] == kk; q++) {
             const int2 p2 = pr[idx[q]];
-            pr2[q] = p2;
-            const short si = (short)(grp[p2.x] == ga ? gs[p2.x] : B + gs[p2.x]);
-            const short sj = (short)(grp[p2.y] == ga ? gs[p2.y] : B + gs[p2.y]);
-            ps[q] = make_short2(si, sj);
+            const unsigned char si = (unsigned char)(grp[p2.x] == ga ? gs[p2.x] : B + gs[p2.x]);
+            const unsigned char sj = (unsigned char)(grp[p2.y] == ga ? gs[p2.y] : B + gs[p2.y]);
+            t.pr[q] = p2;
+            t.ps[q] = make_uchar2(si, sj);
+            t.ts[row + si] = p2.x;
+            t.ts[row + sj] = p2.y;
         }
-        for (size_t u = start; u + 1 < q;) {
-            const short2 a0 = ps[u];
-            bool found = false;
-            for (size_t v = u + 1; v < q && !found; v++) {
-                const short2 b0 = ps[v];
-                if (a0.x != b0.x && a0.x != b0.y && a0.y != b0.x && a0.y != b0.y) {
-                    std::swap(ps[u + 1], ps[v]);
-                    std::swap(pr2[u + 1], pr2[v]);
-                    found = true;
-                }
-            }
-            u += found ? 2 : 1;
-        }
-        // z: the tile's row of the sphere lists (tiles may be dealt to shards)
-        tl.push_back(make_int4((int)start, (int)(q - start), (int)tl.size(), ga == gb ? 1 : 0));
-    }
-    pr.swap(pr2);
-    if (!ts.empty()) {
-        CK(c->tsph.alloc(ts.size()));
-        CK(c->pslot.alloc(ps.size()));
-        CK(cudaMemcpy(c->tsph.p, ts.data(), sizeof(int) * ts.size(), cudaMemcpyHostToDevice));
-        CK(cudaMemcpy(c->pslot.p, ps.data(), sizeof(short2) * ps.size(), cudaMemcpyHostToDevice));
+        t.tl.push_back(make_int4((int)start, (int)(q - start), (int)t.tl.size(), 0));
     }
     return MSTMG_OK;
 }
 
+// node_selection (fft:654-825) with target box = the sphere-centre extents,
+// the near-pair list, the node translations and the kernel spectra.
 int fft_build(mstmg_ctx* c)
 {
     FftState& F = *c->fft;
@@ -832,25 +737,19 @@ int fft_build(mstmg_ctx* c)
             for (int j : members[(size_t)(sx - 1) + (size_t)F.cd[0] * ((sy - 1) + (size_t)F.cd[1] * (sz - 1))])
                 if (j > i) pr.push_back(make_int2(i, j));
         }
-    // Grouped tiles for the tiled kernel (one sphere order it supports): the
-    // spheres, taken cell by cell, form groups of TILE_B; a tile holds the
-    // near pairs between two groups (or inside one), its spheres listed by
-    // slot, so the near pairs of nearby spheres share the tiles' output
-    // accumulation as the block tiles of a whole cluster do.
-    std::vector<int4> tl;
-    {
-        const int lmin = *std::min_element(c->order.begin(), c->order.end());
-        c->tiled = !c->opts.generic_kernel && lmin == c->lmax && lmin >= c->opts.translation_switch_order && tiled_supported(c->lmax, 1) &&
-                   !pr.empty();
-        c->tile_L = c->lmax;
-        if (c->tiled) {
-            if (int rg = group_tiles(c, members, pr, tl)) return rg;
-        } else {
-            c->tsph.release();
-            c->pslot.release();
-        }
+    // Tiles of the near pairs: the spheres, taken cell by cell, form the
+    // groups, so the near pairs of nearby spheres share the tiles' output
+    // accumulation as the tiles of a whole cluster do.
+    const int lmin = *std::min_element(c->order.begin(), c->order.end());
+    c->tiled = !c->opts.generic_kernel && lmin == c->lmax && lmin >= c->opts.translation_switch_order && tiled_order(c->lmax) && !pr.empty();
+    TileSet ts;
+    if (!c->opts.generic_kernel) {
+        std::vector<int> flat;
+        for (const auto& cm : members) flat.insert(flat.end(), cm.begin(), cm.end());
+        if (int rg = group_tiles(c, flat, pr, ts)) return rg;
+        pr.swap(ts.pr);
     }
-    int rc = upload_pairs(c, pr, (int)pr.size(), tl);   // synchronises: the host vectors above are done with
+    int rc = upload_pairs(c, pr, (int)pr.size(), c->opts.generic_kernel ? nullptr : &ts);   // synchronises: the host vectors above are done with
     if (rc) return rc;
     // node translations
     std::vector<long long> joff(n + 1);
@@ -1092,7 +991,6 @@ extern "C" int mstmg_time_translation(mstmg_ctx* c, int prec, int nrhs, int reps
     if (ms) *ms = t / reps;
     return check_kernel_err(c);
 }
-
 
 template int translate<float>(mstmg_ctx*, const zf*, zf*, int, unsigned, int);
 template int translate<double>(mstmg_ctx*, const zd*, zd*, int, unsigned, int);

@@ -603,10 +603,10 @@ extern "C" int mstmg_operator_bytes(const mstmg_ctx* c, int prec, double* stored
 {
     if (!c) return MSTMG_ERR_ARG;
     double es = prec == 0 ? 8.0 : 4.0;
-    // with host spheres the stored records include the regular translations
-    // between hosts and the spheres they hold (FP64 only)
+    // FP64 records serve the passes of either precision; with host spheres
+    // they include the regular translations between hosts and the spheres they hold
     const double hb = c->hs.on() ? (double)c->hs.hunits * 8.0 : 0.0;
-    if (stored) *stored = ((prec != 0 && c->row32) ? (double)c->npairs * c->row32 * es : (double)c->op_units * es) + hb;
+    if (stored) *stored = (double)c->op_units * 8.0 + hb;
     if (canonical) {
         auto canon = [&](int a, int b) {
             int nmn = std::min(a, b), nmx = std::max(a, b);
@@ -952,6 +952,8 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
     // orientation, an ensemble), whose steps are launch-bound on small
     // clusters: not with kernel timing (events) or the FFT path (cuFFT plans)
     bool graphs = gw.graphs_ok && (seg || S <= 2) && !c->timing && !(c->fft && c->fft->on);
+    // the rotation passes' columns (the tensor-core passes take the wider groups)
+    if (int rw = ensure_wide(c, std::max(2, tc_eligible(c) ? std::min(S, TC_MIN_COLS) : S))) return rw;
     if (graphs && gw.graph_gen != c->layout_gen) {
         gw.drop_graphs();
         gw.graph_gen = c->layout_gen;
@@ -1164,9 +1166,8 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
                     if ((r2 = translate_many<float>(c, gw.XP.p, gw.Y.p, 2, 0u))) return r2;
                     launch_eg_apply(sm, an32, ne, ldv, na, gw.act.p, seg->off, seg->len, gw.XP.p, gw.Y.p, gw.W.p, c->nsm, c->st);
                 } else {
-                    const int npad = na <= 2 ? na : ((na + 3) / 4) * 4;   // whole FP32 chunks
-                    launch_gm_gather(ne, m1, j, na, npad, gw.act.p, gw.V.p, gw.XP.p, c->nsm, c->st);
-                    if ((r2 = translate_many<float>(c, gw.XP.p, gw.Y.p, npad, 0u))) return r2;
+                    launch_gm_gather(ne, m1, j, na, na, gw.act.p, gw.V.p, gw.XP.p, c->nsm, c->st);
+                    if ((r2 = translate_many<float>(c, gw.XP.p, gw.Y.p, na, 0u))) return r2;
                     gm_apply_ctx(c, sm, an32, ne, na, gw.XP.p, gw.Y.p, gw.W.p);
                 }
                 CK(cudaMemsetAsync(gw.h.p, 0, sizeof(double) * (O1 + hn), c->st));

@@ -22,8 +22,7 @@
 #include "bicg.cuh"
 #include "sphere_kernels.cuh"
 #include "tables.h"
-#include "translate_tiled.cuh"
-#include "translate_rows.cuh"
+#include "translate_mma.cuh"
 #include "postproc.cuh"
 #include "mrhs.cuh"
 #include "ranorient.cuh"
@@ -311,8 +310,7 @@ struct HostSpheres {
     int nzp = 0;
     DevBuf<long long> hopoff;
     DevBuf<double> hop64, hmed;
-    DevBuf<float> hop32;
-    bool hops_ready = false, hops32_ready = false;
+    bool hops_ready = false;
     bool on() const { return nhosted > 0; }
 };
 
@@ -338,22 +336,22 @@ struct mstmg_ctx {
     DevBuf<float> an32;
     DevBuf<int2> pairs;
     DevBuf<long long> opoff;
+    // tiles of the pairs (translate_mma.cu; none with opts.generic_kernel): the
+    // tiles by launch group, each group with its strides' largest order
+    bool tiled = false;      // clusters of one order in 3..10: tiles may be dealt to shards, tensor-core images
     DevBuf<int4> tiles;
-    int ntiles = 0;
-    // grouped tiles (the FFT path's near pairs): spheres of each tile by slot
-    // and the slots of each pair; empty for block tiles
-    DevBuf<int> tsph;
-    DevBuf<short2> pslot;
-    bool tiled = false;   // monodisperse cluster: pairs stored in tile order for the fast kernel
-    int tile_L = 0;       // the sphere order of the tiled pairs (the cluster's; with host spheres, the held spheres')
-    int row32 = 0;        // tiled: floats per FP32 row record (translate_rows.cuh); 0: FP32 records as FP64
+    DevBuf<int> tsph;        // spheres of each tile row by slot
+    DevBuf<MmaPair> tpairs;  // per pair, in tile order
+    struct TileGroup { int first, count, L, uniform, maxrec; };
+    std::vector<TileGroup> tgroups;   // of this shard's tiles
+    int tslots = 0;
     // pair shard (mstmg_set_pair_shard): this context translates the tiles
     // t with t % nshards == shard; all tiles kept on the host
     int shard = 0, nshards = 1;
-    std::vector<int4> tiles_host;
-    DevBuf<double> op64;
-    DevBuf<float> op32;
-    bool ops64_ready = false, ops32_ready = false;
+    std::vector<int4> tiles_host;           // w: the tile's group
+    std::vector<TileGroup> tgroups_host;
+    DevBuf<double> op64;   // operator records, read by FP64 and FP32 passes
+    bool ops64_ready = false, ops32_ready = false;   // records (and dense FP64); dense FP32
     // mixed fixed-orientation solve: the two polarisations as a many-system
     // residual-replacement solve, its work kept across solves
     MultiWork<double> fo64;
@@ -372,11 +370,11 @@ struct mstmg_ctx {
     DevBuf<double> d_cfg_xg, cfg_qtot;
     GmresWork ens_gm;
     int ens_ldv = 0;
-    int chunk32 = 0;   // FP32 columns per tiled chunk chosen by timing (0: not yet)
     DevBuf<double> vcc, fnr, rfnr, bcofd;
     DevBuf<zd> opgen_xi;   // Hankel functions of every pair while the operators are generated
     int vn = 0;
     DevBuf<int> err;
+    DevBuf<zd> wide;   // FP64 copies of an FP32 pass's columns, x then y
     DevBuf<zd> X64, Y64, pmnp, amnp, pw0, drot, vec64, bvec64;
     DevBuf<zf> X32, Y32, vec32, rvec32;
     DevBuf<double> part, qeff, qtot, small;
@@ -448,15 +446,30 @@ int reject_sharded(const mstmg_ctx* c, const char* fn);
 int reject_hosts(const mstmg_ctx* c, const char* fn);
 int apply_shard(mstmg_ctx* c);
 int check_kernel_err(mstmg_ctx* c);
-int upload_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np, const std::vector<int4>& tl);
+// Pairs grouped in tiles: the pairs between two groups of up to 4 spheres (or
+// inside one), tile after tile
+struct TileSet {
+    std::vector<int2> pr;    // the pairs, i < j
+    std::vector<uchar2> ps;  // their slots
+    std::vector<int4> tl;    // (first pair, pairs, row of ts, 0)
+    std::vector<int> ts;     // the tiles' spheres, `slots` a row by slot, -1: none
+    int slots = 0;
+};
+int tile_group_size(const mstmg_ctx* c, long long npairs, int L);
+int upload_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np, const TileSet* ts);
+inline bool tiled_order(int L) { return L >= 3 && L <= 10; }
 int ensure_gentran(mstmg_ctx* c, int lm);
 int setup_layout(mstmg_ctx* c);
 // capi_pass.cu
 DenseArgs dense_args(mstmg_ctx* c);
 int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force);
 int ensure_ops(mstmg_ctx* c, int prec, bool force);
-template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int nrhs, unsigned contran, int nchunk = 1);
-int fp32_chunk(mstmg_ctx* c, const zf* x, zf* y, int ncols, unsigned pattern2);
+template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period = 32);
+// Columns from which a plain (no conjugate-transpose column) FP32 pass goes to
+// the tensor cores: one M tile costs the same for 1 or 128 columns, and at 12
+// columns it already beats the rotation kernel.
+#define TC_MIN_COLS 12
+int ensure_wide(mstmg_ctx* c, int ncols);
 bool tc_eligible(const mstmg_ctx* c);
 int ensure_tc(mstmg_ctx* c);
 int tc_translate(mstmg_ctx* c, const zf* x, zf* y, int ncols);
@@ -470,7 +483,7 @@ template <typename T> int translate_hosts(mstmg_ctx* c, const cpx<T>* x, cpx<T>*
 template <typename T> void mie_all(mstmg_ctx* c, int idir, int conj_in, const cpx<T>* x, cpx<T>* y);
 template <typename T> int fft_far(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran);
 int fft_build(mstmg_ctx* c);
-int group_tiles(mstmg_ctx* c, const std::vector<std::vector<int>>& members, std::vector<int2>& pr, std::vector<int4>& tl);
+int group_tiles(mstmg_ctx* c, const std::vector<int>& members, const std::vector<int2>& pr, TileSet& t);
 // capi_origin.cu
 mstmg::Tables& big_tables();   // the reference's large constant tables (this thread's copy)
 // capi_solve.cu

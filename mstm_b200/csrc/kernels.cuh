@@ -8,9 +8,7 @@ struct OpGenArgs {
     const double* pos;       // 3N
     const int* order;        // N
     const long long* opoff;  // per pair, in storage units
-    double* op64;            // may be null
-    float* op32;             // may be null
-    int row32;               // > 0: op32 holds row records (translate_rows.cuh) of one order, row32 floats each
+    double* op64;
     const double* vcc;       // vcc_const(vn, vn(vn+2), 0:2vn)
     int vnmax;
     const double* fnr;       // fnr[k] = sqrt(k)
@@ -32,15 +30,15 @@ template <typename T> struct TransArgs {
     const int2* pairs;
     const int* order;
     const int* offset;       // sphere_offset (complex units)
-    const T* ops;
-    const long long* opoff;  // storage units
+    const double* ops;
+    const long long* opoff;  // doubles
     const cpx<T>* x;         // ld x nrhs
     cpx<T>* y;               // ld x nrhs, accumulated
     int ld;
     int nrhs;
     unsigned contran;        // bit r set: rhs r is a conjugate-transpose product
     int lmax;                // largest order (smem strides)
-    int maxrec;              // largest operator record, storage units
+    int maxrec;              // largest operator record, doubles
     int* err;
     int uniform = 0;         // 1: every pair has both orders lmax
 };

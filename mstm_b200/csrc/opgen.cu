@@ -22,17 +22,17 @@
 // into a scratch of 2 LMAX + 1 complex per pair; the Wigner-d rows (serial in
 // the degree and the restricted index, parallel over the other index) one
 // warp per pair; the axial blocks one CTA per pair, a thread per (m, n, l).
-// Record layout (units of the storage type T, double or float):
-//   [0,2)            e^{i phi}
-//   [2, 2+R)         E_1, O_1, E_2, O_2, ...   (row-major, restricted index first)
-//   [2+R, 2+R+2Z)    Z_0[p=0], Z_1[p=0], Z_1[p=1], Z_2[p=0], ... complex, [row n][col l]
-//   padding to a multiple of 4 units.
-// FP32 records of clusters of one sphere order (the tiled passes) use the row
-// layout of translate_rows.cuh instead: the same values, rows 16-byte aligned.
+// Record layout (doubles; R rotation values, oplayout.cuh):
+//   [0, H)           e^{i m phi}, then e^{-i m phi}, m = 0 .. nmax (H = 4 nmax + 4)
+//   [H, H+R)         E_1, O_1, E_2, O_2, ...   (row-major, restricted index first;
+//                    O_n has the rows and columns of E_n, k = 0 and m = 0 zero)
+//   [zb, zb+2Z)      Z_0[p=0], Z_1[p=0], Z_1[p=1], Z_2[p=0], ... complex, [row n][col l];
+//                    zb is H+R rounded up to an even number
+//   zeros up to zb and to a multiple of 4 doubles.
+// Passes of either precision read these records.
 #include "common.cuh"
 #include "special.cuh"
 #include "kernels.cuh"
-#include "translate_rows.cuh"
 
 #define DW (2 * MSTMG_LMAX + 1)
 #define XIW (2 * MSTMG_LMAX + 1)   // Hankel orders w = 0 .. nt + ns <= 2 LMAX per pair
@@ -87,23 +87,18 @@ __global__ void __launch_bounds__(128) opgen_pair_kernel(OpGenArgs a)
             atomicExch(a.err, MSTMG_ERR_UNSUPPORTED);
             continue;
         }
-        const long long off = a.opoff[q];
-        if (a.op64) {
-            a.op64[off] = g.ephi.x;
-            a.op64[off + 1] = g.ephi.y;
-        }
-        if (a.op32 && a.row32) {
-            // row records: the powers e^{i m phi}, m = 0..nt, by the recurrence in FP64
-            float* h = a.op32 + (long long)q * a.row32;
-            zd e = mk(1.0, 0.0);
-            for (int m = 0; m <= g.nt; m++) {
-                h[2 * m] = (float)e.x;
-                h[2 * m + 1] = (float)e.y;
-                e = e * g.ephi;
-            }
-        } else if (a.op32) {
-            a.op32[off] = (float)g.ephi.x;
-            a.op32[off + 1] = (float)g.ephi.y;
+        // e^{i m phi} by the recurrence (ephicoef)
+        double* h = a.op64 + a.opoff[q];
+        if (op_z_base(g.nmax, g.nmin) > op_head(g.nmax) + op_rot_size(g.nmax, g.nmin)) h[op_z_base(g.nmax, g.nmin) - 1] = 0.0;
+        const int units = op_record_units(g.nt, g.ns);
+        for (int k = op_z_base(g.nmax, g.nmin) + 2 * op_z_offset(g.nmin + 1, g.nt, g.ns); k < units; k++) h[k] = 0.0;
+        zd e = mk(1.0, 0.0);
+        for (int m = 0; m <= g.nmax; m++) {
+            h[2 * m] = e.x;
+            h[2 * m + 1] = e.y;
+            h[2 * (g.nmax + 1 + m)] = e.x;
+            h[2 * (g.nmax + 1 + m) + 1] = -e.y;
+            e = g.ephi * e;
         }
         zd* xi = a.xi + (size_t)q * XIW;
         const int nl = g.nt + g.ns;
@@ -134,10 +129,7 @@ __global__ void __launch_bounds__(128) opgen_rot_kernel(OpGenArgs a)
         if (!g.ok) continue;
         const int nmin = g.nmin, nmax = g.nmax;
         const double ct = g.ct;
-        const long long off = a.opoff[q];
-        double* rec64 = a.op64 ? a.op64 + off : nullptr;
-        float* rec32 = (a.op32 && !a.row32) ? a.op32 + off : nullptr;
-        float* row32 = (a.op32 && a.row32) ? a.op32 + (size_t)q * a.row32 : nullptr;
+        double* rec64 = a.op64 + a.opoff[q];
         const double sbe = (fabs(ct) >= 1.0) ? 0.0 : sqrt(fabs((1.0 + ct) * (1.0 - ct)));
         const double cbe2 = 0.5 * (1.0 + ct), sbe2 = 0.5 * (1.0 - ct);
         for (int k = lane; k < 2 * MSTMG_LMAX + 3; k += 32) {
@@ -195,39 +187,16 @@ __global__ void __launch_bounds__(128) opgen_rot_kernel(OpGenArgs a)
                 __syncwarp();
             }
             // fold into E_n, O_n
-            const int roff = 2 + op_rot_offset(n, nmin);
-            const int ne = (kk + 1) * (n + 1), no = kk * n;
-            // row and column of flat element e by a float reciprocal: e < 2^10 and
+            const int roff = op_head(nmax) + op_rot_offset(n, nmin);
+            const int ne = (kk + 1) * (n + 1);
+            // row and column of element e by a float reciprocal: e < 2^10 and
             // e / (n + 1) sits at least 1 / (2 (n + 1)) from the next integer
-            const float rn1 = 1.0f / (float)(n + 1), rn = 1.0f / (float)n;
-            for (int e = lane; e < ne + no; e += 32) {
-                double v;
-                if (e < ne) {
-                    const int rr_ = (int)(((float)e + 0.5f) * rn1), f = e - rr_ * (n + 1);
-                    const double dp = D[rr_ * DW + (f + MSTMG_LMAX)];
-                    v = (f == 0) ? 0.5 * dp : 0.5 * (dp + pm1(f) * D[rr_ * DW + (-f + MSTMG_LMAX)]);
-                } else {
-                    const int e2 = e - ne;
-                    const int qq = (int)(((float)e2 + 0.5f) * rn);
-                    const int rr_ = 1 + qq, f = 1 + e2 - qq * n;
-                    const double dp = D[rr_ * DW + (f + MSTMG_LMAX)];
-                    v = 0.5 * (dp - pm1(f) * D[rr_ * DW + (-f + MSTMG_LMAX)]);
-                }
-                if (rec64) rec64[roff + e] = v;
-                if (rec32) rec32[roff + e] = (float)v;
-                if (row32) {
-                    // row layout: row k of degree n is [E(k,0), 0, E(k,1), O(k,1), ..., E(k,n), O(k,n)]
-                    int k, slot;
-                    if (e < ne) {
-                        k = (int)(((float)e + 0.5f) * rn1);
-                        slot = 2 * (e - k * (n + 1));
-                    } else {
-                        const int qq = (int)(((float)(e - ne) + 0.5f) * rn);
-                        k = 1 + qq;
-                        slot = 2 * (1 + (e - ne) - qq * n) + 1;
-                    }
-                    row32[rr_rot_off(n, nmax) + k * rr_rw(n) + slot] = (float)v;
-                }
+            const float rn1 = 1.0f / (float)(n + 1);
+            for (int e = lane; e < ne; e += 32) {
+                const int rr_ = (int)(((float)e + 0.5f) * rn1), f = e - rr_ * (n + 1);
+                const double dp = D[rr_ * DW + (f + MSTMG_LMAX)], dm = pm1(f) * D[rr_ * DW + (-f + MSTMG_LMAX)];
+                rec64[roff + e] = f == 0 ? 0.5 * dp : 0.5 * (dp + dm);
+                rec64[roff + ne + e] = f == 0 || rr_ == 0 ? 0.0 : 0.5 * (dp - dm);
             }
             __syncwarp();
         }
@@ -249,11 +218,8 @@ __global__ void __launch_bounds__(128) opgen_axial_kernel(OpGenArgs a)
         __syncthreads();   // the previous pair's reads of xs are done
         for (int k = threadIdx.x; k <= nt + ns; k += blockDim.x) xs[k] = a.xi[(size_t)q * XIW + k];
         __syncthreads();
-        const long long off = a.opoff[q];
-        double* rec64 = a.op64 ? a.op64 + off : nullptr;
-        float* rec32 = (a.op32 && !a.row32) ? a.op32 + off : nullptr;
-        float* row32 = (a.op32 && a.row32) ? a.op32 + (size_t)q * a.row32 : nullptr;
-        const int zbase = 2 + op_rot_size(g.nmax, nmin);
+        double* rec64 = a.op64 + a.opoff[q];
+        const int zbase = op_z_base(g.nmax, nmin);
         // walk the blocks forward: block m holds rc(m) elements, mode-1 copies
         // after the mode-0 ones for m > 0 (op_z_offset)
         int m = 0, e = threadIdx.x, zoff = 0;
@@ -277,35 +243,11 @@ __global__ void __launch_bounds__(128) opgen_axial_kernel(OpGenArgs a)
             s2 = imul(s2);
             const zd v0 = s1 + s2, v1 = s1 - s2;
             const int zo = zbase + 2 * (zoff + e);
-            if (rec64) {
-                rec64[zo] = v0.x;
-                rec64[zo + 1] = v0.y;
-                if (m > 0) {
-                    rec64[zo + 2 * rc] = v1.x;
-                    rec64[zo + 2 * rc + 1] = v1.y;
-                }
-            }
-            if (row32) {
-                // row layout: m = 0 rows of Z_0(n, .); m > 0 rows of (Z_m^0, Z_m^1)(n, l) pairs
-                if (m == 0) {
-                    float* z = row32 + rr_z_off(0, nt) + (n - 1) * rr_zw0(nt) + 2 * (l - 1);
-                    z[0] = (float)v0.x;
-                    z[1] = (float)v0.y;
-                } else {
-                    float* z = row32 + rr_z_off(m, nt) + (n - m1) * 4 * rr_zq(cols) + 4 * (l - m1);
-                    z[0] = (float)v0.x;
-                    z[1] = (float)v0.y;
-                    z[2] = (float)v1.x;
-                    z[3] = (float)v1.y;
-                }
-            }
-            if (rec32) {
-                rec32[zo] = (float)v0.x;
-                rec32[zo + 1] = (float)v0.y;
-                if (m > 0) {
-                    rec32[zo + 2 * rc] = (float)v1.x;
-                    rec32[zo + 2 * rc + 1] = (float)v1.y;
-                }
+            rec64[zo] = v0.x;
+            rec64[zo + 1] = v0.y;
+            if (m > 0) {
+                rec64[zo + 2 * rc] = v1.x;
+                rec64[zo + 2 * rc + 1] = v1.y;
             }
             e += blockDim.x;
         }

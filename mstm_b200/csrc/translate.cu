@@ -73,8 +73,8 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
     int* zoff = roff + (MSTMG_LMAX + 2);                        // lm+2 ints
     int* flag = zoff + (MSTMG_LMAX + 2);                        // 1 int
     cpx<T>* ephm = (cpx<T>*)(sm + 256);                         // 2*LMAX+1 entries, index q+LMAX
-    T* opb = (T*)(sm + 256 + 2 * sizeof(cpx<T>) * (2 * MSTMG_LMAX + 1) + 64);
-    opb = (T*)(((uintptr_t)opb + 127) & ~(uintptr_t)127);
+    double* opb = (double*)(sm + 256 + 2 * sizeof(cpx<T>) * (2 * MSTMG_LMAX + 1) + 64);
+    opb = (double*)(((uintptr_t)opb + 127) & ~(uintptr_t)127);
     cpx<T>* bufA = (cpx<T>*)(opb + 2 * (size_t)a.maxrec);       // s/t, later g
     const int szA = lm * 2 * (lm + 1);                          // per (inst, p)
     cpx<T>* bufB = bufA + (size_t)NI * 2 * szA;                 // a'
@@ -94,7 +94,7 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             int q = q0 + b * G;
             if (q < a.npairs) {
                 int i = a.pairs[q].x, j = a.pairs[q].y;
-                uint32_t bytes = (uint32_t)(op_record_units(a.order[i], a.order[j]) * sizeof(T));
+                uint32_t bytes = (uint32_t)(op_record_units(a.order[i], a.order[j]) * sizeof(double));
                 mbar_arrive_expect_tx(&bar[b], bytes);
                 bulk_g2s(opb + (size_t)b * a.maxrec, a.ops + a.opoff[q], bytes, &bar[b]);
             }
@@ -111,26 +111,22 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             mbar_wait_bounded(&bar[b ^ 1], ((t + 1) >> 1) & 1);
             return;
         }
-        const T* rec = opb + (size_t)b * a.maxrec;
+        const double* rec = opb + (size_t)b * a.maxrec;
         const int i = a.pairs[q].x, j = a.pairs[q].y;
         const int noi = UNI ? LM : a.order[i], noj = UNI ? LM : a.order[j];
         const int nmin = noi < noj ? noi : noj, nmax = noi > noj ? noi : noj;
         if (noi != prev_noi || noj != prev_noj) {
             if (tid <= lm + 1) {
-                roff[tid] = (tid >= 1 && tid <= nmax) ? 2 + op_rot_offset(tid, nmin) : 0;
-                zoff[tid] = (tid <= nmin) ? 2 + op_rot_size(nmax, nmin) + 2 * op_z_offset(tid, noi, noj) : 0;
+                roff[tid] = (tid >= 1 && tid <= nmax) ? op_head(nmax) + op_rot_offset(tid, nmin) : 0;
+                zoff[tid] = (tid <= nmin) ? op_z_base(nmax, nmin) + 2 * op_z_offset(tid, noi, noj) : 0;
             }
             prev_noi = noi;
             prev_noj = noj;
         }
-        if (tid == 0) {
-            cpx<T> ep = mk(rec[0], rec[1]);
+        if (tid <= nmax) {
             cpx<T>* e = ephm + MSTMG_LMAX;
-            e[0] = mk((T)1, (T)0);
-            for (int m = 1; m <= nmax; m++) {
-                e[m] = ep * e[m - 1];
-                e[-m] = cj(e[m]);
-            }
+            e[tid] = mk((T)rec[2 * tid], (T)rec[2 * tid + 1]);
+            e[-tid] = cj(e[tid]);
         }
         __syncthreads();
         const cpx<T>* e = ephm + MSTMG_LMAX;
@@ -175,15 +171,15 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             int nsrc = dir ? noi : noj;
             int kk = n < nmin ? n : nmin;
             if (n > nsrc || k > kk) continue;
-            const T* E = rec + roff[n];
-            const T* O = E + (kk + 1) * (n + 1);
+            const double* E = rec + roff[n];
+            const double* O = E + (kk + 1) * (n + 1);
             const cpx<T>* st = bufA + (size_t)(inst * 2 + p) * szA + (n - 1) * 2 * (lm + 1);
             cpx<T> P = mk((T)0, (T)0), Q = mk((T)0, (T)0);
-            const T* Er = E + k * (n + 1);
-            for (int m = 0; m <= n; m++) P = P + Er[m] * st[m];
+            const double* Er = E + k * (n + 1);
+            for (int m = 0; m <= n; m++) P = P + (T)Er[m] * st[m];
             if (k > 0) {
-                const T* Or = O + (k - 1) * n;
-                for (int m = 1; m <= n; m++) Q = Q + Or[m - 1] * st[lm + 1 + m];
+                const double* Or = O + k * (n + 1);
+                for (int m = 1; m <= n; m++) Q = Q + (T)Or[m] * st[lm + 1 + m];
             }
             cpx<T>* ap = bufB + (size_t)(inst * 2 + p) * szB + (n - 1) * (2 * lm + 1) + lm;
             ap[k] = P + Q;
@@ -206,19 +202,19 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             if (row > ntg) continue;
             int rows = noi - m1 + 1, cols = noj - m1 + 1;
             int pz = (am == 0) ? 0 : (m > 0 ? p : 1 - p);
-            const T* zb = rec + zoff[am] + 2 * pz * rows * cols;
+            const double* zb = rec + zoff[am] + 2 * pz * rows * cols;
             const cpx<T>* ap = bufB + (size_t)(inst * 2 + p) * szB + lm + m;   // ap[(n-1)*(2lm+1)]
             cpx<T> g = mk((T)0, (T)0);
             if (dir == 0) {
-                const T* zr = zb + 2 * (row - m1) * cols;
+                const double* zr = zb + 2 * (row - m1) * cols;
                 for (int l = m1; l <= noj; l++) {
-                    cpx<T> z = mk(zr[2 * (l - m1)], zr[2 * (l - m1) + 1]);
+                    cpx<T> z = mk((T)zr[2 * (l - m1)], (T)zr[2 * (l - m1) + 1]);
                     g = g + z * ap[(l - 1) * (2 * lm + 1)];
                 }
             } else {
                 for (int n = m1; n <= noi; n++) {
-                    const T* zz = zb + 2 * ((n - m1) * cols + (row - m1));
-                    cpx<T> z = mk(zz[0], zz[1]);
+                    const double* zz = zb + 2 * ((n - m1) * cols + (row - m1));
+                    cpx<T> z = mk((T)zz[0], (T)zz[1]);
                     g = g + ap[(n - 1) * (2 * lm + 1)] * z;
                 }
             }
@@ -239,18 +235,18 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             int kk = n < nmin ? n : nmin;
             int sop = dir, top = (a.contran >> r) & 1;
             int im = sop ? -1 : 1;
-            const T* E = rec + roff[n];
-            const T* O = E + (kk + 1) * (n + 1);
+            const double* E = rec + roff[n];
+            const double* O = E + (kk + 1) * (n + 1);
             const cpx<T>* g = bufA + (size_t)(inst * 2 + p) * szA + (n - 1) * (2 * lm + 1) + lm;
             // g'(k) = sum_m g(m) d(m,k): the m=0 term enters once, the +-m
             // pairs through s(m)=g(m)+(-1)^m g(-m) and t(m)=g(m)-(-1)^m g(-m).
-            cpx<T> P = g[0] * E[k];
+            cpx<T> P = g[0] * (T)E[k];
             cpx<T> Q = mk((T)0, (T)0);
             for (int m = 1; m <= kk; m++) {
                 T sg = (m & 1) ? (T)-1 : (T)1;
                 cpx<T> gp = g[m], gm = sg * g[-m];
-                P = P + E[m * (n + 1) + k] * (gp + gm);
-                if (k > 0) Q = Q + O[(m - 1) * n + (k - 1)] * (gp - gm);
+                P = P + (T)E[m * (n + 1) + k] * (gp + gm);
+                if (k > 0) Q = Q + (T)O[m * (n + 1) + k] * (gp - gm);
             }
             cpx<T>* ys = a.y + (size_t)r * a.ld + a.offset[tgt];
             if (k == 0) {
@@ -271,7 +267,7 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
             if (qn < a.npairs) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 int in = a.pairs[qn].x, jn = a.pairs[qn].y;
-                uint32_t bytes = (uint32_t)(op_record_units(a.order[in], a.order[jn]) * sizeof(T));
+                uint32_t bytes = (uint32_t)(op_record_units(a.order[in], a.order[jn]) * sizeof(double));
                 mbar_arrive_expect_tx(&bar[b], bytes);
                 bulk_g2s(opb + (size_t)b * a.maxrec, a.ops + a.opoff[qn], bytes, &bar[b]);
             }
@@ -282,7 +278,7 @@ template <typename T, int NT, int LM, bool UNI> __global__ void __launch_bounds_
 template <typename T> size_t translate_smem_bytes(int lmax, int nrhs, int maxrec)
 {
     size_t head = 256 + 2 * sizeof(cpx<T>) * (2 * MSTMG_LMAX + 1) + 64 + 128;
-    size_t ops = 2 * (size_t)maxrec * sizeof(T);
+    size_t ops = 2 * (size_t)maxrec * sizeof(double);
     int NI = 2 * nrhs;
     size_t bufs = (size_t)NI * 2 * (lmax * 2 * (lmax + 1) + lmax * (2 * lmax + 1)) * sizeof(cpx<T>);
     return head + ops + bufs;
@@ -310,8 +306,22 @@ template <typename T, int NT, int LM, bool UNI = false> static void launch_trans
 
 // Pairs of small orders leave most of a 256-thread CTA idle in every phase:
 // two-warp CTAs up to order 6.  a.lmax (1 .. MSTMG_LMAX) picks the instance.
-template <typename T> void launch_translate(const TransArgs<T>& a, int nsm, cudaStream_t st)
+template <typename T> void launch_translate(const TransArgs<T>& a0, int nsm, cudaStream_t st)
 {
+    TransArgs<T> a = a0;
+    // columns that do not fit the shared memory together go one launch after the other
+    while (a.nrhs > 1 && translate_smem_bytes<T>(a.lmax, a.nrhs, a.maxrec) > 227 * 1024) a.nrhs = (a.nrhs + 1) / 2;
+    if (a.nrhs < a0.nrhs) {
+        const int w = a.nrhs;
+        for (int k = 0; k < a0.nrhs; k += w) {
+            a.nrhs = w < a0.nrhs - k ? w : a0.nrhs - k;
+            a.x = a0.x + (size_t)k * a0.ld;
+            a.y = a0.y + (size_t)k * a0.ld;
+            a.contran = a0.contran >> k;
+            launch_translate(a, nsm, st);
+        }
+        return;
+    }
     static_assert(MSTMG_LMAX == 16, "one instance per order up to MSTMG_LMAX");
     if (a.uniform) {
         switch (a.lmax) {

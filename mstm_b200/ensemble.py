@@ -41,14 +41,12 @@ def ensemble_configs(count, seed=4, nmin=50, nmax=400, x=1.5, m=1.6 + 0.005j, fv
 
 class Autotuner:
     """Per size class (sphere count rounded to 50, sphere order, precision), the
-    pass that serves the many-column solves: the tensor-core pass (dense TF32
-    hi/lo operators), or the rotation kernels with their CTAs per SM, FP32
-    column chunk and kernel family (tiled or order-generic), chosen by timing
-    one translation pass over the column count of a T-matrix group."""
+    pass that serves the many-column solves: the tensor-core pass of dense
+    TF32 hi/lo operators, or the rotation kernels (FP64 tensor-core tiles, or
+    the order-generic kernel), chosen by timing one translation pass over the
+    column count of a T-matrix group."""
 
-    CANDIDATES = [dict(tensor_core=0)] + \
-                 [dict(tensor_core=-1, tile_ctas_per_sm=c, fp32_chunk=k, generic_kernel=0) for c in (0, 2) for k in (2, 4)] + \
-                 [dict(tensor_core=-1, tile_ctas_per_sm=0, fp32_chunk=0, generic_kernel=1)]
+    CANDIDATES = [dict(tensor_core=0), dict(tensor_core=-1, generic_kernel=0), dict(tensor_core=-1, generic_kernel=1)]
 
     def __init__(self, reps=3):
         self.reps = reps
