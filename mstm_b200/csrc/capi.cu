@@ -668,7 +668,6 @@ int setup_layout(mstmg_ctx* c)
     CK(c->vec32.alloc(2LL * 7 * ne));
     CK(c->rvec32.alloc(2LL * ne));
     CK(c->pw0.alloc(2LL * 2 * lm * (lm + 2)));
-    CK(c->drot.alloc(3LL * (lm * (lm + 2) + 1)));
     CK(c->part.alloc(3LL * c->nsm * 4 + 16));
     CK(c->qeff.alloc(9LL * n));
     CK(c->qtot.alloc(9));
@@ -864,7 +863,7 @@ extern "C" void mstmg_ctx_destroy(mstmg_ctx* c)
     for (auto* b : d) b->release();
     DevBuf<int>* ib[] = {&c->d_order, &c->d_offset, &c->d_mie_offset, &c->slot, &c->slot_full, &c->err};
     for (auto* b : ib) b->release();
-    DevBuf<zd>* zb[] = {&c->an, &c->an_inv, &c->X64, &c->Y64, &c->pmnp, &c->amnp, &c->pw0, &c->drot, &c->vec64, &c->bvec64};
+    DevBuf<zd>* zb[] = {&c->an, &c->an_inv, &c->X64, &c->Y64, &c->pmnp, &c->amnp, &c->pw0, &c->vec64, &c->bvec64};
     for (auto* b : zb) b->release();
     DevBuf<zf>* fb[] = {&c->X32, &c->Y32, &c->vec32, &c->rvec32};
     for (auto* b : fb) b->release();

@@ -8,7 +8,7 @@
 // scatprops:262-281): all spheres, or those outside every other sphere
 static void planewave_ctx(mstmg_ctx* c, double alpha, double sinc, int dir)
 {
-    launch_planewave(alpha, sinc, dir, c->lmax, c->neqns, c->slot_full.p, c->d_order.p, c->d_offset.p, c->pos.p, c->pw0.p, c->drot.p,
+    launch_planewave(alpha, sinc, dir, c->lmax, c->neqns, c->slot_full.p, c->d_order.p, c->d_offset.p, c->pos.p, c->pw0.p,
                      c->pmnp.p, c->st, c->n, c->hs.on() ? c->hs.d_outside.p : nullptr);
 }
 

@@ -375,7 +375,7 @@ struct mstmg_ctx {
     int vn = 0;
     DevBuf<int> err;
     DevBuf<zd> wide;   // FP64 copies of an FP32 pass's columns, x then y
-    DevBuf<zd> X64, Y64, pmnp, amnp, pw0, drot, vec64, bvec64;
+    DevBuf<zd> X64, Y64, pmnp, amnp, pw0, vec64, bvec64;
     DevBuf<zf> X32, Y32, vec32, rvec32;
     DevBuf<double> part, qeff, qtot, small;
     DevBuf<BicgScalars> sc;

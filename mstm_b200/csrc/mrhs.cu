@@ -10,6 +10,7 @@
 // system in a fixed order, so results do not depend on the other systems.
 #include "mrhs.cuh"
 #include "special.cuh"
+#include "qeffcoef.cuh"
 
 #define MB 256
 
@@ -666,40 +667,30 @@ __global__ void tm_rhs_kernel(int l, zd* P0)
 // G (may be null): the exciting fields of the columns (host spheres: the
 // interaction without the Mie multiply plus the incident field), else
 // A^{-1} a; rext (may be null): the index around each sphere, else rimed
-__global__ void tm_qeff_kernel(int nsph, int ncols, const int* order, const int* offset, const int* mie_offset, const double* radius,
-                               zd rimed, const zd* an_inv, const zd* A, const zd* P, int ld, double* qcol, const zd* G, const double* rext)
+// One CTA a sphere and a share of the columns, the sphere's coefficients once
+// for all of them; a thread per (sphere, column) took 152 us for 60 spheres of
+// order 8.
+__global__ void __launch_bounds__(QEFF_NT) tm_qeff_kernel(int nsph, int ncols, const int* order, const int* offset, const int* mie_offset,
+                                                          const double* radius, zd rimed, const zd* an_inv, const zd* A, const zd* P,
+                                                          int ld, double* qcol, const zd* G, const double* rext)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nsph * ncols) return;
-    const int c = t / nsph, i = t - c * nsph;
+    __shared__ QeffCoef co;
+    __shared__ double red[2 * 3];
+    const int i = blockIdx.x;
     const int L = order[i], off = offset[i], hb = L * (L + 2);
     const double xsp = radius[i];
     const zd ri0 = rext ? mk(rext[2 * i], rext[2 * i + 1]) : rimed;
-    const zd xri = xsp * ri0;
     const zd rib = cdivr(2.0, cdivr(1.0, ri0) + cdivr(1.0, ri0));
-    zd psi[MSTMG_LMAX + 2], xi[MSTMG_LMAX + 2], scr[2 * (MSTMG_LMAX + 2)];   // sphere orders are at most MSTMG_LMAX
-    mstm_cricbessel(L, xri, psi, scr);
-    mstm_crichankel(L, xri, xi, scr);
-    const zd* a = A + (size_t)c * ld + off;
-    const zd* f = P + (size_t)c * ld + off;
+    qeff_coefficients(co, L, xsp, ri0);
     const zd* Ai = an_inv + mie_offset[i];
-    double qe = 0.0, qa = 0.0, qi = 0.0;
-    const zd cterm = imul(cdiv(cj(cdivr(1.0, ri0)), ri0));
-    for (int n = 1; n <= L; n++) {
-        zd psip = psi[n - 1] - cdiv((double)n * psi[n], xri);
-        zd xip = xi[n - 1] - cdiv((double)n * xi[n], xri);
-        zd aam[4], ggm[4], agm[4];
-        for (int s = 1; s <= 2; s++)
-            for (int u = 1; u <= 2; u++) {
-                double sg = pm1(s) * pm1(u);
-                int kk = (s - 1) + 2 * (u - 1);
-                aam[kk] = cterm * (xip * cj(xi[n]) - sg * (xi[n] * cj(xip)));
-                ggm[kk] = cterm * (psip * cj(psi[n]) - sg * (psi[n] * cj(psip)));
-                agm[kk] = cterm * (xip * cj(psi[n]) - sg * (xi[n] * cj(psip)));
-            }
-        const zd* Ain = Ai + 4 * (n - 1);
-        for (int m = -n; m <= n; m++) {
-            int a0 = aidx(m, n, 0, L);
+    for (int c = blockIdx.y; c < ncols; c += gridDim.y) {
+        const zd* a = A + (size_t)c * ld + off;
+        const zd* f = P + (size_t)c * ld + off;
+        double q[3] = {0.0, 0.0, 0.0};   // qe, qa, qi
+        for (int a0 = threadIdx.x; a0 < hb; a0 += QEFF_NT) {
+            const int n = slot_degree(a0, L);
+            const zd *aam = co.aam[n - 1], *ggm = co.ggm[n - 1], *agm = co.agm[n - 1];
+            const zd* Ain = Ai + 4 * (n - 1);
             zd av[2] = {a[a0], a[a0 + hb]};
             zd gv[2] = {Ain[0] * av[0] + Ain[2] * av[1], Ain[1] * av[0] + Ain[3] * av[1]};
             if (G) {
@@ -708,20 +699,21 @@ __global__ void tm_qeff_kernel(int nsph, int ncols, const int* order, const int*
                 gv[1] = gc[a0 + hb];
             }
             zd fv[2] = {f[a0], f[a0 + hb]};
+#pragma unroll
             for (int s = 0; s < 2; s++)
+#pragma unroll
                 for (int u = 0; u < 2; u++) {
-                    int kk = s + 2 * u;
-                    zd crib = cj(rib) + pm1(s + u) * rib;
-                    qi += (ggm[kk] * fv[s] * cj(rib * fv[u])).x;
-                    qa += (aam[kk] * av[s] * cj(rib * av[u]) + ggm[kk] * gv[s] * cj(rib * gv[u]) + agm[kk] * av[s] * cj(gv[u]) * crib).x;
-                    qe += (agm[kk] * av[s] * cj(fv[u]) * crib).x;
+                    const int kk = s + 2 * u;
+                    const zd crib = cj(rib) + pm1(s + u) * rib;
+                    q[2] += (ggm[kk] * fv[s] * cj(rib * fv[u])).x;
+                    q[1] += (aam[kk] * av[s] * cj(rib * av[u]) + ggm[kk] * gv[s] * cj(rib * gv[u]) + agm[kk] * av[s] * cj(gv[u]) * crib).x;
+                    q[0] += (agm[kk] * av[s] * cj(fv[u]) * crib).x;
                 }
         }
+        qeff_reduce<3>(q, red);
+        if (threadIdx.x == 0)   // qs = qi (the reference's 10-22 patch)
+            for (int j = 0; j < 3; j++) qcol[3 * ((size_t)i + (size_t)nsph * c) + j] = q[j] * 2.0 / xsp / xsp;
     }
-    double* q = qcol + 3 * ((size_t)i + (size_t)nsph * c);
-    q[0] = qe * 2.0 / xsp / xsp;
-    q[1] = qa * 2.0 / xsp / xsp;
-    q[2] = qi * 2.0 / xsp / xsp;   // qs = qi (the reference's 10-22 patch)
 }
 
 // One block: per sphere add the columns in order, then the weighted total in sphere order.
@@ -928,8 +920,10 @@ void launch_tm_rhs(int l, zd* P0, cudaStream_t st)
 void launch_tm_qeff(int nsph, int ncols, const int* order, const int* offset, const int* mie_offset, const double* radius, zd rimed,
                     const zd* an_inv, const zd* A, const zd* P, int ld, double* qcol, cudaStream_t st, const zd* G, const double* rext)
 {
-    int tot = nsph * ncols;
-    tm_qeff_kernel<<<(tot + 63) / 64, 64, 0, st>>>(nsph, ncols, order, offset, mie_offset, radius, rimed, an_inv, A, P, ld, qcol, G, rext);
+    // about 8 CTAs an SM: a few columns share a CTA's coefficients
+    int gy = (8 * 148 + nsph - 1) / nsph;
+    if (gy > ncols) gy = ncols;
+    tm_qeff_kernel<<<dim3(nsph, gy), QEFF_NT, 0, st>>>(nsph, ncols, order, offset, mie_offset, radius, rimed, an_inv, A, P, ld, qcol, G, rext);
     launch_counter() += 1;
 }
 void launch_tm_qsum(int nsph, int ncols, const double* qcol, const double* radius, double xv, double* sq, double* qsum, cudaStream_t st)

@@ -6,11 +6,11 @@
 // not allocate in the middle of its own stream work.  For them
 // mstmg_planewave_noalloc computes the same coefficients as mstmg_planewave
 // (no context, no cudaMalloc): the caller passes device input and output
-// buffers, and the two small intermediate tables live in the file-scope
-// device array below.
+// buffers, and the small intermediate table lives in the file-scope device
+// array below.
 //
 // The array is a fixed, modest size (enough for sphere order MSTMG_LMAX = 16,
-// about 32 KB) and every GPU that loads the library holds it until the
+// about 18 KB) and every GPU that loads the library holds it until the
 // process exits.  Its device address is looked up with cudaGetSymbolAddress
 // on every call made outside stream capture, with the calling thread's
 // current device and context (a context that was destroyed and made again
@@ -28,9 +28,8 @@
 #include "sphere_kernels.cuh"
 
 #define NOALLOC_PW0 (2 * 2 * MSTMG_LMAX * (MSTMG_LMAX + 2))       // pw0: nb(L) x 2 polarisations
-#define NOALLOC_DROT (3 * (MSTMG_LMAX * (MSTMG_LMAX + 2) + 1))    // Wigner-d table with |m| <= 1
 
-static __device__ __align__(256) zd g_pw_scratch[NOALLOC_PW0 + NOALLOC_DROT];
+static __device__ __align__(256) zd g_pw_scratch[NOALLOC_PW0];
 
 namespace {
 std::mutex g_mu;
@@ -38,7 +37,7 @@ zd* g_scratch_ptr[64] = {nullptr};
 }
 void mstmg_internal_set_error(const std::string& msg);   // message for mstmg_last_error (capi.cu)
 
-__global__ void planewave_common_kernel(double alpha, zd cb, int nodr, zd* pw0, zd* drot);
+__global__ void planewave_common_kernel(double alpha, zd cb, int nodr, zd* pw0);
 
 // Per-sphere phase for spheres that all have order L (layerplanewavecoef without
 // plane boundaries, december2023/mstm-modules-33.f90:3901-3965).
@@ -125,8 +124,7 @@ extern "C" int mstmg_planewave_noalloc(int nsphere, int order, const double* pos
     zd a = cdiv(mk(sinc, 0.0), riinc);
     zd cbinc = csqrtd((mk(1.0, 0.0) - a) * (mk(1.0, 0.0) + a)) * (double)(3 - 2 * dir);
     zd* pw0 = scratch;
-    zd* drot = scratch + NOALLOC_PW0;
-    planewave_common_kernel<<<1, 32, 0, st>>>(alpha, cbinc, order, pw0, drot);
+    planewave_common_kernel<<<1, PLANEWAVE_NT, 0, st>>>(alpha, cbinc, order, pw0);
     long long ne = (long long)nsphere * 2 * order * (order + 2);
     planewave_phase_uniform_kernel<<<(unsigned)((ne + 255) / 256), 256, 0, st>>>(nsphere, order, pos, pw0, cbinc, riinc, sinc, alpha,
                                                                                   (zd*)pmnp);

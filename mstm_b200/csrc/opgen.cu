@@ -103,6 +103,11 @@ __global__ void __launch_bounds__(128) opgen_pair_kernel(OpGenArgs a)
         zd* xi = a.xi + (size_t)q * XIW;
         const int nl = g.nt + g.ns;
         const zd z = a.pmed ? mk(g.r * a.pmed[2 * q], g.r * a.pmed[2 * q + 1]) : mk(g.r * a.rimed_re, g.r * a.rimed_im);
+        if (mstm_bessel_real(nl, z, xi)) {
+            if (a.regular)
+                for (int k = 0; k <= nl; k++) xi[k].y = 0.0;
+            continue;
+        }
         if (a.regular) mstm_cricbessel(nl, z, xi, hs);
         else mstm_crichankel(nl, z, xi, hs);
         for (int k = 0; k <= nl; k++) xi[k] = cdiv(xi[k], z);

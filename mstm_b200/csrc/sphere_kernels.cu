@@ -3,6 +3,7 @@
 // coefficient generation and the final cross-section sums run in FP64.
 #include "common.cuh"
 #include "special.cuh"
+#include "qeffcoef.cuh"
 #include "kernels.cuh"
 #include "sphere_kernels.cuh"
 
@@ -180,100 +181,83 @@ void launch_mie_coefs(int n, const double* radius, const double* ri, double mre,
 // lmax into pw0(nb(lmax), 2 polarisations), then per sphere the phase of
 // layerplanewavecoef without plane boundaries (modules:3901-3965).
 // ---------------------------------------------------------------------------
-__global__ void planewave_common_kernel(double alpha, zd cb, int nodr, zd* pw0, zd* drot /* 3*(nodr(nodr+2)+1) */)
+// One CTA, a thread per column k = -n..n of the degree, rows m = 0, +-1 of the
+// degree in shared memory (rows beyond are not used): latency bound, two
+// barriers a degree.  On one thread the square roots and divisions of every
+// (n, k) stood in line: 81 us at order 7, 290 us at order 14; now 11 and 20 us.
+__global__ void __launch_bounds__(PLANEWAVE_NT) planewave_common_kernel(double alpha, zd cb, int nodr, zd* pw0)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
     // crotcoef(cb, kmax=1, nodr) (modules:1187-1246)
-    const int kmax = 1, ld = 3;
-    int nd = nodr * (nodr + 2) + 1;
-    for (int k = 0; k < ld * nd; k++) drot[k] = mk(0.0, 0.0);
-#define DC(m, nk) drot[((m) + kmax) + ld * (nk)]
-    zd sbe = csqrtd((mk(1.0, 0.0) + cb) * (mk(1.0, 0.0) - cb));
-    zd cbe2 = 0.5 * (mk(1.0, 0.0) + cb), sbe2 = 0.5 * (mk(1.0, 0.0) - cb);
-    zd dk0s[2 * MSTMG_LMAX + 3], dk01s[2 * MSTMG_LMAX + 3];
-    zd* dk0 = dk0s + (MSTMG_LMAX + 1);
-    zd* dk01 = dk01s + (MSTMG_LMAX + 1);
-    for (int k = 0; k < 2 * MSTMG_LMAX + 3; k++) { dk0s[k] = mk(0.0, 0.0); dk01s[k] = mk(0.0, 0.0); }
-    int in = 1;
-    dk0[0] = mk(1.0, 0.0);
+    __shared__ double sq[2 * MSTMG_LMAX + 3];
+    __shared__ zd dk0s[2 * MSTMG_LMAX + 1], row1[2 * MSTMG_LMAX + 1], ea[MSTMG_LMAX + 1];
+    static_assert(PLANEWAVE_NT >= 2 * MSTMG_LMAX + 3, "a thread per column and per square root");
+    const int k = (int)threadIdx.x - MSTMG_LMAX, nb = 2 * nodr * (nodr + 2);
+    zd* dk0 = dk0s + MSTMG_LMAX;
+    zd* v1 = row1 + MSTMG_LMAX;
+    const zd sbe = csqrtd((mk(1.0, 0.0) + cb) * (mk(1.0, 0.0) - cb));
+    const zd cbe2 = 0.5 * (mk(1.0, 0.0) + cb), sbe2 = 0.5 * (mk(1.0, 0.0) - cb);
+    if (threadIdx.x < 2 * MSTMG_LMAX + 3) sq[threadIdx.x] = sqrt((double)threadIdx.x);
+    if (threadIdx.x == PLANEWAVE_NT - 1) {
+        // ealpham: powers of e^{i alpha} as ephicoef builds them
+        const zd ep = mk(cos(alpha), sin(alpha));
+        zd pw = mk(1.0, 0.0);
+        for (int q = 0; q <= nodr; q++) {
+            ea[q] = pw;
+            pw = ep * pw;
+        }
+    }
+    zd d0 = mk(k == 0 ? 1.0 : 0.0, 0.0), d01 = mk(0.0, 0.0);   // dk0, dk01 of this column
     zd sben = mk(1.0, 0.0);
-    DC(0, 0) = mk(1.0, 0.0);
     // bcof(n,n) = sqrt((2n)!/(n!)^2), built by the same recurrence as numconstants::init
     double bnn = 1.0;
+    __syncthreads();
     for (int n = 1; n <= nodr; n++) {
-        bnn = sqrt((double)(n + n)) * sqrt((double)(n + n - 1)) * bnn / sqrt((double)n) / sqrt((double)n);
-        int knmax = n < kmax ? n : kmax;
-        int nn1 = n * (n + 1);
-        in = -in;
-        {
-            zd tq = sben * sbe;   // sben = sben*sbe/2
-            sben = mk(tq.x / 2.0, tq.y / 2.0);
+        const double in = pm1(n);
+        bnn = sq[n + n] * sq[n + n - 1] * bnn / sq[n] / sq[n];
+        const zd tq = sben * sbe;   // sben = sben*sbe/2
+        sben = mk(tq.x / 2.0, tq.y / 2.0);
+        const bool on = k >= -n && k <= n;
+        if (k == n || k == -n) {
+            d0 = (in * sben) * bnn;
+            if (k == -n) d0 = in * d0;
+            d01 = mk(0.0, 0.0);
+        } else if (on) {
+            const zd dkt = d01;
+            d01 = d0;
+            const double c1 = (double)(n + n - 1), c2 = sq[n - k - 1] * sq[n + k - 1], c3 = sq[n + k] * sq[n - k];
+            const zd num = (cb * c1) * d01 - c2 * dkt;
+            d0 = mk(num.x / c3, num.y / c3);
         }
-        dk0[n] = ((double)in * sben) * bnn;
-        dk0[-n] = (double)in * dk0[n];
-        dk01[n] = mk(0.0, 0.0);
-        dk01[-n] = mk(0.0, 0.0);
-        DC(0, nn1 + n) = dk0[n];
-        DC(0, nn1 - n) = dk0[-n];
-        for (int k = -n + 1; k <= n - 1; k++) {
-            int kn = nn1 + k;
-            zd dkt = dk01[k];
-            dk01[k] = dk0[k];
-            double c1 = (double)(n + n - 1), c2 = sqrt((double)(n - k - 1)) * sqrt((double)(n + k - 1));
-            double c3 = sqrt((double)(n + k)) * sqrt((double)(n - k));
-            zd num = (cb * c1) * dk01[k] - c2 * dkt;
-            dk0[k] = mk(num.x / c3, num.y / c3);
-            DC(0, kn) = dk0[k];
+        if (on) dk0[k] = d0;
+        __syncthreads();
+        if (on) {
+            const double fmn = 1.0 / sq[n] / sq[n + 1];
+            const zd dkm1 = (k == -n) ? mk(0.0, 0.0) : dk0[k - 1], dkn1 = (k == n) ? mk(0.0, 0.0) : dk0[k + 1];
+            const zd v = (sq[n + k] * sq[n - k + 1]) * cbe2 * dkm1 - (sq[n - k] * sq[n + k + 1]) * sbe2 * dkn1 - ((double)k * sbe) * d0;
+            v1[k] = v * fmn;
         }
-        int im = 1;
-        for (int m = 1; m <= knmax; m++) {
-            im = -im;
-            double fmn = 1.0 / sqrt((double)(n - m + 1)) / sqrt((double)(n + m));
-            int m1 = m - 1;
-            zd dkm0 = mk(0.0, 0.0);
-            for (int k = -n; k <= n; k++) {
-                int kn = nn1 + k;
-                zd dkm1 = dkm0;
-                dkm0 = DC(m1, kn);
-                zd dkn1 = (k == n) ? mk(0.0, 0.0) : DC(m1, kn + 1);
-                zd v = (sqrt((double)(n + k)) * sqrt((double)(n - k + 1))) * cbe2 * dkm1 -
-                       (sqrt((double)(n - k)) * sqrt((double)(n + k + 1))) * sbe2 * dkn1 - ((double)k * sbe) * DC(m1, kn);
-                DC(m, kn) = v * fmn;
-                DC(-m, nn1 - k) = DC(m, kn) * (pm1(k) * im);
-            }
-        }
-    }
-    int nb = 2 * nodr * (nodr + 2);
-    // tau(0:nodr+1,nodr,2) then the LR combination
-    for (int n = 1; n <= nodr; n++) {
-        int nn1 = n * (n + 1);
-        double fnm = sqrt((double)(n + n + 1) / 2.0) / 4.0;
-        zd cin;
-        {
-            int e = (n + 1) % 4;
-            zd ipw = (e == 0) ? mk(1.0, 0.0) : (e == 1 ? mk(0.0, 1.0) : (e == 2 ? mk(-1.0, 0.0) : mk(0.0, -1.0)));
-            cin = 4.0 * ipw;
-        }
-        for (int m = -n; m <= n; m++) {
-            int mn = nn1 + m;
-            zd tau1 = -fnm * (-DC(-1, mn) + DC(1, mn));
-            zd tau2 = -fnm * (DC(-1, mn) + DC(1, mn));
-            zd taulr[2] = {(tau1 + tau2) * 0.5, (tau1 - tau2) * 0.5};
-            // ealpham(-m): powers of e^{i alpha} as ephicoef builds them
-            zd ea;
-            zd ep = mk(cos(alpha), sin(alpha));
-            zd pw = mk(1.0, 0.0);
-            for (int q = 1; q <= (m < 0 ? -m : m); q++) pw = ep * pw;
-            ea = (m <= 0) ? pw : cj(pw);
+        __syncthreads();
+        // tau(m,n,2), m = k, then the LR combination; row -1 is
+        // D(-1,m) = -(-1)^m D(1,-m)
+        if (on) {
+            const int m = k;
+            const zd dp = v1[m], dm = v1[-m] * (-pm1(m));
+            const double fnm = sqrt((double)(n + n + 1) / 2.0) / 4.0;
+            const int e = (n + 1) % 4;
+            const zd ipw = (e == 0) ? mk(1.0, 0.0) : (e == 1 ? mk(0.0, 1.0) : (e == 2 ? mk(-1.0, 0.0) : mk(0.0, -1.0)));
+            const zd cin = 4.0 * ipw;
+            const zd tau1 = -fnm * (-dm + dp);
+            const zd tau2 = -fnm * (dm + dp);
+            const zd taulr[2] = {(tau1 + tau2) * 0.5, (tau1 - tau2) * 0.5};
+            const zd em = (m <= 0) ? ea[-m] : cj(ea[m]);
             for (int p = 1; p <= 2; p++) {
-                double sp = -pm1(p);
-                int ai = aidx(m, n, p - 1, nodr);
-                pw0[ai] = -(cin * taulr[p - 1] * ea);
-                pw0[nb + ai] = sp * imul(cin * taulr[p - 1] * ea);
+                const double sp = -pm1(p);
+                const int ai = aidx(m, n, p - 1, nodr);
+                pw0[ai] = -(cin * taulr[p - 1] * em);
+                pw0[nb + ai] = sp * imul(cin * taulr[p - 1] * em);
             }
         }
     }
-#undef DC
 }
 
 // outside (may be null): 1 for the spheres outside every other; the others,
@@ -308,12 +292,12 @@ __global__ void planewave_phase_kernel(int nslots2, const int* slot_sphere, cons
 }
 
 void launch_planewave(double alpha, double sinc, int dir, int lmax, int neqns, const int* slot_full, const int* order,
-                      const int* offset, const double* pos, zd* pw0, zd* drot, zd* pmnp, cudaStream_t st, int nreal, const int* outside)
+                      const int* offset, const double* pos, zd* pw0, zd* pmnp, cudaStream_t st, int nreal, const int* outside)
 {
     zd riinc = mk(1.0, 0.0);
     zd a = cdiv(mk(sinc, 0.0), riinc);
     zd cbinc = csqrtd((mk(1.0, 0.0) - a) * (mk(1.0, 0.0) + a)) * (double)(3 - 2 * dir);
-    planewave_common_kernel<<<1, 32, 0, st>>>(alpha, cbinc, lmax, pw0, drot);
+    planewave_common_kernel<<<1, PLANEWAVE_NT, 0, st>>>(alpha, cbinc, lmax, pw0);
     planewave_phase_kernel<<<(neqns + 255) / 256, 256, 0, st>>>(neqns, slot_full, order, offset, pos, lmax, pw0, cbinc, riinc,
                                                                  sinc, alpha, pmnp, neqns, nreal, outside);
     launch_counter() += 2;
@@ -443,89 +427,71 @@ template void launch_hmie<float>(int, int, const int*, const int*, const int*, c
 // With host spheres (gmnp given) the exciting field is the interaction
 // without the Mie multiply plus the incident field, and each sphere sits in
 // the index rext around it (qefficiencyfactors, scatprops:807-840).
-__global__ void qeff_kernel(int nsph, const int* order, const int* offset, const int* mie_offset, const double* radius, zd rimed,
-                            const zd* an_inv, const zd* amnp, const zd* pmnp0, int ld, double* qeff, const double* rext, const zd* gmnp)
+// One CTA a sphere, its (m, n) slots over the threads, the coefficients of each
+// degree once in shared memory: latency bound.  One thread a sphere summed
+// every slot in line and kept the Bessel arrays in local memory: 135 us for 20
+// spheres of order 7 and 417 us for 40 of order 14; now 11 and 15 us.
+__global__ void __launch_bounds__(QEFF_NT) qeff_kernel(int nsph, const int* order, const int* offset, const int* mie_offset,
+                                                       const double* radius, zd rimed, const zd* an_inv, const zd* amnp, const zd* pmnp0,
+                                                       int ld, double* qeff, const double* rext, const zd* gmnp)
 {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nsph) return;
-    int L = order[i], off = offset[i];
-    double xsp = radius[i];
-    zd ri0 = rext ? mk(rext[2 * i], rext[2 * i + 1]) : rimed;
-    zd xri = xsp * ri0;
-    zd rib = cdivr(2.0, cdivr(1.0, ri0) + cdivr(1.0, ri0));
-    zd psi[MIE_NMAX], xi[MIE_NMAX], scr[2 * MIE_NMAX];
-    mstm_cricbessel(L, xri, psi, scr);
-    mstm_crichankel(L, xri, xi, scr);
-    double qe[3] = {0, 0, 0}, qa[3] = {0, 0, 0}, qi[3] = {0, 0, 0};
+    __shared__ QeffCoef co;
+    __shared__ double red[2 * 9];
+    const int i = blockIdx.x;
+    const int L = order[i], off = offset[i];
+    const double xsp = radius[i];
+    const zd ri0 = rext ? mk(rext[2 * i], rext[2 * i + 1]) : rimed;
+    const zd rib = cdivr(2.0, cdivr(1.0, ri0) + cdivr(1.0, ri0));
+    qeff_coefficients(co, L, xsp, ri0);
+    double q[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};   // qe, qa, qi, three each
     const zd* Ai = an_inv + mie_offset[i];
-    int hb = L * (L + 2);
-    for (int n = 1; n <= L; n++) {
-        zd psip = psi[n - 1] - cdiv((double)n * psi[n], xri);
-        zd xip = xi[n - 1] - cdiv((double)n * xi[n], xri);
-        zd aam[4], ggm[4], agm[4];
-        zd cterm = imul(cdiv(cj(cdivr(1.0, ri0)), ri0));
-        for (int s = 1; s <= 2; s++) {
-            double ss = pm1(s);
-            for (int t = 1; t <= 2; t++) {
-                double st = pm1(t);
-                int k = (s - 1) + 2 * (t - 1);
-                aam[k] = cterm * (xip * cj(xi[n]) - (ss * st) * (xi[n] * cj(xip)));
-                ggm[k] = cterm * (psip * cj(psi[n]) - (ss * st) * (psi[n] * cj(psip)));
-                agm[k] = cterm * (xip * cj(psi[n]) - (ss * st) * (xi[n] * cj(psip)));
-            }
-        }
+    const int hb = L * (L + 2);
+    for (int a0 = threadIdx.x; a0 < hb; a0 += QEFF_NT) {
+        const int n = slot_degree(a0, L);
+        const zd *aam = co.aam[n - 1], *ggm = co.ggm[n - 1], *agm = co.agm[n - 1];
         const zd* Ain = Ai + 4 * (n - 1);
-        for (int m = -n; m <= n; m++) {
-            int a0 = aidx(m, n, 0, L);
-            zd av[2][2], gv[2][2], fv[2][2];   // [pol][mode]
-            for (int pol = 0; pol < 2; pol++) {
-                zd x0 = amnp[(size_t)pol * ld + off + a0], x1 = amnp[(size_t)pol * ld + off + a0 + hb];
-                av[pol][0] = x0;
-                av[pol][1] = x1;
-                if (gmnp) {
-                    gv[pol][0] = gmnp[(size_t)pol * ld + off + a0];
-                    gv[pol][1] = gmnp[(size_t)pol * ld + off + a0 + hb];
-                } else {
-                    // onemiecoeffmult with the inverse: g(p) = sum_q Ainv(p,q) a(q)
-                    gv[pol][0] = Ain[0] * x0 + Ain[2] * x1;
-                    gv[pol][1] = Ain[1] * x0 + Ain[3] * x1;
-                }
-                fv[pol][0] = pmnp0[(size_t)pol * ld + off + a0];
-                fv[pol][1] = pmnp0[(size_t)pol * ld + off + a0 + hb];
+        zd av[2][2], gv[2][2], fv[2][2];   // [pol][mode]
+        for (int pol = 0; pol < 2; pol++) {
+            zd x0 = amnp[(size_t)pol * ld + off + a0], x1 = amnp[(size_t)pol * ld + off + a0 + hb];
+            av[pol][0] = x0;
+            av[pol][1] = x1;
+            if (gmnp) {
+                gv[pol][0] = gmnp[(size_t)pol * ld + off + a0];
+                gv[pol][1] = gmnp[(size_t)pol * ld + off + a0 + hb];
+            } else {
+                // onemiecoeffmult with the inverse: g(p) = sum_q Ainv(p,q) a(q)
+                gv[pol][0] = Ain[0] * x0 + Ain[2] * x1;
+                gv[pol][1] = Ain[1] * x0 + Ain[3] * x1;
             }
-            for (int p1 = 0; p1 < 2; p1++)
-                for (int p2 = 0; p2 < 2; p2++) {
-                    int k;
-                    double cst;
-                    if (p1 == 0 && p2 == 0) { k = 0; cst = 1.0; }
-                    else if (p1 == 1 && p2 == 1) { k = 1; cst = 1.0; }
-                    else { k = 2; cst = 0.5; }
-                    for (int s = 0; s < 2; s++)
-                        for (int t = 0; t < 2; t++) {
-                            int mk_ = s + 2 * t;
-                            double sgn = pm1(s + t);
-                            zd crib = cj(rib) + sgn * rib;
-                            qi[k] = qi[k] + (cst * (ggm[mk_] * fv[p1][s] * cj(rib * fv[p2][t]))).x;
-                            qa[k] = qa[k] + (cst * (aam[mk_] * av[p1][s] * cj(rib * av[p2][t]) + ggm[mk_] * gv[p1][s] * cj(rib * gv[p2][t]) +
-                                                    agm[mk_] * av[p1][s] * cj(gv[p2][t]) * crib)).x;
-                            qe[k] = qe[k] + (cst * (agm[mk_] * av[p1][s] * cj(fv[p2][t]) * crib)).x;
-                        }
-                }
+            fv[pol][0] = pmnp0[(size_t)pol * ld + off + a0];
+            fv[pol][1] = pmnp0[(size_t)pol * ld + off + a0 + hb];
         }
+#pragma unroll
+        for (int p1 = 0; p1 < 2; p1++)
+#pragma unroll
+            for (int p2 = 0; p2 < 2; p2++) {
+                const int k = p1 == p2 ? p1 : 2;
+                const double cst = p1 == p2 ? 1.0 : 0.5;
+#pragma unroll
+                for (int s = 0; s < 2; s++)
+#pragma unroll
+                    for (int t = 0; t < 2; t++) {
+                        const int mk_ = s + 2 * t;
+                        const zd crib = cj(rib) + pm1(s + t) * rib;
+                        q[6 + k] += (cst * (ggm[mk_] * fv[p1][s] * cj(rib * fv[p2][t]))).x;
+                        q[3 + k] += (cst * (aam[mk_] * av[p1][s] * cj(rib * av[p2][t]) + ggm[mk_] * gv[p1][s] * cj(rib * gv[p2][t]) +
+                                            agm[mk_] * av[p1][s] * cj(gv[p2][t]) * crib)).x;
+                        q[k] += (cst * (agm[mk_] * av[p1][s] * cj(fv[p2][t]) * crib)).x;
+                    }
+            }
     }
-    double qeffi[3][3];
-    for (int k = 0; k < 3; k++) {
-        qi[k] = qi[k] * 2.0 / xsp / xsp;
-        qe[k] = qe[k] * 2.0 / xsp / xsp;
-        qa[k] = qa[k] * 2.0 / xsp / xsp;
-        qeffi[0][k] = qe[k];
-        qeffi[1][k] = qa[k];
-        qeffi[2][k] = qi[k];
-    }
-    for (int q = 0; q < 3; q++) {
-        qeff[q + 3 * (0 + 3 * i)] = 0.5 * (qeffi[q][0] + qeffi[q][1]);
-        qeff[q + 3 * (1 + 3 * i)] = qeffi[q][0];
-        qeff[q + 3 * (2 + 3 * i)] = qeffi[q][1];
+    qeff_reduce<9>(q, red);
+    if (threadIdx.x != 0) return;
+    for (int k = 0; k < 9; k++) q[k] = q[k] * 2.0 / xsp / xsp;
+    for (int j = 0; j < 3; j++) {
+        qeff[j + 3 * (0 + 3 * i)] = 0.5 * (q[3 * j] + q[3 * j + 1]);
+        qeff[j + 3 * (1 + 3 * i)] = q[3 * j];
+        qeff[j + 3 * (2 + 3 * i)] = q[3 * j + 1];
     }
 }
 
@@ -555,22 +521,27 @@ __global__ void __launch_bounds__(QTOT_NT) qtot_kernel(int nsph, const double* r
     }
 }
 
-// totals over the spheres of each configuration of an ensemble (one thread
-// a configuration, the spheres summed in order as qtotcalc does)
-__global__ void qtot_configs_kernel(int nc, const int* cfg_start, const double* radius, const double* qeff, const double* xg, double* qtot)
+// totals over the spheres of each configuration of an ensemble, one warp a
+// configuration (one thread each left the loads of its spheres in line:
+// 77 us for 48 configurations of 15 to 40 spheres)
+__global__ void __launch_bounds__(128) qtot_configs_kernel(int nc, const int* cfg_start, const double* radius, const double* qeff,
+                                                           const double* xg, double* qtot)
 {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (k >= nc) return;
     double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int i = cfg_start[k]; i < cfg_start[k + 1]; i++)
+    for (int i = cfg_start[k] + lane; i < cfg_start[k + 1]; i += 32)
         for (int q = 0; q < 9; q++) s[q] = s[q] + qeff[q + 9 * i] * radius[i] * radius[i] / (xg[k] * xg[k]);
+    for (int q = 0; q < 9; q++)
+        for (int w = 16; w > 0; w >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], w);
+    if (lane != 0) return;
     for (int pol = 0; pol < 3; pol++) s[2 + 3 * pol] = s[0 + 3 * pol] + s[2 + 3 * pol] - s[1 + 3 * pol];
     for (int q = 0; q < 9; q++) qtot[q + 9 * k] = s[q];
 }
 
 void launch_qtot_configs(int nc, const int* cfg_start, const double* radius, const double* qeff, const double* xg, double* qtot, cudaStream_t st)
 {
-    qtot_configs_kernel<<<(nc + 63) / 64, 64, 0, st>>>(nc, cfg_start, radius, qeff, xg, qtot);
+    qtot_configs_kernel<<<(nc + 3) / 4, 128, 0, st>>>(nc, cfg_start, radius, qeff, xg, qtot);
     launch_counter() += 1;
 }
 
@@ -579,31 +550,49 @@ void launch_qtot_configs(int nc, const int* cfg_start, const double* radius, con
 // both scaled by the area ratio, written into qeff's absorption rows as the
 // reference does; the totals over the spheres outside every other.
 // qv: scratch of 3 nsph doubles.
-// held[hstart[i] .. hstart[i+1]): the spheres sphere i holds, in order
+// held[hstart[i] .. hstart[i+1]): the spheres sphere i holds, in order; a warp
+// sums them (one thread took 390 us for a host of 600)
 __global__ void __launch_bounds__(QTOT_NT) qtot_hosts_kernel(int nsph, const double* radius, const int* host, const int* hstart,
                                                              const int* held, double* qeff, double* qv, double xg, double* qtot)
 {
     __shared__ double red[9][QTOT_NT];
-    for (int i = threadIdx.x; i < nsph; i += QTOT_NT)
-        for (int p = 0; p < 3; p++) {
-            double v = qeff[1 + 3 * (p + 3 * i)];
-            for (int q = hstart[i]; q < hstart[i + 1]; q++) {
-                const int j = held[q];
-                v = v - qeff[1 + 3 * (p + 3 * j)] * radius[j] * radius[j] / (radius[i] * radius[i]);
-            }
-            qv[p + 3 * i] = v;
+    __shared__ int hlist[QTOT_NT], nh;
+    // spheres that hold others, gathered per QTOT_NT spheres, one warp each
+    auto each_holder = [&](auto body) {
+        for (int i0 = 0; i0 < nsph; i0 += QTOT_NT) {
+            const int i = i0 + threadIdx.x;
+            if (threadIdx.x == 0) nh = 0;
+            __syncthreads();
+            if (i < nsph && hstart[i + 1] > hstart[i]) hlist[atomicAdd(&nh, 1)] = i;
+            __syncthreads();
+            for (int h = threadIdx.x >> 5; h < nh; h += QTOT_NT / 32) body(hlist[h]);
+            __syncthreads();
         }
-    __syncthreads();
-    for (int i = threadIdx.x; i < nsph; i += QTOT_NT)
-        for (int p = 0; p < 3; p++) {
-            double v = qv[p + 3 * i];
-            for (int q = hstart[i]; q < hstart[i + 1]; q++) {
-                const int j = held[q];
-                v = v + qv[p + 3 * j] * radius[j] * radius[j] / (radius[i] * radius[i]);
-            }
-            qeff[1 + 3 * (p + 3 * i)] = v;
+    };
+    const int lane = threadIdx.x & 31;
+    // sum over the spheres i holds of q (element p + 3 j scaled) times (r_j / r_i)^2
+    auto held_sum = [&](int i, auto q) {
+        double v[3] = {0.0, 0.0, 0.0};
+        for (int h = hstart[i] + lane; h < hstart[i + 1]; h += 32) {
+            const int j = held[h];
+            for (int p = 0; p < 3; p++) v[p] += q(p + 3 * j) * radius[j] * radius[j] / (radius[i] * radius[i]);
         }
+        for (int p = 0; p < 3; p++)
+            for (int w = 16; w > 0; w >>= 1) v[p] += __shfl_xor_sync(0xffffffffu, v[p], w);
+        return lane == 0 ? v[0] : (lane == 1 ? v[1] : v[2]);   // lanes 0..2: p
+    };
+    for (int e = threadIdx.x; e < 3 * nsph; e += QTOT_NT) qv[e] = qeff[1 + 3 * e];
     __syncthreads();
+    each_holder([&](int i) {
+        const double v = held_sum(i, [&](int e) { return qeff[1 + 3 * e]; });
+        if (lane < 3) qv[lane + 3 * i] -= v;
+    });
+    for (int e = threadIdx.x; e < 3 * nsph; e += QTOT_NT) qeff[1 + 3 * e] = qv[e];
+    __syncthreads();
+    each_holder([&](int i) {
+        const double v = held_sum(i, [&](int e) { return qv[e]; });
+        if (lane < 3) qeff[1 + 3 * (lane + 3 * i)] += v;
+    });
     double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
     for (int i = threadIdx.x; i < nsph; i += QTOT_NT)
         if (host[i] < 0)
@@ -627,7 +616,7 @@ void launch_qeff(int nsph, const int* order, const int* offset, const int* mie_o
                  const zd* amnp, const zd* pmnp0, int ld, double* qeff, double xg, double* qtot, cudaStream_t st, const double* rext,
                  const zd* gmnp, const int* host, double* qv, const int* hstart, const int* held)
 {
-    qeff_kernel<<<(nsph + 63) / 64, 64, 0, st>>>(nsph, order, offset, mie_offset, radius, rimed, an_inv, amnp, pmnp0, ld, qeff, rext, gmnp);
+    qeff_kernel<<<nsph, QEFF_NT, 0, st>>>(nsph, order, offset, mie_offset, radius, rimed, an_inv, amnp, pmnp0, ld, qeff, rext, gmnp);
     if (host) qtot_hosts_kernel<<<1, QTOT_NT, 0, st>>>(nsph, radius, host, hstart, held, qeff, qv, xg, qtot);
     else qtot_kernel<<<1, QTOT_NT, 0, st>>>(nsph, radius, qeff, xg, qtot);
     launch_counter() += 2;

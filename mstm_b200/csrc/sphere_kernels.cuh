@@ -11,8 +11,9 @@ void launch_mie_coefs(int n, const double* radius, const double* ri, double mre,
                       const int* mie_offset, const int* hoff, zd* an, zd* an_inv, float* an32, zd* dn, zd* un, zd* vn, double* qext,
                       double* qabs, cudaStream_t st);
 // outside (null: every sphere): 1 for the spheres the incident wave reaches
+#define PLANEWAVE_NT 64   // threads of planewave_common_kernel
 void launch_planewave(double alpha, double sinc, int dir, int lmax, int neqns, const int* slot_full, const int* order,
-                      const int* offset, const double* pos, zd* pw0, zd* drot, zd* pmnp, cudaStream_t st, int nreal = 0,
+                      const int* offset, const double* pos, zd* pw0, zd* pmnp, cudaStream_t st, int nreal = 0,
                       const int* outside = nullptr);
 // Mie multiply with host spheres' second blocks at hoff[i] (>= 0)
 template <typename T>
