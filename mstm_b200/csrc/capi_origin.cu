@@ -556,9 +556,9 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     if (rc) return rc;
     const size_t nblkt = 2 * (size_t)T * (T + 2);
     const int W = 2 * T + 1;
-    DevBuf<zd> dT, trace, dm, dmcf, fm;
+    DevBuf<zd> dT, trace, dm, dmcf, bg, bcf, part;
     DevBuf<float2> tc;
-    DevBuf<double> dsm, dsmat, vscr, dscr, dbcd;
+    DevBuf<double> dsm, dsmat, vtab, dscr, dbcd;
     CK(dT.alloc(nblkt * nblkt));
     CK(copy_in(dT.p, tmat, sizeof(zd) * nblkt * nblkt, c->st));
     CK(tc.alloc(nblkt * nblkt));
@@ -567,9 +567,12 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     CK(dmcf.alloc(ro_dm_elems(T)));
     CK(cudaMemsetAsync(dm.p, 0, sizeof(zd) * ro_dm_elems(T), c->st));
     CK(cudaMemsetAsync(dmcf.p, 0, sizeof(zd) * ro_dm_elems(T), c->st));
-    CK(fm.alloc((size_t)W * 2 * 3 * T * 2 * T * 2));
+    const RoSizes rz = ro_sizes(T);
+    CK(bg.alloc(rz.bg));
+    CK(bcf.alloc(rz.bcf));
+    CK(part.alloc(rz.part));
     CK(dsm.alloc(2 * 16 * (size_t)W));
-    CK(vscr.alloc(ro_vscr_doubles(T, c->nsm)));
+    CK(vtab.alloc(rz.vtab));
     const int nang = nangles > 0 ? nangles : 1;
     CK(dscr.alloc((size_t)nang * (16 * (2 * T) + 40)));
     CK(dsmat.alloc(16 * (size_t)nang));
@@ -583,16 +586,20 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     a.trace = trace.p;
     a.dm = dm.p;
     a.dmcf = dmcf.p;
-    a.fm = fm.p;
+    a.bg = bg.p;
+    a.bcf = bcf.p;
+    a.part = part.p;
+    a.bgi = rz.bgi;
+    a.vw0 = 0;
     a.sm = dsm.p;
     a.smcf = dsm.p + 16 * W;
     a.bcof = bt.bc.p;
     a.fnr = bt.fnr.p;
     a.nbc = bt.nbc;
-    a.vscr = vscr.p;
+    a.vtab = vtab.p;
     a.rimed_re = c->opts.medium_re;
     if (launch_ranorient(a, dT.p, nangles, dbcd.p, dscr.p, dsmat.p, c->nsm, c->st) != 0) {
-        set_err("mstmg_ranorient_scattering: t_matrix_order too large for the shared-memory layout");
+        set_err("mstmg_ranorient_scattering: t_matrix_order too large for the kernels (at most " + std::to_string(RO_ORDER_MAX) + ")");
         return MSTMG_ERR_UNSUPPORTED;
     }
     CK(cudaGetLastError());
