@@ -55,11 +55,10 @@ static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps,
         }
     for (int k = 0; k < 3; k++) r0[k] = r0[k] / (double)nout;
     DevBuf<zd> tscr;
-    const int sstride = 3 * (200 + MSTMG_LMAX + 4);
     CK(dtord.alloc(n));
-    CK(tscr.alloc(tranorder_scratch(n, sstride)));
-    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc.p, bt.fnr.p, bt.nbc, tscr.p, sstride,
-                     dtord.p, c->st);
+    CK(tscr.alloc(tranorder_scratch(n)));
+    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc.p, bt.fnr.p, bt.nbc, tscr.p, dtord.p,
+                     c->st);
     tord.resize(n);
     CK(cudaMemcpyAsync(tord.data(), dtord.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -186,8 +185,8 @@ extern "C" int mstmg_scattering(mstmg_ctx* c, const double* amnp, double trans_e
     CK(copy_in(dsrc.p, amnp, sizeof(zd) * 2 * (size_t)ne, c->st));
     CK(da0.alloc(2 * (size_t)nb0));
     CK(cudaMemsetAsync(da0.p, 0, sizeof(zd) * 2 * (size_t)nb0, c->st));
-    int grid = std::min(n, c->nsm * 2);
-    size_t stride = merge_scratch_per_cta(T, L);
+    int grid = std::min(n, c->nsm * 3);
+    size_t stride = merge_scratch_per_cta(T, L, 2);
     CK(mscr.alloc((size_t)grid * stride));
     MergeArgs ma = merge_args(c, rt, bt, r0, dtord.p);
     ma.T = T;
@@ -202,14 +201,12 @@ extern "C" int mstmg_scattering(mstmg_ctx* c, const double* amnp, double trans_e
     CK(cudaGetLastError());
     // GSF expansion and scattering matrix
     const int W = 2 * T + 1;
-    DevBuf<double> ds, fscr, cscr, dsm;
+    DevBuf<double> ds, dsm;
     CK(ds.alloc(4 * 16 * (size_t)W));
     CK(cudaMemsetAsync(ds.p, 0, sizeof(double) * 4 * 16 * (size_t)W, c->st));
-    CK(fscr.alloc(fosm_scratch_doubles(T)));
-    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, fscr.p, c->st);
-    CK(cscr.alloc(fosmcalc_scratch_doubles(T, nangles)));
+    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
     CK(dsm.alloc(16 * (size_t)nangles));
-    launch_fosmcalc(T, nangles, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, bt.fnr.p, rt.bcd.p, cscr.p, dsm.p, c->st);
+    launch_fosmcalc(T, nangles, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, bt.fnr.p, rt.bcd.p, dsm.p, c->st);
     CK(cudaGetLastError());
     double s0[2];
     CK(cudaMemcpyAsync(&s0[0], ds.p + 0, sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -235,13 +232,12 @@ extern "C" int mstmg_gsf_coefficients(mstmg_ctx* c, int t_matrix_order, const do
     const size_t nb0 = 2 * (size_t)T * (T + 2);
     const int W = 2 * T + 1;
     DevBuf<zd> da0;
-    DevBuf<double> ds, fscr;
+    DevBuf<double> ds;
     CK(da0.alloc(2 * nb0));
     CK(copy_in(da0.p, amnp0, sizeof(zd) * 2 * nb0, c->st));
     CK(ds.alloc(4 * 16 * (size_t)W));
     CK(cudaMemsetAsync(ds.p, 0, sizeof(double) * 4 * 16 * (size_t)W, c->st));
-    CK(fscr.alloc(fosm_scratch_doubles(T)));
-    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, fscr.p, c->st);
+    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
     CK(cudaGetLastError());
     CK(copy_out(coef, ds.p, sizeof(double) * 4 * 16 * (size_t)W, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -365,7 +361,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
     RegTables rtm, rtd;   // merge: spheres -> origin; distribute: origin -> spheres
     if ((rc = build_reg_tables(c, TM, L, rtm)) || (rc = build_reg_tables(c, L, TM, rtd))) return rc;
     const int grid = std::min(n, c->nsm * 2);
-    const size_t strm = merge_scratch_per_cta(TM, L), strd = merge_scratch_per_cta(L, TM);
+    const size_t strm = merge_scratch_per_cta(TM, L, Sord), strd = merge_scratch_per_cta(L, TM, Sord);
     DevBuf<zd> mscr, P0, PK, B64, A0, dT, X64;
     DevBuf<double> qcol, dsq, qsum, rr;
     DevBuf<zf> B32;
@@ -413,6 +409,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
             launch_tm_rhs(q, P0.p, c->st);
             MergeArgs md = merge_args(c, rtd, bt, r0, dtord.p);
             md.mode = 1;
+            md.lsrc = q;
             md.out = PK.p + (size_t)col0 * ne;
             md.ldo = ne;
             md.T = q;
@@ -558,7 +555,7 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     const int W = 2 * T + 1;
     DevBuf<zd> dT, trace, dm, dmcf, bg, bcf, part;
     DevBuf<float2> tc;
-    DevBuf<double> dsm, dsmat, vtab, dscr, dbcd;
+    DevBuf<double> dsm, dsmat, vtab, dbcd;
     CK(dT.alloc(nblkt * nblkt));
     CK(copy_in(dT.p, tmat, sizeof(zd) * nblkt * nblkt, c->st));
     CK(tc.alloc(nblkt * nblkt));
@@ -574,7 +571,6 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     CK(dsm.alloc(2 * 16 * (size_t)W));
     CK(vtab.alloc(rz.vtab));
     const int nang = nangles > 0 ? nangles : 1;
-    CK(dscr.alloc((size_t)nang * (16 * (2 * T) + 40)));
     CK(dsmat.alloc(16 * (size_t)nang));
     std::vector<double> bd(2 * T + 4);
     for (int k = 0; k < (int)bd.size(); k++) bd[k] = big_tables().bc(k, k);
@@ -598,7 +594,7 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     a.nbc = bt.nbc;
     a.vtab = vtab.p;
     a.rimed_re = c->opts.medium_re;
-    if (launch_ranorient(a, dT.p, nangles, dbcd.p, dscr.p, dsmat.p, c->nsm, c->st) != 0) {
+    if (launch_ranorient(a, dT.p, nangles, dbcd.p, dsmat.p, c->nsm, c->st) != 0) {
         set_err("mstmg_ranorient_scattering: t_matrix_order too large for the kernels (at most " + std::to_string(RO_ORDER_MAX) + ")");
         return MSTMG_ERR_UNSUPPORTED;
     }

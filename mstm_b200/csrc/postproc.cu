@@ -17,9 +17,10 @@
 #include "special.cuh"
 #include "postproc.cuh"
 #include "vcoupling.cuh"
+#include "gsfrows.cuh"
 #include <algorithm>
 
-#define PP_NT 128
+#define PP_NT 256
 
 // vector-coupling coefficients: vc_func / vc_uprec of vcoupling.cuh
 
@@ -35,19 +36,21 @@ __device__ __forceinline__ zd ipow_z(int k)
 // n, exactly as the reference's loop does, and stops at the first order whose
 // partial sum meets the criterion.
 // ---------------------------------------------------------------------------
-#define TRANORDER_WPB 4
-__global__ void __launch_bounds__(32 * TRANORDER_WPB) tranorder_kernel(int nsph, const double* pos, const int* order, double ox,
-                                                                       double oy, double oz, double rire, double eps, int maxt,
-                                                                       VCTab tab, zd* scratch, int sstride, int* tord)
+// One Bessel evaluation serves all 32 orders, and each lane's coupling row lies
+// in shared memory; with an evaluation per order and rows in global scratch
+// the kernel took 1224 us for 350 spheres; now 47 us.
+#define TRANORDER_NLIM 200
+#define TRANORDER_ROW (TRANORDER_NLIM + 31 + MSTMG_LMAX + 2)
+__global__ void __launch_bounds__(32) tranorder_kernel(int nsph, const double* pos, const int* order, double ox, double oy, double oz,
+                                                       double rire, double eps, int maxt, VCTab tab, zd* scratch, int* tord)
 {
-    __shared__ double terms[TRANORDER_WPB][32];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const int gw = blockIdx.x * TRANORDER_WPB + wib, nw = gridDim.x * TRANORDER_WPB;
-    const int nlim = 200;
-    zd* xi = scratch + ((size_t)gw * 32 + lane) * sstride;
-    zd* scr = xi + (nlim + MSTMG_LMAX + 2);
-    double* vc1 = (double*)(scr + (nlim + MSTMG_LMAX + 2));
-    for (int i = gw; i < nsph; i += nw) {
+    extern __shared__ __align__(16) unsigned char tr_smem[];
+    zd* xs = reinterpret_cast<zd*>(tr_smem);                  // j_l(z) i^l
+    double* vc1 = reinterpret_cast<double*>(xs + TRANORDER_ROW) + threadIdx.x * TRANORDER_ROW;
+    __shared__ double terms[32];
+    const int lane = threadIdx.x;
+    zd* xi_own = scratch + ((size_t)blockIdx.x * 32 + lane) * 2 * TRANORDER_ROW;   // the complex routine's arrays
+    for (int i = blockIdx.x; i < nsph; i += gridDim.x) {
         const int lmax = order[i];
         const double dx = pos[3 * i] - ox, dy = pos[3 * i + 1] - oy, dz = pos[3 * i + 2] - oz;
         const double r = sqrt(dx * dx + dy * dy + dz * dz);
@@ -56,12 +59,24 @@ __global__ void __launch_bounds__(32 * TRANORDER_WPB) tranorder_kernel(int nsph,
             const zd z = mk(r * rire, 0.0);
             double sum = 0.0;
             int found = 0;
-            for (int n0 = 1; n0 <= nlim && !found; n0 += 32) {
+            for (int n0 = 1; n0 <= TRANORDER_NLIM && !found; n0 += 32) {
                 const int n = n0 + lane;
+                int shared_xi = 0;
+                __syncwarp();
+                if (lane == 0) shared_xi = mstm_bessel_real(min(n0 + 31, TRANORDER_NLIM) + lmax, z, xs);
+                shared_xi = __shfl_sync(0xffffffffu, shared_xi, 0);
+                __syncwarp();
+                if (shared_xi)
+                    for (int l = lane; l <= min(n0 + 31, TRANORDER_NLIM) + lmax; l += 32) xs[l] = mk(xs[l].x, 0.0) * ipow_z(l);
+                __syncwarp();
                 double term = 0.0;
-                if (n <= nlim) {
-                    mstm_cricbessel(n + lmax, z, xi, scr);
-                    for (int l = 0; l <= n + lmax; l++) xi[l] = cdiv(xi[l], z) * ipow_z(l);
+                if (n <= TRANORDER_NLIM) {
+                    const zd* xi = xs;
+                    if (!shared_xi) {
+                        mstm_cricbessel(n + lmax, z, xi_own, xi_own + TRANORDER_ROW);
+                        for (int l = 0; l <= n + lmax; l++) xi_own[l] = cdiv(xi_own[l], z) * ipow_z(l);
+                        xi = xi_own;
+                    }
                     const int l = lmax;
                     const zd c = (tab.fr(n + n + 1) * tab.fr(l + l + 1)) * ipow_z(n - l);
                     vc_func(tab, -1, n, 1, l, vc1);
@@ -76,11 +91,11 @@ __global__ void __launch_bounds__(32 * TRANORDER_WPB) tranorder_kernel(int nsph,
                     b = c * b;
                     term = (a * cj(a) + b * cj(b)).x;
                 }
-                terms[wib][lane] = term;
+                terms[lane] = term;
                 __syncwarp();
                 if (lane == 0)
-                    for (int k = 0; k < 32 && n0 + k <= nlim; k++) {
-                        sum = sum + terms[wib][k];
+                    for (int k = 0; k < 32 && n0 + k <= TRANORDER_NLIM; k++) {
+                        sum = sum + terms[k];
                         if (fabs(1.0 - sum) < eps) {
                             found = n0 + k;
                             break;
@@ -89,7 +104,7 @@ __global__ void __launch_bounds__(32 * TRANORDER_WPB) tranorder_kernel(int nsph,
                 found = __shfl_sync(0xffffffffu, found, 0);
                 __syncwarp();
             }
-            nmax = found ? found : nlim;
+            nmax = found ? found : TRANORDER_NLIM;
             nmax = max(nmax, lmax);
         }
         if (lane == 0) tord[i] = min(nmax, maxt);
@@ -101,15 +116,25 @@ __global__ void __launch_bounds__(32 * TRANORDER_WPB) tranorder_kernel(int nsph,
 // MERGE_PC columns), spheres grid-strided, scratch per CTA.  Per sphere the
 // translation's tables are made once -- e^{i m phi} powers, the regular
 // radial functions, the Wigner-d rows (rotcoef recurrence) and the axial
-// blocks of every degree m (first row and last column by the
-// vector-coupling sums, the interior by the three-term recurrence, as
-// axialtrancoefrecurrence fills them) -- and then applied to the chunk's
-// columns together: forward rotation, axial translation, back rotation,
-// each phase one barrier for all the columns.
+// blocks of every degree m -- and then applied to the chunk's columns
+// together: forward rotation, axial translation, back rotation, each phase
+// one barrier for all the columns.
+// The tables are latency bound, so each is split where it has no recurrence:
+// a thread owns a column of the m = 0 rows through every degree, a warp owns a
+// degree of the other rows (its two last rows in shared memory, no barrier),
+// and every axial element is its own vector-coupling sum (the reference's
+// three-term recurrence over n gives the same numbers).  With CTA-wide
+// barriers at every step of every recurrence, through global scratch, a launch
+// took 318 us for the columns of one order of a T matrix of 60 spheres and
+// 1330 us for 350 spheres of order 9 merged to one origin expansion; now 124
+// and 287 us.
+// Source expansions whose only nonzero degrees are lsrc and up (the unit
+// fields of one order that a T matrix distributes) skip the degrees below.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
 {
-    const int tid = threadIdx.x;
+    extern __shared__ __align__(16) unsigned char mg_smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int T = a.T;
     zd* base = a.scratch + ((size_t)blockIdx.y * gridDim.x + blockIdx.x) * a.scratch_stride;
     const bool dist = (a.mode == 1);
@@ -121,6 +146,7 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
         const int L = dist ? T : Li;                       // source order
         const int nt = dist ? Li : min(T, a.tord[i]);      // target order
         const int nmin = min(L, nt), nmax = max(L, nt);
+        const int l0 = max(1, a.lsrc);                     // first source degree
         const int W = 2 * nmin + 1;
         const double sv = dist ? -1.0 : 1.0;               // translation vector: target - source
         const double rv0 = sv * (a.r0[0] - a.pos[3 * i]), rv1 = sv * (a.r0[1] - a.pos[3 * i + 1]), rv2 = sv * (a.r0[2] - a.pos[3 * i + 2]);
@@ -130,15 +156,11 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
         zd* xi = base;                                        // nt+L+2
         zd* hs = xi + (nmax + L + 4);                         // Bessel scratch 2*(nt+L+2)
         zd* eph = hs + 2 * (nmax + L + 4);                    // e^{i m phi}, m = -nmax..nmax
-        double* D = (double*)(eph + (2 * nmax + 1));          // Wigner rows: per degree n, W x (2n+1), restricted index first
-        size_t dsz = 0;
-        for (int n = 0; n <= nmax; n++) dsz += (size_t)W * (2 * n + 1);
-        double* dk0 = D + dsz + 1 + (nmax + 1);
-        double* dk01 = dk0 + (2 * nmax + 3);
-        int* dofs = (int*)(dk01 + (nmax + 2));                // offsets of D per degree, nmax + 2 ints
-        zd* Zall = (zd*)(dofs + ((nmax + 3 + 3) & ~3));       // axial blocks, per degree ma: 2 x nt x L
-        zd* AP = Zall + (size_t)(nmin + 1) * 2 * nt * L;      // a'(k, l, q) per column: PC x 2 x L x W
-        zd* G = AP + (size_t)MERGE_PC * 2 * L * W;            // g(m, n, q) per column: PC x 2 x nt x W
+        double* D = (double*)(eph + (2 * nmax + 1));          // Wigner rows: per degree n, W x (2n+1) at W n n, restricted index first
+        zd* Zall = (zd*)(D + ((size_t)W * (nmax + 1) * (nmax + 1) + 1) / 2 * 2);   // axial blocks, per degree ma: 2 x nt x L
+        zd* AP = Zall + (size_t)(nmin + 1) * 2 * nt * L;      // a'(k, l, q) per column: np x 2 x L x W
+        zd* G = AP + (size_t)np * 2 * L * W;                  // g(m, n, q) per column: np x 2 x nt x W
+        zd* XP = G + (size_t)np * 2 * nt * W;                 // x(m, l, q) e^{i m phi} per column: np x 2 x L (L + 2)
         const zd* src = a.amnp;
         __syncthreads();
         if (rr < 1.0e-12) {
@@ -170,139 +192,123 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
         const double r = sqrt(rr);
         const double ct = rv2 / r;
         const zd ephi = (rv0 == 0.0 && rv1 == 0.0) ? mk(1.0, 0.0) : mk(rv0 / sqrt(rv0 * rv0 + rv1 * rv1), rv1 / sqrt(rv0 * rv0 + rv1 * rv1));
-        // Bessel functions psi_n(r)/r (cricbessel), n = 0..nt+L; e^{i m phi}; degree offsets of D
-        if (tid == 0) {
-            zd z = mk(r * a.rimed_re, r * a.rimed_im);
-            mstm_cricbessel(nt + L, z, xi, hs);
-            for (int k = 0; k <= nt + L; k++) xi[k] = cdiv(xi[k], z);
+        // Bessel functions psi_n(r)/r (cricbessel), n = 0..nt+L; e^{i m phi}
+        if (tid == PP_NT - 1) {
+            const zd z = mk(r * a.rimed_re, r * a.rimed_im);
+            if (mstm_bessel_real(nt + L, z, xi))
+                for (int k = 0; k <= nt + L; k++) xi[k].y = 0.0;
+            else {
+                mstm_cricbessel(nt + L, z, xi, hs);
+                for (int k = 0; k <= nt + L; k++) xi[k] = cdiv(xi[k], z);
+            }
         }
-        if (tid == 32) {
+        if (tid == PP_NT - 33) {
             zd* e = eph + nmax;
-            e[0] = mk(1.0, 0.0);
+            zd em = mk(1.0, 0.0);
+            e[0] = em;
             for (int m = 1; m <= nmax; m++) {
-                e[m] = ephi * e[m - 1];
-                e[-m] = cj(e[m]);
+                em = ephi * em;
+                e[m] = em;
+                e[-m] = cj(em);
             }
         }
-        if (tid == 64) {
-            int o = W;   // degree 0 occupies W x 1 but only its centre matters
-            dofs[0] = 0;
-            for (int n = 1; n <= nmax; n++) {
-                dofs[n] = o;
-                o += W * (2 * n + 1);
-            }
-        }
-        // Wigner-d rows by the rotcoef recurrence (kmax = nmin, nmax)
-        {
-            double sbe = (fabs(ct) >= 1.0) ? 0.0 : sqrt(fabs((1.0 + ct) * (1.0 - ct)));
-            double cbe2 = 0.5 * (1.0 + ct), sbe2 = 0.5 * (1.0 - ct);
-            for (int k = tid; k < 2 * nmax + 3; k += PP_NT) { dk0[k - (nmax + 1)] = 0.0; dk01[k - (nmax + 1)] = 0.0; }
-            __syncthreads();
-            if (tid == 0) { dk0[0] = 1.0; D[0] = 1.0; }
-            __syncthreads();
-            int sgn = 1;
-            double sben = 1.0;
-            size_t doff = (size_t)W;
-            for (int n = 1; n <= nmax; n++) {
-                int kk = min(n, nmin);
-                int ld = 2 * n + 1;
-                double* Dn = D + doff;
-                sgn = -sgn;
+        // Wigner-d rows by the rotcoef recurrence (kmax = nmin, nmax), of the
+        // degrees the rotations use
+        auto used = [&](int n) { return n <= nt || (n >= l0 && n <= L); };
+        const double sbe = (fabs(ct) >= 1.0) ? 0.0 : sqrt(fabs((1.0 + ct) * (1.0 - ct)));
+        const double cbe2 = 0.5 * (1.0 + ct), sbe2 = 0.5 * (1.0 - ct);
+        for (int k = tid - nmax; k <= nmax; k += PP_NT) {
+            const int ak = abs(k);
+            double d0 = 1.0, d01 = 0.0, sben = 1.0;
+            for (int n = 1; n <= ak; n++) {
                 sben = sben * sbe / 2.0;
                 if (sben < 1.0e-30) sben = 0.0;
-                double newv[4];
-                int cnt = 0;
-                for (int k = -n + 1 + tid; k <= n - 1; k += PP_NT) {
-                    newv[cnt++] = (ct * (double)(n + n - 1) * dk0[k] - a.fnr[n - k - 1] * a.fnr[n + k - 1] * dk01[k]) / (a.fnr[n + k] * a.fnr[n - k]);
+            }
+            if (ak > 0) {
+                d0 = pm1(ak) * sben * a.bcofd[ak];
+                if (k < 0) d0 = pm1(ak) * d0;
+                if (used(ak)) D[(size_t)W * ak * ak + nmin * (2 * ak + 1) + k + ak] = d0;
+            }
+            for (int n = ak + 1; n <= nmax; n++) {
+                const double v = (ct * (double)(n + n - 1) * d0 - a.fnr[n - k - 1] * a.fnr[n + k - 1] * d01) / (a.fnr[n + k] * a.fnr[n - k]);
+                d01 = d0;
+                d0 = v;
+                if (used(n)) D[(size_t)W * n * n + nmin * (2 * n + 1) + k + n] = v;
+            }
+        }
+        // phase (shift_op = F: e^{+i m phi} on the source) needs eph: after the barrier
+        __syncthreads();
+        {
+            double* row0 = reinterpret_cast<double*>(mg_smem) + (size_t)warp * 2 * (2 * nmax + 3);
+            double* row1 = row0 + 2 * nmax + 3;
+            for (int n = nmax - warp; n >= 1; n -= PP_NT / 32) {
+                if (!used(n)) continue;
+                const int kk = min(n, nmin), ld = 2 * n + 1;
+                double* Dn = D + (size_t)W * n * n + nmin * ld + n;   // (m, k) at m ld + k
+                double *cur = row0, *nxt = row1;                      // column k at k + n + 1, a zero at either end
+                for (int k = -n + lane; k <= n; k += 32) cur[k + n + 1] = Dn[k];
+                if (lane < 2) {
+                    row0[lane * (ld + 1)] = 0.0;
+                    row1[lane * (ld + 1)] = 0.0;
                 }
-                __syncthreads();
-                cnt = 0;
-                for (int k = -n + 1 + tid; k <= n - 1; k += PP_NT) {
-                    dk01[k] = dk0[k];
-                    dk0[k] = newv[cnt++];
-                }
-                if (tid == 0) {
-                    dk0[n] = sgn * sben * a.bcofd[n];
-                    dk0[-n] = sgn * dk0[n];
-                    dk01[n] = 0.0;
-                    dk01[-n] = 0.0;
-                }
-                __syncthreads();
-                for (int k = -n + tid; k <= n; k += PP_NT) Dn[(0 + nmin) * ld + (k + n)] = dk0[k];
-                __syncthreads();
-                int im = 1;
+                double fm = 0.0;   // of m = lane + 1
+                if (lane < kk) fm = 1.0 / a.fnr[n - lane] / a.fnr[n + lane + 1];
+                __syncwarp();
                 for (int m = 1; m <= kk; m++) {
-                    im = -im;
-                    double fmn = 1.0 / a.fnr[n - m + 1] / a.fnr[n + m];
-                    for (int k = -n + tid; k <= n; k += PP_NT) {
-                        double dkm1 = (k == -n) ? 0.0 : Dn[(m - 1 + nmin) * ld + (k - 1 + n)];
-                        double dkn1 = (k == n) ? 0.0 : Dn[(m - 1 + nmin) * ld + (k + 1 + n)];
-                        double v = (a.fnr[n + k] * a.fnr[n - k + 1] * cbe2 * dkm1 - a.fnr[n - k] * a.fnr[n + k + 1] * sbe2 * dkn1 -
-                                    (double)k * sbe * Dn[(m - 1 + nmin) * ld + (k + n)]) * fmn;
-                        Dn[(m + nmin) * ld + (k + n)] = v;
-                        Dn[(-m + nmin) * ld + (-k + n)] = v * pm1(k) * im;
+                    const double fmn = __shfl_sync(0xffffffffu, fm, m - 1), im = pm1(m);
+                    for (int k = -n + lane; k <= n; k += 32) {
+                        const double v = (a.fnr[n + k] * a.fnr[n - k + 1] * cbe2 * cur[k + n] - a.fnr[n - k] * a.fnr[n + k + 1] * sbe2 * cur[k + n + 2] -
+                                          (double)k * sbe * cur[k + n + 1]) * fmn;
+                        nxt[k + n + 1] = v;
+                        Dn[m * ld + k] = v;
+                        Dn[-m * ld - k] = v * pm1(k) * im;
                     }
-                    __syncthreads();
-                }
-                doff += (size_t)W * ld;
-            }
-        }
-        __syncthreads();
-        // axial blocks of every degree ma (regular functions), kept for all columns
-        for (int ma = 0; ma <= nmin; ma++) {
-            zd* Z = Zall + (size_t)ma * 2 * nt * L;
-            int m1 = max(1, ma);
-            int rows = nt - m1 + 1, cols = L - m1 + 1;
-            // first row n = m1 and last column l = L
-            for (int e = tid; e < cols + (rows - 1); e += PP_NT) {
-                int n, l;
-                if (e < cols) { n = m1; l = m1 + e; }
-                else { n = m1 + 1 + (e - cols); l = L; }
-                int wmin = abs(n - l), wmax = n + l, ml = l * (l + 1) + ma;
-                zd s1 = mk(0.0, 0.0), s2 = mk(0.0, 0.0);
-                for (int w = wmin; w <= wmax; w += 2) s1 = s1 + a.vcc[(n - 1) + (size_t)a.vcT * ((ml - 1) + (size_t)a.vcML * w)] * xi[w];
-                for (int w = wmin + 1; w <= wmax - 1; w += 2) s2 = s2 + a.vcc[(n - 1) + (size_t)a.vcT * ((ml - 1) + (size_t)a.vcML * w)] * xi[w];
-                s2 = imul(s2);
-                Z[(0 * nt + (n - 1)) * L + (l - 1)] = s1 + s2;
-                Z[(1 * nt + (n - 1)) * L + (l - 1)] = s1 - s2;
-            }
-            __syncthreads();
-            if (m1 < min(nt, L)) {
-                for (int n = m1; n <= nt - 1; n++) {
-                    for (int e = tid; e < 2 * (L - m1); e += PP_NT) {
-                        int pp = e / (L - m1), l = m1 + e % (L - m1);
-                        double sp = (pp == 0) ? 1.0 : -1.0;
-#define ZA(nn, ll) Z[(pp * nt + ((nn) - 1)) * L + ((ll) - 1)]
-#define FC(arr, mm, ll) arr[((mm) + a.fcN) + (2 * a.fcN + 1) * ((ll) - 1)]
-                        zd v = -(ZA(n, l + 1) * FC(a.fnp1, ma, l)) + imul(sp * (FC(a.fnc, ma, l) - FC(a.fnc, ma, n)) * ZA(n, l));
-                        if (l >= m1 + 1) v = v + ZA(n, l - 1) * FC(a.fnm1, ma, l);
-                        if (n > m1) v = v + ZA(n - 1, l) * FC(a.fnm1, ma, n);
-                        double dd = FC(a.fnp1, ma, n);
-                        ZA(n + 1, l) = mk(v.x / dd, v.y / dd);
-#undef ZA
-#undef FC
-                    }
-                    __syncthreads();
+                    __syncwarp();
+                    double* t = cur;
+                    cur = nxt;
+                    nxt = t;
                 }
             }
         }
-        __syncthreads();
+        // axial blocks of every degree ma (regular functions), kept for all columns:
+        // every element its vector-coupling sum, n fastest as the table lies
+        for (int e = tid; e < (nmin + 1) * (L - l0 + 1) * nt; e += PP_NT) {
+            const int n = e % nt + 1, l = l0 + (e / nt) % (L - l0 + 1), ma = e / (nt * (L - l0 + 1));
+            if (n < ma || l < ma) continue;
+            const int wmin = abs(n - l), wmax = n + l, ml = l * (l + 1) + ma;
+            const double* vc = a.vcc + (n - 1) + (size_t)a.vcT * (ml - 1);
+            const size_t vw = (size_t)a.vcT * a.vcML;
+            zd s1 = vc[vw * wmin] * xi[wmin], s2 = mk(0.0, 0.0);
+#pragma unroll 2
+            for (int w = wmin + 1; w < wmax; w += 2) {
+                s2 = s2 + vc[vw * w] * xi[w];
+                s1 = s1 + vc[vw * (w + 1)] * xi[w + 1];
+            }
+            s2 = imul(s2);
+            zd* Z = Zall + (size_t)ma * 2 * nt * L + (n - 1) * L + (l - 1);
+            Z[0] = s1 + s2;
+            Z[nt * L] = s1 - s2;
+        }
         const zd* e = eph + nmax;
-        // phase (shift_op = F: e^{+i m phi} on the source) and forward rotation of degrees l <= L, every column
-        for (int it = tid; it < np * 2 * L * W; it += PP_NT) {
-            const int pc = it / (2 * L * W), ee = it - pc * (2 * L * W);
-            int q = ee / (L * W);
-            int rem = ee - q * L * W;
-            int l = rem / W + 1;
-            int k = rem % W - nmin;
-            int n1 = min(l, nt);
+        const int xl = L * (L + 2);
+        for (int it = tid; it < np * 2 * xl; it += PP_NT) {
+            const int pc = it / (2 * xl), q = (it / xl) % 2, loc = it % xl;
+            const int row = loc % (L + 2), col = loc / (L + 2) + 1;
+            const int l = row <= col ? col : row - 1, m = row <= col ? row : -col;
+            if (l >= l0) XP[((size_t)pc * 2 + q) * xl + l * l - 1 + l + m] = src[(size_t)(p0 + pc) * a.ld + soff + (size_t)q * xl + loc] * e[m];
+        }
+        __syncthreads();
+        // forward rotation of the source degrees, every column
+        for (int it = tid; it < np * 2 * (L - l0 + 1) * W; it += PP_NT) {
+            const int k = it % W - nmin, l = l0 + (it / W) % (L - l0 + 1), pq = it / (W * (L - l0 + 1));
             zd acc = mk(0.0, 0.0);
-            if (abs(k) <= n1) {
-                const double* Dl = D + dofs[l];
-                const zd* x = src + (size_t)(p0 + pc) * a.ld + soff;
-                for (int m = -l; m <= l; m++) acc = acc + Dl[(k + nmin) * (2 * l + 1) + (m + l)] * (x[aidx(m, l, q, L)] * e[m]);
+            if (abs(k) <= min(l, nt)) {
+                const double* Dl = D + (size_t)W * l * l + (k + nmin) * (2 * l + 1);
+                const zd* x = XP + (size_t)pq * xl + l * l - 1;
+#pragma unroll 4
+                for (int m = 0; m <= 2 * l; m++) acc = acc + Dl[m] * x[m];
             }
-            AP[(((size_t)pc * 2 + q) * L + (l - 1)) * W + (k + nmin)] = acc;
+            AP[((size_t)pq * L + (l - 1)) * W + (k + nmin)] = acc;
         }
         __syncthreads();
         // g(+ma, n, p) = Z[mode p] a'(+ma) ; g(-ma, n, p) = Z[mode 1-p] a'(-ma), every degree ma and column
@@ -328,7 +334,7 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
                 const zd* Z = Zall + (size_t)ma * 2 * nt * L;
                 const zd* ap = AP + ((size_t)pc * 2 + pm) * L * W;
                 zd acc = mk(0.0, 0.0);
-                for (int l = m1; l <= L; l++) acc = acc + Z[(pz * nt + (n - 1)) * L + (l - 1)] * ap[(l - 1) * W + (mm + nmin)];
+                for (int l = max(m1, l0); l <= L; l++) acc = acc + Z[(pz * nt + (n - 1)) * L + (l - 1)] * ap[(l - 1) * W + (mm + nmin)];
                 G[(((size_t)pc * 2 + pm) * nt + (n - 1)) * W + (mm + nmin)] = acc;
             }
         }
@@ -337,11 +343,12 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
         for (int it = tid; it < np * nt * (nt + 2); it += PP_NT) {
             const int pc = it / (nt * (nt + 2)), ee = it - pc * (nt * (nt + 2));
             const int p = p0 + pc;
-            int n = 1;
+            int n = (int)sqrtf((float)(ee + 1));   // n n - 1 <= ee < (n + 1)(n + 1) - 1
             while (n * (n + 2) <= ee) n++;
+            while (n * n - 1 > ee) n--;
             int k = ee - (n * n - 1) - n;   // -n..n
             int n1 = min(n, L);
-            const double* Dn = D + dofs[n];
+            const double* Dn = D + (size_t)W * n * n;
             zd gq[2];
             for (int pm = 0; pm < 2; pm++) {
                 const zd* g = G + ((size_t)pc * 2 + pm) * nt * W;
@@ -367,105 +374,111 @@ __global__ void __launch_bounds__(PP_NT) merge_kernel(MergeArgs a)
 }
 
 // ---------------------------------------------------------------------------
-// fosmexpansion: one warp per (n, l); lanes over m, 32 at a time.  For each
-// (p, q, w) the lanes' contributions go to the same few table elements, so
-// the warp adds them up first (a butterfly over the lanes) and one lane
-// issues the atomics into the global tables.
+// fosmexpansion: one CTA per (n, l).  The terms of (m, p, q) in the elements
+// of degree w are a weight without w times a coupling coefficient of (m, w),
+// so that each element is a matrix-vector product over m: per chunk of FO_MC
+// orders m, a thread per coupling row (three kinds) fills shared memory, a warp
+// forms the weights (summed over the (p, q) of one parity of p + q: that
+// parity against n + l + w decides the element), then a thread per w sums
+// over m.  With the lanes over m and a butterfly per (p, q, w) the kernel took
+// 2.63 ms for the 350-sphere aggregate of order 9 (rows in strided global
+// scratch); now 0.44 ms.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_allsum(double v)
+#define FO_MC 32
+#define FO_NT 128
+__global__ void __launch_bounds__(FO_NT) fosm_kernel(int ntot, int mc, const zd* a0, VCTab tab, double* s00, double* s02, double* sp22,
+                                                     double* sm22)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-__global__ void __launch_bounds__(32) fosm_kernel(int ntot, const zd* a0, VCTab tab, double* s00, double* s02, double* sp22, double* sm22, double* vscr)
-{
-  const int lane = threadIdx.x;
-  double* base = vscr + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 5 * (2 * ntot + 2);
-  double* cm1p1 = base;
-  double* cm1m1 = cm1p1 + (2 * ntot + 2);
-  double* cmmpm = cm1m1 + (2 * ntot + 2);
-  double* cmmm2pm = cmmpm + (2 * ntot + 2);
-  double* cmmp2pm = cmmm2pm + (2 * ntot + 2);
-  for (int nl = blockIdx.x; nl < ntot * ntot; nl += gridDim.x) {
-    int n = nl / ntot + 1, l = nl % ntot + 1;
-    const int nb = 2 * ntot * (ntot + 2);
-    const int half = ntot * (ntot + 2);
-    int wmin = abs(n - l), wmax = n + l;
-    zd fnl = sqrt((double)((n + n + 1) * (l + l + 1))) * ipow_z(l - n);
-    int mm = min(n, l + 2);
-    // the m-independent couplings, once per (n, l)
-    vc_func(tab, -1, n, 1, l, cm1p1);
-    vc_func(tab, -1, n, -1, l, cm1m1);
-    for (int m0 = -mm; m0 <= mm; m0 += 32) {
-        const int m = m0 + lane;
-        const bool act = m <= mm;
-        if (act && abs(m) <= l) vc_func(tab, -m, n, m, l, cmmpm);
-        else for (int w = 0; w <= n + l; w++) cmmpm[w] = 0.0;
-        if (act && abs(-2 + m) <= l) vc_func(tab, -m, n, -2 + m, l, cmmm2pm);
-        else for (int w = 0; w <= n + l; w++) cmmm2pm[w] = 0.0;
-        if (act && abs(2 + m) <= l) vc_func(tab, -m, n, 2 + m, l, cmmp2pm);
-        else for (int w = 0; w <= n + l; w++) cmmp2pm[w] = 0.0;
-        double m1m = pm1(m);
-        auto A = [&](int pol, int mq, int nq, int p) -> zd {
-            if (!act || mq < -nq || mq > nq) return mk(0.0, 0.0);
-            return a0[(size_t)pol * nb + aidx(mq, nq, 0, ntot) + (size_t)half * p];
-        };
-        for (int p = 1; p <= 2; p++)
-            for (int q = 1; q <= 2; q++) {
-                double m1mq = pm1(m + q);
-                double m1mnpl = pm1(m + n + p + l);
-                zd a1n = A(0, m, n, p - 1), a2n = A(1, m, n, p - 1);
-                zd a1l = A(0, m, l, q - 1), a2l = A(1, m, l, q - 1);
-                zd a1122 = a1n * cj(a1l) + a2n * cj(a2l);
-                zd a2112 = a2n * cj(a1l) - a1n * cj(a2l);
-                zd a1p2 = (a1n + imul(a2n)) * cj(A(0, m - 2, l, q - 1) - imul(A(1, m - 2, l, q - 1)));
-                zd a1m2 = (a1n - imul(a2n)) * cj(A(0, m + 2, l, q - 1) + imul(A(1, m + 2, l, q - 1)));
-                for (int w = wmin; w <= wmax; w++) {
-                    double m1w = pm1(w);
-                    bool ev = ((n + l + w + p + q) % 2 == 0);   // one parity for the whole warp
-#define SS(arr, i, j) (&arr[((i) - 1) + 4 * ((j) - 1) + 16 * w])
-                    // this lane's terms of the five elements (n, l, w, p, q) feeds
-                    double v0, v1 = 0.0, v2 = 0.0, v3 = 0.0, v4 = 0.0;
-                    if (ev) v0 = -((m1m * fnl) * a1122 * (cm1p1[w] * cmmpm[w])).x / 2.0;
-                    else v0 = (imul(mk(0.5, 0.0)) * (m1m * fnl) * a2112 * (cm1p1[w] * cmmpm[w])).x;
-                    if (w >= 2) {
-                        if (ev) {
-                            v1 = -((m1mq * a1122) * fnl * (cm1m1[w] * cmmpm[w])).x / 2.0;
-                            v2 = -((m1m * a1p2) * fnl * (cm1p1[w] * cmmm2pm[w])).x / 4.0
-                                 - ((m1m * a1m2) * fnl * (cm1p1[w] * cmmp2pm[w])).x / 4.0;
-                        } else {
-                            v1 = (imul(mk(-0.5, 0.0)) * (m1mq * a2112) * fnl * (cm1m1[w] * cmmpm[w])).y;
-                            v2 = ((m1m * a1p2) * fnl * (cm1p1[w] * cmmm2pm[w])).y / 4.0
-                                 - ((m1m * a1m2) * fnl * (cm1p1[w] * cmmp2pm[w])).y / 4.0;
-                        }
-                        v3 = -((m1mnpl * m1w * a1p2) * fnl * (cm1m1[w] * cmmm2pm[w])).x / 8.0
-                             - ((m1mq * a1m2) * fnl * (cm1m1[w] * cmmp2pm[w])).x / 8.0;
-                        v4 = -((m1mq * a1p2) * fnl * (cm1m1[w] * cmmm2pm[w])).x / 8.0
-                             - ((m1mnpl * m1w * a1m2) * fnl * (cm1m1[w] * cmmp2pm[w])).x / 8.0;
-                    }
-                    v0 = warp_allsum(v0);
-                    if (w >= 2) {
-                        v1 = warp_allsum(v1);
-                        v2 = warp_allsum(v2);
-                        v3 = warp_allsum(v3);
-                        v4 = warp_allsum(v4);
-                    }
-                    if (lane == 0) {
-                        atomicAdd(ev ? SS(s00, 1, 1) : SS(s00, 4, 4), v0);
-                        if (w >= 2) {
-                            atomicAdd(ev ? SS(s02, 2, 1) : SS(s02, 3, 4), v1);
-                            atomicAdd(ev ? SS(s02, 1, 2) : SS(s02, 4, 3), v2);
-                            atomicAdd(SS(sm22, 2, 2), v3);
-                            atomicAdd(SS(sp22, 2, 2), v4);
-                        }
-                    }
-#undef SS
-                }
+    extern __shared__ __align__(16) double fo_smem[];
+    // weights of (m, parity of p + q): on cmmpm for n + l + w of the same
+    // parity (0, 1) and the other (2, 3), on cmmm2pm, cmmp2pm likewise (4..7),
+    // and the four of the w >= 2 diagonal elements, both parities (8..11)
+    __shared__ double wt[FO_MC][2][12];
+    const int tid = threadIdx.x, VL = 2 * ntot + 2;
+    double* c1[2] = {fo_smem, fo_smem + VL};   // cm1p1, cm1m1
+    double* rows = fo_smem + 2 * VL;           // [kind][m][w]
+    // large (n, l) first
+    const int nl = ntot * ntot - 1 - (int)blockIdx.x, n = nl / ntot + 1, l = nl % ntot + 1;
+    const int nb = 2 * ntot * (ntot + 2), half = ntot * (ntot + 2);
+    const int wmin = abs(n - l), wmax = n + l, mm = min(n, l + 2);
+    const zd fnl = sqrt((double)((n + n + 1) * (l + l + 1))) * ipow_z(l - n);
+    if (tid >= 96 && tid < 98) vc_func(tab, -1, n, tid == 96 ? 1 : -1, l, c1[tid - 96]);   // independent of m
+    for (int m0 = -mm; m0 <= mm; m0 += mc) {
+        const int cnt = min(mc, mm - m0 + 1);
+        if (tid < 96) {
+            const int kind = tid / 32, j = tid % 32, m = m0 + j, k = m + (kind == 0 ? 0 : (kind == 1 ? -2 : 2));
+            if (j < cnt) {
+                double* v = rows + (size_t)(kind * mc + j) * VL;
+                if (abs(k) <= l) vc_func(tab, -m, n, k, l, v);
+                else
+                    for (int w = wmin; w <= wmax; w++) v[w] = 0.0;
             }
+        } else if (tid - 96 < cnt) {
+            const int m = m0 + tid - 96;
+            auto A = [&](int pol, int mq, int nq, int p) -> zd {
+                if (mq < -nq || mq > nq) return mk(0.0, 0.0);
+                return a0[(size_t)pol * nb + aidx(mq, nq, 0, ntot) + (size_t)half * p];
+            };
+            const double m1m = pm1(m);
+            for (int c = 0; c < 2; c++) {
+                double w[12];
+                for (int e = 0; e < 12; e++) w[e] = 0.0;
+                for (int p = 1; p <= 2; p++) {
+                    const int q = c == 0 ? p : 3 - p;
+                    const double m1mq = pm1(m + q), m1mnpl = pm1(m + n + p + l);
+                    const zd a1n = A(0, m, n, p - 1), a2n = A(1, m, n, p - 1), a1l = A(0, m, l, q - 1), a2l = A(1, m, l, q - 1);
+                    const zd a1122 = (a1n * cj(a1l) + a2n * cj(a2l)) * fnl, a2112 = (a2n * cj(a1l) - a1n * cj(a2l)) * fnl;
+                    const zd a1p2 = (a1n + imul(a2n)) * cj(A(0, m - 2, l, q - 1) - imul(A(1, m - 2, l, q - 1))) * fnl;
+                    const zd a1m2 = (a1n - imul(a2n)) * cj(A(0, m + 2, l, q - 1) + imul(A(1, m + 2, l, q - 1))) * fnl;
+                    w[0] += -m1m * a1122.x / 2.0;       // cm1p1: s00(1,1)
+                    w[1] += -m1mq * a1122.x / 2.0;      // cm1m1: s02(2,1)
+                    w[2] += -m1m * a2112.y / 2.0;       // cm1p1: s00(4,4)
+                    w[3] += -m1mq * a2112.x / 2.0;      // cm1m1: s02(3,4)
+                    w[4] += -m1m * a1p2.x / 4.0;        // cm1p1: s02(1,2)
+                    w[5] += -m1m * a1m2.x / 4.0;
+                    w[6] += m1m * a1p2.y / 4.0;         // cm1p1: s02(4,3)
+                    w[7] += -m1m * a1m2.y / 4.0;
+                    w[8] += -m1mnpl * a1p2.x / 8.0;     // cm1m1: sm22(2,2), times (-1)^w on cmmm2pm
+                    w[9] += -m1mq * a1m2.x / 8.0;
+                    w[10] += -m1mq * a1p2.x / 8.0;      // cm1m1: sp22(2,2), times (-1)^w on cmmp2pm
+                    w[11] += -m1mnpl * a1m2.x / 8.0;
+                }
+                for (int e = 0; e < 12; e++) wt[tid - 96][c][e] = w[e];
+            }
+        }
+        __syncthreads();
+        for (int w = wmin + tid; w <= wmax; w += FO_NT) {
+            const int ev = (n + l + w) & 1, od = 1 - ev;
+            const double m1w = pm1(w);
+            double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            for (int j = 0; j < cnt; j++) {
+                const double c0 = rows[(size_t)j * VL + w], cm = rows[(size_t)(mc + j) * VL + w], cp = rows[(size_t)(2 * mc + j) * VL + w];
+                const double *we = wt[j][ev], *wo = wt[j][od];
+                t[0] += we[0] * c0;
+                t[1] += we[1] * c0;
+                t[2] += wo[2] * c0;
+                t[3] += wo[3] * c0;
+                t[4] += we[4] * cm + we[5] * cp;
+                t[5] += wo[6] * cm + wo[7] * cp;
+                t[6] += m1w * (we[8] + wo[8]) * cm + (we[9] + wo[9]) * cp;
+                t[7] += (we[10] + wo[10]) * cm + m1w * (we[11] + wo[11]) * cp;
+            }
+            const double p1 = c1[0][w], q1 = c1[1][w];
+#define SS(arr, i, j) (&arr[((i) - 1) + 4 * ((j) - 1) + 16 * w])
+            atomicAdd(SS(s00, 1, 1), p1 * t[0]);
+            atomicAdd(SS(s00, 4, 4), p1 * t[2]);
+            if (w >= 2) {
+                atomicAdd(SS(s02, 2, 1), q1 * t[1]);
+                atomicAdd(SS(s02, 3, 4), q1 * t[3]);
+                atomicAdd(SS(s02, 1, 2), p1 * t[4]);
+                atomicAdd(SS(s02, 4, 3), p1 * t[5]);
+                atomicAdd(SS(sm22, 2, 2), q1 * t[6]);
+                atomicAdd(SS(sp22, 2, 2), q1 * t[7]);
+            }
+#undef SS
+        }
+        __syncthreads();
     }
-  }
 }
 
 // the sign patches and the 1/(2 m_medium) factor of fosmexpansion
@@ -483,82 +496,38 @@ __global__ void fosm_patch_kernel(int ntot, double* s00, double* s02, double* sp
         for (int e = 0; e < 16; e++) S[k][e + 16 * w] = 0.5 * S[k][e + 16 * w] / scale;
 }
 
-// fosmcalc at each angle: one CTA per angle; rotcoef(ct, 2, 2ntot) by the
-// degree recurrence, then the sum over w and the element patches
-__global__ void fosmcalc_kernel(int ntot, int nang, const double* s00, const double* s02, const double* sp22,
-                                const double* sm22, const double* fnr, const double* bcofd, double* dscr, double* smat)
+// fosmcalc at each angle: one CTA per angle; the functions of every degree
+// (gsfrows.cuh), then the sum over w and the element patches
+__global__ void __launch_bounds__(GSF_NT) fosmcalc_kernel(int ntot, int nang, const double* s00, const double* s02, const double* sp22,
+                                                          const double* sm22, const double* fnr, const double* bcofd, double* smat)
 {
-    int ia = blockIdx.x;
+    extern __shared__ __align__(16) double gsf_smem[];
+    const int ia = blockIdx.x;
     if (ia >= nang) return;
-    const int nmax = 2 * ntot, kmax = 2;
     // polar angle as scattering_matrix_calculation forms it (input:3039-3043), pi as MSTM stores it
     double ct = cos(MSTMG_REF_PI / 180.0 * (0.0 + (180.0 - 0.0) * (double)ia / (double)(nang - 1)));
     if (ct == 1.0) ct = 0.9999999;
     if (ct == -1.0) ct = -0.9999999;
-    double* dk0 = dscr + (size_t)ia * (16 * nmax + 40) + (nmax + 1);
-    double* dk01 = dk0 + (2 * nmax + 3);
-    double* dc = dk01 + (2 * nmax + 3);   // rows m = -2..2 of the current degree, columns k = -nmax..nmax
-    const int W = 2 * nmax + 1;
-#define DCR(m, k) dc[((m) + 2) * W + ((k) + nmax)]
+    const int nmax = 2 * ntot;
+    gsf_columns(nmax, ct, fnr, bcofd, gsf_smem);
+    __shared__ double red[GSF_NT / 16][16];
     __shared__ double acc[16];
-    if (threadIdx.x < 16) acc[threadIdx.x] = 0.0;
-    double sbe = (fabs(ct) >= 1.0) ? 0.0 : sqrt(fabs((1.0 + ct) * (1.0 - ct)));
-    double cbe2 = 0.5 * (1.0 + ct), sbe2 = 0.5 * (1.0 - ct);
-    for (int k = threadIdx.x; k < 2 * nmax + 3; k += blockDim.x) { dk0[k - (nmax + 1)] = 0.0; dk01[k - (nmax + 1)] = 0.0; }
-    __syncthreads();
-    if (threadIdx.x == 0) dk0[0] = 1.0;
-    __syncthreads();
-    // degree 0: dc(0,0) = 1 -> the w = 0 term
-    if (threadIdx.x < 16) acc[threadIdx.x] += s00[threadIdx.x] * 1.0;
-    int sgn = 1;
-    double sben = 1.0;
-    for (int n = 1; n <= nmax; n++) {
-        int kk = min(n, kmax);
-        sgn = -sgn;
-        sben = sben * sbe / 2.0;
-        if (sben < 1.0e-30) sben = 0.0;
-        double newv[8];
-        int cnt = 0;
-        for (int k = -n + 1 + (int)threadIdx.x; k <= n - 1; k += blockDim.x)
-            newv[cnt++] = (ct * (double)(n + n - 1) * dk0[k] - fnr[n - k - 1] * fnr[n + k - 1] * dk01[k]) / (fnr[n + k] * fnr[n - k]);
-        __syncthreads();
-        cnt = 0;
-        for (int k = -n + 1 + (int)threadIdx.x; k <= n - 1; k += blockDim.x) {
-            dk01[k] = dk0[k];
-            dk0[k] = newv[cnt++];
-        }
-        if (threadIdx.x == 0) {
-            dk0[n] = sgn * sben * bcofd[n];
-            dk0[-n] = sgn * dk0[n];
-            dk01[n] = 0.0;
-            dk01[-n] = 0.0;
-        }
-        __syncthreads();
-        for (int k = -n + (int)threadIdx.x; k <= n; k += blockDim.x) DCR(0, k) = dk0[k];
-        __syncthreads();
-        int im = 1;
-        for (int m = 1; m <= kk; m++) {
-            im = -im;
-            double fmn = 1.0 / fnr[n - m + 1] / fnr[n + m];
-            for (int k = -n + (int)threadIdx.x; k <= n; k += blockDim.x) {
-                double dkm1 = (k == -n) ? 0.0 : DCR(m - 1, k - 1);
-                double dkn1 = (k == n) ? 0.0 : DCR(m - 1, k + 1);
-                double v = (fnr[n + k] * fnr[n - k + 1] * cbe2 * dkm1 - fnr[n - k] * fnr[n + k + 1] * sbe2 * dkn1 -
-                            (double)k * sbe * DCR(m - 1, k)) * fmn;
-                DCR(m, k) = v;
-                DCR(-m, -k) = v * pm1(k) * im;
-            }
-            __syncthreads();
-        }
-        // terms: w = n uses dc(0, n(n+1)) [k=0 column]; dc(0,n(n+1)+2), dc(+-2, n(n+1)+2) [k=2]
-        if (threadIdx.x < 16) {
-            int e = threadIdx.x;
-            double v = s00[e + 16 * n] * DCR(0, 0);
-            if (n >= 2) v += s02[e + 16 * n] * DCR(0, 2) + sp22[e + 16 * n] * DCR(2, 2) + sm22[e + 16 * n] * DCR(-2, 2);
-            acc[e] += v;
-        }
-        __syncthreads();
+    const int e = threadIdx.x % 16, part = threadIdx.x / 16;
+    double v = part == 0 ? s00[e] * 1.0 : 0.0;   // degree 0: dc(0,0) = 1
+    // terms: w = n uses dc(0, n(n+1)) [k=0 column]; dc(0,n(n+1)+2), dc(+-2, n(n+1)+2) [k=2]
+    for (int n = 1 + part; n <= nmax; n += GSF_NT / 16) {
+        const double* g = gsf_smem + GSF_ROW * n;
+        v += s00[e + 16 * n] * g[GSF_D00];
+        if (n >= 2) v += s02[e + 16 * n] * g[GSF_D02] + sp22[e + 16 * n] * g[GSF_D22] + sm22[e + 16 * n] * g[GSF_DM22];
     }
+    red[part][e] = v;
+    __syncthreads();
+    if (threadIdx.x < 16) {
+        double t = 0.0;
+        for (int p = 0; p < GSF_NT / 16; p++) t += red[p][threadIdx.x];
+        acc[threadIdx.x] = t;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
         double sm[16];
         for (int e = 0; e < 16; e++) sm[e] = acc[e];
@@ -576,7 +545,6 @@ __global__ void fosmcalc_kernel(int ntot, int nang, const double* s00, const dou
 #undef SM
         for (int e = 0; e < 16; e++) smat[(size_t)ia * 16 + e] = sm[e];
     }
-#undef DCR
 }
 
 // scatteringmatrix (scatprops:1498-1573) with normalize_s11 = .false. at the
@@ -726,54 +694,57 @@ __global__ void __launch_bounds__(PS_NT) planesm_kernel(PlaneSmArgs a)
     }
 }
 
-// blocks of TRANORDER_WPB warps, at most one warp per SM's worth (148) in all
-int tranorder_blocks(int nsph) { return std::max(1, (std::min(nsph, 148) + TRANORDER_WPB - 1) / TRANORDER_WPB); }
-size_t tranorder_scratch(int nsph, int sstride) { return (size_t)tranorder_blocks(nsph) * TRANORDER_WPB * 32 * (size_t)sstride; }
+// a warp per sphere, three to an SM (68 KB of shared memory each)
+int tranorder_blocks(int nsph) { return std::max(1, std::min(nsph, 3 * 148)); }
+size_t tranorder_scratch(int nsph) { return (size_t)tranorder_blocks(nsph) * 32 * 2 * TRANORDER_ROW; }
 
 void launch_tranorder(int nsph, const double* pos, const int* order, const double* origin, double rire, double eps, int maxt,
-                      const double* bcof, const double* fnr, int nbc, zd* scratch, int sstride, int* tord, cudaStream_t st)
+                      const double* bcof, const double* fnr, int nbc, zd* scratch, int* tord, cudaStream_t st)
 {
     VCTab t{bcof, fnr, nbc};
-    tranorder_kernel<<<tranorder_blocks(nsph), 32 * TRANORDER_WPB, 0, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire,
-                                                                            eps, maxt, t, scratch, sstride, tord);
+    const int smem = (int)(sizeof(zd) * TRANORDER_ROW + sizeof(double) * 32 * TRANORDER_ROW);
+    cudaFuncSetAttribute(tranorder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    tranorder_kernel<<<tranorder_blocks(nsph), 32, smem, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire, eps, maxt, t,
+                                                               scratch, tord);
     launch_counter() += 1;
 }
 
-size_t merge_scratch_per_cta(int T, int L)
+size_t merge_scratch_per_cta(int T, int L, int npol)
 {
-    int nmin = std::min(T, L), nmax = std::max(T, L), W = 2 * nmin + 1;
-    size_t dsz = 0;
-    for (int n = 0; n <= nmax; n++) dsz += (size_t)W * (2 * n + 1);
-    size_t z = (size_t)(nmax + L + 4) * 3 + (2 * nmax + 1);             // xi + Bessel scratch + e^{i m phi}
-    size_t dbl = dsz + 1 + 2 * (2 * nmax + 3) + 8 + (nmax + 8) / 2 + 2;  // D + dk arrays + degree offsets
-    size_t zz = (size_t)(nmin + 1) * 2 * T * L + (size_t)MERGE_PC * (2 * (size_t)L * W + 2 * (size_t)T * W);
-    return z + (dbl + 1) / 2 + zz + 8;                                  // in zd units
+    const size_t nmin = std::min(T, L), nmax = std::max(T, L), W = 2 * nmin + 1, np = std::min(npol, MERGE_PC);
+    const size_t z = (nmax + L + 4) * 3 + (2 * nmax + 1);               // xi + Bessel scratch + e^{i m phi}
+    const size_t dbl = (W * (nmax + 1) * (nmax + 1) + 1) / 2 * 2;       // D
+    const size_t zz = (nmin + 1) * 2 * T * L + np * (2 * (size_t)L * W + 2 * (size_t)T * W + 2 * (size_t)L * (L + 2));
+    return z + dbl / 2 + zz + 8;                                        // in zd units
 }
 int merge_chunks(int npol) { return (npol + MERGE_PC - 1) / MERGE_PC; }
 
 void launch_merge(const MergeArgs& a, int grid, cudaStream_t st)
 {
-    merge_kernel<<<dim3(grid, merge_chunks(a.npol)), PP_NT, 0, st>>>(a);
+    // two rows of the Wigner recurrence a warp; orders reach MSTMG_LMAX and T
+    const int nmax = std::max(a.T, MSTMG_LMAX), smem = (int)sizeof(double) * (PP_NT / 32) * 2 * (2 * nmax + 3);
+    cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    merge_kernel<<<dim3(grid, merge_chunks(a.npol)), PP_NT, smem, st>>>(a);
     launch_counter() += 1;
 }
 
-int fosm_grid(int ntot) { return std::min(ntot * ntot, 148 * 8); }
-size_t fosm_scratch_doubles(int ntot) { return (size_t)fosm_grid(ntot) * 32 * 5 * (2 * ntot + 2); }
-size_t fosmcalc_scratch_doubles(int ntot, int nang) { return (size_t)nang * (16 * (2 * ntot) + 40); }
-
 void launch_fosm(int ntot, const zd* a0, const double* bcof, const double* fnr, int nbc, double* s00, double* s02, double* sp22,
-                 double* sm22, double* vscr, cudaStream_t st)
+                 double* sm22, cudaStream_t st)
 {
     VCTab t{bcof, fnr, nbc};
-    fosm_kernel<<<fosm_grid(ntot), 32, 0, st>>>(ntot, a0, t, s00, s02, sp22, sm22, vscr);
+    // FO_MC orders m a chunk while three rows of each fit 200 KB (order 128)
+    const int row = (int)sizeof(double) * (2 * ntot + 2), mc = std::max(1, std::min(FO_MC, (200 * 1024 - 2 * row) / (3 * row)));
+    const int smem = row * (2 + 3 * mc);
+    cudaFuncSetAttribute(fosm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    fosm_kernel<<<ntot * ntot, FO_NT, smem, st>>>(ntot, mc, a0, t, s00, s02, sp22, sm22);
     fosm_patch_kernel<<<(2 * ntot + 1 + 63) / 64, 64, 0, st>>>(ntot, s00, s02, sp22, sm22, 1.0);
     launch_counter() += 2;
 }
 
 void launch_fosmcalc(int ntot, int nang, const double* s00, const double* s02, const double* sp22, const double* sm22,
-                     const double* fnr, const double* bcofd, double* dscr, double* smat, cudaStream_t st)
+                     const double* fnr, const double* bcofd, double* smat, cudaStream_t st)
 {
-    fosmcalc_kernel<<<nang, 128, 0, st>>>(ntot, nang, s00, s02, sp22, sm22, fnr, bcofd, dscr, smat);
+    fosmcalc_kernel<<<nang, GSF_NT, gsf_smem_bytes(2 * ntot), st>>>(ntot, nang, s00, s02, sp22, sm22, fnr, bcofd, smat);
     launch_counter() += 1;
 }
 

@@ -34,26 +34,24 @@ struct MergeArgs {
     const double* bcofd;
     zd* scratch;
     size_t scratch_stride;  // zd units per CTA
+    int lsrc = 1;           // source degrees below lsrc are zero
     const int* active = nullptr;   // with host spheres: 1 for the spheres merged or distributed to (those outside every other)
 };
 
-size_t tranorder_scratch(int nsph, int sstride);   // complex values of scratch launch_tranorder needs
+size_t tranorder_scratch(int nsph);   // complex values of scratch launch_tranorder needs
 void launch_tranorder(int nsph, const double* pos, const int* order, const double* origin, double rire, double eps, int maxt,
-                      const double* bcof, const double* fnr, int nbc, zd* scratch, int sstride, int* tord, cudaStream_t st);
+                      const double* bcof, const double* fnr, int nbc, zd* scratch, int* tord, cudaStream_t st);
 #define MERGE_PC 16   // columns a CTA of the merge kernel translates together
 // zd units of merge-kernel scratch per CTA; a launch of `grid` CTAs per chunk
 // of MERGE_PC columns needs grid * merge_chunks(npol) of them
-size_t merge_scratch_per_cta(int T, int L);
+size_t merge_scratch_per_cta(int T, int L, int npol);
 int merge_chunks(int npol);
 // grid CTAs over the spheres times merge_chunks(npol) column chunks
 void launch_merge(const MergeArgs& a, int grid, cudaStream_t st);
-int fosm_grid(int ntot);
-size_t fosm_scratch_doubles(int ntot);
-size_t fosmcalc_scratch_doubles(int ntot, int nang);
 void launch_fosm(int ntot, const zd* a0, const double* bcof, const double* fnr, int nbc, double* s00, double* s02, double* sp22,
-                 double* sm22, double* vscr, cudaStream_t st);
+                 double* sm22, cudaStream_t st);
 void launch_fosmcalc(int ntot, int nang, const double* s00, const double* s02, const double* sp22, const double* sm22,
-                     const double* fnr, const double* bcofd, double* dscr, double* smat, cudaStream_t st);
+                     const double* fnr, const double* bcofd, double* smat, cudaStream_t st);
 
 // scatteringmatrix at the directions i = ldim..udim of scattering_matrix_calculation
 #define PS_TMAX 200

@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "ranorient.cuh"
 #include "vcoupling.cuh"
+#include "gsfrows.cuh"
 
 namespace {
 
@@ -361,104 +362,48 @@ __global__ void ro_sum_kernel(RoArgs a)
 }
 
 // ranorienscatmatrixcalc at theta_i = i pi/(nang-1) (pi as the reference stores it)
-__global__ void ro_calc_kernel(int nodrexp, int nang, const double* smc, const double* fnr, const double* bcofd, double* dscr, double* smat)
+__global__ void __launch_bounds__(GSF_NT) ro_calc_kernel(int nmax, int nang, const double* smc, const double* fnr, const double* bcofd,
+                                                         double* smat)
 {
+    extern __shared__ __align__(16) double gsf_smem[];
     const int ia = blockIdx.x;
     if (ia >= nang) return;
-    const int nmax = nodrexp, kmax = 2, W = 2 * nmax + 1;
     const double ct = cos((double)ia * MSTMG_REF_PI / (double)(nang - 1));
-    double* dk0 = dscr + (size_t)ia * (16 * nmax + 40) + (nmax + 1);
-    double* dk01 = dk0 + (2 * nmax + 3);
-    double* dc = dk01 + (2 * nmax + 3);   // rows m = -2..2 of the current degree, columns k = -nmax..nmax
-#define DCR(m, k) dc[((m) + 2) * W + ((k) + nmax)]
-#define SC(i, j, n) smc[((i) - 1) + 4 * ((j) - 1) + 16 * (n)]
+    gsf_columns(nmax, ct, fnr, bcofd, gsf_smem);
+    // a warp per element of the upper set, lanes over the degrees
     __shared__ double so[16];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#define SC(i, j, n) smc[((i) - 1) + 4 * ((j) - 1) + 16 * (n)]
+    for (int el = warp; el < 16; el += GSF_NT / 32) {
+        const int i = el % 4 + 1, j = el / 4 + 1;
+        double v = 0.0;
+        for (int n = lane; n <= nmax; n += 32) {
+            const double* g = gsf_smem + GSF_ROW * n;
+            const double d00 = n ? g[GSF_D00] : 1.0;   // degree 0: dc(0,0) = 1
+            if ((i == 1 || i == 4) && (j == 1 || j == 4)) v += d00 * SC(i, j, n);
+            if (n < 2) continue;
+            // dc(k, n(n+1)+m) of rotcoef(ct, 2, nodrexp) is the table's (k, m)
+            const double d20 = g[GSF_D20], d2m = g[GSF_D2M], d2p = g[GSF_D22];
+            if ((i == 1 && (j == 2 || j == 3)) || (i == 2 && j == 4) || (i == 3 && j == 4) || (i == 4 && j == 2)) v += d20 * SC(i, j, n);
+            if (i == 2 && j == 2) v += d2m * SC(2, 2, n) + d2p * SC(3, 3, n);
+            if (i == 2 && j == 3) v += d2p * SC(2, 3, n) + d2p * SC(3, 2, n);
+            if (i == 3 && j == 3) v += -d2m * SC(2, 2, n) + d2p * SC(3, 3, n);
+            if (i == 3 && j == 2) v += d2p * SC(2, 3, n) - d2p * SC(3, 2, n);
+        }
+        for (int x = 16; x > 0; x >>= 1) v += __shfl_xor_sync(0xffffffffu, v, x);
+        if (lane == 0) so[el] = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
 #define SO(i, j) so[((i) - 1) + 4 * ((j) - 1)]
-    if (threadIdx.x < 16) so[threadIdx.x] = 0.0;
-    const double sbe = (fabs(ct) >= 1.0) ? 0.0 : sqrt(fabs((1.0 + ct) * (1.0 - ct)));
-    const double cbe2 = 0.5 * (1.0 + ct), sbe2 = 0.5 * (1.0 - ct);
-    for (int k = threadIdx.x; k < 2 * nmax + 3; k += blockDim.x) { dk0[k - (nmax + 1)] = 0.0; dk01[k - (nmax + 1)] = 0.0; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        dk0[0] = 1.0;
-        // degree 0: dc(0,0) = 1
-        SO(1, 1) = SO(1, 1) + SC(1, 1, 0);
-        SO(1, 4) = SO(1, 4) + SC(1, 4, 0);
-        SO(4, 1) = SO(4, 1) + SC(4, 1, 0);
-        SO(4, 4) = SO(4, 4) + SC(4, 4, 0);
-    }
-    __syncthreads();
-    int sgn = 1;
-    double sben = 1.0;
-    for (int n = 1; n <= nmax; n++) {
-        int kk = min(n, kmax);
-        sgn = -sgn;
-        sben = sben * sbe / 2.0;
-        if (sben < 1.0e-30) sben = 0.0;
-        double newv[8];
-        int cnt = 0;
-        for (int k = -n + 1 + (int)threadIdx.x; k <= n - 1; k += blockDim.x)
-            newv[cnt++] = (ct * (double)(n + n - 1) * dk0[k] - fnr[n - k - 1] * fnr[n + k - 1] * dk01[k]) / (fnr[n + k] * fnr[n - k]);
-        __syncthreads();
-        cnt = 0;
-        for (int k = -n + 1 + (int)threadIdx.x; k <= n - 1; k += blockDim.x) {
-            dk01[k] = dk0[k];
-            dk0[k] = newv[cnt++];
-        }
-        if (threadIdx.x == 0) {
-            dk0[n] = sgn * sben * bcofd[n];
-            dk0[-n] = sgn * dk0[n];
-            dk01[n] = 0.0;
-            dk01[-n] = 0.0;
-        }
-        __syncthreads();
-        for (int k = -n + (int)threadIdx.x; k <= n; k += blockDim.x) DCR(0, k) = dk0[k];
-        __syncthreads();
-        int im = 1;
-        for (int m = 1; m <= kk; m++) {
-            im = -im;
-            double fmn = 1.0 / fnr[n - m + 1] / fnr[n + m];
-            for (int k = -n + (int)threadIdx.x; k <= n; k += blockDim.x) {
-                double dkm1 = (k == -n) ? 0.0 : DCR(m - 1, k - 1);
-                double dkn1 = (k == n) ? 0.0 : DCR(m - 1, k + 1);
-                double v = (fnr[n + k] * fnr[n - k + 1] * cbe2 * dkm1 - fnr[n - k] * fnr[n + k + 1] * sbe2 * dkn1 -
-                            (double)k * sbe * DCR(m - 1, k)) * fmn;
-                DCR(m, k) = v;
-                DCR(-m, -k) = v * pm1(k) * im;
-            }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) {
-            // dc(k, n(n+1)+m) of rotcoef(ct, 2, nodrexp) is DCR(k, m) here
-            double d00 = DCR(0, 0);
-            SO(1, 1) = SO(1, 1) + d00 * SC(1, 1, n);
-            SO(1, 4) = SO(1, 4) + d00 * SC(1, 4, n);
-            SO(4, 1) = SO(4, 1) + d00 * SC(4, 1, n);
-            SO(4, 4) = SO(4, 4) + d00 * SC(4, 4, n);
-            if (n >= 2) {
-                double d20 = DCR(2, 0), d2m = DCR(2, -2), d2p = DCR(2, 2);
-                SO(1, 2) = SO(1, 2) + d20 * SC(1, 2, n);
-                SO(2, 4) = SO(2, 4) + d20 * SC(2, 4, n);
-                SO(3, 4) = SO(3, 4) + d20 * SC(3, 4, n);
-                SO(1, 3) = SO(1, 3) + d20 * SC(1, 3, n);
-                SO(3, 1) = SO(1, 3) + d20 * SC(3, 1, n);   // as the reference writes it
-                SO(4, 2) = SO(4, 2) + d20 * SC(4, 2, n);
-                SO(2, 2) = SO(2, 2) + d2m * SC(2, 2, n) + d2p * SC(3, 3, n);
-                SO(2, 3) = SO(2, 3) + d2p * SC(2, 3, n) + d2p * SC(3, 2, n);
-                SO(3, 3) = SO(3, 3) - d2m * SC(2, 2, n) + d2p * SC(3, 3, n);
-                SO(3, 2) = SO(3, 2) + d2p * SC(2, 3, n) - d2p * SC(3, 2, n);
-            }
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
+        // as the reference writes it: each degree starts from the new (1,3)
+        SO(3, 1) = nmax >= 2 ? SO(1, 3) + gsf_smem[GSF_ROW * nmax + GSF_D20] * SC(3, 1, nmax) : 0.0;
         SO(2, 1) = SO(1, 2);
         SO(4, 3) = -SO(3, 4);
+#undef SO
         for (int e = 0; e < 16; e++) smat[16 * (size_t)ia + e] = so[e];
     }
-#undef DCR
 #undef SC
-#undef SO
 }
 
 // items from i0 on whose bm and vector-coupling rows fit the buffers; nodr
@@ -495,7 +440,7 @@ RoSizes ro_sizes(int nodr)
 }
 size_t ro_dm_elems(int nodr) { return (size_t)(2 * nodr + 3) * 3 * nodr * 2 * nodr * 2; }
 
-int launch_ranorient(const RoArgs& args, const zd* tmat, int nang, const double* bcofd, double* dscr, double* smat, int nsm, cudaStream_t st)
+int launch_ranorient(const RoArgs& args, const zd* tmat, int nang, const double* bcofd, double* smat, int nsm, cudaStream_t st)
 {
     RoArgs a = args;
     const int nodr = a.nodr;
@@ -529,7 +474,7 @@ int launch_ranorient(const RoArgs& args, const zd* tmat, int nang, const double*
     ro_dm_kernel<true><<<dim3(nu3, nt * nt, 1), 256, 0, st>>>(a, 0, 2 * nodr + 1);
     ro_coef_kernel<<<dim3(nodr, 2 * nodr + 1), RO_CT, sm_co, st>>>(a);
     ro_sum_kernel<<<2 * nodr + 1, 32, 0, st>>>(a);
-    if (nang > 1) ro_calc_kernel<<<nang, 64, 0, st>>>(2 * nodr, nang, a.sm, a.fnr, bcofd, dscr, smat);
+    if (nang > 1) ro_calc_kernel<<<nang, GSF_NT, gsf_smem_bytes(2 * nodr), st>>>(2 * nodr, nang, a.sm, a.fnr, bcofd, smat);
     launch_counter() += (nang > 1) ? 4 : 3;
     return 0;
 }

@@ -36,4 +36,4 @@ RoSizes ro_sizes(int nodr);
 size_t ro_vtab_w(int nodr);
 size_t ro_dm_elems(int nodr);
 // returns -1 for orders above RO_ORDER_MAX
-int launch_ranorient(const RoArgs& a, const zd* tmat, int nang, const double* bcofd, double* dscr, double* smat, int nsm, cudaStream_t st);
+int launch_ranorient(const RoArgs& a, const zd* tmat, int nang, const double* bcofd, double* smat, int nsm, cudaStream_t st);

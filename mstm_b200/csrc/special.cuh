@@ -107,9 +107,9 @@ __host__ __device__ inline void mstm_cspherebessel(int n, zd z, zd* csj, zd* csy
 }
 
 // h_k = j_k(z) + i y_k(z), k = 0 .. n, for real z: every pair distance and
-// sphere radius in a lossless medium.  Returns false, writing nothing, for
-// arguments it leaves to the complex routines (Im z != 0, or so small that
-// y_n or the backward values could leave the range of a double).
+// sphere radius in a lossless medium.  Returns false for arguments it leaves to
+// the complex routines (Im z != 0, or so small that y_n or the backward values
+// could leave the range of a double: |y| above 1e140; h is then partly written).
 // y_k runs forward (it dominates from k = z on); j_k runs forward too while
 // the turning point k = z lies beyond n, else backward from an order m with
 // |y_m| > 1e10 |y_n|, where j_m/j_n < 1e-20, scaled to the larger of j_0 and
@@ -123,7 +123,7 @@ __host__ __device__ inline void mstm_cspherebessel(int n, zd z, zd* csj, zd* csy
 __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
 {
     const double z = zc.x;
-    if (zc.y != 0.0 || !(z >= MSTM_REAL_BESSEL_MIN) || n > 2 * MSTMG_LMAX) return false;
+    if (zc.y != 0.0 || !(z >= MSTM_REAL_BESSEL_MIN)) return false;
     double sn, cs;
     sincos(z, &sn, &cs);
     const double rz = 1.0 / z;
@@ -153,6 +153,7 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
     if (n == 1) lim = 1.0e10 * fabs(yb);
     while (m < n || fabs(yb) < lim) {
         const double yn = (double)(2 * m + 1) * rz * yb - ya;
+        if (fabs(yn) > 1.0e140) return false;
         ya = yb;
         yb = yn;
         m++;
