@@ -22,25 +22,38 @@ mstmg::Tables& big_tables()
     return *big;
 }
 
-// Device copies of the bcof / sqrt tables of big_tables().
+// The context's device copies of big_tables(), made by the first call that
+// needs them: bcof (side nbc + 1), sqrt, bcof(n, n) for n <= nbc.
 struct BigTablesDev {
-    DevBuf<double> bc, fnr;
+    const double *bc = nullptr, *fnr = nullptr, *bcd = nullptr;
     int nbc = 420;
 };
 static int upload_big(mstmg_ctx* c, BigTablesDev& d)
 {
-    mstmg::Tables& big = big_tables();
-    CK(d.bc.alloc(big.bcof.size()));
-    CK(d.fnr.alloc(big.fnr.size()));
-    CK(cudaMemcpyAsync(d.bc.p, big.bcof.data(), sizeof(double) * big.bcof.size(), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(d.fnr.p, big.fnr.data(), sizeof(double) * big.fnr.size(), cudaMemcpyHostToDevice, c->st));
+    std::lock_guard<std::mutex> lk(c->big_mu);
+    if (!c->big_ready) {
+        mstmg::Tables& big = big_tables();
+        std::vector<double> bd(d.nbc + 1);
+        for (int k = 0; k <= d.nbc; k++) bd[k] = big.bc(k, k);
+        CK(c->big_bc.alloc(big.bcof.size()));
+        CK(c->big_fnr.alloc(big.fnr.size()));
+        CK(c->big_bcd.alloc(bd.size()));
+        CK(cudaMemcpyAsync(c->big_bc.p, big.bcof.data(), sizeof(double) * big.bcof.size(), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->big_fnr.p, big.fnr.data(), sizeof(double) * big.fnr.size(), cudaMemcpyHostToDevice, c->st));
+        CK(cudaMemcpyAsync(c->big_bcd.p, bd.data(), sizeof(double) * bd.size(), cudaMemcpyHostToDevice, c->st));
+        CK(cudaStreamSynchronize(c->st));
+        c->big_ready = true;
+    }
+    d.bc = c->big_bc.p;
+    d.fnr = c->big_fnr.p;
+    d.bcd = c->big_bcd.p;
     return MSTMG_OK;
 }
 
 // Cluster origin (mean position of the spheres) and the order each sphere
 // needs to reach it (tranordertest, modules:1896-1942, capped at max_t_order);
 // T = max(min(L, max_t_order), those orders)  (input:1179-1197).
-static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps, int max_t_order, double* r0, DevBuf<int>& dtord,
+static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps, int max_t_order, double* r0, CallScratch& ws, TmpBuf<int>& dtord,
                          std::vector<int>& tord, int* T)
 {
     const int n = c->n;
@@ -54,10 +67,10 @@ static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps,
             for (int k = 0; k < 3; k++) r0[k] = r0[k] + c->hpos[3 * (size_t)i + k];
         }
     for (int k = 0; k < 3; k++) r0[k] = r0[k] / (double)nout;
-    DevBuf<zd> tscr;
+    TmpBuf<zd> tscr(ws);
     CK(dtord.alloc(n));
     CK(tscr.alloc(tranorder_scratch(n)));
-    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc.p, bt.fnr.p, bt.nbc, tscr.p, dtord.p,
+    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc, bt.fnr, bt.nbc, tscr.p, dtord.p,
                      c->st);
     tord.resize(n);
     CK(cudaMemcpyAsync(tord.data(), dtord.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c->st));
@@ -73,59 +86,20 @@ static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps,
     return MSTMG_OK;
 }
 
-// Constant tables of a regular translation from source orders <= Ls to target
-// orders <= Tt (the vcc_const combination of axialtrancoefinit, modules:1680-1722,
-// the recurrence factors of axialtrancoefrecurrence up to max(Tt, Ls), and bcof(n,n)).
+// Constants of a regular translation from source orders <= Ls to target orders
+// <= Tt (the vcc_const combination of axialtrancoefinit, modules:1680-1722).
 struct RegTables {
-    DevBuf<double> vcc, f1, f2, f3, bcd;
-    int vcT = 0, vcML = 0, FN = 0;
+    explicit RegTables(CallScratch& ws) : vcc(ws) {}
+    TmpBuf<double> vcc;
+    int vcT = 0, vcML = 0;
 };
-static int build_reg_tables(mstmg_ctx* c, int Tt, int Ls, RegTables& r)
+static int build_reg_tables(mstmg_ctx* c, const BigTablesDev& bt, int Tt, int Ls, RegTables& r)
 {
-    mstmg::Tables& big = big_tables();
-    std::vector<double> vcc((size_t)Tt * Ls * (Ls + 2) * (Tt + Ls + 1), 0.0), vc1(2 * (Tt + Ls) + 4), vc2(2 * (Tt + Ls) + 4);
-    for (int nn = 1; nn <= Tt; nn++)
-        for (int l = 1; l <= Ls; l++) {
-            double c1 = big.fnr[nn + nn + 1] * big.fnr[l + l + 1];
-            big.vcfunc(-1, nn, 1, l, vc2.data());
-            int wmin = std::abs(nn - l), wmax = nn + l, nlmin = std::min(l, nn);
-            for (int m = -nlmin; m <= nlmin; m++) {
-                int ml = l * (l + 1) + m;
-                double c2 = -c1 * ((m & 1) ? -1.0 : 1.0);
-                big.vcfunc(-m, nn, m, l, vc1.data());
-                for (int w = wmin; w <= wmax; w++) {
-                    int e = ((nn - l + w) % 4 + 4) % 4;
-                    double ri = (e == 0 || e == 1) ? 1.0 : -1.0;
-                    vcc[(size_t)(nn - 1) + (size_t)Tt * ((size_t)(ml - 1) + (size_t)Ls * (Ls + 2) * w)] = c2 * vc1[w] * vc2[w] * ri;
-                }
-            }
-        }
-    const int FN = std::max(Tt, Ls);
-    size_t nf = (size_t)(2 * FN + 1) * FN;
-    std::vector<double> f1(nf, 0.0), f2(nf, 0.0), f3(nf, 0.0);
-    const std::vector<double>& fr = big.fnr;
-    for (int m = -FN; m <= FN; m++)
-        for (int l = std::max(1, std::abs(m)); l <= FN; l++) {
-            size_t ix = (size_t)(m + FN) + (2 * FN + 1) * (size_t)(l - 1);
-            int lp1 = l + 1, lm1 = l - 1;
-            f1[ix] = fr[lm1] * fr[lp1] * fr[l - m] * fr[l + m] / fr[lm1 + l] / fr[l + lp1] / (double)l;
-            f2[ix] = (double)m / (double)l / (double)lp1;
-            f3[ix] = fr[l] * fr[l + 2] * fr[lp1 - m] * fr[lp1 + m] / fr[l + lp1] / fr[l + l + 3] / (double)lp1;
-        }
-    std::vector<double> bd(Tt + Ls + 4);
-    for (int k = 0; k < (int)bd.size(); k++) bd[k] = big.bc(k, k);
-    auto up = [&](DevBuf<double>& d, const std::vector<double>& h) -> int {
-        CK(d.alloc(h.size()));
-        CK(cudaMemcpyAsync(d.p, h.data(), sizeof(double) * h.size(), cudaMemcpyHostToDevice, c->st));
-        return MSTMG_OK;
-    };
-    int rc;
-    if ((rc = up(r.vcc, vcc)) || (rc = up(r.f1, f1)) || (rc = up(r.f2, f2)) || (rc = up(r.f3, f3)) || (rc = up(r.bcd, bd))) return rc;
-    // the host vectors are freed on return: wait for the copies
-    CK(cudaStreamSynchronize(c->st));
+    CK(r.vcc.alloc((size_t)Tt * Ls * (Ls + 2) * (Tt + Ls + 1)));
+    launch_regular_couplings(Tt, Ls, bt.bc, bt.fnr, bt.nbc, r.vcc.p, c->st);
+    CK(cudaGetLastError());
     r.vcT = Tt;
     r.vcML = Ls * (Ls + 2);
-    r.FN = FN;
     return MSTMG_OK;
 }
 
@@ -148,12 +122,8 @@ static MergeArgs merge_args(mstmg_ctx* c, const RegTables& rt, const BigTablesDe
     ma.vcc = rt.vcc.p;
     ma.vcT = rt.vcT;
     ma.vcML = rt.vcML;
-    ma.fnm1 = rt.f1.p;
-    ma.fnc = rt.f2.p;
-    ma.fnp1 = rt.f3.p;
-    ma.fcN = rt.FN;
-    ma.fnr = bt.fnr.p;
-    ma.bcofd = rt.bcd.p;
+    ma.fnr = bt.fnr;
+    ma.bcofd = bt.bcd;
     ma.active = c->hs.on() ? c->hs.d_outside.p : nullptr;
     return ma;
 }
@@ -168,19 +138,20 @@ extern "C" int mstmg_scattering(mstmg_ctx* c, const double* amnp, double trans_e
         return MSTMG_ERR_ARG;
     }
     const int n = c->n, L = c->lmax;
+    CallScratch ws(c->pool, c->st);
     BigTablesDev bt;
     int rc = upload_big(c, bt);
     if (rc) return rc;
     double r0[3];
-    DevBuf<int> dtord;
+    TmpBuf<int> dtord(ws);
     std::vector<int> tord;
     int T = 0;
-    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, dtord, tord, &T))) return rc;
-    RegTables rt;
-    if ((rc = build_reg_tables(c, T, L, rt))) return rc;
+    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, ws, dtord, tord, &T))) return rc;
+    RegTables rt(ws);
+    if ((rc = build_reg_tables(c, bt, T, L, rt))) return rc;
     // merge to the common origin
     const int ne = c->neqns, nb0 = 2 * T * (T + 2);
-    DevBuf<zd> dsrc, da0, mscr;
+    TmpBuf<zd> dsrc(ws), da0(ws), mscr(ws);
     CK(dsrc.alloc(2 * (size_t)ne));
     CK(copy_in(dsrc.p, amnp, sizeof(zd) * 2 * (size_t)ne, c->st));
     CK(da0.alloc(2 * (size_t)nb0));
@@ -201,12 +172,12 @@ extern "C" int mstmg_scattering(mstmg_ctx* c, const double* amnp, double trans_e
     CK(cudaGetLastError());
     // GSF expansion and scattering matrix
     const int W = 2 * T + 1;
-    DevBuf<double> ds, dsm;
+    TmpBuf<double> ds(ws), dsm(ws);
     CK(ds.alloc(4 * 16 * (size_t)W));
     CK(cudaMemsetAsync(ds.p, 0, sizeof(double) * 4 * 16 * (size_t)W, c->st));
-    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
+    launch_fosm(T, da0.p, bt.bc, bt.fnr, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
     CK(dsm.alloc(16 * (size_t)nangles));
-    launch_fosmcalc(T, nangles, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, bt.fnr.p, rt.bcd.p, dsm.p, c->st);
+    launch_fosmcalc(T, nangles, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, bt.fnr, bt.bcd, dsm.p, c->st);
     CK(cudaGetLastError());
     double s0[2];
     CK(cudaMemcpyAsync(&s0[0], ds.p + 0, sizeof(double), cudaMemcpyDeviceToHost, c->st));
@@ -226,18 +197,19 @@ extern "C" int mstmg_gsf_coefficients(mstmg_ctx* c, int t_matrix_order, const do
         set_err("mstmg_gsf_coefficients: bad arguments");
         return MSTMG_ERR_ARG;
     }
+    CallScratch ws(c->pool, c->st);
     BigTablesDev bt;
     int rc = upload_big(c, bt);
     if (rc) return rc;
     const size_t nb0 = 2 * (size_t)T * (T + 2);
     const int W = 2 * T + 1;
-    DevBuf<zd> da0;
-    DevBuf<double> ds;
+    TmpBuf<zd> da0(ws);
+    TmpBuf<double> ds(ws);
     CK(da0.alloc(2 * nb0));
     CK(copy_in(da0.p, amnp0, sizeof(zd) * 2 * nb0, c->st));
     CK(ds.alloc(4 * 16 * (size_t)W));
     CK(cudaMemsetAsync(ds.p, 0, sizeof(double) * 4 * 16 * (size_t)W, c->st));
-    launch_fosm(T, da0.p, bt.bc.p, bt.fnr.p, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
+    launch_fosm(T, da0.p, bt.bc, bt.fnr, bt.nbc, ds.p, ds.p + 16 * W, ds.p + 32 * W, ds.p + 48 * W, c->st);
     CK(cudaGetLastError());
     CK(copy_out(coef, ds.p, sizeof(double) * 4 * 16 * (size_t)W, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -256,19 +228,15 @@ extern "C" int mstmg_scattering_plane(mstmg_ctx* c, int t_matrix_order, const do
         set_err("mstmg_scattering_plane: t_matrix_order above 200 is not supported");
         return MSTMG_ERR_UNSUPPORTED;
     }
-    mstmg::Tables& big = big_tables();
-    std::vector<double> bd(T + 1);
-    for (int k = 0; k <= T; k++) bd[k] = big.bc(k, k);
+    CallScratch ws(c->pool, c->st);
+    BigTablesDev bt;
+    if (int rc = upload_big(c, bt)) return rc;
     const size_t nb0 = 2 * (size_t)T * (T + 2);
     const int nang = udim - ldim + 1;
-    DevBuf<double> dfnr, dbd, dsm;
-    DevBuf<zd> da0;
-    CK(dfnr.alloc(2 * T + 2));
-    CK(dbd.alloc(T + 1));
+    TmpBuf<double> dsm(ws);
+    TmpBuf<zd> da0(ws);
     CK(da0.alloc(2 * nb0));
     CK(dsm.alloc(16 * (size_t)nang));
-    CK(cudaMemcpyAsync(dfnr.p, big.fnr.data(), sizeof(double) * (2 * T + 2), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemcpyAsync(dbd.p, bd.data(), sizeof(double) * (T + 1), cudaMemcpyHostToDevice, c->st));
     CK(copy_in(da0.p, amnp0, sizeof(zd) * 2 * nb0, c->st));
     PlaneSmArgs a;
     a.T = T;
@@ -280,8 +248,8 @@ extern "C" int mstmg_scattering_plane(mstmg_ctx* c, int t_matrix_order, const do
     a.alpha = alpha;
     a.rotate = rotate_plane ? 1 : 0;
     a.rimed_re = c->opts.medium_re;
-    a.fnr = dfnr.p;
-    a.bcofd = dbd.p;
+    a.fnr = bt.fnr;
+    a.bcofd = bt.bcd;
     a.smat = dsm.p;
     launch_planesm(a, c->st);
     CK(cudaGetLastError());
@@ -297,13 +265,14 @@ extern "C" int mstmg_t_matrix_order(mstmg_ctx* c, double trans_eps, int max_t_or
         set_err("mstmg_t_matrix_order: bad arguments");
         return MSTMG_ERR_ARG;
     }
+    CallScratch ws(c->pool, c->st);
     BigTablesDev bt;
     int rc = upload_big(c, bt);
     if (rc) return rc;
     double r0[3];
-    DevBuf<int> dtord;
+    TmpBuf<int> dtord(ws);
     int T = 0;
-    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, dtord, c->tord, &T))) {
+    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, ws, dtord, c->tord, &T))) {
         c->tord.clear();
         return rc;
     }
@@ -344,6 +313,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
     const int TM_GROUP = 256;
     auto cols_of = [](int q) { return 2 * (2 * q + 1); };
     const int nblkt = 2 * TM * (TM + 2), Sord = cols_of(TM), Smax = grouped ? std::max(Sord, TM_GROUP) : Sord;
+    CallScratch ws(c->pool, c->st);
     BigTablesDev bt;
     if ((rc = upload_big(c, bt))) return rc;
     // the cluster origin: the mean of the spheres outside every other (input:1166-1177)
@@ -355,15 +325,16 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
             for (int k = 0; k < 3; k++) r0[k] = r0[k] + c->hpos[3 * (size_t)i + k];
         }
     for (int k = 0; k < 3; k++) r0[k] = r0[k] / (double)nout;
-    DevBuf<int> dtord;
+    TmpBuf<int> dtord(ws);
     CK(dtord.alloc(n));
     CK(cudaMemcpyAsync(dtord.p, c->tord.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->st));
-    RegTables rtm, rtd;   // merge: spheres -> origin; distribute: origin -> spheres
-    if ((rc = build_reg_tables(c, TM, L, rtm)) || (rc = build_reg_tables(c, L, TM, rtd))) return rc;
+    RegTables rtm(ws), rtd(ws);   // merge: spheres -> origin; distribute: origin -> spheres
+    if ((rc = build_reg_tables(c, bt, TM, L, rtm)) || (rc = build_reg_tables(c, bt, L, TM, rtd))) return rc;
     const int grid = std::min(n, c->nsm * 2);
     const size_t strm = merge_scratch_per_cta(TM, L, Sord), strd = merge_scratch_per_cta(L, TM, Sord);
-    DevBuf<zd> mscr, P0, PK, B64, A0, dT, X64;
-    DevBuf<double> qcol, dsq, qsum, rr;
+    TmpBuf<zd> mscr(ws), P0(ws), PK(ws), B64(ws), A0(ws), dT(ws), X64(ws);
+    TmpBuf<double> qcol(ws), dsq(ws), qsum(ws);
+    DevBuf<double> rr;
     DevBuf<zf> B32;
     DevBuf<int> idx;
     CK(mscr.alloc((size_t)grid * merge_chunks(Sord) * std::max(strm, strd)));
@@ -377,7 +348,18 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
     CK(dsq.alloc((size_t)3 * n));
     CK(cudaMemsetAsync(dsq.p, 0, sizeof(double) * 3 * n, c->st));
     CK(qsum.alloc(3));
-    MultiWork<double> w64;
+    MultiWork<double>& w64 = c->tm64;
+    // given back at the end where it is large, as the workspace is
+    struct Trim {
+        MultiWork<double>& w;
+        ~Trim()
+        {
+            if (sizeof(zd) * (w.vec.n + w.XP.n + w.YP.n) <= CALL_POOL_MAX) return;
+            w.vec.release();
+            w.XP.release();
+            w.YP.release();
+        }
+    } trim{w64};
     MultiWork<float> w32;
     if ((rc = w64.init(Smax, ne, c->nsm, !mixed))) return rc;
     GmresWork& gw = c->tm_gm;
@@ -522,9 +504,10 @@ extern "C" int mstmg_tmatrix_qext_qsca(mstmg_ctx* c, int t_matrix_order, const d
         return MSTMG_ERR_ARG;
     }
     const size_t nblkt = 2 * (size_t)t_matrix_order * (t_matrix_order + 2);
-    DevBuf<zd> dT;
-    DevBuf<float> tc;
-    DevBuf<double> out;
+    CallScratch ws(c->pool, c->st);
+    TmpBuf<zd> dT(ws);
+    TmpBuf<float> tc(ws);
+    TmpBuf<double> out(ws);
     CK(dT.alloc(nblkt * nblkt));
     CK(tc.alloc(2 * nblkt * nblkt));
     CK(out.alloc(2));
@@ -548,14 +531,15 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
         set_err("mstmg_ranorient_scattering: bad arguments (1 <= t_matrix_order <= 60, nangles 0 or >= 2)");
         return MSTMG_ERR_ARG;
     }
+    CallScratch ws(c->pool, c->st);
     BigTablesDev bt;
     int rc = upload_big(c, bt);
     if (rc) return rc;
     const size_t nblkt = 2 * (size_t)T * (T + 2);
     const int W = 2 * T + 1;
-    DevBuf<zd> dT, trace, dm, dmcf, bg, bcf, part;
-    DevBuf<float2> tc;
-    DevBuf<double> dsm, dsmat, vtab, dbcd;
+    TmpBuf<zd> dT(ws), trace(ws), dm(ws), dmcf(ws), bg(ws), bcf(ws), part(ws);
+    TmpBuf<float2> tc(ws);
+    TmpBuf<double> dsm(ws), dsmat(ws), vtab(ws);
     CK(dT.alloc(nblkt * nblkt));
     CK(copy_in(dT.p, tmat, sizeof(zd) * nblkt * nblkt, c->st));
     CK(tc.alloc(nblkt * nblkt));
@@ -572,10 +556,6 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     CK(vtab.alloc(rz.vtab));
     const int nang = nangles > 0 ? nangles : 1;
     CK(dsmat.alloc(16 * (size_t)nang));
-    std::vector<double> bd(2 * T + 4);
-    for (int k = 0; k < (int)bd.size(); k++) bd[k] = big_tables().bc(k, k);
-    CK(dbcd.alloc(bd.size()));
-    CK(cudaMemcpyAsync(dbcd.p, bd.data(), sizeof(double) * bd.size(), cudaMemcpyHostToDevice, c->st));
     RoArgs a;
     a.nodr = T;
     a.tc = tc.p;
@@ -589,12 +569,12 @@ extern "C" int mstmg_ranorient_scattering(mstmg_ctx* c, int t_matrix_order, cons
     a.vw0 = 0;
     a.sm = dsm.p;
     a.smcf = dsm.p + 16 * W;
-    a.bcof = bt.bc.p;
-    a.fnr = bt.fnr.p;
+    a.bcof = bt.bc;
+    a.fnr = bt.fnr;
     a.nbc = bt.nbc;
     a.vtab = vtab.p;
     a.rimed_re = c->opts.medium_re;
-    if (launch_ranorient(a, dT.p, nangles, dbcd.p, dsmat.p, c->nsm, c->st) != 0) {
+    if (launch_ranorient(a, dT.p, nangles, bt.bcd, dsmat.p, c->nsm, c->st) != 0) {
         set_err("mstmg_ranorient_scattering: t_matrix_order too large for the kernels (at most " + std::to_string(RO_ORDER_MAX) + ")");
         return MSTMG_ERR_UNSUPPORTED;
     }

@@ -9,6 +9,7 @@
 //                   expansion) and the T matrix (tmatrix_solution, random
 //                   orientation)
 #pragma once
+#include <mutex>
 #include <algorithm>
 #include <complex>
 #include <cstdio>
@@ -71,6 +72,86 @@ template <typename T> struct DevBuf {
         p = nullptr;
         n = 0;
     }
+};
+
+// Device workspace of the calls that post-process a solution (capi_origin.cu),
+// kept by the context: blocks that a call fills from the front and hands back
+// at its end, up to CALL_POOL_MAX bytes (blocks beyond are freed then; all of
+// them with the context).  Each call used to allocate and free 14 to 45
+// buffers: 3.3 ms of a 5.4 ms scattering call, 11.6 ms of a 111 ms T matrix.
+// One call at a time has the blocks; one that finds them taken by another
+// thread works in blocks of its own.
+#define CALL_POOL_MAX ((size_t)1 << 30)
+#define CALL_POOL_BLOCK ((size_t)32 << 20)
+struct CallPool {
+    struct Block {
+        char* p;
+        size_t n;
+    };
+    std::mutex mu;
+    std::vector<Block> blocks;
+    ~CallPool()
+    {
+        for (auto& b : blocks) cudaFree(b.p);
+    }
+};
+class CallScratch {
+public:
+    CallScratch(CallPool& pool, cudaStream_t st) : lk_(pool.mu, std::try_to_lock), st_(st)
+    {
+        blocks_ = lk_.owns_lock() ? &pool.blocks : &own_;
+    }
+    CallScratch(const CallScratch&) = delete;
+    CallScratch& operator=(const CallScratch&) = delete;
+    ~CallScratch()
+    {
+        cudaStreamSynchronize(st_);   // an error return may leave work that uses the blocks
+        size_t sum = 0;
+        for (auto& b : *blocks_) sum += b.n;
+        while (!blocks_->empty() && (blocks_ == &own_ || sum > CALL_POOL_MAX)) {
+            sum -= blocks_->back().n;
+            cudaFree(blocks_->back().p);
+            blocks_->pop_back();
+        }
+    }
+    cudaError_t alloc(void** out, size_t bytes)
+    {
+        bytes = (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
+        for (size_t k = 0; k < blocks_->size(); k++) {
+            if (used_.size() <= k) used_.push_back(0);
+            if ((*blocks_)[k].n - used_[k] >= bytes) {
+                *out = (*blocks_)[k].p + used_[k];
+                used_[k] += bytes;
+                return cudaSuccess;
+            }
+        }
+        CallPool::Block b{nullptr, std::max(bytes, CALL_POOL_BLOCK)};
+        cudaError_t e = cudaMalloc((void**)&b.p, b.n);
+        if (e != cudaSuccess && b.n > bytes) {   // no room for a whole block
+            cudaGetLastError();
+            b.n = bytes;
+            e = cudaMalloc((void**)&b.p, b.n);
+        }
+        if (e != cudaSuccess) return e;
+        blocks_->push_back(b);
+        used_.resize(blocks_->size(), 0);
+        used_.back() = bytes;
+        *out = b.p;
+        return cudaSuccess;
+    }
+
+private:
+    std::unique_lock<std::mutex> lk_;
+    cudaStream_t st_;
+    std::vector<CallPool::Block> own_, *blocks_;
+    std::vector<size_t> used_;
+};
+// a buffer of a call's workspace
+template <typename T> struct TmpBuf {
+    explicit TmpBuf(CallScratch& w) : ws(w) {}
+    CallScratch& ws;
+    T* p = nullptr;
+    cudaError_t alloc(size_t count) { return ws.alloc((void**)&p, sizeof(T) * count); }
 };
 
 template <typename T> struct BicgVecs {
@@ -362,6 +443,12 @@ struct mstmg_ctx {
     GmresWork fo_gm;   // mixed_solver 2
     bool fo_gm_ready = false;
     GmresWork tm_gm;   // mixed_solver 2, T-matrix columns: kept across calls (sized for the largest order)
+    MultiWork<double> tm64;   // FP64 work of the T-matrix columns, kept likewise while below CALL_POOL_MAX
+    CallPool pool;
+    // the reference's constant tables on the device: bcof, square roots, bcof(n, n)
+    std::mutex big_mu;
+    DevBuf<double> big_bc, big_fnr, big_bcd;
+    bool big_ready = false;
     // ensembles (mstmg_ensemble_create): configuration c holds spheres
     // cfg_start[c] .. cfg_start[c+1]-1; no pairs between configurations
     std::vector<int> cfg_start, cfg_of;

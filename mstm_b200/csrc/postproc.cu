@@ -112,6 +112,35 @@ __global__ void __launch_bounds__(32) tranorder_kernel(int nsph, const double* p
 }
 
 // ---------------------------------------------------------------------------
+// coupling constants of a regular translation (axialtrancoefinit,
+// modules:1680-1722): one CTA per (n, l), a thread per degree m and one for
+// the m-independent row, rows in shared memory (min(n, l) <= MSTMG_LMAX: one
+// side is a sphere).  The host took 2 ms for the tables of a 350-sphere
+// scattering matrix before the first kernel that reads them could start.
+// ---------------------------------------------------------------------------
+#define RC_NT 64
+static_assert(RC_NT >= 2 * MSTMG_LMAX + 2, "a thread per degree m and one more");
+__global__ void __launch_bounds__(RC_NT) regular_couplings_kernel(int Tt, int Ls, VCTab tab, double* vcc)
+{
+    extern __shared__ __align__(16) double rc_smem[];
+    const int n = Tt - (int)blockIdx.x, l = Ls - (int)blockIdx.y, VL = Tt + Ls + 1;
+    const int nlmin = min(n, l), wmin = abs(n - l), wmax = n + l, nm = 2 * nlmin + 1;
+    const int r = threadIdx.x;
+    if (r < nm) vc_func(tab, nlmin - r, n, r - nlmin, l, rc_smem + r * VL);   // vcfunc(-m,n,m,l), m = r - nlmin
+    else if (r == nm) vc_func(tab, -1, n, 1, l, rc_smem + nm * VL);
+    __syncthreads();
+    const double c1 = tab.fr(n + n + 1) * tab.fr(l + l + 1);
+    const double* v2 = rc_smem + nm * VL;
+    const int nw = wmax - wmin + 1;
+    for (int e = threadIdx.x; e < nm * nw; e += RC_NT) {
+        const int q = e / nw, w = wmin + e % nw, m = q - nlmin, ml = l * (l + 1) + m;
+        const int ph = ((n - l + w) % 4 + 4) % 4;
+        const double ri = (ph == 0 || ph == 1) ? 1.0 : -1.0;
+        vcc[(size_t)(n - 1) + (size_t)Tt * ((size_t)(ml - 1) + (size_t)Ls * (Ls + 2) * w)] = -c1 * pm1(m) * rc_smem[q * VL + w] * v2[w] * ri;
+    }
+}
+
+// ---------------------------------------------------------------------------
 // merge to / distribute from the common origin: CTAs over (sphere, chunk of
 // MERGE_PC columns), spheres grid-strided, scratch per CTA.  Per sphere the
 // translation's tables are made once -- e^{i m phi} powers, the regular
@@ -706,6 +735,15 @@ void launch_tranorder(int nsph, const double* pos, const int* order, const doubl
     cudaFuncSetAttribute(tranorder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     tranorder_kernel<<<tranorder_blocks(nsph), 32, smem, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire, eps, maxt, t,
                                                                scratch, tord);
+    launch_counter() += 1;
+}
+
+void launch_regular_couplings(int Tt, int Ls, const double* bcof, const double* fnr, int nbc, double* vcc, cudaStream_t st)
+{
+    VCTab t{bcof, fnr, nbc};
+    const int smem = (int)sizeof(double) * (2 * std::min(Tt, Ls) + 2) * (Tt + Ls + 1);
+    cudaFuncSetAttribute(regular_couplings_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    regular_couplings_kernel<<<dim3(Tt, Ls), RC_NT, smem, st>>>(Tt, Ls, t, vcc);
     launch_counter() += 1;
 }
 

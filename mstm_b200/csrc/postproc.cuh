@@ -26,10 +26,6 @@ struct MergeArgs {
     int ld0;
     const double* vcc;      // vcc_const slice (n <= vcT, ml <= vcML, w <= vcT + L)
     int vcT, vcML;
-    const double* fnm1;     // (-fcN..fcN, 1..fcN)
-    const double* fnc;
-    const double* fnp1;
-    int fcN;
     const double* fnr;
     const double* bcofd;
     zd* scratch;
@@ -41,6 +37,8 @@ struct MergeArgs {
 size_t tranorder_scratch(int nsph);   // complex values of scratch launch_tranorder needs
 void launch_tranorder(int nsph, const double* pos, const int* order, const double* origin, double rire, double eps, int maxt,
                       const double* bcof, const double* fnr, int nbc, zd* scratch, int* tord, cudaStream_t st);
+// vcc_const of source orders <= Ls, target orders <= Tt: vcc[(n-1) + Tt ((ml-1) + Ls (Ls+2) w)]
+void launch_regular_couplings(int Tt, int Ls, const double* bcof, const double* fnr, int nbc, double* vcc, cudaStream_t st);
 #define MERGE_PC 16   // columns a CTA of the merge kernel translates together
 // zd units of merge-kernel scratch per CTA; a launch of `grid` CTAs per chunk
 // of MERGE_PC columns needs grid * merge_chunks(npol) of them
