@@ -589,7 +589,7 @@ template <typename T> int fft_far(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int 
             set_err("FFT translation: forward transform failed");
             return MSTMG_ERR_CUDA;
         }
-        launch_fft_mul<T>(F.nbN, F.N8, w, F.H.p, A.p, G.p, c->nsm, c->st);
+        launch_fft_mul<T>(F.nbN, F.N8, w, F.H.p, A.p, G.p, c->st);
         if (sizeof(T) == 8) fr = cufftExecZ2Z(F.plan[pi][w], (cufftDoubleComplex*)G.p, (cufftDoubleComplex*)G.p, CUFFT_INVERSE);
         else fr = cufftExecC2C(F.plan[pi][w], (cufftComplex*)G.p, (cufftComplex*)G.p, CUFFT_INVERSE);
         if (fr != CUFFT_SUCCESS) {

@@ -20,6 +20,7 @@
 //                      all columns                                 fft:827-899
 //   fft_n2s_kernel     node coefficients -> sphere (1/N of the inverse FFT
 //                      folded in), shifted back, added to y
+#include <type_traits>
 #include "common.cuh"
 #include "gentran.cuh"
 #include "fftpath.cuh"
@@ -174,20 +175,39 @@ __global__ void fft_round_kernel(size_t n, const zd* in, float2* out)
         out[e] = make_float2((float)in[e].x, (float)in[e].y);
 }
 
-template <typename T> struct c2 { typedef double2 t; };
-template <> struct c2<float> { typedef float2 t; };
+// 8 or 16 bytes in one load
+__device__ __forceinline__ zf ldc(const zf* p)
+{
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return mk(v.x, v.y);
+}
+__device__ __forceinline__ zd ldc(const zd* p)
+{
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    return mk(v.x, v.y);
+}
 
-// sphere -> node: A[col][p][k][slot_i] += sum_m Jsn_i(k, m, p) (S x_i)(m, p)
-template <typename T>
-__global__ void __launch_bounds__(FFT_NT) fft_s2n_kernel(FftMArgs a, const cpx<T>* J, const cpx<T>* x, int ld, int ncol, unsigned contran,
-                                                         cpx<T>* A)
+#define FFT_MB 8   // J records of a thread in flight, the last few of a share included
+
+// The three kernels below are bound by the J records (read once a pass), the
+// kernel spectra H (likewise) and the caches: a fixed number of columns NC
+// keeps the sums in registers (a runtime count kept them in local memory).
+// For 2500 spheres of order 7 and two FP32 columns they took 75 (s2n), 154
+// (mul) and 41 us (n2s); now 24, 49 and 28.
+
+// sphere -> node: A[col][p][k][slot_i] += sum_m Jsn_i(k, m, p) (S x_i)(m, p).
+// One CTA a sphere; a thread has an element (p, k) and one of the shares the
+// sum over m is cut into so that every thread works.
+template <typename T, int NC>
+__global__ void __launch_bounds__(FFT_MT) fft_s2n_kernel(FftMArgs a, const cpx<T>* J, const cpx<T>* x, int ld, unsigned contran, cpx<T>* A)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
-    cpx<T>* xs = reinterpret_cast<cpx<T>*>(smraw);   // ncol x 2 nb
+    cpx<T>* xs = reinterpret_cast<cpx<T>*>(smraw);   // NC x 2 nbmax
     const int i = blockIdx.x;
     const int L = a.order[i], nb = L * (L + 2), No = a.No, nbN = No * (No + 2);
+    cpx<T>* ps = xs + NC * 2 * a.nbmax;              // NC x FFT_MT partial sums
     const size_t N8 = a.N8;
-    for (int e = threadIdx.x; e < ncol * 2 * nb; e += FFT_NT) {
+    for (int e = threadIdx.x; e < NC * 2 * nb; e += FFT_MT) {
         int c = e / (2 * nb), el = e % (2 * nb);
         int p = el / nb, idx = el % nb;
         cpx<T> v = x[(size_t)c * ld + a.offset[i] + el];
@@ -203,76 +223,139 @@ __global__ void __launch_bounds__(FFT_NT) fft_s2n_kernel(FftMArgs a, const cpx<T
     }
     __syncthreads();
     const cpx<T>* Ji = J + a.joff[i];
-    const int slot = a.slot[i];
-    for (int e = threadIdx.x; e < 2 * nbN; e += FFT_NT) {
-        int p = e / nbN, k = e % nbN;
-        cpx<T> acc[4];
-        for (int c = 0; c < ncol; c++) acc[c] = mk((T)0, (T)0);
-        for (int m = 0; m < nb; m++) {
-            cpx<T> j = Ji[k + (size_t)nbN * (m + (size_t)nb * p)];
-            for (int c = 0; c < ncol; c++) acc[c] = acc[c] + j * xs[c * 2 * nb + p * nb + m];
+    const int slot = a.slot[i], items = 2 * nbN;
+    const int nsh = max(1, FFT_MT / items), mper = (nb + nsh - 1) / nsh;
+    for (int e0 = 0; e0 < items; e0 += FFT_MT) {
+        const int cnt = min(items - e0, FFT_MT), sh = threadIdx.x / cnt, e = e0 + threadIdx.x % cnt;
+        const int p = e / nbN, k = e % nbN;
+        cpx<T> acc[NC];
+        for (int c = 0; c < NC; c++) acc[c] = mk((T)0, (T)0);
+        if (sh < nsh) {
+            const cpx<T>* Jp = Ji + k + (size_t)nbN * nb * p;
+            const cpx<T>* xp = xs + p * nb;
+            const int m1 = min(nb, (sh + 1) * mper);
+            for (int m = sh * mper; m < m1; m += FFT_MB) {
+                cpx<T> j[FFT_MB];
+#pragma unroll
+                for (int u = 0; u < FFT_MB; u++) j[u] = m + u < m1 ? ldc(Jp + (size_t)nbN * (m + u)) : mk((T)0, (T)0);
+#pragma unroll
+                for (int u = 0; u < FFT_MB; u++)
+                    if (m + u < m1)
+#pragma unroll
+                        for (int c = 0; c < NC; c++) acc[c] = acc[c] + j[u] * xp[c * 2 * nb + m + u];
+            }
         }
-        for (int c = 0; c < ncol; c++) {
-            cpx<T>* dst = A + ((size_t)(c * 2 + p) * nbN + k) * N8 + slot;
-            atomicAdd(&dst->x, acc[c].x);
-            atomicAdd(&dst->y, acc[c].y);
+        if (nsh > 1) {
+            for (int c = 0; c < NC; c++) ps[c * FFT_MT + threadIdx.x] = acc[c];
+            __syncthreads();
+            if (sh == 0)
+                for (int c = 0; c < NC; c++)
+                    for (int q = 1; q < nsh; q++) acc[c] = acc[c] + ps[c * FFT_MT + threadIdx.x + q * cnt];
         }
+        if (sh == 0)
+            for (int c = 0; c < NC; c++) {
+                cpx<T>* dst = A + ((size_t)(c * 2 + p) * nbN + k) * N8 + slot;
+                atomicAdd(&dst->x, acc[c].x);
+                atomicAdd(&dst->y, acc[c].y);
+            }
     }
 }
 
 // per frequency f: G[col][p][l][f] = sum_n H[p][l][n][f] A[col][p][n][f].
-// Row (p, l) = blockIdx.y, frequencies over threads: every H element is read
-// once, coalesced along f, and the A rows are shared through the caches by
-// the 2 nbN rows of a frequency block.
-template <typename T>
-__global__ void __launch_bounds__(FFT_NT) fft_mul_kernel(int nbN, size_t N8, int ncol, const float2* H, const cpx<T>* A, cpx<T>* G)
+// A thread has one f and R rows l of one p (blockIdx.y): every H element is
+// read once, coalesced along f, and each A value serves R rows from a register.
+template <typename T, int NC, int R>
+__global__ void __launch_bounds__(FFT_NT) fft_mul_kernel(int nbN, size_t N8, const float2* H, const cpx<T>* A, cpx<T>* G)
 {
-    const int pl = blockIdx.y, p = pl / nbN, l = pl - p * nbN;
-    const float2* h = H + (size_t)pl * nbN * N8;
-    for (size_t f = blockIdx.x * (size_t)FFT_NT + threadIdx.x; f < N8; f += (size_t)gridDim.x * FFT_NT) {
-        cpx<T> acc[4];
-        for (int c = 0; c < ncol; c++) acc[c] = mk((T)0, (T)0);
+    const int ng = (nbN + R - 1) / R, p = blockIdx.y / ng, l0 = (blockIdx.y - p * ng) * R, nr = min(R, nbN - l0);
+    const size_t f = blockIdx.x * (size_t)FFT_NT + threadIdx.x;
+    if (f >= N8) return;
+    const float2* h = H + ((size_t)(p * nbN + l0) * nbN) * N8 + f;
+    const cpx<T>* Ap = A + (size_t)p * nbN * N8 + f;
+    const size_t cs = (size_t)2 * nbN * N8;   // a column
+    cpx<T> acc[R][NC];
+#pragma unroll
+    for (int r = 0; r < R; r++)
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[r][c] = mk((T)0, (T)0);
+    auto rows = [&](auto full) {
+#pragma unroll 2
         for (int n = 0; n < nbN; n++) {
-            const float2 hh = h[(size_t)n * N8 + f];
-            const cpx<T> hv = mk((T)hh.x, (T)hh.y);
-            for (int c = 0; c < ncol; c++) acc[c] = acc[c] + hv * A[((size_t)(c * 2 + p) * nbN + n) * N8 + f];
+            cpx<T> av[NC];
+            float2 hv[R];
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (full || r < nr) hv[r] = __ldcs(&h[((size_t)r * nbN + n) * N8]);
+#pragma unroll
+            for (int c = 0; c < NC; c++) av[c] = ldc(Ap + c * cs + (size_t)n * N8);
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (full || r < nr)
+#pragma unroll
+                    for (int c = 0; c < NC; c++) acc[r][c] = acc[r][c] + mk((T)hv[r].x, (T)hv[r].y) * av[c];
         }
-        for (int c = 0; c < ncol; c++) G[((size_t)(c * 2 + p) * nbN + l) * N8 + f] = acc[c];
-    }
+    };
+    if (nr == R) rows(std::true_type());
+    else rows(std::false_type());
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (r < nr)
+#pragma unroll
+            for (int c = 0; c < NC; c++) G[c * cs + (size_t)(p * nbN + l0 + r) * N8 + f] = acc[r][c];
 }
 
-// node -> sphere: y_i += S (Jns_i g_node / N8)
-template <typename T>
-__global__ void __launch_bounds__(FFT_NT) fft_n2s_kernel(FftMArgs a, const cpx<T>* J, const cpx<T>* G, int ncol, unsigned contran, cpx<T>* y,
-                                                         int ld)
+// node -> sphere: y_i += S (Jns_i g_node / N8); the sum over k in shares as in s2n
+template <typename T, int NC>
+__global__ void __launch_bounds__(FFT_MT) fft_n2s_kernel(FftMArgs a, const cpx<T>* J, const cpx<T>* G, unsigned contran, cpx<T>* y, int ld)
 {
     extern __shared__ __align__(16) unsigned char smraw[];
     const int i = blockIdx.x;
     const int L = a.order[i], nb = L * (L + 2), No = a.No, nbN = No * (No + 2);
-    cpx<T>* gs = reinterpret_cast<cpx<T>*>(smraw);   // ncol x 2 nbN
-    cpx<T>* ys = gs + 4 * 2 * nbN;                    // ncol x 2 nb
+    cpx<T>* gs = reinterpret_cast<cpx<T>*>(smraw);   // NC x 2 nbN
+    cpx<T>* ys = gs + NC * 2 * nbN;                   // NC x 2 nbmax
+    cpx<T>* ps = ys + NC * 2 * a.nbmax;               // NC x FFT_MT partial sums
     const size_t N8 = a.N8;
     const int slot = a.slot[i];
     const T inv = (T)(1.0 / (double)N8);
-    for (int e = threadIdx.x; e < ncol * 2 * nbN; e += FFT_NT) {
-        int c = e / (2 * nbN), el = e % (2 * nbN);
-        cpx<T> v = G[((size_t)c * 2 * nbN + el) * N8 + slot];
+    for (int e = threadIdx.x; e < NC * 2 * nbN; e += FFT_MT) {
+        const cpx<T> v = ldc(G + (size_t)e * N8 + slot);
         gs[e] = mk(v.x * inv, v.y * inv);
     }
     __syncthreads();
     const cpx<T>* Ji = J + a.joff[i];
-    for (int e = threadIdx.x; e < 2 * nb; e += FFT_NT) {
-        int p = e / nb, m = e % nb;
-        cpx<T> acc[4];
-        for (int c = 0; c < ncol; c++) acc[c] = mk((T)0, (T)0);
-        for (int k = 0; k < nbN; k++) {
-            cpx<T> j = Ji[m + (size_t)nb * (k + (size_t)nbN * p)];
-            for (int c = 0; c < ncol; c++) acc[c] = acc[c] + j * gs[c * 2 * nbN + p * nbN + k];
+    const int items = 2 * nb, nsh = max(1, FFT_MT / items), kper = (nbN + nsh - 1) / nsh;
+    for (int e0 = 0; e0 < items; e0 += FFT_MT) {
+        const int cnt = min(items - e0, FFT_MT), sh = threadIdx.x / cnt, e = e0 + threadIdx.x % cnt;
+        const int p = e / nb, m = e % nb;
+        cpx<T> acc[NC];
+        for (int c = 0; c < NC; c++) acc[c] = mk((T)0, (T)0);
+        if (sh < nsh) {
+            const cpx<T>* Jp = Ji + m + (size_t)nb * nbN * p;
+            const cpx<T>* gp = gs + p * nbN;
+            const int k1 = min(nbN, (sh + 1) * kper);
+            for (int k = sh * kper; k < k1; k += FFT_MB) {
+                cpx<T> j[FFT_MB];
+#pragma unroll
+                for (int u = 0; u < FFT_MB; u++) j[u] = k + u < k1 ? ldc(Jp + (size_t)nb * (k + u)) : mk((T)0, (T)0);
+#pragma unroll
+                for (int u = 0; u < FFT_MB; u++)
+                    if (k + u < k1)
+#pragma unroll
+                        for (int c = 0; c < NC; c++) acc[c] = acc[c] + j[u] * gp[c * 2 * nbN + k + u];
+            }
         }
-        for (int c = 0; c < ncol; c++) ys[c * 2 * nb + e] = acc[c];
+        if (nsh > 1) {
+            for (int c = 0; c < NC; c++) ps[c * FFT_MT + threadIdx.x] = acc[c];
+            __syncthreads();
+            if (sh == 0)
+                for (int c = 0; c < NC; c++)
+                    for (int q = 1; q < nsh; q++) acc[c] = acc[c] + ps[c * FFT_MT + threadIdx.x + q * cnt];
+        }
+        if (sh == 0)
+            for (int c = 0; c < NC; c++) ys[c * 2 * nb + e] = acc[c];
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < ncol * 2 * nb; e += FFT_NT) {
+    for (int e = threadIdx.x; e < NC * 2 * nb; e += FFT_MT) {
         int c = e / (2 * nb), el = e % (2 * nb);
         int p = el / nb, idx = el % nb;
         cpx<T> v = ys[e];
@@ -306,35 +389,50 @@ void launch_fft_round(size_t n, const zd* in, float2* out, cudaStream_t st)
     fft_round_kernel<<<(int)std::min<size_t>((n + 255) / 256, 148 * 32), 256, 0, st>>>(n, in, out);
     launch_counter() += 1;
 }
+// f(number of columns as a constant), 1 .. 4
+template <typename F> static void with_columns(int ncol, F f)
+{
+    switch (ncol) {
+    case 1: f(std::integral_constant<int, 1>()); break;
+    case 2: f(std::integral_constant<int, 2>()); break;
+    case 3: f(std::integral_constant<int, 3>()); break;
+    default: f(std::integral_constant<int, 4>()); break;
+    }
+}
 template <typename T>
 void launch_fft_s2n(const FftMArgs& a, const cpx<T>* J, const cpx<T>* x, int ld, int ncol, unsigned contran, cpx<T>* A, cudaStream_t st)
 {
-    size_t smem = sizeof(cpx<T>) * 4 * 2 * a.nbmax;
-    cudaFuncSetAttribute(fft_s2n_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fft_s2n_kernel<T><<<a.nsph, FFT_NT, smem, st>>>(a, J, x, ld, ncol, contran, A);
+    const int smem = (int)sizeof(cpx<T>) * ncol * (2 * a.nbmax + FFT_MT);
+    with_columns(ncol, [&](auto nc) {
+        auto k = fft_s2n_kernel<T, decltype(nc)::value>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        k<<<a.nsph, FFT_MT, smem, st>>>(a, J, x, ld, contran, A);
+    });
     launch_counter() += 1;
 }
-template <typename T> void launch_fft_mul(int nbN, size_t N8, int ncol, const float2* H, const cpx<T>* A, cpx<T>* G, int nsm, cudaStream_t st)
+template <typename T> void launch_fft_mul(int nbN, size_t N8, int ncol, const float2* H, const cpx<T>* A, cpx<T>* G, cudaStream_t st)
 {
-    const int rows = 2 * nbN;
-    const int want = std::max(1, nsm * 16 / rows);   // about 16 CTAs per SM over all rows
-    int g = (int)std::min<size_t>((N8 + FFT_NT - 1) / FFT_NT, (size_t)want);
-    fft_mul_kernel<T><<<dim3(g, rows), FFT_NT, 0, st>>>(nbN, N8, ncol, H, A, G);
+    // rows a thread: as many as leave two CTAs' registers to an SM
+    constexpr int R = sizeof(T) == 4 ? 8 : 4;
+    const dim3 g((unsigned)((N8 + FFT_NT - 1) / FFT_NT), 2 * ((nbN + R - 1) / R));
+    with_columns(ncol, [&](auto nc) { fft_mul_kernel<T, decltype(nc)::value, R><<<g, FFT_NT, 0, st>>>(nbN, N8, H, A, G); });
     launch_counter() += 1;
 }
 template <typename T>
 void launch_fft_n2s(const FftMArgs& a, const cpx<T>* J, const cpx<T>* G, int ncol, unsigned contran, cpx<T>* y, int ld, cudaStream_t st)
 {
-    const int nbN = a.No * (a.No + 2);
-    size_t smem = sizeof(cpx<T>) * 4 * 2 * (nbN + a.nbmax);
-    cudaFuncSetAttribute(fft_n2s_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    fft_n2s_kernel<T><<<a.nsph, FFT_NT, smem, st>>>(a, J, G, ncol, contran, y, ld);
+    const int nbN = a.No * (a.No + 2), smem = (int)sizeof(cpx<T>) * ncol * (2 * nbN + 2 * a.nbmax + FFT_MT);
+    with_columns(ncol, [&](auto nc) {
+        auto k = fft_n2s_kernel<T, decltype(nc)::value>;
+        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        k<<<a.nsph, FFT_MT, smem, st>>>(a, J, G, contran, y, ld);
+    });
     launch_counter() += 1;
 }
 
 template void launch_fft_s2n<double>(const FftMArgs&, const zd*, const zd*, int, int, unsigned, zd*, cudaStream_t);
 template void launch_fft_s2n<float>(const FftMArgs&, const zf*, const zf*, int, int, unsigned, zf*, cudaStream_t);
-template void launch_fft_mul<double>(int, size_t, int, const float2*, const zd*, zd*, int, cudaStream_t);
-template void launch_fft_mul<float>(int, size_t, int, const float2*, const zf*, zf*, int, cudaStream_t);
+template void launch_fft_mul<double>(int, size_t, int, const float2*, const zd*, zd*, cudaStream_t);
+template void launch_fft_mul<float>(int, size_t, int, const float2*, const zf*, zf*, cudaStream_t);
 template void launch_fft_n2s<double>(const FftMArgs&, const zd*, const zd*, int, unsigned, zd*, int, cudaStream_t);
 template void launch_fft_n2s<float>(const FftMArgs&, const zf*, const zf*, int, unsigned, zf*, int, cudaStream_t);

@@ -4,6 +4,7 @@
 #include "gentran.cuh"
 
 #define FFT_NT 128
+#define FFT_MT 256   // threads of the sphere <-> node kernels: shares of each sum at node order 5 and below
 #define FFT_NBN_MAX 440   // node order <= 20
 
 struct FftJArgs {
@@ -42,6 +43,6 @@ void launch_fft_hbuild(const FftHArgs& a, int nsm, cudaStream_t st);
 void launch_fft_round(size_t n, const zd* in, float2* out, cudaStream_t st);
 template <typename T>
 void launch_fft_s2n(const FftMArgs& a, const cpx<T>* J, const cpx<T>* x, int ld, int ncol, unsigned contran, cpx<T>* A, cudaStream_t st);
-template <typename T> void launch_fft_mul(int nbN, size_t N8, int ncol, const float2* H, const cpx<T>* A, cpx<T>* G, int nsm, cudaStream_t st);
+template <typename T> void launch_fft_mul(int nbN, size_t N8, int ncol, const float2* H, const cpx<T>* A, cpx<T>* G, cudaStream_t st);
 template <typename T>
 void launch_fft_n2s(const FftMArgs& a, const cpx<T>* J, const cpx<T>* G, int ncol, unsigned contran, cpx<T>* y, int ld, cudaStream_t st);
