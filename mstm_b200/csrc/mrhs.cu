@@ -96,54 +96,125 @@ __global__ void __launch_bounds__(MB) gm_apply_kernel(SlotMaps sm, const zf* an,
     }
 }
 
-// h[i S + s] += V_{s,i}^H W[:, k] (and hacc likewise when given), i = blockIdx.y
-__global__ void __launch_bounds__(MB) gm_dots_kernel(int ld, int S, int m1, const int* act, const zf* V, const zf* W, double* h, double* hacc,
-                                                     const int* len)
+// one 8-byte load
+__device__ __forceinline__ cpx<double> ldw(const zf* p)
 {
-    const int i = blockIdx.y, k = blockIdx.z, s = act[k];
-    const zf* v = V + ((size_t)s * m1 + i) * ld;
-    const zf* w = W + (size_t)k * ld;
-    const int ne = len ? len[s] : ld;
-    double acc[2] = {0.0, 0.0};
-    for (int e = blockIdx.x * MB + threadIdx.x; e < ne; e += gridDim.x * MB) {
-        const cpx<double> x = upd_(v[e]), y = upd_(w[e]);
-        acc[0] += x.x * y.x + x.y * y.y;
-        acc[1] += x.x * y.y - x.y * y.x;
-    }
-    double out[2];
-    mblock_store<2>(acc, out);
-    if (threadIdx.x == 0) {
-        const size_t o = 2 * ((size_t)i * S + s);
-        atomicAdd(&h[o], out[0]);
-        atomicAdd(&h[o + 1], out[1]);
-        if (hacc) {
-            atomicAdd(&hacc[o], out[0]);
-            atomicAdd(&hacc[o + 1], out[1]);
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    return mk((double)v.x, (double)v.y);
+}
+
+// Dots of W[:, k] with GM_DI vectors V_{s,i0}, ... at once (fewer at the end):
+// bound by reading V, w is read once for all of them.  CTAs of 128 threads:
+// with 256 (two sums of a warp more to wait for, fewer CTAs an SM) 13 vectors
+// of 2 columns of 315,000 values took 47 us against 27, V not in L2.
+#define GM_DI 4
+#define GM_DT 128         // threads
+#define GM_CHUNK 1024     // elements of a device-driven item: 8 a thread
+#define GV_N 64           // steps of a restart cycle the one-block kernels keep in shared memory and registers
+#define GM_HS 512         // 8 KB of coefficients; longer restart cycles read the rest from global memory
+__device__ __forceinline__ void gm_dots_part(int e0, int e1, int step, int ni, const zf* v, int ld, const zf* w, int i0, int S, int s,
+                                             double* h, double* hacc)
+{
+    double acc[2 * GM_DI];
+#pragma unroll
+    for (int q = 0; q < 2 * GM_DI; q++) acc[q] = 0.0;
+    if (ni == GM_DI) {
+#pragma unroll 2
+        for (int e = e0; e < e1; e += step) {
+            const cpx<double> y = ldw(w + e);
+#pragma unroll
+            for (int q = 0; q < GM_DI; q++) {
+                const cpx<double> x = ldw(v + (size_t)q * ld + e);
+                acc[2 * q] = fma(x.y, y.y, fma(x.x, y.x, acc[2 * q]));
+                acc[2 * q + 1] = fma(-x.y, y.x, fma(x.x, y.y, acc[2 * q + 1]));
+            }
+        }
+    } else {
+#pragma unroll 2
+        for (int e = e0; e < e1; e += step) {
+            const cpx<double> y = ldw(w + e);
+#pragma unroll
+            for (int q = 0; q < GM_DI - 1; q++)
+                if (q < ni) {
+                    const cpx<double> x = ldw(v + (size_t)q * ld + e);
+                    acc[2 * q] = fma(x.y, y.y, fma(x.x, y.x, acc[2 * q]));
+                    acc[2 * q + 1] = fma(-x.y, y.x, fma(x.x, y.y, acc[2 * q + 1]));
+                }
         }
     }
+    // the eight sums over a warp in nine exchanges: each halves the values a
+    // lane still carries, so that lane l ends with value l >> 2
+    static_assert(GM_DI == 4, "eight sums");
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int half = 4, bit = 16; half >= 1; half >>= 1, bit >>= 1)
+#pragma unroll
+        for (int q = 0; q < half; q++) {
+            const bool up = lane & bit;
+            const double mine = up ? acc[q + half] : acc[q], give = up ? acc[q] : acc[q + half];
+            acc[q] = mine + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 2);
+    acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], 1);
+    __shared__ double sh[2 * GM_DI][GM_DT / 32];
+    if ((lane & 3) == 0) sh[lane >> 2][threadIdx.x >> 5] = acc[0];
+    __syncthreads();
+    const int q = threadIdx.x;
+    if (q < 2 * ni) {
+        double t = 0.0;
+#pragma unroll
+        for (int w_ = 0; w_ < GM_DT / 32; w_++) t += sh[q][w_];
+        const size_t o = 2 * ((size_t)(i0 + (q >> 1)) * S + s) + (q & 1);
+        atomicAdd(&h[o], t);
+        if (hacc) atomicAdd(&hacc[o], t);
+    }
+}
+
+// h[i S + s] += V_{s,i}^H W[:, k] for i < kp1 (and hacc likewise when given), i / GM_DI = blockIdx.y
+__global__ void __launch_bounds__(GM_DT) gm_dots_kernel(int ld, int S, int m1, int kp1, const int* act, const zf* V, const zf* W, double* h,
+                                                     double* hacc, const int* len)
+{
+    const int i0 = blockIdx.y * GM_DI, k = blockIdx.z, s = act[k];
+    gm_dots_part(blockIdx.x * GM_DT + threadIdx.x, len ? len[s] : ld, gridDim.x * GM_DT, min(GM_DI, kp1 - i0), V + ((size_t)s * m1 + i0) * ld, ld,
+                 W + (size_t)k * ld, i0, S, s, h, hacc);
 }
 
 // W[:, k] -= sum_{i < kp1} V_{s,i} h[i S + s] (FP64 accumulation per
 // element); nrm[s] += |W[:, k]|^2 of the result when nrm is given; with
-// jp, kp1 = *jp + 1
+// jp, kp1 = *jp + 1.  The first GM_HS coefficients in shared memory and four
+// vectors' loads in flight: reading V bounds it.  With 4-byte loads and the
+// coefficients from global memory in each step it took 25 us a step of the
+// 2500-sphere FFT solve and 46 us for 256 columns of 9600; now 17 and 37 (the
+// dots: 31 to 16 and 27 to 19).
 __global__ void __launch_bounds__(MB) gm_update_kernel(int ld, int S, int m1, int kp1, const int* act, const zf* V, const double* h, zf* W,
                                                       double* nrm, const int* len, const int* jp)
 {
+    __shared__ double2 hs[GM_HS];
     const int k = blockIdx.y, s = act[k];
     if (jp) kp1 = *jp + 1;
+    const int ks = min(kp1, GM_HS);
+    for (int i = threadIdx.x; i < ks; i += MB) hs[i] = make_double2(h[2 * ((size_t)i * S + s)], h[2 * ((size_t)i * S + s) + 1]);
+    __syncthreads();
     const zf* vs = V + (size_t)s * m1 * ld;
     zf* w = W + (size_t)k * ld;
     const int ne = len ? len[s] : ld;
     double n2[1] = {0.0};
     for (int e = blockIdx.x * MB + threadIdx.x; e < ne; e += gridDim.x * MB) {
-        cpx<double> x = upd_(w[e]);
-        for (int i = 0; i < kp1; i++) {
-            const cpx<double> t = upd_(vs[(size_t)i * ld + e]) * mk(h[2 * ((size_t)i * S + s)], h[2 * ((size_t)i * S + s) + 1]);
+        cpx<double> x = ldw(w + e);
+        const zf* v = vs + e;
+#pragma unroll 4
+        for (int i = 0; i < ks; i++) {
+            const cpx<double> t = ldw(v + (size_t)i * ld) * mk(hs[i].x, hs[i].y);
+            x.x -= t.x;
+            x.y -= t.y;
+        }
+        for (int i = ks; i < kp1; i++) {
+            const cpx<double> t = ldw(v + (size_t)i * ld) * mk(h[2 * ((size_t)i * S + s)], h[2 * ((size_t)i * S + s) + 1]);
             x.x -= t.x;
             x.y -= t.y;
         }
         const zf r = mk((float)x.x, (float)x.y);
-        w[e] = r;
+        *reinterpret_cast<float2*>(w + e) = make_float2(r.x, r.y);
         n2[0] += (double)r.x * r.x + (double)r.y * r.y;
     }
     if (nrm) {
@@ -983,7 +1054,8 @@ void launch_gm_apply(const SlotMaps& sm, const zf* an, int ld, int a, const zf* 
 void launch_gm_dots(int ld, int S, int m1, int kp1, int a, const int* act, const zf* V, const zf* W, double* h, double* hacc, int nsm,
                     cudaStream_t st, const int* len)
 {
-    gm_dots_kernel<<<dim3(multi_grid(ld, kp1 * a, nsm), kp1, a), MB, 0, st>>>(ld, S, m1, act, V, W, h, hacc, len);
+    const int ng = (kp1 + GM_DI - 1) / GM_DI;
+    gm_dots_kernel<<<dim3(multi_grid(ld, ng * a, 2 * nsm), ng, a), GM_DT, 0, st>>>(ld, S, m1, kp1, act, V, W, h, hacc, len);
     launch_counter() += 1;
 }
 void launch_gm_update(int ld, int S, int m1, int kp1, int a, const int* act, const zf* V, const double* h, zf* W, double* nrm, int nsm,
@@ -1044,99 +1116,119 @@ void launch_eg_combine(int ne, int ldv, int S, int m1, int kp1, int a, const int
 // WHILE node that the Givens kernel clears; the host synchronises once per
 // cycle.  Same arithmetic as the host's rotations (FP64).
 // ---------------------------------------------------------------------------
-// h[i S + s] (+ hacc) += V_{s,i}^H W[:, k] for i <= *jp: items (i, k, chunk)
-// over a fixed grid, partial dots over chunks of `chunk` elements
-__global__ void __launch_bounds__(MB) gm_dots_dev_kernel(int ld, int S, int m1, int a, const int* act, const int* jp, const zf* V, const zf* W,
+// h[i S + s] (+ hacc) += V_{s,i}^H W[:, k] for i <= *jp: items (GM_DI values
+// of i, k, chunk) over a fixed grid, partial dots over chunks of `chunk` elements
+__global__ void __launch_bounds__(GM_DT) gm_dots_dev_kernel(int ld, int S, int m1, int a, const int* act, const int* jp, const zf* V, const zf* W,
                                                         double* h, double* hacc, const int* len, int chunk)
 {
-    const int kp1 = *jp + 1;
+    const int kp1 = *jp + 1, ng = (kp1 + GM_DI - 1) / GM_DI;
     const int nch = (ld + chunk - 1) / chunk;
-    const long long nitem = (long long)kp1 * a * nch;
+    const long long nitem = (long long)ng * a * nch;
     for (long long it = blockIdx.x; it < nitem; it += gridDim.x) {
         const int ch = (int)(it % nch);
         const int k = (int)((it / nch) % a);
-        const int i = (int)(it / ((long long)nch * a));
+        const int i0 = (int)(it / ((long long)nch * a)) * GM_DI;
         const int s = act[k];
-        const int ne = len ? len[s] : ld;
-        const zf* v = V + ((size_t)s * m1 + i) * ld;
-        const zf* w = W + (size_t)k * ld;
-        double acc[2] = {0.0, 0.0};
-        const int e1 = min(ne, (ch + 1) * chunk);
-        for (int e = ch * chunk + threadIdx.x; e < e1; e += MB) {
-            const cpx<double> x = upd_(v[e]), y = upd_(w[e]);
-            acc[0] += x.x * y.x + x.y * y.y;
-            acc[1] += x.x * y.y - x.y * y.x;
-        }
-        double out[2];
-        mblock_store<2>(acc, out);
-        if (threadIdx.x == 0) {
-            const size_t o = 2 * ((size_t)i * S + s);
-            atomicAdd(&h[o], out[0]);
-            atomicAdd(&h[o + 1], out[1]);
-            if (hacc) {
-                atomicAdd(&hacc[o], out[0]);
-                atomicAdd(&hacc[o + 1], out[1]);
-            }
-        }
-        __syncthreads();   // mblock_store's shared slots are reused by the next item
+        gm_dots_part(ch * chunk + threadIdx.x, min(len ? len[s] : ld, (ch + 1) * chunk), GM_DT, min(GM_DI, kp1 - i0),
+                     V + ((size_t)s * m1 + i0) * ld, ld, W + (size_t)k * ld, i0, S, s, h, hacc);
+        __syncthreads();   // the shared slots are reused by the next item
     }
 }
 
-// One block: the Givens step of every alive system (thread k for system
-// act[k]), as the host does it: the Hessenberg column of step j (h1) and
-// the norm of the new vector (h0[s]), the earlier rotations, the new one,
-// the least-squares right-hand side g; a system stops when its residual
+// One block: the Givens step of every alive system, as the host does it: the
+// Hessenberg column of step j (h1) and the norm of the new vector (h0[s]), the
+// earlier rotations, the new one, the least-squares right-hand side g; a system
+// stops when its residual
 // estimate |g_{j+1}|^2 falls below target[s] or its Krylov space is
 // invariant (status 2 when the column is zero).  Thread 0 then advances j and
 // sets the cycle's WHILE condition: some system alive and j < jmax.
+// Up to eight systems have a warp each: its lanes bring the column and the
+// earlier rotations to shared memory, one lane runs the chain there (two
+// systems, 20 rotations: 6.6 us against 12.6 with the chain in global
+// memory).  More systems, or longer cycles, have a thread each, side by side
+// (96 systems: 8.5 us; by warps in turn 37).
 __global__ void __launch_bounds__(256) gm_givens_kernel(int S, int m, int a, const int* act, const double* h0, const double* h1, GmDevState d,
                                                        cudaGraphConditionalHandle cond)
 {
     __shared__ int cnt;
+    __shared__ double2 sh_col[256 / 32][GV_N], sh_sn[256 / 32][GV_N];
+    __shared__ double sh_cs[256 / 32][GV_N];
     if (threadIdx.x == 0) cnt = 0;
     __syncthreads();
-    const int j = *d.j, m1 = m + 1;
-    for (int k = threadIdx.x; k < a; k += blockDim.x) {
-        const int s = act[k];
-        if (!d.alive[s]) continue;
-        double2* col = d.Rm + ((size_t)s * m + j) * m1;
-        double cn = 0.0;
-        for (int i = 0; i <= j; i++) {
-            const size_t o = 2 * ((size_t)i * S + s);
-            col[i] = make_double2(h1[o], h1[o + 1]);
-            cn += h1[o] * h1[o] + h1[o + 1] * h1[o + 1];
-        }
-        const double hsub = sqrt(fmax(h0[s], 0.0));
-        const double* cs = d.cs + (size_t)s * m;
-        const double2* sn = d.sn + (size_t)s * m;
-        for (int i = 0; i < j; i++) {   // the earlier rotations
+    const int j = *d.j, m1 = m + 1, lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    // the earlier rotations; the rotated diagonal entry is returned
+    auto chain = [&](double2* col, const double* cs, const double2* sn) {
+        double2 a0 = col[0];
+#pragma unroll 4
+        for (int i = 0; i < j; i++) {
             const double ci = cs[i];
-            const double2 si = sn[i], a0 = col[i], a1 = col[i + 1];
+            const double2 si = sn[i], a1 = col[i + 1];
             // t = ci a0 + si a1; a1' = -conj(si) a0 + ci a1
-            const double2 t = make_double2(ci * a0.x + si.x * a1.x - si.y * a1.y, ci * a0.y + si.x * a1.y + si.y * a1.x);
-            col[i + 1] = make_double2(-(si.x * a0.x + si.y * a0.y) + ci * a1.x, -(si.x * a0.y - si.y * a0.x) + ci * a1.y);
-            col[i] = t;
+            col[i] = make_double2(ci * a0.x + si.x * a1.x - si.y * a1.y, ci * a0.y + si.x * a1.y + si.y * a1.x);
+            a0 = make_double2(-(si.x * a0.x + si.y * a0.y) + ci * a1.x, -(si.x * a0.y - si.y * a0.x) + ci * a1.y);
         }
-        const double aa = hypot(col[j].x, col[j].y), rho = sqrt(aa * aa + hsub * hsub);
+        return a0;
+    };
+    // the new rotation of system s, cn the squared norm of its column
+    auto finish = [&](int s, double2* col, double2 aj, double cn) {
+        const double hsub = sqrt(fmax(h0[s], 0.0));
+        const double aa = hypot(aj.x, aj.y), rho = sqrt(aa * aa + hsub * hsub);
+        col[j] = aj;
         if (rho == 0.0) {   // A v_j = 0: the operator is singular
             d.status[s] = 2;
             d.alive[s] = 0;
-            continue;
+            return;
         }
-        const double2 ph = aa > 0.0 ? make_double2(col[j].x / aa, col[j].y / aa) : make_double2(1.0, 0.0);
+        const double2 ph = aa > 0.0 ? make_double2(aj.x / aa, aj.y / aa) : make_double2(1.0, 0.0);
         const double cj = aa / rho;
         const double2 sj = make_double2(ph.x * hsub / rho, ph.y * hsub / rho);
         d.cs[(size_t)s * m + j] = cj;
         d.sn[(size_t)s * m + j] = sj;
         col[j] = make_double2(ph.x * rho, ph.y * rho);
         double2* g = d.g + (size_t)s * m1;
-        const double2 gj = g[j];
-        g[j + 1] = make_double2(-(sj.x * gj.x + sj.y * gj.y), -(sj.x * gj.y - sj.y * gj.x));   // -conj(sj) gj
+        const double2 gj = g[j], gn = make_double2(-(sj.x * gj.x + sj.y * gj.y), -(sj.x * gj.y - sj.y * gj.x));   // -conj(sj) gj
+        g[j + 1] = gn;
         g[j] = make_double2(cj * gj.x, cj * gj.y);
         d.kk[s] = j + 1;
-        const double e2 = g[j + 1].x * g[j + 1].x + g[j + 1].y * g[j + 1].y;
+        const double e2 = gn.x * gn.x + gn.y * gn.y;
         if (e2 >= d.target[s] && hsub > 1.0e-13 * sqrt(cn + hsub * hsub)) atomicAdd(&cnt, 1);
         else d.alive[s] = 0;
+    };
+    if (a <= 256 / 32 && j < GV_N) {
+        const int s = wp < a ? act[wp] : -1;
+        if (s >= 0 && d.alive[s]) {
+            double2* gcol = d.Rm + ((size_t)s * m + j) * m1;
+            double cn = 0.0;
+            for (int i = lane; i <= j; i += 32) {
+                const size_t o = 2 * ((size_t)i * S + s);
+                sh_col[wp][i] = make_double2(h1[o], h1[o + 1]);
+                cn += h1[o] * h1[o] + h1[o + 1] * h1[o + 1];
+                if (i < j) {
+                    sh_cs[wp][i] = d.cs[(size_t)s * m + i];
+                    sh_sn[wp][i] = d.sn[(size_t)s * m + i];
+                }
+            }
+            for (int x = 16; x > 0; x >>= 1) cn += __shfl_xor_sync(0xffffffffu, cn, x);
+            __syncwarp();
+            double2 aj = make_double2(0.0, 0.0);
+            if (lane == 0) aj = chain(sh_col[wp], sh_cs[wp], sh_sn[wp]);
+            __syncwarp();
+            for (int i = lane; i < j; i += 32) gcol[i] = sh_col[wp][i];
+            if (lane == 0) finish(s, gcol, aj, cn);
+        }
+    } else {
+        for (int k = threadIdx.x; k < a; k += blockDim.x) {
+            const int s = act[k];
+            if (!d.alive[s]) continue;
+            double2* col = d.Rm + ((size_t)s * m + j) * m1;
+            double cn = 0.0;
+            for (int i = 0; i <= j; i++) {
+                const size_t o = 2 * ((size_t)i * S + s);
+                col[i] = make_double2(h1[o], h1[o + 1]);
+                cn += h1[o] * h1[o] + h1[o + 1] * h1[o + 1];
+            }
+            finish(s, col, chain(col, d.cs + (size_t)s * m, d.sn + (size_t)s * m), cn);
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -1145,30 +1237,56 @@ __global__ void __launch_bounds__(256) gm_givens_kernel(int S, int m, int a, con
     }
 }
 
-// The cycle's least-squares solutions R y = g (back substitution per system,
-// thread k for system act[k]) into y[i S + s] (complex as 2 doubles, zero past
-// kk[s]; y zeroed by the caller), and *kmax = the largest kk.
+// The cycle's least-squares solutions R y = g (back substitution, a warp for
+// system act[k]) into y[i S + s] (complex as 2 doubles, zero past kk[s]; y
+// zeroed by the caller), and *kmax = the largest kk.  Column by column: lane
+// i mod 32 holds the right-hand side of row i, the column's loads are
+// contiguous and do not wait for the solution (one thread row by row took
+// 102 us at 30 steps).
 __global__ void __launch_bounds__(256) gm_backsolve_kernel(int S, int m, int a, const int* act, GmDevState d, double* y, int* kmax)
 {
-    const int m1 = m + 1;
-    for (int k = threadIdx.x + blockIdx.x * blockDim.x; k < a; k += blockDim.x * gridDim.x) {
-        const int s = act[k], ks = d.kk[s];
-        atomicMax(kmax, ks);
-        const double2* R = d.Rm + (size_t)s * m * m1;   // column l at R + l m1
-        const double2* g = d.g + (size_t)s * m1;
-        for (int i = ks - 1; i >= 0; i--) {
-            double2 t = g[i];
-            for (int l = i + 1; l < ks; l++) {
-                const double2 r = R[(size_t)l * m1 + i];
-                const double yx = y[2 * ((size_t)l * S + s)], yy = y[2 * ((size_t)l * S + s) + 1];
-                t.x -= r.x * yx - r.y * yy;
-                t.y -= r.x * yy + r.y * yx;
+    const int m1 = m + 1, lane = threadIdx.x & 31;
+    const int k = (int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (k >= a) return;
+    const int s = act[k], ks = d.kk[s];
+    if (lane == 0) atomicMax(kmax, ks);
+    const double2* R = d.Rm + (size_t)s * m * m1;   // column l at R + l m1
+    const double2* g = d.g + (size_t)s * m1;
+    // rows in blocks of GV_N, the last block first; the columns of later blocks
+    // are subtracted before a block's own
+    for (int r0 = (ks - 1) / GV_N * GV_N; r0 >= 0; r0 -= GV_N) {
+        const int nr = min(ks - r0, GV_N);
+        double2 t[GV_N / 32];
+#pragma unroll
+        for (int q = 0; q < GV_N / 32; q++) t[q] = lane + 32 * q < nr ? g[r0 + lane + 32 * q] : make_double2(0.0, 0.0);
+        auto subtract = [&](const double2* col, int n, double2 v) {   // rows r0 .. r0 + n - 1 of a column
+#pragma unroll
+            for (int q = 0; q < GV_N / 32; q++)
+                if (lane + 32 * q < n) {
+                    const double2 r = col[r0 + lane + 32 * q];
+                    t[q].x -= r.x * v.x - r.y * v.y;
+                    t[q].y -= r.x * v.y + r.y * v.x;
+                }
+        };
+        for (int l = ks - 1; l >= r0 + nr; l--)
+            subtract(R + (size_t)l * m1, nr, make_double2(y[2 * ((size_t)l * S + s)], y[2 * ((size_t)l * S + s) + 1]));
+#pragma unroll
+        for (int q = GV_N / 32 - 1; q >= 0; q--)
+#pragma unroll 2
+            for (int r = 31; r >= 0; r--) {
+                const int i = 32 * q + r;
+                if (i >= nr) continue;
+                const double2 d0 = R[(size_t)(r0 + i) * m1 + r0 + i];
+                const double den = d0.x * d0.x + d0.y * d0.y;
+                const double tx = __shfl_sync(0xffffffffu, t[q].x, r), ty = __shfl_sync(0xffffffffu, t[q].y, r);
+                const double2 v = make_double2((tx * d0.x + ty * d0.y) / den, (ty * d0.x - tx * d0.y) / den);
+                if (lane == 0) {
+                    y[2 * ((size_t)(r0 + i) * S + s)] = v.x;
+                    y[2 * ((size_t)(r0 + i) * S + s) + 1] = v.y;
+                }
+                subtract(R + (size_t)(r0 + i) * m1, i, v);
             }
-            const double2 d0 = R[(size_t)i * m1 + i];
-            const double den = d0.x * d0.x + d0.y * d0.y;
-            y[2 * ((size_t)i * S + s)] = (t.x * d0.x + t.y * d0.y) / den;
-            y[2 * ((size_t)i * S + s) + 1] = (t.y * d0.x - t.x * d0.y) / den;
-        }
+        __syncwarp();
     }
 }
 
@@ -1187,7 +1305,7 @@ void launch_eg_gather_dev(int ne, int ldv, int m1, int a, const int* act, const 
 void launch_gm_dots_dev(int ld, int S, int m1, int a, const int* act, const int* jp, const zf* V, const zf* W, double* h, double* hacc,
                         int nsm, cudaStream_t st, const int* len)
 {
-    gm_dots_dev_kernel<<<4 * nsm, MB, 0, st>>>(ld, S, m1, a, act, jp, V, W, h, hacc, len, 8192);
+    gm_dots_dev_kernel<<<8 * nsm, GM_DT, 0, st>>>(ld, S, m1, a, act, jp, V, W, h, hacc, len, GM_CHUNK);
     launch_counter() += 1;
 }
 void launch_gm_update_dev(int ld, int S, int m1, int a, const int* act, const int* jp, const zf* V, const double* h, zf* W, double* nrm,
@@ -1210,7 +1328,7 @@ void launch_gm_givens(int S, int m, int a, const int* act, const double* h0, con
 }
 void launch_gm_backsolve(int S, int m, int a, const int* act, const GmDevState& d, double* y, int* kmax, cudaStream_t st)
 {
-    gm_backsolve_kernel<<<(a + 255) / 256, 256, 0, st>>>(S, m, a, act, d, y, kmax);
+    gm_backsolve_kernel<<<(a + 7) / 8, 256, 0, st>>>(S, m, a, act, d, y, kmax);
     launch_counter() += 1;
 }
 void launch_gm_combine_dev(int ld, int S, int m1, int a, const int* act, const zf* V, const double* y, const int* kp1, zd* X, int nsm,
