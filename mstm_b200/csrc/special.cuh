@@ -153,13 +153,13 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
     if (n == 1) lim = 1.0e10 * fabs(yb);
     while (m < n || fabs(yb) < lim) {
         const double yn = (double)(2 * m + 1) * rz * yb - ya;
-        if (fabs(yn) > 1.0e140) return false;
         ya = yb;
         yb = yn;
         m++;
         if (m <= n) h[m].y = yb;
         if (m == n) lim = 1.0e10 * fabs(yb);
     }
+    if (!(fabs(yb) <= 1.0e140)) return false;
     double fa = 0.0, fb = 1.0e-150;   // orders m+1, m
     for (int k = m; k >= 1; k--) {
         if (k <= n) h[k].x = fb;
