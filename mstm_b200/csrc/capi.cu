@@ -643,6 +643,18 @@ int setup_layout(mstmg_ctx* c)
     mstmg::Tables tb(6 * lm + 6);
     std::vector<double> vcc, f1, f2, f3;
     tb.axial_constants(lm, vcc, f1, f2, f3);
+    // by term of the sums for the generator's lanes: [k][m][n][l], w = |n - l| + k
+    {
+        std::vector<double> by((size_t)(2 * lm + 1) * (lm + 1) * lm * lm, 0.0);
+        for (int k = 0; k <= 2 * lm; k++)
+            for (int m = 0; m <= lm; m++)
+                for (int n = std::max(1, m); n <= lm; n++)
+                    for (int l = std::max(1, m); l <= lm; l++)
+                        if (k <= 2 * std::min(n, l))
+                            by[(((size_t)k * (lm + 1) + m) * lm + n - 1) * lm + l - 1] =
+                                vcc[(size_t)(n - 1) + (size_t)lm * ((size_t)(l * (l + 1) + m - 1) + (size_t)lm * (lm + 2) * (std::abs(n - l) + k))];
+        vcc.swap(by);
+    }
     c->vn = lm;
     std::vector<double> bd(lm + 2, 0.0);
     for (int k = 0; k <= lm + 1; k++) bd[k] = tb.bc(k, k);

@@ -9,7 +9,7 @@ struct OpGenArgs {
     const int* order;        // N
     const long long* opoff;  // per pair, in storage units
     double* op64;
-    const double* vcc;       // vcc_const(vn, vn(vn+2), 0:2vn)
+    const double* vcc;       // vcc_const by term: [k][m >= 0][n][l], w = |n - l| + k, (2 vn + 1)(vn + 1) vn vn values
     int vnmax;
     const double* fnr;       // fnr[k] = sqrt(k)
     const double* rfnr;      // 1 / sqrt(k) (k >= 1)

@@ -21,7 +21,7 @@
 // the Riccati-Hankel functions xi_w / z (serial in w) one thread per pair,
 // into a scratch of 2 LMAX + 1 complex per pair; the Wigner-d rows (serial in
 // the degree and the restricted index, parallel over the other index) one
-// warp per pair; the axial blocks one CTA per pair, a thread per (m, n, l).
+// warp per pair; the axial blocks one CTA per AX_P pairs, a thread per (m, n, l).
 // Record layout (doubles; R rotation values, oplayout.cuh):
 //   [0, H)           e^{i m phi}, then e^{-i m phi}, m = 0 .. nmax (H = 4 nmax + 4)
 //   [H, H+R)         E_1, O_1, E_2, O_2, ...   (row-major, restricted index first;
@@ -208,54 +208,95 @@ __global__ void __launch_bounds__(128) opgen_rot_kernel(OpGenArgs a)
     }
 }
 
-// axial translation blocks (itype 3, outgoing; itype 1, regular, with the
-// Bessel functions in the scratch), one CTA per pair: the
-// pair's xi_w / z staged in shared memory, thread t takes the mode-0
-// elements t, t + 128, ... of the concatenated blocks Z_0, Z_1, ...
+// Axial translation blocks (itype 3, outgoing; itype 1, regular, with the
+// Bessel functions in the scratch) of AX_P consecutive pairs per CTA, their
+// xi_w / z side by side in shared memory: thread t takes the mode-0 elements
+// t, t + 128, ... of the concatenated blocks Z_0, Z_1, ..., for all the pairs
+// when their orders agree, else for one after the other.  The table lies by
+// term, degree m, n and l, so that the lanes (consecutive l) read it
+// contiguously and every value serves AX_P pairs; one pair a CTA from a table
+// by w, n fastest, took 1.62 ms for the 124,750 pairs of 500 spheres of order
+// 9 (its records alone, 1.3 GB, take 0.2 ms to write).
+#define AX_P 4
+template <int NP> __device__ __forceinline__ void axial_blocks(const OpGenArgs& a, int nt, int ns, double* const* rec, const zd (*xs)[AX_P], int p0)
+{
+    const int nmin = nt < ns ? nt : ns, nmax = nt > ns ? nt : ns, vn = a.vnmax;
+    const int zbase = op_z_base(nmax, nmin);
+    const size_t ks = (size_t)(vn + 1) * vn * vn;   // one term of the sums further
+    // walk the blocks forward: block m holds rc(m) elements, mode-1 copies
+    // after the mode-0 ones for m > 0 (op_z_offset)
+    int m = 0, e = threadIdx.x, zoff = 0;
+    while (m <= nmin) {
+        const int m1 = m < 1 ? 1 : m;
+        const int cols = ns - m1 + 1, rc = (nt - m1 + 1) * cols;
+        if (e >= rc) {
+            e -= rc;
+            zoff += (m == 0 ? 1 : 2) * rc;
+            m++;
+            continue;
+        }
+        const int qn = (int)(((float)e + 0.5f) * (1.0f / (float)cols));   // e / cols (e < 2^10)
+        const int n = m1 + qn, l = m1 + e - qn * cols;
+        const int wmin = n > l ? n - l : l - n, nw = n < l ? n : l;   // terms w = wmin, wmin + 1, ..., wmin + 2 nw
+        const double* vc = a.vcc + ((size_t)m * vn + (n - 1)) * vn + (l - 1);
+        const zd(*x)[AX_P] = xs + wmin;
+        zd s1[NP], s2[NP];
+        {
+            const double v = *vc;
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                s1[p] = v * x[0][p0 + p];
+                s2[p] = mk(0.0, 0.0);
+            }
+        }
+#pragma unroll 2
+        for (int k = 0; k < nw; k++) {
+            const double v2 = vc[ks * (2 * k + 1)], v1 = vc[ks * (2 * k + 2)];
+#pragma unroll
+            for (int p = 0; p < NP; p++) {
+                s2[p] = s2[p] + v2 * x[2 * k + 1][p0 + p];
+                s1[p] = s1[p] + v1 * x[2 * k + 2][p0 + p];
+            }
+        }
+        const int zo = zbase + 2 * (zoff + e);
+#pragma unroll
+        for (int p = 0; p < NP; p++) {
+            const zd t = imul(s2[p]), v0 = s1[p] + t, v1 = s1[p] - t;
+            double* r = rec[p0 + p];
+            *reinterpret_cast<double2*>(r + zo) = make_double2(v0.x, v0.y);   // an even offset of a record aligned to 32 bytes
+            if (m > 0) *reinterpret_cast<double2*>(r + zo + 2 * rc) = make_double2(v1.x, v1.y);
+        }
+        e += blockDim.x;
+    }
+}
+
 __global__ void __launch_bounds__(128) opgen_axial_kernel(OpGenArgs a)
 {
-    __shared__ zd xs[XIW];
-    const int vn = a.vnmax;
-    for (int q = blockIdx.x; q < a.npairs; q += gridDim.x) {
-        const PairGeom g = pair_geom(a, q);
-        if (!g.ok) continue;   // uniform over the CTA
-        const int nt = g.nt, ns = g.ns, nmin = g.nmin;
-        __syncthreads();   // the previous pair's reads of xs are done
-        for (int k = threadIdx.x; k <= nt + ns; k += blockDim.x) xs[k] = a.xi[(size_t)q * XIW + k];
-        __syncthreads();
-        double* rec64 = a.op64 + a.opoff[q];
-        const int zbase = op_z_base(g.nmax, nmin);
-        // walk the blocks forward: block m holds rc(m) elements, mode-1 copies
-        // after the mode-0 ones for m > 0 (op_z_offset)
-        int m = 0, e = threadIdx.x, zoff = 0;
-        while (m <= nmin) {
-            const int m1 = m < 1 ? 1 : m;
-            const int cols = ns - m1 + 1, rc = (nt - m1 + 1) * cols;
-            if (e >= rc) {
-                e -= rc;
-                zoff += (m == 0 ? 1 : 2) * rc;
-                m++;
-                continue;
-            }
-            const int qn = (int)(((float)e + 0.5f) * (1.0f / (float)cols));   // e / cols (e < 2^10)
-            const int n = m1 + qn, l = m1 + e - qn * cols;
-            const int wmin = n > l ? n - l : l - n, wmax = n + l, ml = l * (l + 1) + m;
-            const double* vc = a.vcc + (size_t)(n - 1) + (size_t)vn * (size_t)(ml - 1);
-            const size_t ws = (size_t)vn * vn * (vn + 2);
-            zd s1 = mk(0.0, 0.0), s2 = mk(0.0, 0.0);
-            for (int w = wmin; w <= wmax; w += 2) s1 = s1 + vc[ws * w] * xs[w];
-            for (int w = wmin + 1; w <= wmax - 1; w += 2) s2 = s2 + vc[ws * w] * xs[w];
-            s2 = imul(s2);
-            const zd v0 = s1 + s2, v1 = s1 - s2;
-            const int zo = zbase + 2 * (zoff + e);
-            rec64[zo] = v0.x;
-            rec64[zo + 1] = v0.y;
-            if (m > 0) {
-                rec64[zo + 2 * rc] = v1.x;
-                rec64[zo + 2 * rc + 1] = v1.y;
-            }
-            e += blockDim.x;
+    __shared__ zd xs[XIW][AX_P];
+    __shared__ int nts[AX_P], nss[AX_P];   // orders; 0 for coincident centres and past the last pair
+    __shared__ double* rec[AX_P];
+    for (int q0 = blockIdx.x * AX_P; q0 < a.npairs; q0 += gridDim.x * AX_P) {
+        __syncthreads();   // the previous pairs' reads are done
+        if (threadIdx.x < AX_P) {
+            const int q = q0 + threadIdx.x;
+            const bool in = q < a.npairs;
+            const PairGeom g = pair_geom(a, in ? q : q0);
+            nts[threadIdx.x] = in && g.ok ? g.nt : 0;
+            nss[threadIdx.x] = in && g.ok ? g.ns : 0;
+            rec[threadIdx.x] = a.op64 + a.opoff[in ? q : q0];
         }
+        __syncthreads();
+        bool same = nts[0] > 0;
+        for (int p = 1; p < AX_P; p++) same = same && nts[p] == nts[0] && nss[p] == nss[0];
+        for (int t = threadIdx.x; t < AX_P * XIW; t += blockDim.x) {
+            const int p = t / XIW, k = t % XIW;
+            if (nts[p] > 0 && k <= nts[p] + nss[p]) xs[k][p] = a.xi[(size_t)(q0 + p) * XIW + k];
+        }
+        __syncthreads();
+        if (same) axial_blocks<AX_P>(a, nts[0], nss[0], rec, xs, 0);
+        else
+            for (int p = 0; p < AX_P; p++)
+                if (nts[p] > 0) axial_blocks<1>(a, nts[p], nss[p], rec, xs, p);
     }
 }
 
@@ -277,7 +318,7 @@ void launch_opgen(const OpGenArgs& a, int nsm, cudaStream_t st)
     int b2 = (a.npairs + warps - 1) / warps;
     if (b2 > nsm * 16) b2 = nsm * 16;
     opgen_rot_kernel<<<b2, warps * 32, smem, st>>>(a);
-    int b3 = a.npairs < nsm * 16 ? a.npairs : nsm * 16;
+    const int ng = (a.npairs + AX_P - 1) / AX_P, b3 = ng < nsm * 16 ? ng : nsm * 16;
     opgen_axial_kernel<<<b3, 128, 0, st>>>(a);
     launch_counter() += 3;
 }
