@@ -414,7 +414,7 @@ static int fixed_orientation_impl(mstmg_ctx* c, double alpha, double sinc, int d
         zd* xs[2] = {c->amnp.p, c->amnp.p + ne};
         zd* bs[2] = {bvec, bvec + ne};
         if (xinit != c->amnp.p)
-            for (int p = 0; p < 2; p++) CK(cudaMemcpyAsync(xs[p], bs[p], sizeof(zd) * ne, cudaMemcpyDeviceToDevice, c->st));
+            CK(cudaMemcpyAsync(xs[0], bvec, sizeof(zd) * 2 * (size_t)ne, cudaMemcpyDeviceToDevice, c->st));
         if (c->opts.mixed_solver == 1) {
             rc = solve_mixed(c, bs, xs, eps, niter, it, er, st);
         } else if (c->opts.mixed_solver == 2) {
@@ -991,36 +991,43 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
         c->passes32 += nstep * dev_passes_per_step;
         dev_act.clear();
     };
+    // the systems in gw.act.p on the device; copied again only when they change
+    std::vector<int> on_dev;
+    auto put_act = [&](const std::vector<int>& v) -> cudaError_t {
+        if (v == on_dev) return cudaSuccess;
+        on_dev = v;
+        return cudaMemcpyAsync(gw.act.p, v.data(), sizeof(int) * v.size(), cudaMemcpyHostToDevice, c->st);
+    };
     for (int cyc = 0; cyc <= c->opts.max_outer && !act.empty(); cyc++) {
         // FP64 true residuals of the cycle's systems into R (FP32, by system,
         // or the two columns of an ensemble)
         int a = (int)act.size();
+        CK(put_act(act));
         if (seg) {
-            CK(cudaMemcpyAsync(gw.act.p, act.data(), sizeof(int) * a, cudaMemcpyHostToDevice, c->st));
             if ((rc = translate_many<double>(c, X, c->Y64.p, 2, 0u))) return rc;
             CK(cudaMemsetAsync(gw.rr.p, 0, sizeof(double) * 2 * S, c->st));
             launch_eg_resid(sm, c->an.p, ne, ldv, a, gw.act.p, seg->off, seg->len, B, X, c->Y64.p, gw.R.p, gw.rr.p, c->nsm, c->st);
         } else {
             const int apad = a == 1 ? 1 : ((a + 1) / 2) * 2;
-            CK(cudaMemcpyAsync(w64.act.p, act.data(), sizeof(int) * a, cudaMemcpyHostToDevice, c->st));
             if (x_zero && cyc == 0) {
                 // H 0 = 0: the residual is B
                 CK(cudaMemsetAsync(w64.YP.p, 0, sizeof(zd) * (size_t)ne * apad, c->st));
             } else {
-                launch_m_gather<double>(ne, a, apad, w64.act.p, X, w64.XP.p, c->nsm, c->st);
+                launch_m_gather<double>(ne, a, apad, gw.act.p, X, w64.XP.p, c->nsm, c->st);
                 if ((rc = translate_many<double>(c, w64.XP.p, w64.YP.p, apad, 0u))) return rc;
             }
             if (c->hs.on()) {
                 // host spheres: the Mie multiply apart, the residual kernel takes M H x
                 for (int k = 0; k < a; k++) mie_all<double>(c, 1, 0, w64.YP.p + (size_t)k * ne, w64.YP.p + (size_t)k * ne);
-                launch_m_resid<float>(sm, nullptr, ne, a, w64.act.p, B, X, w64.YP.p, gw.R.p, w64.part.p, gw.rr.p, c->nsm, c->st, 1);
+                launch_m_resid<float>(sm, nullptr, ne, a, gw.act.p, B, X, w64.YP.p, gw.R.p, w64.part.p, gw.rr.p, c->nsm, c->st, 1);
             } else {
-                launch_m_resid<float>(sm, c->an.p, ne, a, w64.act.p, B, X, w64.YP.p, gw.R.p, w64.part.p, gw.rr.p, c->nsm, c->st, 1);
+                launch_m_resid<float>(sm, c->an.p, ne, a, gw.act.p, B, X, w64.YP.p, gw.R.p, w64.part.p, gw.rr.p, c->nsm, c->st, 1);
             }
         }
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(hrr.data(), gw.rr.p, sizeof(double) * 2 * S, cudaMemcpyDeviceToHost, c->st));
+        CK(cudaMemcpyAsync(gw.hback, gw.rr.p, sizeof(double) * gw.back_doubles(), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
+        hrr.assign(gw.hback, gw.hback + 2 * (size_t)S);
         c->host_syncs++;
         (*outer_count)++;
         fold_device_cycle();
@@ -1033,10 +1040,6 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
         act = keep;
         a = (int)act.size();
         if (a == 0 || cyc == c->opts.max_outer) break;
-        CK(cudaMemcpyAsync(gw.act.p, act.data(), sizeof(int) * a, cudaMemcpyHostToDevice, c->st));
-        // v_0 = r / |r|
-        if (seg) launch_eg_start(ne, ldv, m1, a, gw.act.p, seg->off, seg->len, gw.R.p, gw.rr.p, 1.0e-35, gw.V.p, c->nsm, c->st);
-        else launch_gm_scale(ne, m1, 0, a, gw.act.p, 1, gw.R.p, gw.rr.p, 2, 1.0e-35, gw.V.p, c->nsm, c->st);
         long long room = cap;
         for (int s : act) {
             const double beta2 = hrr[2 * s];
@@ -1049,26 +1052,34 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
         }
         cur = act;
         const int jmax = (int)std::min<long long>(m, room);
-        if (graphs && jmax > 0) {
+        const bool device_cycle = graphs && jmax > 0;
+        if (device_cycle) {
+            // one copy starts the cycle: targets, |r|, the active systems, jmax
+            std::fill(gw.hout, gw.hout + gw.out_doubles(), 0.0);
+            int* oi = gw.out_ints();
+            for (int k = 0; k < a; k++) {
+                const int s = act[k];
+                gw.hout[s] = gw.target[s];
+                gw.hout[S + s] = std::sqrt(hrr[2 * s]);
+                oi[k] = s;
+                oi[S + s] = 1;
+            }
+            oi[2 * S] = jmax;
+            CK(cudaMemcpyAsync(gw.dtarget.p, gw.hout, sizeof(double) * gw.out_doubles(), cudaMemcpyHostToDevice, c->st));
+            on_dev = act;
+            launch_gm_cycle_start(S, m1, gw.dbeta.p, gw.dev(), c->st);
+        } else {
+            CK(put_act(act));
+        }
+        // v_0 = r / |r|
+        if (seg) launch_eg_start(ne, ldv, m1, a, gw.act.p, seg->off, seg->len, gw.R.p, gw.rr.p, 1.0e-35, gw.V.p, c->nsm, c->st);
+        else launch_gm_scale(ne, m1, 0, a, gw.act.p, 1, gw.R.p, gw.rr.p, 2, 1.0e-35, gw.V.p, c->nsm, c->st);
+        if (device_cycle) {
             // the whole cycle on the device: one graph launch, its Arnoldi
             // step repeated under a conditional WHILE node until every system
             // has left or jmax steps are done; then the least-squares
             // solutions and the corrections, with no synchronisation
             const int na = a;
-            std::vector<int> alive(S, 0);
-            std::vector<double2> g0((size_t)S * m1, make_double2(0.0, 0.0));
-            for (int s : act) {
-                alive[s] = 1;
-                g0[(size_t)s * m1] = make_double2(std::sqrt(hrr[2 * s]), 0.0);
-            }
-            const int zero = 0;
-            CK(cudaMemcpyAsync(gw.dalive.p, alive.data(), sizeof(int) * S, cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(gw.dg.p, g0.data(), sizeof(double2) * g0.size(), cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(gw.dtarget.p, gw.target.data(), sizeof(double) * S, cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(gw.dj.p, &zero, sizeof(int), cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemcpyAsync(gw.djmax.p, &jmax, sizeof(int), cudaMemcpyHostToDevice, c->st));
-            CK(cudaMemsetAsync(gw.dkk.p, 0, sizeof(int) * S, c->st));
-            CK(cudaMemsetAsync(gw.dstatus.p, 0, sizeof(int) * S, c->st));
             auto it = gw.cycles.find(na);
             if (it == gw.cycles.end()) {
                 cudaGraph_t gr = nullptr, body = nullptr;
@@ -1138,20 +1149,14 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
                 dev_passes_per_step = it->second.passes32_per_step;
                 // least-squares solutions on the device, summed into X
                 GmDevState d = gw.dev();
-                CK(cudaMemsetAsync(h2, 0, sizeof(double) * HP, c->st));
-                CK(cudaMemsetAsync(gw.dkmax.p, 0, sizeof(int), c->st));
                 launch_gm_backsolve(S, m, na, gw.act.p, d, h2, gw.dkmax.p, c->st);
                 if (seg) launch_eg_combine_dev(ne, ldv, S, m1, na, gw.act.p, seg->off, seg->len, gw.V.p, h2, gw.dkmax.p, X, c->nsm, c->st);
                 else launch_gm_combine_dev(ne, S, m1, na, gw.act.p, gw.V.p, h2, gw.dkmax.p, X, c->nsm, c->st);
                 CK(cudaGetLastError());
-                CK(cudaMemcpyAsync(gw.hkk, gw.dkk.p, sizeof(int) * S, cudaMemcpyDeviceToHost, c->st));
-                CK(cudaMemcpyAsync(gw.hkk + S, gw.dstatus.p, sizeof(int) * S, cudaMemcpyDeviceToHost, c->st));
-                CK(cudaMemcpyAsync(gw.hkk + 2 * S, gw.dj.p, sizeof(int), cudaMemcpyDeviceToHost, c->st));
-                dev_act = act;
+                dev_act = act;   // its counts come home with the next residuals
                 continue;
             }
             // capture failed: the host-driven steps below
-            CK(cudaMemcpyAsync(gw.act.p, act.data(), sizeof(int) * a, cudaMemcpyHostToDevice, c->st));
         }
         for (int j = 0; j < jmax && !cur.empty(); j++) {
             const int na = (int)cur.size();
@@ -1256,7 +1261,7 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
             }
             if (next.size() != cur.size()) {
                 cur = next;
-                if (!cur.empty()) CK(cudaMemcpyAsync(gw.act.p, cur.data(), sizeof(int) * cur.size(), cudaMemcpyHostToDevice, c->st));
+                if (!cur.empty()) CK(put_act(cur));
             }
         }
         // least-squares solutions (zero-padded to the longest), summed into X
@@ -1277,7 +1282,7 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
                 }
                 steps[s] += ks;
             }
-            CK(cudaMemcpyAsync(gw.act.p, act.data(), sizeof(int) * a, cudaMemcpyHostToDevice, c->st));
+            CK(put_act(act));
             CK(cudaMemcpyAsync(h2, gw.ybuf.data(), sizeof(double) * 2 * (size_t)kmax * S, cudaMemcpyHostToDevice, c->st));
             if (seg) launch_eg_combine(ne, ldv, S, m1, kmax, a, gw.act.p, seg->off, seg->len, gw.V.p, h2, X, c->nsm, c->st);
             else launch_gm_combine(ne, S, m1, kmax, a, gw.act.p, gw.V.p, h2, X, c->nsm, c->st);
@@ -1285,6 +1290,7 @@ int solve_multi_gmres(mstmg_ctx* c, MultiWork<double>& w64, GmresWork& gw, int S
         }
     }
     if (!dev_act.empty()) {
+        CK(cudaMemcpyAsync(gw.hback, gw.rr.p, sizeof(double) * gw.back_doubles(), cudaMemcpyDeviceToHost, c->st));
         CK(cudaStreamSynchronize(c->st));
         c->host_syncs++;
         fold_device_cycle();

@@ -245,9 +245,23 @@ struct GmresWork {
     int S = 0, m = 0, ne = 0;
     DevBuf<zf> V, W, XP, Y, R;
     // h: S squared norms (padded to even), then two Gram-Schmidt passes of (m + 1) S complex
-    DevBuf<double> h, rr;
-    DevBuf<int> act;
+    DevBuf<double> h;
     double* hh = nullptr;   // pinned host copy of the norms and the first pass
+    // Small state, in two blocks that each travel in one copy: back, the
+    // residuals of a cycle's start (rr) with the counts of the device-driven
+    // cycle before it; out, what starts a device-driven cycle.  hback and
+    // hout are the pinned copies.  (As separate pageable copies and memsets
+    // they were 22 calls a solve of two cycles.)
+    template <typename T> struct At {
+        T* p = nullptr;
+    };
+    DevBuf<double> small;
+    At<double> rr, dtarget, dbeta;
+    At<int> act, dj, djmax, dalive, dkk, dstatus, dkmax;
+    double *hback = nullptr, *hout = nullptr;
+    size_t back_doubles() const { return 2 * (size_t)S + (size_t)S + 1; }          // rr; kk, status, j
+    size_t out_doubles() const { return 2 * (size_t)S + (size_t)S + 1; }           // target, beta; act, alive, jmax, kmax
+    int* out_ints() const { return reinterpret_cast<int*>(hout + 2 * (size_t)S); }
     std::vector<std::complex<double>> Rm, g, sn;   // per system: rotated Hessenberg (m x (m + 1)), rhs, rotations
     std::vector<double> cs, target, ybuf;
     std::vector<int> kk;
@@ -265,10 +279,9 @@ struct GmresWork {
     // Arnoldi cycles driven on the device (two-column solves): the state of
     // the rotations in device memory and one graph per active-system count,
     // the step under a conditional WHILE node (mrhs.cu, gm_givens_kernel)
-    DevBuf<int> dj, djmax, dalive, dkk, dstatus, dkmax;
-    DevBuf<double> dtarget, dcs;
+    DevBuf<double> dcs;
     DevBuf<double2> dsn, dg, dRm;
-    int* hkk = nullptr;   // pinned: kk, status of every system and the steps of the last device cycle
+    int* hkk = nullptr;   // in hback: kk, status of every system and the steps of the last device cycle
     struct CycleGraph {
         cudaGraphExec_t exec;
         long long launches_per_step;
@@ -290,7 +303,7 @@ struct GmresWork {
     {
         drop_graphs();
         if (hh) cudaFreeHost(hh);
-        if (hkk) cudaFreeHost(hkk);
+        if (hback) cudaFreeHost(hback);
     }
     size_t off1() const { return (size_t)(S + (S & 1)); }
     size_t hpass() const { return (size_t)(m + 1) * S * 2; }
@@ -332,26 +345,30 @@ struct GmresWork {
         CK(Y.alloc((size_t)spad * ne));
         CK(R.alloc((size_t)S * ne));
         CK(h.alloc(off1() + 2 * hpass()));
-        CK(rr.alloc(2 * (size_t)S));
-        CK(act.alloc(S));
+        CK(small.alloc(back_doubles() + out_doubles()));
+        rr.p = small.p;
+        dkk.p = reinterpret_cast<int*>(rr.p + 2 * (size_t)S);
+        dstatus.p = dkk.p + S;
+        dj.p = dstatus.p + S;
+        dtarget.p = small.p + back_doubles();
+        dbeta.p = dtarget.p + S;
+        act.p = reinterpret_cast<int*>(dbeta.p + S);
+        dalive.p = act.p + S;
+        djmax.p = dalive.p + S;
+        dkmax.p = djmax.p + 1;
         if (hh) cudaFreeHost(hh);
         hh = nullptr;
         CK(cudaMallocHost((void**)&hh, sizeof(double) * (off1() + hpass())));
         dRm.release();
-        CK(dj.alloc(1));
-        CK(djmax.alloc(1));
-        CK(dkmax.alloc(1));
-        CK(dalive.alloc(S));
-        CK(dkk.alloc(S));
-        CK(dstatus.alloc(S));
-        CK(dtarget.alloc(S));
         CK(dcs.alloc((size_t)S * m));
         CK(dsn.alloc((size_t)S * m));
         CK(dg.alloc((size_t)S * (m + 1)));
         CK(dRm.alloc((size_t)S * m * (m + 1)));
-        if (hkk) cudaFreeHost(hkk);
-        hkk = nullptr;
-        CK(cudaMallocHost((void**)&hkk, sizeof(int) * (2 * (size_t)S + 1)));
+        if (hback) cudaFreeHost(hback);
+        hback = nullptr;
+        CK(cudaMallocHost((void**)&hback, sizeof(double) * (back_doubles() + out_doubles())));
+        hout = hback + back_doubles();
+        hkk = reinterpret_cast<int*>(hback + 2 * (size_t)S);
         Rm.assign((size_t)S * m * (m + 1), 0.0);
         g.assign((size_t)S * (m + 1), 0.0);
         sn.assign((size_t)S * m, 0.0);

@@ -1238,8 +1238,8 @@ __global__ void __launch_bounds__(256) gm_givens_kernel(int S, int m, int a, con
 }
 
 // The cycle's least-squares solutions R y = g (back substitution, a warp for
-// system act[k]) into y[i S + s] (complex as 2 doubles, zero past kk[s]; y
-// zeroed by the caller), and *kmax = the largest kk.  Column by column: lane
+// system act[k]) into y[i S + s] (complex as 2 doubles, zero from kk[s] to the
+// cycle's last step), and *kmax = the largest kk.  Column by column: lane
 // i mod 32 holds the right-hand side of row i, the column's loads are
 // contiguous and do not wait for the solution (one thread row by row took
 // 102 us at 30 steps).
@@ -1250,6 +1250,10 @@ __global__ void __launch_bounds__(256) gm_backsolve_kernel(int S, int m, int a, 
     if (k >= a) return;
     const int s = act[k], ks = d.kk[s];
     if (lane == 0) atomicMax(kmax, ks);
+    for (int i = ks + lane; i < *d.j; i += 32) {
+        y[2 * ((size_t)i * S + s)] = 0.0;
+        y[2 * ((size_t)i * S + s) + 1] = 0.0;
+    }
     const double2* R = d.Rm + (size_t)s * m * m1;   // column l at R + l m1
     const double2* g = d.g + (size_t)s * m1;
     // rows in blocks of GV_N, the last block first; the columns of later blocks
@@ -1290,6 +1294,22 @@ __global__ void __launch_bounds__(256) gm_backsolve_kernel(int S, int m, int a, 
     }
 }
 
+// Start of a device-driven cycle: no steps, every system's right-hand side
+// |r| e_0 (g_{j+1} is written by step j before it is read).
+__global__ void __launch_bounds__(256) gm_cycle_start_kernel(int S, int m1, const double* beta, GmDevState d)
+{
+    const int s = blockIdx.x * 256 + threadIdx.x;
+    if (s == 0) *d.j = 0;
+    if (s >= S) return;
+    d.kk[s] = 0;
+    d.status[s] = 0;
+    d.g[(size_t)s * m1] = make_double2(beta[s], 0.0);
+}
+void launch_gm_cycle_start(int S, int m1, const double* beta, const GmDevState& d, cudaStream_t st)
+{
+    gm_cycle_start_kernel<<<(S + 255) / 256, 256, 0, st>>>(S, m1, beta, d);
+    launch_counter() += 1;
+}
 void launch_gm_gather_dev(int ld, int m1, int a, int apad, const int* act, const int* jp, const int* alive, const zf* V, zf* XP, int nsm,
                           cudaStream_t st)
 {

@@ -101,6 +101,7 @@ struct GmDevState {
     double2* g;      // per system: m + 1 least-squares right-hand side
     double2* Rm;     // per system: m rotated Hessenberg columns of m + 1
 };
+void launch_gm_cycle_start(int S, int m1, const double* beta, const GmDevState& d, cudaStream_t st);
 void launch_gm_gather_dev(int ld, int m1, int a, int apad, const int* act, const int* jp, const int* alive, const zf* V, zf* XP, int nsm,
                           cudaStream_t st);
 void launch_eg_gather_dev(int ne, int ldv, int m1, int a, const int* act, const int* off, const int* len, const int* jp, const int* alive,
