@@ -215,8 +215,9 @@ __global__ void __launch_bounds__(128) opgen_rot_kernel(OpGenArgs a)
 // when their orders agree, else for one after the other.  The table lies by
 // term, degree m, n and l, so that the lanes (consecutive l) read it
 // contiguously and every value serves AX_P pairs; one pair a CTA from a table
-// by w, n fastest, took 1.62 ms for the 124,750 pairs of 500 spheres of order
-// 9 (its records alone, 1.3 GB, take 0.2 ms to write).
+// by w, n fastest, took 1.62 ms for the 124,750 pairs of 500 spheres of order 9
+// (their 1.3 GB of blocks take 0.2 ms to write) and 0.34 ms for 180,000 of
+// order 3; now 1.04 and 0.10 ms.
 #define AX_P 4
 template <int NP> __device__ __forceinline__ void axial_blocks(const OpGenArgs& a, int nt, int ns, double* const* rec, const zd (*xs)[AX_P], int p0)
 {
@@ -270,16 +271,17 @@ template <int NP> __device__ __forceinline__ void axial_blocks(const OpGenArgs& 
     }
 }
 
-__global__ void __launch_bounds__(128) opgen_axial_kernel(OpGenArgs a)
+// grp: pairs a CTA takes, AX_P or 1
+__global__ void __launch_bounds__(128) opgen_axial_kernel(OpGenArgs a, int grp)
 {
     __shared__ zd xs[XIW][AX_P];
     __shared__ int nts[AX_P], nss[AX_P];   // orders; 0 for coincident centres and past the last pair
     __shared__ double* rec[AX_P];
-    for (int q0 = blockIdx.x * AX_P; q0 < a.npairs; q0 += gridDim.x * AX_P) {
+    for (int q0 = blockIdx.x * grp; q0 < a.npairs; q0 += gridDim.x * grp) {
         __syncthreads();   // the previous pairs' reads are done
         if (threadIdx.x < AX_P) {
             const int q = q0 + threadIdx.x;
-            const bool in = q < a.npairs;
+            const bool in = (int)threadIdx.x < grp && q < a.npairs;
             const PairGeom g = pair_geom(a, in ? q : q0);
             nts[threadIdx.x] = in && g.ok ? g.nt : 0;
             nss[threadIdx.x] = in && g.ok ? g.ns : 0;
@@ -318,7 +320,10 @@ void launch_opgen(const OpGenArgs& a, int nsm, cudaStream_t st)
     int b2 = (a.npairs + warps - 1) / warps;
     if (b2 > nsm * 16) b2 = nsm * 16;
     opgen_rot_kernel<<<b2, warps * 32, smem, st>>>(a);
-    const int ng = (a.npairs + AX_P - 1) / AX_P, b3 = ng < nsm * 16 ? ng : nsm * 16;
-    opgen_axial_kernel<<<b3, 128, 0, st>>>(a);
+    // pairs together once they fill the chip with groups; 780 pairs of order 14
+    // take 76 us in groups and 62 alone, 20,503 of order 9 193 and 290
+    const int grp = a.npairs >= AX_P * 8 * nsm ? AX_P : 1;
+    const int ng = (a.npairs + grp - 1) / grp, b3 = ng < nsm * 16 ? ng : nsm * 16;
+    opgen_axial_kernel<<<b3, 128, 0, st>>>(a, grp);
     launch_counter() += 3;
 }
