@@ -40,12 +40,97 @@ template <int K> __device__ __forceinline__ void block_reduce_store(double (&v)[
 
 template <typename T> __device__ __forceinline__ cpx<double> up(cpx<T> a) { return mk((double)a.x, (double)a.y); }
 
+// Sums of nparts partials of K values over one warp, in a fixed order: lanes
+// over the partials, then a butterfly (one thread reading them in line took
+// 8 us for the 79 partials of 203 spheres).
+template <int K> __device__ __forceinline__ void warp_parts(int nparts, const double* part, double* s)
+{
+#pragma unroll 4
+    for (int b = threadIdx.x; b < nparts; b += 32)
+#pragma unroll
+        for (int k = 0; k < K; k++) s[k] += __ldcg(part + K * b + k);   // another CTA may just have written it
+#pragma unroll
+    for (int k = 0; k < K; k++)
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], x);
+}
+
+// The scalars after a reduction, by one warp:
+// mode 0: after init   (csk = sum cr*cr, enorm = sum |b|^2; stop if csk == 0)
+// mode 1: after post   (cak = sum conj(w) cap; alpha = csk/cak or breakdown)
+// mode 2: after upd1   (csk2, eerr; stop test; beta = csk2/csk; csk = csk2)
+__device__ inline void bicg_finish(int mode, int nparts, const double* part, BicgScalars* sc, double eps, int normalize)
+{
+    double s[3] = {0.0, 0.0, 0.0};
+    if (mode == 1) warp_parts<2>(nparts, part, s);
+    else warp_parts<3>(nparts, part, s);
+    if (threadIdx.x != 0) return;
+    if (mode == 0) {
+        sc->csk[0] = s[0];
+        sc->csk[1] = s[1];
+        sc->enorm = normalize ? s[2] : 1.0;
+        sc->stop = (s[0] == 0.0 && s[1] == 0.0) ? 1 : 0;
+        sc->breakdown = 0;
+        sc->eerr = 0.0;
+        sc->done = 0;
+    } else if (mode == 1) {
+        zd cak = mk(s[0], s[1]);
+        if (cabsd(cak) != 0.0) {
+            zd a = cdiv(mk(sc->csk[0], sc->csk[1]), cak);
+            sc->alpha[0] = a.x;
+            sc->alpha[1] = a.y;
+        } else {
+            sc->breakdown = 1;
+        }
+    } else {
+        if (sc->breakdown) return;
+        double eerr = s[2] / sc->enorm;
+        sc->eerr = eerr;
+        zd csk = mk(sc->csk[0], sc->csk[1]);
+        if (eerr < eps || cabsd(csk) == 0.0) {
+            sc->stop = 1;
+        } else {
+            zd csk2 = mk(s[0], s[1]);
+            zd b = cdiv(csk2, csk);
+            sc->beta[0] = b.x;
+            sc->beta[1] = b.y;
+            sc->csk_prev[0] = csk.x;
+            sc->csk_prev[1] = csk.y;
+            sc->csk[0] = csk2.x;
+            sc->csk[1] = csk2.y;
+        }
+    }
+}
+
+__global__ void fin_kernel(int mode, int nparts, const double* part, BicgScalars* sc, double eps, int normalize)
+{
+    bicg_finish(mode, nparts, part, sc, eps, normalize);
+}
+
+// After a CTA stored its partials: the last one to do so finishes the
+// reduction (a launch for one warp took 3.2 us and the gap before it).
+__device__ __forceinline__ void last_cta_finish(int mode, const double* part, BicgScalars* sc, double eps, int normalize)
+{
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        last = atomicAdd(&sc->done, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (last && threadIdx.x < 32) {
+        __threadfence();
+        if (threadIdx.x == 0) sc->done = 0;
+        bicg_finish(mode, (int)gridDim.x, part, sc, eps, normalize);
+    }
+}
+
 // cap = p - M*y0 (Mie multiply, idir=1), caw = w - conj(y1); partial sum conj(w)*cap.
 // an == null: y0 already holds M*y0 (the host-sphere Mie multiply runs apart)
 template <typename T>
 __global__ void __launch_bounds__(RB) post_kernel(int nslots, const int* slot_sphere, const int* order, const int* offset,
                                                   const int* mie_offset, const cpx<T>* an, const cpx<T>* p, const cpx<T>* w,
-                                                  const cpx<T>* y0, const cpx<T>* y1, cpx<T>* cap, cpx<T>* caw, double* part)
+                                                  const cpx<T>* y0, const cpx<T>* y1, cpx<T>* cap, cpx<T>* caw, double* part,
+                                                  BicgScalars* sc)
 {
     double acc[2] = {0.0, 0.0};
     for (int e = blockIdx.x * RB + threadIdx.x; e < nslots; e += gridDim.x * RB) {
@@ -72,6 +157,7 @@ __global__ void __launch_bounds__(RB) post_kernel(int nslots, const int* slot_sp
         acc[1] += w0.x * d0.y - w0.y * d0.x + w1.x * d1.y - w1.y * d1.x;
     }
     block_reduce_store<2>(acc, part + 2 * blockIdx.x);
+    last_cta_finish(1, part, sc, 0.0, 1);
 }
 
 // Initial residual: cr = b - x + M*y0 ; cq = conj(cr) ; cw = cq ; cp = cr.
@@ -121,8 +207,8 @@ __global__ void __launch_bounds__(RB) init_kernel(int nslots, const int* slot_sp
 
 // x += a p ; r -= a cap ; q -= conj(a) caw ; partials sum conj(q)*r, sum |r|^2
 template <typename T>
-__global__ void __launch_bounds__(RB) upd1_kernel(int n, const BicgScalars* sc, cpx<T>* x, cpx<T>* r, cpx<T>* q, const cpx<T>* p,
-                                                  const cpx<T>* cap, const cpx<T>* caw, double* part)
+__global__ void __launch_bounds__(RB) upd1_kernel(int n, BicgScalars* sc, cpx<T>* x, cpx<T>* r, cpx<T>* q, const cpx<T>* p,
+                                                  const cpx<T>* cap, const cpx<T>* caw, double* part, double eps)
 {
     double acc[3] = {0.0, 0.0, 0.0};
     if (!sc->breakdown) {
@@ -141,6 +227,7 @@ __global__ void __launch_bounds__(RB) upd1_kernel(int n, const BicgScalars* sc, 
         }
     }
     block_reduce_store<3>(acc, part + 3 * blockIdx.x);
+    last_cta_finish(2, part, sc, eps, 1);
 }
 
 // p = r + b p ; w = q + conj(b) w   (skipped once the system stopped)
@@ -156,64 +243,29 @@ __global__ void __launch_bounds__(RB) upd2_kernel(int n, const BicgScalars* sc, 
     }
 }
 
-// Sums of nparts partials of K values over one warp, in a fixed order: lanes
-// over the partials, then a butterfly (one thread reading them in line took
-// 8 us for the 79 partials of 203 spheres).
-template <int K> __device__ __forceinline__ void warp_parts(int nparts, const double* part, double* s)
+// The same, and the next pass's columns with it: x0 = p, x1 = the transposed
+// Mie multiply of conj(w) (mie_kernel with idir -1, conj_in 1): one launch for
+// an update, a copy and a multiply (2.4 + 1.7 + 2.6 us at 203 spheres).
+template <typename T>
+__global__ void __launch_bounds__(RB) upd2_columns_kernel(SlotMaps sm, const cpx<T>* an, const BicgScalars* sc, cpx<T>* p, cpx<T>* w,
+                                                          const cpx<T>* r, const cpx<T>* q, cpx<T>* x0, cpx<T>* x1)
 {
-#pragma unroll 4
-    for (int b = threadIdx.x; b < nparts; b += 32)
-#pragma unroll
-        for (int k = 0; k < K; k++) s[k] += part[K * b + k];
-#pragma unroll
-    for (int k = 0; k < K; k++)
-#pragma unroll
-        for (int x = 16; x > 0; x >>= 1) s[k] += __shfl_xor_sync(0xffffffffu, s[k], x);
-}
-
-// one warp
-// mode 0: after init   (csk = sum cr*cr, enorm = sum |b|^2; stop if csk == 0)
-// mode 1: after post   (cak = sum conj(w) cap; alpha = csk/cak or breakdown)
-// mode 2: after upd1   (csk2, eerr; stop test; beta = csk2/csk; csk = csk2)
-__global__ void fin_kernel(int mode, int nparts, const double* part, BicgScalars* sc, double eps, int normalize)
-{
-    double s[3] = {0.0, 0.0, 0.0};
-    if (mode == 1) warp_parts<2>(nparts, part, s);
-    else warp_parts<3>(nparts, part, s);
-    if (threadIdx.x != 0) return;
-    if (mode == 0) {
-        sc->csk[0] = s[0];
-        sc->csk[1] = s[1];
-        sc->enorm = normalize ? s[2] : 1.0;
-        sc->stop = (s[0] == 0.0 && s[1] == 0.0) ? 1 : 0;
-        sc->breakdown = 0;
-        sc->eerr = 0.0;
-    } else if (mode == 1) {
-        zd cak = mk(s[0], s[1]);
-        if (cabsd(cak) != 0.0) {
-            zd a = cdiv(mk(sc->csk[0], sc->csk[1]), cak);
-            sc->alpha[0] = a.x;
-            sc->alpha[1] = a.y;
-        } else {
-            sc->breakdown = 1;
-        }
-    } else {
-        if (sc->breakdown) return;
-        double eerr = s[2] / sc->enorm;
-        sc->eerr = eerr;
-        zd csk = mk(sc->csk[0], sc->csk[1]);
-        if (eerr < eps || cabsd(csk) == 0.0) {
-            sc->stop = 1;
-        } else {
-            zd csk2 = mk(s[0], s[1]);
-            zd b = cdiv(csk2, csk);
-            sc->beta[0] = b.x;
-            sc->beta[1] = b.y;
-            sc->csk_prev[0] = csk.x;
-            sc->csk_prev[1] = csk.y;
-            sc->csk[0] = csk2.x;
-            sc->csk[1] = csk2.y;
-        }
+    if (sc->stop || sc->breakdown) return;
+    const cpx<T> b = mk((T)sc->beta[0], (T)sc->beta[1]), bc = cj(b);
+    for (int e = blockIdx.x * RB + threadIdx.x; e < sm.nslots; e += gridDim.x * RB) {
+        const int i = sm.slot[e], L = sm.order[i], hb = L * (L + 2), loc = e - sm.offset[i] / 2;
+        const int row = loc % (L + 2), col = loc / (L + 2) + 1, n = (row <= col) ? col : row - 1;
+        const int k0 = sm.offset[i] + loc, k1 = k0 + hb;
+        const cpx<T> p0 = r[k0] + b * p[k0], p1 = r[k1] + b * p[k1], w0 = q[k0] + bc * w[k0], w1 = q[k1] + bc * w[k1];
+        p[k0] = p0;
+        p[k1] = p1;
+        w[k0] = w0;
+        w[k1] = w1;
+        x0[k0] = p0;
+        x0[k1] = p1;
+        const cpx<T>* A = an + sm.mie_offset[i] + 4 * (n - 1);
+        x1[k0] = A[0] * cj(w0) + A[1] * cj(w1);
+        x1[k1] = A[2] * cj(w0) + A[3] * cj(w1);
     }
 }
 
@@ -308,9 +360,8 @@ void launch_post(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* p, const cp
                  cpx<T>* cap, cpx<T>* caw, double* part, BicgScalars* sc, int nsm, cudaStream_t st)
 {
     int g = grid_for(sm.nslots, nsm);
-    post_kernel<T><<<g, RB, 0, st>>>(sm.nslots, sm.slot, sm.order, sm.offset, sm.mie_offset, an, p, w, y0, y1, cap, caw, part);
-    fin_kernel<<<1, 32, 0, st>>>(1, g, part, sc, 0.0, 1);
-    launch_counter() += 2;
+    post_kernel<T><<<g, RB, 0, st>>>(sm.nslots, sm.slot, sm.order, sm.offset, sm.mie_offset, an, p, w, y0, y1, cap, caw, part, sc);
+    launch_counter() += 1;
 }
 template <typename T>
 void launch_init(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* b, const cpx<T>* x, const cpx<T>* y0, int have_y, cpx<T>* r,
@@ -322,14 +373,14 @@ void launch_init(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* b, const cp
     launch_counter() += 2;
 }
 template <typename T>
-void launch_upd(int n, cpx<T>* x, cpx<T>* r, cpx<T>* q, cpx<T>* p, cpx<T>* w, const cpx<T>* cap, const cpx<T>* caw, double* part,
-                BicgScalars* sc, double eps, int nsm, cudaStream_t st)
+void launch_upd(const SlotMaps& sm, const cpx<T>* an, int n, cpx<T>* x, cpx<T>* r, cpx<T>* q, cpx<T>* p, cpx<T>* w, const cpx<T>* cap,
+                const cpx<T>* caw, double* part, BicgScalars* sc, double eps, cpx<T>* x0, cpx<T>* x1, int nsm, cudaStream_t st)
 {
     int g = grid_for(n, nsm);
-    upd1_kernel<T><<<g, RB, 0, st>>>(n, sc, x, r, q, p, cap, caw, part);
-    fin_kernel<<<1, 32, 0, st>>>(2, g, part, sc, eps, 1);
-    upd2_kernel<T><<<g, RB, 0, st>>>(n, sc, p, w, r, q);
-    launch_counter() += 3;
+    upd1_kernel<T><<<g, RB, 0, st>>>(n, sc, x, r, q, p, cap, caw, part, eps);
+    if (x0) upd2_columns_kernel<T><<<grid_for(sm.nslots, nsm), RB, 0, st>>>(sm, an, sc, p, w, r, q, x0, x1);
+    else upd2_kernel<T><<<g, RB, 0, st>>>(n, sc, p, w, r, q);
+    launch_counter() += 2;
 }
 
 template <typename T, typename TB>
@@ -358,8 +409,8 @@ template void launch_post<double>(const SlotMaps&, const zd*, const zd*, const z
 template void launch_post<float>(const SlotMaps&, const zf*, const zf*, const zf*, const zf*, const zf*, zf*, zf*, double*, BicgScalars*, int, cudaStream_t);
 template void launch_init<double>(const SlotMaps&, const zd*, const zd*, const zd*, const zd*, int, zd*, zd*, zd*, zd*, double*, BicgScalars*, int, int, cudaStream_t);
 template void launch_init<float>(const SlotMaps&, const zf*, const zf*, const zf*, const zf*, int, zf*, zf*, zf*, zf*, double*, BicgScalars*, int, int, cudaStream_t);
-template void launch_upd<double>(int, zd*, zd*, zd*, zd*, zd*, const zd*, const zd*, double*, BicgScalars*, double, int, cudaStream_t);
-template void launch_upd<float>(int, zf*, zf*, zf*, zf*, zf*, const zf*, const zf*, double*, BicgScalars*, double, int, cudaStream_t);
+template void launch_upd<double>(const SlotMaps&, const zd*, int, zd*, zd*, zd*, zd*, zd*, const zd*, const zd*, double*, BicgScalars*, double, zd*, zd*, int, cudaStream_t);
+template void launch_upd<float>(const SlotMaps&, const zf*, int, zf*, zf*, zf*, zf*, zf*, const zf*, const zf*, double*, BicgScalars*, double, zf*, zf*, int, cudaStream_t);
 template void launch_resid<double, double>(const SlotMaps&, const zd*, const zd*, const zd*, const zd*, zd*, double*, double*, int, cudaStream_t);
 template void launch_resid<double, float>(const SlotMaps&, const zd*, const zd*, const zd*, const zd*, zf*, double*, double*, int, cudaStream_t);
 template void launch_conj_copy<double>(int, const zd*, zd*, cudaStream_t);

@@ -6,7 +6,8 @@ struct BicgScalars {
     double csk[2], alpha[2], beta[2];
     double enorm, eerr;
     int stop, breakdown;
-    int pad[2];
+    unsigned done;       // CTAs of the running reduction that have stored their partials
+    int pad;
     double csk_prev[2];   // csk before the last update (residual replacement recomputes beta from it)
 };
 
@@ -25,9 +26,10 @@ void launch_post(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* p, const cp
 template <typename T>
 void launch_init(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* b, const cpx<T>* x, const cpx<T>* y0, int have_y, cpx<T>* r,
                  cpx<T>* p, cpx<T>* w, cpx<T>* q, double* part, BicgScalars* sc, int normalize, int nsm, cudaStream_t st);
+// x0, x1 (may be null): the next pass's columns, p and the transposed Mie multiply of conj(w), are written too
 template <typename T>
-void launch_upd(int n, cpx<T>* x, cpx<T>* r, cpx<T>* q, cpx<T>* p, cpx<T>* w, const cpx<T>* cap, const cpx<T>* caw, double* part,
-                BicgScalars* sc, double eps, int nsm, cudaStream_t st);
+void launch_upd(const SlotMaps& sm, const cpx<T>* an, int n, cpx<T>* x, cpx<T>* r, cpx<T>* q, cpx<T>* p, cpx<T>* w, const cpx<T>* cap,
+                const cpx<T>* caw, double* part, BicgScalars* sc, double eps, cpx<T>* x0, cpx<T>* x1, int nsm, cudaStream_t st);
 template <typename T, typename TB>
 void launch_resid(const SlotMaps& sm, const cpx<T>* an, const cpx<T>* b, const cpx<T>* x, const cpx<T>* y, cpx<TB>* rout, double* part,
                   double* out2, int nsm, cudaStream_t st);

@@ -177,8 +177,9 @@ int ensure_wide(mstmg_ctx* c, int ncols)
 
 // y[:, 0:ncols] = H x[:, 0:ncols]  (y zeroed here); column k is a
 // conjugate-transpose product when bit (k mod period) of contran is set
-// (period 32, one bit a column, or 1, 2 or 4).
-template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period)
+// (period 32, one bit a column, or 1, 2 or 4).  skip (may be null; tiles of
+// pairs only): the pass is empty when either of two device words is not 0.
+template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period, const int* skip)
 {
     NvtxRange nvtx_(sizeof(T) == 8 ? "translation pass FP64" : "translation pass FP32");
     const size_t ld = (size_t)c->neqns;
@@ -245,6 +246,7 @@ template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, in
         a.slots = c->tslots;
         a.err = c->err.p;
         a.ctas_per_sm = c->opts.tile_ctas_per_sm;
+        a.skip = skip;
         for (const auto& g : c->tgroups) {
             if (g.count == 0) continue;
             a.ntiles = g.count;
@@ -992,7 +994,7 @@ extern "C" int mstmg_time_translation(mstmg_ctx* c, int prec, int nrhs, int reps
     return check_kernel_err(c);
 }
 
-template int translate<float>(mstmg_ctx*, const zf*, zf*, int, unsigned, int);
-template int translate<double>(mstmg_ctx*, const zd*, zd*, int, unsigned, int);
+template int translate<float>(mstmg_ctx*, const zf*, zf*, int, unsigned, int, const int*);
+template int translate<double>(mstmg_ctx*, const zd*, zd*, int, unsigned, int, const int*);
 template int translate_many<float>(mstmg_ctx*, const zf*, zf*, int, unsigned);
 template int translate_many<double>(mstmg_ctx*, const zd*, zd*, int, unsigned);

@@ -83,30 +83,56 @@ int bicg_batched(mstmg_ctx* c, int S, const cpx<T>* const* b, BicgVecs<T>* v, bo
     }
     int nact = 0;
     for (int s = 0; s < S; s++) nact += active[s];
+    // One system on tiles of pairs alone: the next pass is queued before the
+    // host reads this iteration's scalars, so that the device does not wait
+    // for it (16 us an iteration); the columns come from the update itself and
+    // the pass is empty if the system has stopped.
+    const bool ahead = S == 1 && !hosts && !c->timing && !c->tgroups_host.empty() && c->ndense == 0 && !c->hs.on() && !(c->fft && c->fft->on);
+    struct Event {
+        cudaEvent_t e = nullptr;
+        ~Event()
+        {
+            if (e) cudaEventDestroy(e);
+        }
+    } scalars;
+    if (ahead) CK(cudaEventCreateWithFlags(&scalars.e, cudaEventDisableTiming));
+    bool queued = false;   // this iteration's pass
     for (int it = 1; it <= niter && nact > 0; it++) {
         int slots[4], a = 0;
         for (int s = 0; s < S; s++)
             if (active[s]) slots[a++] = s;
-        unsigned mask = 0;
-        for (int k = 0; k < a; k++) {
-            int s = slots[k];
-            CK(cudaMemcpyAsync(X + (size_t)(2 * k) * ne, v[s].p, sizeof(cpx<T>) * ne, cudaMemcpyDeviceToDevice, c->st));
-            if (hosts) mie_all(c, -1, 1, (const zd*)v[s].w, (zd*)(X + (size_t)(2 * k + 1) * ne));
-            else launch_mie<T>(sm.nslots, sm.slot, sm.order, sm.offset, sm.mie_offset, an, -1, 1, v[s].w, X + (size_t)(2 * k + 1) * ne, c->st);
-            mask |= 2u << (2 * k);
+        if (!queued) {
+            unsigned mask = 0;
+            for (int k = 0; k < a; k++) {
+                int s = slots[k];
+                CK(cudaMemcpyAsync(X + (size_t)(2 * k) * ne, v[s].p, sizeof(cpx<T>) * ne, cudaMemcpyDeviceToDevice, c->st));
+                if (hosts) mie_all(c, -1, 1, (const zd*)v[s].w, (zd*)(X + (size_t)(2 * k + 1) * ne));
+                else launch_mie<T>(sm.nslots, sm.slot, sm.order, sm.offset, sm.mie_offset, an, -1, 1, v[s].w, X + (size_t)(2 * k + 1) * ne, c->st);
+                mask |= 2u << (2 * k);
+            }
+            rc = translate<T>(c, X, Y, 2 * a, mask);
+            if (rc) return rc;
         }
-        rc = translate<T>(c, X, Y, 2 * a, mask);
-        if (rc) return rc;
+        queued = ahead && it < niter;
         for (int k = 0; k < a; k++) {
             int s = slots[k];
             if (hosts) mie_all(c, 1, 0, (const zd*)(Y + (size_t)(2 * k) * ne), (zd*)(Y + (size_t)(2 * k) * ne));
             launch_post<T>(sm, anf, v[s].p, v[s].w, Y + (size_t)(2 * k) * ne, Y + (size_t)(2 * k + 1) * ne, v[s].cap, v[s].caw, part,
                            c->sc.p + s, c->nsm, c->st);
-            launch_upd<T>(ne, v[s].x, v[s].r, v[s].q, v[s].p, v[s].w, v[s].cap, v[s].caw, part, c->sc.p + s, eps[s], c->nsm, c->st);
+            launch_upd<T>(sm, an, ne, v[s].x, v[s].r, v[s].q, v[s].p, v[s].w, v[s].cap, v[s].caw, part, c->sc.p + s, eps[s],
+                          queued ? X : nullptr, queued ? X + ne : nullptr, c->nsm, c->st);
         }
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(c->h_sc, c->sc.p, sizeof(BicgScalars) * S, cudaMemcpyDeviceToHost, c->st));
-        CK(cudaStreamSynchronize(c->st));
+        int p64 = c->passes64, p32 = c->passes32;
+        if (queued) {
+            CK(cudaEventRecord(scalars.e, c->st));
+            rc = translate<T>(c, X, Y, 2, 2u, 32, &c->sc.p->stop);
+            if (rc) return rc;
+            CK(cudaEventSynchronize(scalars.e));
+        } else {
+            CK(cudaStreamSynchronize(c->st));
+        }
         for (int k = 0; k < a; k++) {
             int s = slots[k];
             iters[s] = it;
@@ -120,6 +146,10 @@ int bicg_batched(mstmg_ctx* c, int S, const cpx<T>* const* b, BicgVecs<T>* v, bo
         }
         nact = 0;
         for (int s = 0; s < S; s++) nact += active[s];
+        if (nact == 0) {   // the pass queued ahead was empty
+            c->passes64 = p64;
+            c->passes32 = p32;
+        }
     }
     for (int s = 0; s < S; s++)
         if (active[s]) iters[s] = niter + 1;   // Fortran DO-loop exit value when the cap is reached

@@ -568,7 +568,7 @@ int setup_layout(mstmg_ctx* c);
 DenseArgs dense_args(mstmg_ctx* c);
 int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force);
 int ensure_ops(mstmg_ctx* c, int prec, bool force);
-template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period = 32);
+template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, int ncols, unsigned contran, int period = 32, const int* skip = nullptr);
 // Columns from which a plain (no conjugate-transpose column) FP32 pass goes to
 // the tensor cores: one M tile costs the same for 1 or 128 columns, and at 12
 // columns it already beats the rotation kernel.

@@ -213,6 +213,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
     const int acs = a.acs;
     const int G = gridDim.x, NI = a.ntiles * a.nchunk;
     if ((int)blockIdx.x >= NI) return;
+    if (a.skip && (a.skip[0] | a.skip[1])) return;
     // everything a product may read past a block's end has to be finite
     for (zd* e = reinterpret_cast<zd*>(recb) - 1 + tid; e < ACC + a.slots * 4 * acs; e += (NW + 1) * 32) *e = mk(0.0, 0.0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");

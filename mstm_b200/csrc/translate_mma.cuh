@@ -40,6 +40,7 @@ struct MmaArgs {
     int* err;
     int recs;               // record buffers (1 or 2, set by the launcher)
     int ctas_per_sm;        // 0: as many as fit
+    const int* skip;        // may be null: the pass does nothing when either of two words is not 0
     // set by the launcher
     int nchunk;
     int bs, bufc, acs;      // source block stride, one work buffer, accumulator mode stride (complex units)
