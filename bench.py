@@ -44,10 +44,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 EPS = 1.0e-12          # squared-norm criterion: ||r||/||b|| < 1e-6
-# DRAM bytes per byte of row records and vectors of the FP32 row-kernel
-# translation pass of 2 columns, from the ncu capture of the 200-sphere
-# aggregate (189.06 MB of 185.0 MB)
-TRAFFIC_PER_ALG_BYTE = 189.06 / 185.0
+# DRAM bytes per byte of records and vectors of the translation pass of 2
+# columns, from the ncu capture of the 200-sphere aggregate (343.5 MB of 338.8 MB)
+TRAFFIC_PER_ALG_BYTE = 343.5 / 338.8
 NITER = 10000
 WORKLOAD = "fractal500"
 METRIC = "solves/s at 1e-6 residual (fractal aggregate N=500, x=2, both polarisations)"
@@ -350,7 +349,7 @@ def run_extras(args, dev, stream):
             # transforms) + x read and y written, for the two columns of an
             # Arnoldi pass
             ms_pass = g.time_translation("mixed", 2, 10)
-            near = g.operator_bytes("fp64")[0] / 2.0   # the near pairs' folded FP32 operator values (row records add padding)
+            near = g.operator_bytes("fp64")[0] / 2.0   # the near pairs' folded operator at 4 B a value (the records hold 8)
             cdim, no = grid["cell_dim"], grid["node_order"]
             nodes = (2 * cdim[0]) * (2 * cdim[1]) * (2 * cdim[2])
             nbn = no * (no + 2)
@@ -425,10 +424,10 @@ def run_extras(args, dev, stream):
     rec = g.operator_bytes("fp64")[0]
     alg = rec + 2 * 2 * g.number_eqns * 16
     pms = row["fp64"]["ms_per_translation_pass_2_columns"]
-    row["fp64"]["pass_roofline"] = {"kernel": "translate_kernel<double, 64, 4> (order-generic, same-host pairs) + the host pairs' launch",
+    row["fp64"]["pass_roofline"] = {"kernel": "translate_mma_kernel<4, 2, 8> (same-host pairs) + translate_kernel (the host's pairs)",
                                     "algorithmic_bytes": alg, "achieved_gbs": round(alg / pms / 1e6, 1),
                                     "frac_of_measured_hbm": round(alg / pms / 1e6 / hbm_peak(), 4),
-                                    "bound": "instruction issue (profiles/translate_generic_fp64_host300.md)"}
+                                    "bound": "latency of a pair's phases"}
     fx = oracle_fixture("host1000")
     if fx is not None:
         row["fp64"]["vs_oracle"] = {"qext": float("%.3g" % abs(r["qtot"][0, 0] / fx["qtot"][0, 0] - 1)),
@@ -570,16 +569,16 @@ def report_line(args, ws, R, ne):
     plain = job_value(ws, args.steps, p["ms_total"])
     # dominant kernel: the FP32 translation pass of the tuned path
     ms32, n32 = m["k32"]
-    stored32, canon32 = m["bytes32"]   # FP32 row-record bytes (as stored), and the reference layout's bytes at 4 B per real
-    folded32 = m["bytes64"][0] / 2.0   # the folded operator values at 4 B each, without the row records' padding
+    stored32, canon32 = m["bytes32"]   # record bytes the pass reads (FP64), and the reference layout's bytes at 4 B per real
+    folded32 = stored32
     # algorithmic bytes per launch, as the canonical matvec bytes define them
     # (the reference layout's stored operator at 4 B per real, read once, +
     # x read + y written; one column per active polarisation: the tuned
     # path's Arnoldi passes carry 2 columns while both polarisations are
     # active, iterations count Arnoldi steps in pairs).  The kernel itself
-    # reads the operator folded by the Wigner and axial symmetries, in row
-    # records (stored32: padding and a phase table on top), which is its DRAM
-    # traffic; the same pass against the folded values is reported beside.
+    # reads the operator folded by the Wigner and axial symmetries, in FP64
+    # records (stored32), which is its DRAM traffic; the same pass against
+    # those bytes is reported beside.
     it = m["stats"]["iterations"]
     n32p = max(1, m["stats"]["passes32"])
     avg_cols = min(2.0, 2.0 * sum(it) / n32p) if sum(it) > 0 else 2.0
@@ -614,14 +613,14 @@ def report_line(args, ws, R, ne):
         "tuned": {"iterations": it, "outer": m["stats"]["outer"], "passes64": m["stats"]["passes64"],
                   "passes32": m["stats"]["passes32"], "qext": m["qtot"][0, 0], "qext_plain": p["qtot"][0, 0],
                   "qext_rel_diff": abs(m["qtot"][0, 0] / p["qtot"][0, 0] - 1)},
-        "roofline": {"kernel": "translate_rows_kernel<9, 2, 0> (FP32 pair translation pass, row kernel)", "bound": "hbm",
+        "roofline": {"kernel": "translate_mma_kernel<9, 3, 4> (pair translation pass of FP32 columns, FP64 tensor cores)", "bound": "hbm",
                      "achieved": round(achieved, 1) if achieved else None, "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 4) if achieved else None,
                      "traffic": round(TRAFFIC_PER_ALG_BYTE * (stored32 + vec_bytes)),
-                     "row_record_bytes": stored32,
+                     "record_bytes": stored32,
                      "traffic_source": "ncu dram__bytes_read+write of this kernel on the 200-sphere aggregate "
-                                       "(profiles/translate_rows_fp32_fractal200.md: 1.02x the row records and vectors "
-                                       "read and written), scaled to this workload's row records",
+                                       "(profiles/translate_mma_aggregate200.md: 1.01x the FP64 records and vectors "
+                                       "read and written), scaled to this workload's records",
                      "peak_source": peak_src,
                      "algorithmic_bytes_per_launch": alg,
                      "algorithmic_bytes_source": "canonical matvec bytes (reference operator layout at 4 B per real, "
@@ -811,8 +810,8 @@ def main():
     ap.add_argument("--workload", default=WORKLOAD)
     ap.add_argument("--precision", default="mixed", choices=["mixed", "fp64", "tc"])
     ap.add_argument("--fp32-chunk", type=int, default=0, help="profiling case: FP32 column chunk (2 or 4; 0 default)")
-    ap.add_argument("--ctas-per-sm", type=int, default=0, help="profiling case: tiled kernel CTAs per SM (0 default)")
-    ap.add_argument("--tile-pairs", type=int, default=0, help="profiling case: 0 the FP32 row kernel (default), 1 or 2 the rotation-tiled kernel with that many pairs per step")
+    ap.add_argument("--ctas-per-sm", type=int, default=0, help="profiling case: most CTAs per SM of the pair kernel (0: as many as fit)")
+    ap.add_argument("--tile-pairs", type=int, default=0, help="accepted without effect")
     ap.add_argument("--nrhs", type=int, default=4)
     ap.add_argument("--tmatrix-case", type=int, default=0, help="profiling case: one T matrix of this many spheres")
     ap.add_argument("--tensor-core", type=int, default=0, help="profiling case: 0 tensor-core passes where they apply, -1 never")
