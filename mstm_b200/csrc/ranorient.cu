@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(RO_NT) ro_bm_kernel(RoArgs a, int i0, int ni)
 // memory at a time, a share of the items (blockIdx.z) a CTA and its sums added
 // with FP64 atomics.  FP64-rate bound: 16 multiply-adds for every four 16-byte
 // shared loads of a thread (2 x 2 outputs).  With a CTA per item adding every
-// product to dm by its own atomics the loop took 32.6 ms for order 22; now 3.8
+// product to dm by its own atomics the loop took 32.6 ms for order 28; now 3.8
 // ms, 2.4 of them the contractions of ro_bm_kernel.
 #define RO_TILE 32
 #define RO_KC 16
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(256) ro_dm_kernel(RoArgs a, int i0, int ni)
 // coefficients take, a warp each, to a.part[part][w][n][12] in the order
 //   aw(0,-1) aw(0,1) bw(0,-1) bw(0,1) aw(2,0) bw(2,0) aw(2,-1) aw(2,1) bw(2,-1) bw(2,1) cw dw
 // One CTA per w with a vcfunc per (ik, n, n1, u) and the sums on one thread
-// took 26.4 ms for order 22; now below 0.7 ms.
+// took 26.4 ms for order 28; now below 0.7 ms.
 #define RO_CT 256
 __global__ void __launch_bounds__(RO_CT) ro_coef_kernel(RoArgs a)
 {
