@@ -286,7 +286,7 @@ int upload_pairs(mstmg_ctx* c, const std::vector<int2>& pr, int np, const TileSe
     c->op_units = u;
     c->maxrec = maxrec;
     c->layout_gen++;
-    c->ops64_ready = c->ops32_ready = false;
+    c->rot_ready = c->dense64_ready = c->dense32_ready = false;
     if (c->tc_state == 1) c->tc_state = 0;
     return MSTMG_OK;
 }
@@ -919,7 +919,7 @@ extern "C" int mstmg_ctx_set_positions(mstmg_ctx* c, const double* pos)
     CK(copy_in(c->pos.p, pos, sizeof(double) * 3 * c->n, c->st));
     if (is_dev(pos)) CK(cudaMemcpy(c->hpos.data(), pos, sizeof(double) * 3 * c->n, cudaMemcpyDeviceToHost));
     else memcpy(c->hpos.data(), pos, sizeof(double) * 3 * c->n);
-    c->ops64_ready = c->ops32_ready = false;
+    c->rot_ready = c->dense64_ready = c->dense32_ready = false;
     if (c->tc_state == 1) c->tc_state = 0;
     if (c->fft && c->fft->on) {
         c->fft->drop_plans();

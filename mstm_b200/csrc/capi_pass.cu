@@ -8,8 +8,6 @@
 // ---------------------------------------------------------------------------
 // operators and the translation pass
 // ---------------------------------------------------------------------------
-// Generate the stored pair operators.  want64 / want32 select the FP64 and
-// FP32 records; both come out of one pass of the generator when both are due.
 DenseArgs dense_args(mstmg_ctx* c)
 {
     DenseArgs d;
@@ -32,37 +30,31 @@ DenseArgs dense_args(mstmg_ctx* c)
     return d;
 }
 
+// Generate the stored pair operators a pass in FP64 (want64) or FP32 (want32)
+// reads, those that are not there yet or with `force` all of them: the dense
+// records of that precision, and the rotation records, which serve both.
 int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
 {
-    if (c->npairs == 0 && c->ndense == 0) return MSTMG_OK;
-    bool need64 = want64 && (force || !c->ops64_ready);
-    bool need32 = want32 && (force || !c->ops32_ready);
-    if (!need64 && !need32) return MSTMG_OK;
-    if (c->ndense > 0) {
+    const bool dense64 = want64 && c->ndense > 0 && (force || !c->dense64_ready);
+    const bool dense32 = want32 && c->ndense > 0 && (force || !c->dense32_ready);
+    if (dense64 || dense32) {
         DenseArgs d = dense_args(c);
         const void* was[2] = {c->dop64.p, c->dop32.p};
-        if (need64) {
+        if (dense64) {
             CK(c->dop64.alloc(c->dense_units));
             d.rec64 = c->dop64.p;
         }
-        if (need32) {
+        if (dense32) {
             CK(c->dop32.alloc(c->dense_units));
             d.rec32 = c->dop32.p;
         }
         if (was[0] != c->dop64.p || was[1] != c->dop32.p) c->layout_gen++;
         launch_dense_gen(d, c->st);
         CK(cudaGetLastError());
+        if (dense64) c->dense64_ready = true;
+        if (dense32) c->dense32_ready = true;
     }
-    if (c->npairs == 0) {
-        if (need64) c->ops64_ready = true;
-        if (need32) c->ops32_ready = true;
-        return MSTMG_OK;
-    }
-    // the rotation records serve the passes of either precision
-    if (!force && c->ops64_ready) {
-        c->ops32_ready = true;
-        return MSTMG_OK;
-    }
+    if (c->npairs == 0 || !(want64 || want32) || (c->rot_ready && !force)) return MSTMG_OK;
     {
         const void* was = c->op64.p;
         CK(c->op64.alloc(c->op_units));
@@ -106,8 +98,7 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
         CK(cudaGetLastError());
         h.hops_ready = true;
     }
-    c->ops64_ready = true;
-    if (need32) c->ops32_ready = true;
+    c->rot_ready = true;
     return MSTMG_OK;
 }
 

@@ -449,7 +449,8 @@ struct mstmg_ctx {
     std::vector<int4> tiles_host;           // w: the tile's group
     std::vector<TileGroup> tgroups_host;
     DevBuf<double> op64;   // operator records, read by FP64 and FP32 passes
-    bool ops64_ready = false, ops32_ready = false;   // records (and dense FP64); dense FP32
+    // generated for the present positions: the rotation (and host) records, the dense records of either precision
+    bool rot_ready = false, dense64_ready = false, dense32_ready = false;
     // mixed fixed-orientation solve: the two polarisations as a many-system
     // residual-replacement solve, its work kept across solves
     MultiWork<double> fo64;
