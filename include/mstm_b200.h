@@ -358,6 +358,13 @@ int mstmg_translation_pass(mstmg_ctx *ctx, int prec, int ncols, const int *con_t
  * usable afterwards. */
 int mstmg_selftest_bounded_wait(int device, int limit, int *status);
 
+/* Diagnostic, no counterpart in the reference: an FP64 translation pass (as
+ * mstmg_translation_pass, on pairs in tiles) in which a wait for the copies of
+ * every CTA's pair number `pair` (from 0) is taken to have run out, although
+ * the copies complete.  *status is the pass's: MSTMG_ERR_CUDA when a CTA came
+ * that far, which leaves y without the tile it was in and the context usable. */
+int mstmg_selftest_pass_wait(mstmg_ctx *ctx, int pair, int ncols, const int *con_tran, const double *x, double *y, int *status);
+
 /* Time `reps` translation passes (nrhs right-hand sides, FP64 (prec 0) or
  * FP32 (prec 1) with every second column a conjugate-transpose product, or
  * (prec 2) plain FP32 columns on the tensor cores) with CUDA events on the

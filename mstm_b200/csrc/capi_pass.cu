@@ -236,6 +236,7 @@ template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, in
         a.period = period;
         a.slots = c->tslots;
         a.err = c->err.p;
+        a.give_up_at = c->give_up_at;
         a.ctas_per_sm = c->opts.tile_ctas_per_sm;
         a.skip = skip;
         for (const auto& g : c->tgroups) {
@@ -935,6 +936,25 @@ extern "C" int mstmg_translation_pass(mstmg_ctx* c, int prec, int ncols, const i
     CK(copy_out(y, y64.p, sizeof(zd) * cols, c->st));
     CK(cudaStreamSynchronize(c->st));
     return check_kernel_err(c);
+}
+
+extern "C" int mstmg_selftest_pass_wait(mstmg_ctx* c, int pair, int ncols, const int* con_tran, const double* x, double* y, int* status)
+{
+    if (!c || !status || pair < 0) {
+        set_err("mstmg_selftest_pass_wait: bad arguments");
+        return MSTMG_ERR_ARG;
+    }
+    if (c->tgroups_host.empty()) {
+        set_err("mstmg_selftest_pass_wait: no pairs on tiles in this context");
+        return MSTMG_ERR_UNSUPPORTED;
+    }
+    c->give_up_at = pair;
+    const int rc = mstmg_translation_pass(c, 0, ncols, con_tran, x, y);
+    c->give_up_at = -1;
+    *status = rc;
+    // a wait that gave up leaves the device as it was; any other CUDA error does not
+    CK(cudaStreamSynchronize(c->st));
+    return rc == MSTMG_ERR_CUDA ? MSTMG_OK : rc;
 }
 
 extern "C" int mstmg_time_translation(mstmg_ctx* c, int prec, int nrhs, int reps, double* ms)

@@ -443,6 +443,7 @@ struct mstmg_ctx {
     struct TileGroup { int first, count, L, uniform, maxrec; };
     std::vector<TileGroup> tgroups;   // of this shard's tiles
     int tslots = 0;
+    int give_up_at = -1;   // mstmg_selftest_pass_wait
     // pair shard (mstmg_set_pair_shard): this context translates the tiles
     // t with t % nshards == shard; all tiles kept on the host
     int shard = 0, nshards = 1;

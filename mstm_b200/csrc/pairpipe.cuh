@@ -29,9 +29,10 @@ __device__ __forceinline__ bool mb_try(uint64_t* bar, uint32_t parity)
                  : "memory");
     return ok != 0;
 }
+constexpr int WAIT_POLLS = 1 << 22;
 // bounded wait: gives up after `limit` polls (the kernels then record
 // MSTMG_ERR_CUDA and return instead of hanging)
-__device__ __forceinline__ bool mb_wait(uint64_t* bar, uint32_t parity, int limit = 1 << 22)
+__device__ __forceinline__ bool mb_wait(uint64_t* bar, uint32_t parity, int limit = WAIT_POLLS)
 {
     for (int it = 0; it < limit; ++it)
         if (mb_try(bar, parity)) return true;

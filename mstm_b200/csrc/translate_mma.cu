@@ -47,6 +47,15 @@
 // FP32 passes run the same kernel, their columns widened before and rounded
 // after: FP64 records, products and sums.
 //
+// A wait that runs out ends the whole CTA: the warp leaves a word in shared
+// memory and goes on; the copying warp looks for it behind phase B's barrier,
+// before it arms that phase's barrier again and before it adds a tile to y; it
+// then issues no more copies, makes the step the last one, waits (bounded) for
+// the copies in flight, sets *err to MSTMG_ERR_CUDA and leaves the tile out of
+// y.  (300 spheres of order 9, 2 columns: 430 -> 440 us, on average 0.6 % over
+// orders 3 to 16; a vote of the CTA in its barriers took 450 us, waits by the
+// copying warp alone 458.)
+//
 // Clusters of one order (3 .. 10) have instances with that order and the
 // units of every warp at compile time; other tiles (mixed or larger orders)
 // run the instances with orders at run time (LC = 0).
@@ -107,6 +116,13 @@ __device__ __forceinline__ int scol(int n, int m, int col) { return col ^ (m & 3
 
 // barrier of the CTA, from the copying warp's code and the others'
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
+// bounded wait of a whole warp
+__device__ __forceinline__ bool mb_wait_warp(uint64_t* bar, uint32_t parity)
+{
+    for (int it = 0; it < WAIT_POLLS; ++it)
+        if (__all_sync(0xffffffffu, mb_try(bar, parity))) return true;
+    return false;
+}
 // y[] += shared values, `bytes` long, by one bulk reduction
 __device__ __forceinline__ void bulk_add(void* dst, const void* src, uint32_t bytes)
 {
@@ -198,7 +214,10 @@ struct Step {
 template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) * 32, MINB) translate_mma_kernel(const __grid_constant__ MmaArgs a)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);              // [0], [1] operators, [2] sources
+    // uniform orders: [0] rotation blocks and sources, [1], [2] axial blocks of
+    // even and odd steps; else [0], [1] operators, [2] sources
+    uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
+    volatile int* gave_up = reinterpret_cast<int*>(sm + 24);      // a wait ran out
     Step* ring = reinterpret_cast<Step*>(sm + 32);                // 4 steps
     int* roff = reinterpret_cast<int*>(sm + 32 + 4 * sizeof(Step));   // per degree: E_n in the record
     int* zoff = roff + MSTMG_LMAX + 2;                            // per order: Z_m in the record
@@ -218,10 +237,11 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
     for (zd* e = reinterpret_cast<zd*>(recb) - 1 + tid; e < ACC + a.slots * 4 * acs; e += (NW + 1) * 32) *e = mk(0.0, 0.0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (tid == 0) {
-        mb_init(&bar[0], 1);
+        mb_init(&bar[0], LC ? 2 : 1);
         mb_init(&bar[1], 1);
         mb_init(&bar[2], 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        *gave_up = a.give_up_at == 0;
     }
 
     // thread 0: the steps in order, fetched two ahead (the next tile's
@@ -266,10 +286,10 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
         bulk_copy(recb + b * op_head(LC), g, h, &bar[0]);
         bulk_copy(body + op_head(LC), g + op_head(LC), r, &bar[0]);
     };
-    auto load_ax = [&](const Step& s) {
+    auto load_ax = [&](const Step& s, int b) {
         constexpr uint32_t z = (op_record_units(LC, LC) - op_z_base(LC, LC)) * 8u;
-        mb_expect(&bar[1], z);
-        bulk_copy(body + op_z_base(LC, LC), a.ops + (size_t)s.rec4 * 4 + op_z_base(LC, LC), z, &bar[1]);
+        mb_expect(&bar[1 + b], z);
+        bulk_copy(body + op_z_base(LC, LC), a.ops + (size_t)s.rec4 * 4 + op_z_base(LC, LC), z, &bar[1 + b]);
     };
     auto load_rec = [&](const Step& s, int b) {
         const int li = s.lls & 255, lj = (s.lls >> 8) & 255;
@@ -281,12 +301,13 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
         const int li = s.lls & 255, lj = (s.lls >> 8) & 255;
         const int c0 = 2 * s.chunk, nr = s.cols >> 2;
         const uint32_t bi = (uint32_t)(2 * li * (li + 2) * 16), bj = (uint32_t)(2 * lj * (lj + 2) * 16);
-        mb_expect(&bar[2], nr * (bi + bj));
+        uint64_t* sb = &bar[LC ? 0 : 2];
+        mb_expect(sb, nr * (bi + bj));
         zd* d = reinterpret_cast<zd*>(buf);
         for (int r = 0; r < nr; r++) {
             const zd* xr = a.x + (size_t)(c0 + r) * a.ld;
-            bulk_copy(d + r * a.bs, xr + s.offj, bj, &bar[2]);         // source of j -> i
-            bulk_copy(d + (2 + r) * a.bs, xr + s.offi, bi, &bar[2]);   // source of i -> j
+            bulk_copy(d + r * a.bs, xr + s.offj, bj, sb);         // source of j -> i
+            bulk_copy(d + (2 + r) * a.bs, xr + s.offi, bi, sb);   // source of i -> j
         }
     };
     cta_sync();
@@ -303,7 +324,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
                     ring[b] = s;
                     if (LC && b == 0) {
                         load_rot(s, 0);
-                        load_ax(s);
+                        load_ax(s, 0);
                     }
                     if (!LC && b < a.recs) load_rec(s, b);
                     if (b == 0) load_src(s, buf0);
@@ -330,20 +351,27 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             __syncwarp();
             for (zd* p = ACC + lane; p < ACC + a.slots * 4 * acs; p += 32) *p = mk(0.0, 0.0);
         };
+        int dead = 0;   // lane 0: 1, a wait ran out; 2, with the next step's record on its way
         unsigned have = 0xffffffffu;
-        for (int t = 0;; t++) {
+        int t = 0;
+        for (;; t++) {
             const Step st = ring[t & 3];
             const int b = t & 1;
             Step nx;
             nx.lls = 0;
             if (lane == 0 && !fetch(nx)) nx.lls = 0;
+            if (due && __any_sync(0xffffffffu, *gave_up)) due = false;   // in C of the last step
             if (due) flush_begin();
             if (!LC && (st.lls & 0xffffu) != have) {
                 have = st.lls & 0xffffu;
                 cta_sync();
             }
             cta_sync();   // B is done
-            const Step& s1 = ring[(t + 1) & 3];
+            Step& s1 = ring[(t + 1) & 3];
+            if (lane == 0 && (*gave_up || t == a.give_up_at)) {
+                dead = !LC && a.recs == 2 && s1.lls ? 2 : 1;
+                s1.lls = 0;   // the other warps read it behind D's barrier
+            }
             if (LC && lane == 0 && s1.lls) {   // E_n and O_n stay in registers for D: the next pair's replace them
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 load_rot(s1, b ^ 1);
@@ -353,12 +381,12 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             if (lane == 0 && s1.lls) {   // the next pair's sources replace a'
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 load_src(s1, b ? buf0 : buf1);
-                if (LC) load_ax(s1);
+                if (LC) load_ax(s1, b ^ 1);
             }
             if (lane == 0) ring[(t + 2) & 3] = nx;
             cta_sync();   // D is done
-            if (!LC && lane == 0) {   // the record after next (with one buffer, the next) replaces this one
-                if (a.recs == 1) nx = ring[(t + 1) & 3];
+            if (!LC && lane == 0 && s1.lls) {   // the record after next (with one buffer, the next) replaces this one
+                if (a.recs == 1) nx = s1;
                 if (nx.lls) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     load_rec(nx, a.recs == 2 ? b : 0);
@@ -369,6 +397,22 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             chunk = st.chunk;
             nr = st.cols >> 2;
             if (!ring[(t + 1) & 3].lls) break;
+        }
+        if (LC && lane == 0 && !dead && *gave_up) dead = 1;   // in C of the last step
+        if (__any_sync(0xffffffffu, dead != 0)) {
+            if (lane == 0) {   // the last phase armed of every barrier
+                const bool next = dead == 2;
+                if (LC) {
+                    mb_wait(&bar[0], t & 1);
+                    for (int k = t; k >= 0 && k > t - 2; k--) mb_wait(&bar[1 + (k & 1)], (k >> 1) & 1);
+                } else {
+                    mb_wait(&bar[a.recs == 2 ? t & 1 : 0], (a.recs == 2 ? t >> 1 : t) & 1);
+                    if (next) mb_wait(&bar[(t + 1) & 1], ((t + 1) >> 1) & 1);
+                    mb_wait(&bar[2], t & 1);
+                }
+                atomicExch(a.err, MSTMG_ERR_CUDA);
+            }
+            return;
         }
         flush_begin();   // the last step ends a tile
         flush_end();
@@ -403,14 +447,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             cta_sync();
         }
         const int par = !LC && a.recs == 2 ? (t >> 1) & 1 : t & 1;
-        if (!mb_wait(&bar[rb], par) || !mb_wait(&bar[2], t & 1)) {
-            if (tid == 0) atomicExch(a.err, MSTMG_ERR_CUDA);
-            // wait (bounded) for the copies in flight, then leave
-            if (LC) mb_wait(&bar[1], par);
-            else if (a.recs == 2) mb_wait(&bar[b ^ 1], ((t + 1) >> 1) & 1);
-            mb_wait(&bar[2], t & 1);
-            return;
-        }
+        if (!mb_wait_warp(&bar[rb], par) || (!LC && !mb_wait_warp(&bar[2], t & 1))) *gave_up = 1;
         const double* rec = LC ? body : recb + (size_t)rb * a.maxrec;
         const zd* hdr = reinterpret_cast<const zd*>(LC ? recb + b * op_head(LC) : rec);   // e^{i m phi}, e^{-i m phi}
         zd* src = b ? buf1 : buf0;    // sources, then s' and t'
@@ -482,11 +519,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
                 });
             }
             cta_sync();
-            if (!mb_wait(&bar[1], t & 1)) {
-                if (tid == 0) atomicExch(a.err, MSTMG_ERR_CUDA);
-                mb_wait(&bar[0], (t + 1) & 1);
-                return;
-            }
+            if (!mb_wait_warp(&bar[1 + b], (t >> 1) & 1)) *gave_up = 1;
 
             // ---- C: axial translation ----
             {

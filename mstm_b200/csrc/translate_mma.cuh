@@ -38,6 +38,7 @@ struct MmaArgs {
     int slots;              // tile slots in use (2, 4 or 8)
     int maxrec;             // largest record of the tiles, doubles
     int* err;
+    int give_up_at;         // -1; self-test: a wait of every CTA's pair number give_up_at is taken to have run out
     int recs;               // record buffers (1 or 2, set by the launcher)
     int ctas_per_sm;        // 0: as many as fit
     const int* skip;        // may be null: the pass does nothing when either of two words is not 0
