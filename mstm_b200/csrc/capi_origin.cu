@@ -348,7 +348,8 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
     CK(dsq.alloc((size_t)3 * n));
     CK(cudaMemsetAsync(dsq.p, 0, sizeof(double) * 3 * n, c->st));
     CK(qsum.alloc(3));
-    MultiWork<double>& w64 = c->tm64;
+    MultiWork<double> own64;
+    MultiWork<double>& w64 = ws.kept() ? c->tm64 : own64;
     // given back at the end where it is large, as the workspace is
     struct Trim {
         MultiWork<double>& w;

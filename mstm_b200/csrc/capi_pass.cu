@@ -159,6 +159,7 @@ int ensure_ops(mstmg_ctx* c, int prec, bool force) { return ensure_ops_both(c, p
 // of a stream capture, which cannot allocate
 int ensure_wide(mstmg_ctx* c, int ncols)
 {
+    std::lock_guard<std::recursive_mutex> lk(c->wide_mu);
     const size_t need = 2 * (size_t)c->neqns * ncols;
     if (c->tgroups_host.empty() || c->wide.n >= need) return MSTMG_OK;
     c->layout_gen++;
@@ -214,6 +215,8 @@ template <typename T> int translate(mstmg_ctx* c, const cpx<T>* x, cpx<T>* y, in
     }
     int rt = 0;
     if (!c->tgroups_host.empty()) {
+        std::unique_lock<std::recursive_mutex> lk(c->wide_mu, std::defer_lock);
+        if (sizeof(T) == 4) lk.lock();
         MmaArgs a;
         a.pairs = c->tpairs.p;
         a.tsph = c->tsph.p;

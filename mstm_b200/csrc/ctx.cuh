@@ -114,6 +114,8 @@ public:
             blocks_->pop_back();
         }
     }
+    // whether this call has what the context keeps
+    bool kept() const { return blocks_ != &own_; }
     cudaError_t alloc(void** out, size_t bytes)
     {
         bytes = (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
@@ -462,8 +464,8 @@ struct mstmg_ctx {
     GmresWork fo_gm;   // mixed_solver 2
     bool fo_gm_ready = false;
     GmresWork tm_gm;   // mixed_solver 2, T-matrix columns: kept across calls (sized for the largest order)
-    MultiWork<double> tm64;   // FP64 work of the T-matrix columns, kept likewise while below CALL_POOL_MAX
     CallPool pool;
+    MultiWork<double> tm64;   // FP64 work of the T-matrix columns, kept likewise while below CALL_POOL_MAX; the call that has the pool has it
     // the reference's constant tables on the device: bcof, square roots, bcof(n, n)
     std::mutex big_mu;
     DevBuf<double> big_bc, big_fnr, big_bcd;
@@ -481,6 +483,7 @@ struct mstmg_ctx {
     int vn = 0;
     DevBuf<int> err;
     DevBuf<zd> wide;   // FP64 copies of an FP32 pass's columns, x then y
+    std::recursive_mutex wide_mu;   // held from its resizing to the launch of its last reader
     DevBuf<zd> X64, Y64, pmnp, amnp, pw0, vec64, bvec64;
     DevBuf<zf> X32, Y32, vec32, rvec32;
     DevBuf<double> part, qeff, qtot, small;
