@@ -47,14 +47,14 @@
 // FP32 passes run the same kernel, their columns widened before and rounded
 // after: FP64 records, products and sums.
 //
-// A wait that runs out ends the whole CTA: the warp leaves a word in shared
-// memory and goes on; the copying warp looks for it behind phase B's barrier,
-// before it arms that phase's barrier again and before it adds a tile to y; it
-// then issues no more copies, makes the step the last one, waits (bounded) for
-// the copies in flight, sets *err to MSTMG_ERR_CUDA and leaves the tile out of
-// y.  (300 spheres of order 9, 2 columns: 430 -> 440 us, on average 0.6 % over
-// orders 3 to 16; a vote of the CTA in its barriers took 450 us, waits by the
-// copying warp alone 458.)
+// A wait that runs out ends the whole CTA: the warp, which waits as one, leaves
+// a word in shared memory and returns; the copying warp looks for it behind
+// phase B's barrier, before it arms that phase's barriers again, and before it
+// adds a tile to y; it then issues no more copies, makes the step the last one,
+// waits (bounded) for the copies in flight, sets *err to MSTMG_ERR_CUDA and
+// leaves the tile out of y.  (500 spheres of order 9, 2 columns: 1172 -> 1198
+// us, 0 to 2 % of a pass at other orders; a vote of the CTA in its barriers
+// took 5 %, waits by the copying warp alone 6 %.)
 //
 // Clusters of one order (3 .. 10) have instances with that order and the
 // units of every warp at compile time; other tiles (mixed or larger orders)
@@ -214,12 +214,15 @@ struct Step {
 template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) * 32, MINB) translate_mma_kernel(const __grid_constant__ MmaArgs a)
 {
     extern __shared__ __align__(128) unsigned char sm[];
-    // uniform orders: [0] rotation blocks and sources, [1], [2] axial blocks of
-    // even and odd steps; else [0], [1] operators, [2] sources
+    // uniform orders: [0] rotation blocks, [1], [2] axial blocks of even and odd
+    // steps, [SRC] sources; else [0], [1] operators, [2] sources.  Up to order 7
+    // rotation blocks and sources share [0] (one wait a pair less: 1 to 2 % of
+    // a pass at orders 5 to 7, but 2 % more at 8 and 9).
+    constexpr int SRC = LC == 0 ? 2 : LC < 8 ? 0 : 3;
     uint64_t* bar = reinterpret_cast<uint64_t*>(sm);
-    volatile int* gave_up = reinterpret_cast<int*>(sm + 24);      // a wait ran out
-    Step* ring = reinterpret_cast<Step*>(sm + 32);                // 4 steps
-    int* roff = reinterpret_cast<int*>(sm + 32 + 4 * sizeof(Step));   // per degree: E_n in the record
+    volatile int* gave_up = reinterpret_cast<int*>(sm + 32);      // a wait ran out
+    Step* ring = reinterpret_cast<Step*>(sm + 48);                // 4 steps
+    int* roff = reinterpret_cast<int*>(sm + 48 + 4 * sizeof(Step));   // per degree: E_n in the record
     int* zoff = roff + MSTMG_LMAX + 2;                            // per order: Z_m in the record
     double* recb = reinterpret_cast<double*>(sm + MMA_HEAD);      // the 16 bytes before are zero
     const int boff = (MMA_HEAD + (LC ? a.maxrec + op_head(LC) : a.recs * a.maxrec) * 8 + 16 * MMA_PAD + 127) & ~127;   // rows of the work buffers are 128-byte aligned
@@ -237,9 +240,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
     for (zd* e = reinterpret_cast<zd*>(recb) - 1 + tid; e < ACC + a.slots * 4 * acs; e += (NW + 1) * 32) *e = mk(0.0, 0.0);
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     if (tid == 0) {
-        mb_init(&bar[0], LC ? 2 : 1);
-        mb_init(&bar[1], 1);
-        mb_init(&bar[2], 1);
+        for (int k = 0; k < 4; k++) mb_init(&bar[k], SRC == 0 && k == 0 ? 2 : 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         *gave_up = a.give_up_at == 0;
     }
@@ -301,13 +302,12 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
         const int li = s.lls & 255, lj = (s.lls >> 8) & 255;
         const int c0 = 2 * s.chunk, nr = s.cols >> 2;
         const uint32_t bi = (uint32_t)(2 * li * (li + 2) * 16), bj = (uint32_t)(2 * lj * (lj + 2) * 16);
-        uint64_t* sb = &bar[LC ? 0 : 2];
-        mb_expect(sb, nr * (bi + bj));
+        mb_expect(&bar[SRC], nr * (bi + bj));
         zd* d = reinterpret_cast<zd*>(buf);
         for (int r = 0; r < nr; r++) {
             const zd* xr = a.x + (size_t)(c0 + r) * a.ld;
-            bulk_copy(d + r * a.bs, xr + s.offj, bj, sb);         // source of j -> i
-            bulk_copy(d + (2 + r) * a.bs, xr + s.offi, bi, sb);   // source of i -> j
+            bulk_copy(d + r * a.bs, xr + s.offj, bj, &bar[SRC]);         // source of j -> i
+            bulk_copy(d + (2 + r) * a.bs, xr + s.offi, bi, &bar[SRC]);   // source of i -> j
         }
     };
     cta_sync();
@@ -404,11 +404,12 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
                 const bool next = dead == 2;
                 if (LC) {
                     mb_wait(&bar[0], t & 1);
+                    if (SRC) mb_wait(&bar[SRC], t & 1);
                     for (int k = t; k >= 0 && k > t - 2; k--) mb_wait(&bar[1 + (k & 1)], (k >> 1) & 1);
                 } else {
                     mb_wait(&bar[a.recs == 2 ? t & 1 : 0], (a.recs == 2 ? t >> 1 : t) & 1);
                     if (next) mb_wait(&bar[(t + 1) & 1], ((t + 1) >> 1) & 1);
-                    mb_wait(&bar[2], t & 1);
+                    mb_wait(&bar[SRC], t & 1);
                 }
                 atomicExch(a.err, MSTMG_ERR_CUDA);
             }
@@ -447,7 +448,10 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             cta_sync();
         }
         const int par = !LC && a.recs == 2 ? (t >> 1) & 1 : t & 1;
-        if (!mb_wait_warp(&bar[rb], par) || (!LC && !mb_wait_warp(&bar[2], t & 1))) *gave_up = 1;
+        if (!mb_wait_warp(&bar[rb], par) || (SRC && !mb_wait_warp(&bar[SRC], t & 1))) {
+            *gave_up = 1;
+            return;
+        }
         const double* rec = LC ? body : recb + (size_t)rb * a.maxrec;
         const zd* hdr = reinterpret_cast<const zd*>(LC ? recb + b * op_head(LC) : rec);   // e^{i m phi}, e^{-i m phi}
         zd* src = b ? buf1 : buf0;    // sources, then s' and t'
@@ -519,7 +523,10 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
                 });
             }
             cta_sync();
-            if (!mb_wait_warp(&bar[1 + b], (t >> 1) & 1)) *gave_up = 1;
+            if (!mb_wait_warp(&bar[1 + b], (t >> 1) & 1)) {
+                *gave_up = 1;
+                return;
+            }
 
             // ---- C: axial translation ----
             {
