@@ -355,10 +355,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
         MultiWork<double>& w;
         ~Trim()
         {
-            if (sizeof(zd) * (w.vec.n + w.XP.n + w.YP.n) <= CALL_POOL_MAX) return;
-            w.vec.release();
-            w.XP.release();
-            w.YP.release();
+            if (w.bytes() > CALL_POOL_MAX) w.release();
         }
     } trim{w64};
     MultiWork<float> w32;

@@ -57,6 +57,7 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
     if (c->npairs == 0 || !(want64 || want32) || (c->rot_ready && !force)) return MSTMG_OK;
     {
         const void* was = c->op64.p;
+        if (c->op64.n < (size_t)c->op_units) c->make_room(sizeof(double) * (size_t)c->op_units);
         CK(c->op64.alloc(c->op_units));
         if (was != c->op64.p) c->layout_gen++;
     }
@@ -334,6 +335,7 @@ int ensure_tc(mstmg_ctx* c)
     }
     rstart[c->n] = (int)rsrc.size();
     const size_t need = ent.size() * tc_himg_floats(g) * sizeof(float);
+    c->make_room(3 * need);
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
     if (need > fr / 3) {

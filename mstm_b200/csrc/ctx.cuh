@@ -9,12 +9,13 @@
 //                   expansion) and the T matrix (tmatrix_solution, random
 //                   orientation)
 #pragma once
-#include <mutex>
 #include <algorithm>
+#include <atomic>
 #include <complex>
 #include <cstdio>
 #include <cstring>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 #include "../../include/mstm_b200.h"
@@ -80,7 +81,9 @@ template <typename T> struct DevBuf {
 // them with the context).  Each call used to allocate and free 14 to 45
 // buffers: 3.3 ms of a 5.4 ms scattering call, 11.6 ms of a 111 ms T matrix.
 // One call at a time has the blocks; one that finds them taken by another
-// thread works in blocks of its own.
+// thread works in blocks of its own.  Where device memory is short the idle
+// ones go: before an allocation here fails, and before the context judges what
+// room there is for operators, images or a basis (mstmg_ctx::make_room).
 #define CALL_POOL_MAX ((size_t)1 << 30)
 #define CALL_POOL_BLOCK ((size_t)32 << 20)
 struct CallPool {
@@ -88,18 +91,20 @@ struct CallPool {
         char* p;
         size_t n;
     };
-    std::mutex mu;
+    std::atomic<bool> taken{false};
     std::vector<Block> blocks;
-    ~CallPool()
+    ~CallPool() { clear(); }
+    void clear()
     {
         for (auto& b : blocks) cudaFree(b.p);
+        blocks.clear();
     }
 };
 class CallScratch {
 public:
-    CallScratch(CallPool& pool, cudaStream_t st) : lk_(pool.mu, std::try_to_lock), st_(st)
+    CallScratch(CallPool& pool, cudaStream_t st) : pool_(pool.taken.exchange(true) ? nullptr : &pool), st_(st)
     {
-        blocks_ = lk_.owns_lock() ? &pool.blocks : &own_;
+        blocks_ = pool_ ? &pool.blocks : &own_;
     }
     CallScratch(const CallScratch&) = delete;
     CallScratch& operator=(const CallScratch&) = delete;
@@ -113,9 +118,10 @@ public:
             cudaFree(blocks_->back().p);
             blocks_->pop_back();
         }
+        if (pool_) pool_->taken = false;
     }
     // whether this call has what the context keeps
-    bool kept() const { return blocks_ != &own_; }
+    bool kept() const { return pool_ != nullptr; }
     cudaError_t alloc(void** out, size_t bytes)
     {
         bytes = (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
@@ -134,6 +140,10 @@ public:
             b.n = bytes;
             e = cudaMalloc((void**)&b.p, b.n);
         }
+        if (e != cudaSuccess && drop_unused()) {
+            cudaGetLastError();
+            e = cudaMalloc((void**)&b.p, b.n);
+        }
         if (e != cudaSuccess) return e;
         blocks_->push_back(b);
         used_.resize(blocks_->size(), 0);
@@ -143,7 +153,20 @@ public:
     }
 
 private:
-    std::unique_lock<std::mutex> lk_;
+    // blocks this call has not used: kept from others, each too small
+    bool drop_unused()
+    {
+        bool any = false;
+        for (size_t k = blocks_->size(); k-- > 0;)
+            if (k >= used_.size() || used_[k] == 0) {
+                cudaFree((*blocks_)[k].p);
+                blocks_->erase(blocks_->begin() + k);
+                if (k < used_.size()) used_.erase(used_.begin() + k);
+                any = true;
+            }
+        return any;
+    }
+    CallPool* pool_;
     cudaStream_t st_;
     std::vector<CallPool::Block> own_, *blocks_;
     std::vector<size_t> used_;
@@ -220,6 +243,13 @@ template <typename T> struct MultiWork {
         m.CAP = b + 5 * cs;
         m.CAW = b + 6 * cs;
         return m;
+    }
+    size_t bytes() const { return sizeof(cpx<T>) * (vec.n + XP.n + YP.n); }
+    void release()
+    {
+        vec.release();
+        XP.release();
+        YP.release();
     }
     // vectors = false: only the packed translation buffers (FP64 residuals of the refinement)
     int init(int S_, int ne, int nsm, bool vectors)
@@ -311,9 +341,11 @@ struct GmresWork {
     size_t hpass() const { return (size_t)(m + 1) * S * 2; }
     // basis length from the free device memory: at most `cap` vectors a
     // system (200 when cap is 0), the basis within a quarter of the free memory
+    static int max_m(int cap) { return cap > 0 ? cap : 200; }
+    static size_t room(int S, int ne, int cap) { return 4 * sizeof(zf) * (size_t)S * ne * (max_m(cap) + 1); }   // for the longest
     static int pick_m(int S, int ne, int cap)
     {
-        const int mmax = cap > 0 ? cap : 200;
+        const int mmax = max_m(cap);
         size_t fr = 0, tot = 0;
         if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) return 0;
         const size_t per = sizeof(zf) * (size_t)S * ne;
@@ -466,6 +498,16 @@ struct mstmg_ctx {
     GmresWork tm_gm;   // mixed_solver 2, T-matrix columns: kept across calls (sized for the largest order)
     CallPool pool;
     MultiWork<double> tm64;   // FP64 work of the T-matrix columns, kept likewise while below CALL_POOL_MAX; the call that has the pool has it
+    // Free what is kept between calls, where the device has not `need` bytes
+    // to spare and no call is using it
+    void make_room(size_t need)
+    {
+        size_t fr = 0, tot = 0;
+        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr >= need || pool.taken.exchange(true)) return;
+        pool.clear();
+        tm64.release();
+        pool.taken = false;
+    }
     // the reference's constant tables on the device: bcof, square roots, bcof(n, n)
     std::mutex big_mu;
     DevBuf<double> big_bc, big_fnr, big_bcd;
