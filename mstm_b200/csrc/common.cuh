@@ -6,12 +6,31 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <atomic>
+#include <map>
+#include <mutex>
+#include <utility>
 
 // Count of kernels launched by this library (all contexts, all threads).
 inline std::atomic<long long>& launch_counter()
 {
     static std::atomic<long long> n{0};
     return n;
+}
+
+// Lets `kernel` be launched with `bytes` of dynamic shared memory on the
+// current device.  The limit belongs to the function and a smaller one replaces
+// a larger one, so that a launch that set its own size could be refused after
+// another thread's call: the largest size asked for stays.
+template <typename... A> inline void allow_smem(void (*kernel)(A...), size_t bytes)
+{
+    static std::mutex mu;
+    static std::map<std::pair<int, const void*>, size_t> most;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::lock_guard<std::mutex> lk(mu);
+    size_t& m = most[{dev, (const void*)kernel}];
+    const size_t want = bytes > m ? bytes : m;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want) == cudaSuccess) m = want;
 }
 
 #define MSTMG_LMAX 16          // largest sphere truncation order the kernels accept

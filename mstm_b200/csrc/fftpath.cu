@@ -405,7 +405,7 @@ void launch_fft_s2n(const FftMArgs& a, const cpx<T>* J, const cpx<T>* x, int ld,
     const int smem = (int)sizeof(cpx<T>) * ncol * (2 * a.nbmax + FFT_MT);
     with_columns(ncol, [&](auto nc) {
         auto k = fft_s2n_kernel<T, decltype(nc)::value>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        allow_smem(k, smem);
         k<<<a.nsph, FFT_MT, smem, st>>>(a, J, x, ld, contran, A);
     });
     launch_counter() += 1;
@@ -424,7 +424,7 @@ void launch_fft_n2s(const FftMArgs& a, const cpx<T>* J, const cpx<T>* G, int nco
     const int nbN = a.No * (a.No + 2), smem = (int)sizeof(cpx<T>) * ncol * (2 * nbN + 2 * a.nbmax + FFT_MT);
     with_columns(ncol, [&](auto nc) {
         auto k = fft_n2s_kernel<T, decltype(nc)::value>;
-        cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        allow_smem(k, smem);
         k<<<a.nsph, FFT_MT, smem, st>>>(a, J, G, contran, y, ld);
     });
     launch_counter() += 1;

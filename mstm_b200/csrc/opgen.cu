@@ -312,11 +312,7 @@ void launch_opgen(const OpGenArgs& a, int nsm, cudaStream_t st)
     opgen_pair_kernel<<<b1, 128, 0, st>>>(a);
     const int warps = 4;
     const size_t smem = sizeof(double) * ROT_WARP_DOUBLES * warps;
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(opgen_rot_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        attr = true;
-    }
+    allow_smem(opgen_rot_kernel, smem);
     int b2 = (a.npairs + warps - 1) / warps;
     if (b2 > nsm * 16) b2 = nsm * 16;
     opgen_rot_kernel<<<b2, warps * 32, smem, st>>>(a);

@@ -738,7 +738,7 @@ void launch_tranorder(int nsph, const double* pos, const int* order, const doubl
 {
     VCTab t{bcof, fnr, nbc};
     const int smem = (int)(sizeof(zd) * TRANORDER_ROW + sizeof(double) * 32 * TRANORDER_ROW);
-    cudaFuncSetAttribute(tranorder_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(tranorder_kernel, smem);
     tranorder_kernel<<<tranorder_blocks(nsph), 32, smem, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire, eps, maxt, t,
                                                                scratch, tord);
     launch_counter() += 1;
@@ -748,7 +748,7 @@ void launch_regular_couplings(int Tt, int Ls, const double* bcof, const double* 
 {
     VCTab t{bcof, fnr, nbc};
     const int smem = (int)sizeof(double) * (2 * std::min(Tt, Ls) + 2) * (Tt + Ls + 1);
-    cudaFuncSetAttribute(regular_couplings_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(regular_couplings_kernel, smem);
     regular_couplings_kernel<<<dim3(Tt, Ls), RC_NT, smem, st>>>(Tt, Ls, t, vcc);
     launch_counter() += 1;
 }
@@ -767,7 +767,7 @@ void launch_merge(const MergeArgs& a, int grid, cudaStream_t st)
 {
     // two rows of the Wigner recurrence a warp; orders reach MSTMG_LMAX and T
     const int nmax = std::max(a.T, MSTMG_LMAX), smem = (int)sizeof(double) * (PP_NT / 32) * 2 * (2 * nmax + 3);
-    cudaFuncSetAttribute(merge_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(merge_kernel, smem);
     merge_kernel<<<dim3(grid, merge_chunks(a.npol)), PP_NT, smem, st>>>(a);
     launch_counter() += 1;
 }
@@ -779,7 +779,7 @@ void launch_fosm(int ntot, const zd* a0, const double* bcof, const double* fnr, 
     // FO_MC orders m a chunk while three rows of each fit 200 KB (order 128)
     const int row = (int)sizeof(double) * (2 * ntot + 2), mc = std::max(1, std::min(FO_MC, (200 * 1024 - 2 * row) / (3 * row)));
     const int smem = row * (2 + 3 * mc);
-    cudaFuncSetAttribute(fosm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    allow_smem(fosm_kernel, smem);
     fosm_kernel<<<ntot * ntot, FO_NT, smem, st>>>(ntot, mc, a0, t, s00, s02, sp22, sm22);
     fosm_patch_kernel<<<(4 * (2 * ntot + 1) + 63) / 64, 64, 0, st>>>(ntot, s00, s02, sp22, sm22, 1.0);
     launch_counter() += 2;

@@ -454,8 +454,8 @@ int launch_ranorient(const RoArgs& args, const zd* tmat, int nang, const double*
     const int nu3 = 3 * (2 * nodr + 3);
     const size_t sm_bm = sizeof(zd) * (4 * nodr + 4) + sizeof(double) * (2 * nodr + 1) * VL;
     const size_t sm_co = sizeof(zd) * 12 * nodr + sizeof(double) * 2 * (2 * nodr + 1) * VL;
-    cudaFuncSetAttribute(ro_bm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_bm);
-    cudaFuncSetAttribute(ro_coef_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm_co);
+    allow_smem(ro_bm_kernel, sm_bm);
+    allow_smem(ro_coef_kernel, sm_co);
     for (int i0 = 0; i0 < nitems;) {
         const int i1 = ro_chunk_end(nodr, i0), ni = i1 - i0;
         int w0 = 0, w1 = 0;

@@ -490,7 +490,7 @@ template <int MTN> static int launch_pass(const TcPassArgs& a, int nsm, cudaStre
     if (nstage > TC_MAXST) nstage = TC_MAXST;
     if (nstage < 2) return -1;
     const size_t smem = 1024 + (size_t)nstage * stg;
-    cudaFuncSetAttribute(tc_pass_kernel<MTN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(tc_pass_kernel<MTN>, smem);
     const long long nunit = 2LL * a.nent;
     const int ntp = (a.nmt + MTN - 1) / MTN;
     int ngroup = nsm / ntp;

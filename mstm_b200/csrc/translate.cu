@@ -288,7 +288,7 @@ template <typename T, int NT, int LM, bool UNI = false> static void launch_trans
 {
     size_t smem = translate_smem_bytes<T>(LM, a.nrhs, a.maxrec);
     auto kern = translate_kernel<T, NT, LM, UNI>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     // as many CTAs per SM as registers and shared memory allow
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, NT, smem) != cudaSuccess) {

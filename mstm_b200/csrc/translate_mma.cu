@@ -939,7 +939,7 @@ template <int LC, int NW, int MINB> int launch_nw(MmaArgs& a, int nsm, cudaStrea
     const size_t smem = work + 8 * (LC ? (size_t)a.maxrec + op_head(LC) : a.recs * (size_t)a.maxrec);
     if (smem > 227 * 1024) return -1;
     auto kern = translate_mma_kernel<LC, NW, MINB>;
-    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    allow_smem(kern, smem);
     int per_sm = (int)((228 * 1024) / (smem + 1024));
     if (per_sm > MINB) per_sm = MINB;
     if (per_sm < 1) per_sm = 1;
