@@ -112,13 +112,15 @@ __host__ __device__ inline void mstm_cspherebessel(int n, zd z, zd* csj, zd* csy
 // could leave the range of a double: |y| above 1e140; h is then partly written).
 // y_k runs forward (it dominates from k = z on); j_k runs forward too while
 // the turning point k = z lies beyond n, else backward from an order m with
-// |y_m| > 1e10 |y_n|, where j_m/j_n < 1e-20, scaled to the larger of j_0 and
-// j_1.  The complex routine finds its start order from log10 estimates, then
+// |y_m| > 1e10 |y_n|, so that j_m/j_n < 1e-10 and what the start at zero leaves
+// in j_n is the product of the two ratios, below 1e-20; scaled to the larger of
+// j_0 and j_1.  The complex routine finds its start order from log10 estimates, then
 // runs two complex divisions a step from m > z, whatever n is: the
 // pair kernel of operator generation went from 69 to 10 us for 190 pairs at
-// n = 14 and from 134 to 19 us for 780 at n = 28.  Largest errors over n <= 32, z from
-// 0.05 to 1000, of the envelope sqrt(j^2 + y^2) for z > k and of j and y
-// below: 3.7e-15 and 3.4e-15 (complex routine: 1.4e-14 and 1.4e-14).
+// n = 14 and from 134 to 19 us for 780 at n = 28.  Largest errors, of the
+// envelope sqrt(j^2 + y^2) for z > k and of j and y below, z from 0.05 to 400:
+// 1.0e-15 and 1.4e-15 for n = 32, 5.7e-15 and 3.4e-15 for n = 216, the largest
+// asked for (complex routine: 5.3e-15 and 4.7e-15, 3.9e-15 and 5.9e-15).
 #define MSTM_REAL_BESSEL_MIN 0.05
 __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
 {
@@ -126,7 +128,10 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
     if (zc.y != 0.0 || !(z >= MSTM_REAL_BESSEL_MIN)) return false;
     double sn, cs;
     sincos(z, &sn, &cs);
-    const double rz = 1.0 / z;
+    // (2 k + 1) / z from 1 / z and what it lacks: the same error of 1 / z in
+    // every step would add up to n / 2 roundings
+    const double rz = 1.0 / z, rl = fma(-rz, z, 1.0) * rz;
+    auto step = [&](int k) { return fma((double)(2 * k + 1), rz, (double)(2 * k + 1) * rl); };
     const double j0 = sn * rz, j1 = (j0 - cs) * rz, y0 = -cs * rz, y1 = (y0 - sn) * rz;
     h[0] = mk(j0, y0);
     if (n < 1) return true;
@@ -134,8 +139,7 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
         double ja = j0, jb = j1, ya = y0, yb = y1;
         h[1] = mk(jb, yb);
         for (int k = 1; k < n; k++) {
-            const double f = (double)(2 * k + 1) * rz;
-            const double jn = f * jb - ja, yn = f * yb - ya;
+            const double f = step(k), jn = fma(f, jb, -ja), yn = fma(f, yb, -ya);
             ja = jb;
             jb = jn;
             ya = yb;
@@ -152,7 +156,7 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
     double lim = 1.0e300;
     if (n == 1) lim = 1.0e10 * fabs(yb);
     while (m < n || fabs(yb) < lim) {
-        const double yn = (double)(2 * m + 1) * rz * yb - ya;
+        const double yn = fma(step(m), yb, -ya);
         ya = yb;
         yb = yn;
         m++;
@@ -163,7 +167,7 @@ __host__ __device__ inline bool mstm_bessel_real(int n, zd zc, zd* h)
     double fa = 0.0, fb = 1.0e-150;   // orders m+1, m
     for (int k = m; k >= 1; k--) {
         if (k <= n) h[k].x = fb;
-        const double fn = (double)(2 * k + 1) * rz * fb - fa;
+        const double fn = fma(step(k), fb, -fa);
         fa = fb;
         fb = fn;
     }
