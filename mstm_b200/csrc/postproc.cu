@@ -126,8 +126,10 @@ __global__ void __launch_bounds__(RC_NT) regular_couplings_kernel(int Tt, int Ls
     const int n = Tt - (int)blockIdx.x, l = Ls - (int)blockIdx.y, VL = Tt + Ls + 1;
     const int nlmin = min(n, l), wmin = abs(n - l), wmax = n + l, nm = 2 * nlmin + 1;
     const int r = threadIdx.x;
-    if (r < nm) vc_func(tab, nlmin - r, n, r - nlmin, l, rc_smem + r * VL);   // vcfunc(-m,n,m,l), m = r - nlmin
-    else if (r == nm) vc_func(tab, -1, n, 1, l, rc_smem + nm * VL);
+    // every axial element is a sum of these, where the reference has most of
+    // them by a recurrence: 0.5 keeps their errors below those it had
+    if (r < nm) vc_func(tab, nlmin - r, n, r - nlmin, l, rc_smem + r * VL, 0.5);   // vcfunc(-m,n,m,l), m = r - nlmin
+    else if (r == nm) vc_func(tab, -1, n, 1, l, rc_smem + nm * VL, 0.5);
     __syncthreads();
     const double c1 = tab.fr(n + n + 1) * tab.fr(l + l + 1);
     const double* v2 = rc_smem + nm * VL;
