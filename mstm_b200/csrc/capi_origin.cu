@@ -53,7 +53,7 @@ static int upload_big(mstmg_ctx* c, BigTablesDev& d)
 // Cluster origin (mean position of the spheres) and the order each sphere
 // needs to reach it (tranordertest, modules:1896-1942, capped at max_t_order);
 // T = max(min(L, max_t_order), those orders)  (input:1179-1197).
-static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps, int max_t_order, double* r0, CallScratch& ws, TmpBuf<int>& dtord,
+static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps, int max_t_order, double* r0, TmpBuf<int>& dtord,
                          std::vector<int>& tord, int* T)
 {
     const int n = c->n;
@@ -67,11 +67,8 @@ static int origin_orders(mstmg_ctx* c, const BigTablesDev& bt, double trans_eps,
             for (int k = 0; k < 3; k++) r0[k] = r0[k] + c->hpos[3 * (size_t)i + k];
         }
     for (int k = 0; k < 3; k++) r0[k] = r0[k] / (double)nout;
-    TmpBuf<zd> tscr(ws);
     CK(dtord.alloc(n));
-    CK(tscr.alloc(tranorder_scratch(n)));
-    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc, bt.fnr, bt.nbc, tscr.p, dtord.p,
-                     c->st);
+    launch_tranorder(n, c->pos.p, c->d_order.p, r0, c->opts.medium_re, trans_eps, max_t_order, bt.bc, bt.fnr, bt.nbc, dtord.p, c->nsm, c->st);
     tord.resize(n);
     CK(cudaMemcpyAsync(tord.data(), dtord.p, sizeof(int) * n, cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -146,7 +143,7 @@ extern "C" int mstmg_scattering(mstmg_ctx* c, const double* amnp, double trans_e
     TmpBuf<int> dtord(ws);
     std::vector<int> tord;
     int T = 0;
-    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, ws, dtord, tord, &T))) return rc;
+    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, dtord, tord, &T))) return rc;
     RegTables rt(ws);
     if ((rc = build_reg_tables(c, bt, T, L, rt))) return rc;
     // merge to the common origin
@@ -272,7 +269,7 @@ extern "C" int mstmg_t_matrix_order(mstmg_ctx* c, double trans_eps, int max_t_or
     double r0[3];
     TmpBuf<int> dtord(ws);
     int T = 0;
-    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, ws, dtord, c->tord, &T))) {
+    if ((rc = origin_orders(c, bt, trans_eps, max_t_order, r0, dtord, c->tord, &T))) {
         c->tord.clear();
         return rc;
     }

@@ -38,18 +38,21 @@ __device__ __forceinline__ zd ipow_z(int k)
 // ---------------------------------------------------------------------------
 // One Bessel evaluation serves all 32 orders, and each lane's coupling row lies
 // in shared memory; with an evaluation per order and rows in global scratch
-// the kernel took 1224 us for 350 spheres; now 47 us.
+// the kernel took 1224 us for 350 spheres; now 47 us.  Arguments the real
+// recurrence leaves to the complex routine have an evaluation per order: each
+// lane in the rest of its coupling row for the first 32 orders, where such
+// arguments meet the criterion, else the lanes in turn with one pair of arrays.
 #define TRANORDER_NLIM 200
 #define TRANORDER_ROW (TRANORDER_NLIM + 31 + MSTMG_LMAX + 2)
 __global__ void __launch_bounds__(32) tranorder_kernel(int nsph, const double* pos, const int* order, double ox, double oy, double oz,
-                                                       double rire, double eps, int maxt, VCTab tab, zd* scratch, int* tord)
+                                                       double rire, double eps, int maxt, VCTab tab, int* tord)
 {
     extern __shared__ __align__(16) unsigned char tr_smem[];
     zd* xs = reinterpret_cast<zd*>(tr_smem);                  // j_l(z) i^l
-    double* vc1 = reinterpret_cast<double*>(xs + TRANORDER_ROW) + threadIdx.x * TRANORDER_ROW;
+    zd* work = xs + TRANORDER_ROW;                            // of the complex routine
+    double* vc1 = reinterpret_cast<double*>(work + TRANORDER_ROW) + threadIdx.x * TRANORDER_ROW;
     __shared__ double terms[32];
     const int lane = threadIdx.x;
-    zd* xi_own = scratch + ((size_t)blockIdx.x * 32 + lane) * 2 * TRANORDER_ROW;   // the complex routine's arrays
     for (int i = blockIdx.x; i < nsph; i += gridDim.x) {
         const int lmax = order[i];
         const double dx = pos[3 * i] - ox, dy = pos[3 * i + 1] - oy, dz = pos[3 * i + 2] - oz;
@@ -70,16 +73,10 @@ __global__ void __launch_bounds__(32) tranorder_kernel(int nsph, const double* p
                     for (int l = lane; l <= min(n0 + 31, TRANORDER_NLIM) + lmax; l += 32) xs[l] = mk(xs[l].x, 0.0) * ipow_z(l);
                 __syncwarp();
                 double term = 0.0;
-                if (n <= TRANORDER_NLIM) {
-                    const zd* xi = xs;
-                    if (!shared_xi) {
-                        mstm_cricbessel(n + lmax, z, xi_own, xi_own + TRANORDER_ROW);
-                        for (int l = 0; l <= n + lmax; l++) xi_own[l] = cdiv(xi_own[l], z) * ipow_z(l);
-                        xi = xi_own;
-                    }
+                if (n <= TRANORDER_NLIM) vc_func(tab, -1, n, 1, lmax, vc1);
+                auto sum_terms = [&](const zd* xi) {
                     const int l = lmax;
                     const zd c = (tab.fr(n + n + 1) * tab.fr(l + l + 1)) * ipow_z(n - l);
-                    vc_func(tab, -1, n, 1, l, vc1);
                     const int wmin = abs(n - l), wmax = n + l;
                     zd a = mk(0.0, 0.0), b = mk(0.0, 0.0);
                     for (int w = wmin; w <= wmax; w++) {
@@ -89,7 +86,25 @@ __global__ void __launch_bounds__(32) tranorder_kernel(int nsph, const double* p
                     }
                     a = c * a;
                     b = c * b;
-                    term = (a * cj(a) + b * cj(b)).x;
+                    return (a * cj(a) + b * cj(b)).x;
+                };
+                auto own_terms = [&](zd* xi, zd* scr) {
+                    mstm_cricbessel(n + lmax, z, xi, scr);
+                    for (int l = 0; l <= n + lmax; l++) xi[l] = cdiv(xi[l], z) * ipow_z(l);
+                    return sum_terms(xi);
+                };
+                constexpr int first = 32 + MSTMG_LMAX + 1;   // values of an order up to 32
+                static_assert(first + 1 + 2 * 2 * first <= TRANORDER_ROW, "a coupling row and two arrays of the first orders");
+                if (shared_xi) {
+                    if (n <= TRANORDER_NLIM) term = sum_terms(xs);
+                } else if (n0 == 1) {
+                    zd* xi = reinterpret_cast<zd*>(vc1 + first + 1);
+                    term = own_terms(xi, xi + first);
+                } else {
+                    for (int q = 0; q < 32; q++) {
+                        if (lane == q && n <= TRANORDER_NLIM) term = own_terms(xs, work);
+                        __syncwarp();
+                    }
                 }
                 terms[lane] = term;
                 __syncwarp();
@@ -731,18 +746,15 @@ __global__ void __launch_bounds__(PS_NT) planesm_kernel(PlaneSmArgs a)
     }
 }
 
-// a warp per sphere, three to an SM (68 KB of shared memory each)
-int tranorder_blocks(int nsph) { return std::max(1, std::min(nsph, 3 * 148)); }
-size_t tranorder_scratch(int nsph) { return (size_t)tranorder_blocks(nsph) * 32 * 2 * TRANORDER_ROW; }
-
 void launch_tranorder(int nsph, const double* pos, const int* order, const double* origin, double rire, double eps, int maxt,
-                      const double* bcof, const double* fnr, int nbc, zd* scratch, int* tord, cudaStream_t st)
+                      const double* bcof, const double* fnr, int nbc, int* tord, int nsm, cudaStream_t st)
 {
     VCTab t{bcof, fnr, nbc};
-    const int smem = (int)(sizeof(zd) * TRANORDER_ROW + sizeof(double) * 32 * TRANORDER_ROW);
+    // a warp per sphere, three to an SM (72 KB of shared memory each)
+    const int smem = (int)(sizeof(zd) * 2 * TRANORDER_ROW + sizeof(double) * 32 * TRANORDER_ROW);
     allow_smem(tranorder_kernel, smem);
-    tranorder_kernel<<<tranorder_blocks(nsph), 32, smem, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire, eps, maxt, t,
-                                                               scratch, tord);
+    tranorder_kernel<<<std::max(1, std::min(nsph, 3 * nsm)), 32, smem, st>>>(nsph, pos, order, origin[0], origin[1], origin[2], rire, eps, maxt,
+                                                                             t, tord);
     launch_counter() += 1;
 }
 

@@ -34,9 +34,8 @@ struct MergeArgs {
     const int* active = nullptr;   // with host spheres: 1 for the spheres merged or distributed to (those outside every other)
 };
 
-size_t tranorder_scratch(int nsph);   // complex values of scratch launch_tranorder needs
 void launch_tranorder(int nsph, const double* pos, const int* order, const double* origin, double rire, double eps, int maxt,
-                      const double* bcof, const double* fnr, int nbc, zd* scratch, int* tord, cudaStream_t st);
+                      const double* bcof, const double* fnr, int nbc, int* tord, int nsm, cudaStream_t st);
 // vcc_const of source orders <= Ls, target orders <= Tt: vcc[(n-1) + Tt ((ml-1) + Ls (Ls+2) w)]
 void launch_regular_couplings(int Tt, int Ls, const double* bcof, const double* fnr, int nbc, double* vcc, cudaStream_t st);
 #define MERGE_PC 16   // columns a CTA of the merge kernel translates together

@@ -44,3 +44,19 @@ def test_operators_take_the_room():
     again = g.ranorientscatmatrix(tm, T)["smat"]   # the workspace comes back
     assert np.abs(again - sm).max() <= 1e-12 * np.abs(sm).max()
     g.close()
+
+
+def test_scattering_matrix_needs_little():
+    """400 spheres of order 3: coefficients, tables and the merge's work take below 64 MB."""
+    import torch
+    from mstm_b200 import api
+    n = 400
+    pos, _ = C.rsa_sphere(n, 1.0, 0.1, seed=n)
+    g = api.SphereCluster(pos * 0.2, np.full(n, 0.2), np.full(n, 1.5 + 0.02j), mie_epsilon=-3.0)
+    h = api.SphereCluster(pos[:4], np.ones(4), np.full(4, 1.5 + 0.02j), mie_epsilon=-3.0)
+    h.scattering(np.ones((h.number_eqns, 2), complex), nangles=5)   # the kernels are loaded
+    before = torch.cuda.mem_get_info()[0]
+    g.scattering(np.ones((g.number_eqns, 2), complex), nangles=5)
+    assert before - torch.cuda.mem_get_info()[0] <= 70e6   # two blocks of 32 MB and some tables
+    g.close()
+    h.close()
