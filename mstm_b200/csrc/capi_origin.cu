@@ -447,7 +447,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
                 G = B64.p;
             }
             launch_tm_qeff(n, S, c->d_order.p, c->d_offset.p, c->d_mie_offset.p, c->rad.p, rimed, c->an_inv.p, Xq, PK.p + (size_t)col0 * ne,
-                           ne, qcol.p, c->st, G, c->hs.on() ? c->hs.d_rext.p : nullptr);
+                           ne, qcol.p, c->nsm, c->st, G, c->hs.on() ? c->hs.d_rext.p : nullptr);
             launch_tm_qsum(n, S, qcol.p, c->rad.p, c->xg, dsq.p, qsum.p, c->st);
             // merge the solutions to the origin: T-matrix columns of order q
             CK(cudaMemsetAsync(A0.p, 0, sizeof(zd) * (size_t)nb * S, c->st));

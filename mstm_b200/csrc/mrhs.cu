@@ -996,10 +996,10 @@ void launch_tm_rhs(int l, zd* P0, cudaStream_t st)
     launch_counter() += 1;
 }
 void launch_tm_qeff(int nsph, int ncols, const int* order, const int* offset, const int* mie_offset, const double* radius, zd rimed,
-                    const zd* an_inv, const zd* A, const zd* P, int ld, double* qcol, cudaStream_t st, const zd* G, const double* rext)
+                    const zd* an_inv, const zd* A, const zd* P, int ld, double* qcol, int nsm, cudaStream_t st, const zd* G, const double* rext)
 {
     // about 8 CTAs an SM: a few columns share a CTA's coefficients
-    int gy = (8 * 148 + nsph - 1) / nsph;
+    int gy = (8 * nsm + nsph - 1) / nsph;
     if (gy > ncols) gy = ncols;
     tm_qeff_kernel<<<dim3(nsph, gy), QEFF_NT, 0, st>>>(nsph, ncols, order, offset, mie_offset, radius, rimed, an_inv, A, P, ld, qcol, G, rext);
     launch_counter() += 1;
