@@ -19,10 +19,11 @@
 // scalar kernels issued one per lane.  Blocks of 1 or 2 x 8 rows and 4-deep
 // products pad the work about twofold (352 MMAs a pair at order 9).
 //
-// What bounds it: the latency of a pair's chain of dependent phases.  Per
-// pair at order 9 the FP64 pipe is busy 1.95k of 2.7k cycles and shared memory
-// about 2k wavefronts, HBM (17 KB of operators) 1.8 TB/s.  Choices that
-// measured (500 spheres of order 9, 2 columns, FP64):
+// What bounds it: the latency of a pair's chain of dependent phases.  Of the
+// 2.7k cycles a pair takes an SM at order 9 the FP64 tensor pipe is busy 50 %,
+// the scalar FP64 pipe 12 %, shared memory 68 %; HBM (17 KB of operators a
+// pair) gives 1.7 TB/s.  Choices that measured (500 spheres of order 9, 2
+// columns, FP64, each against the kernel of its day):
 //   * straight code per warp over units dealt at compile time, few warps a
 //     CTA and several CTAs per SM, against unit loops with index arithmetic
 //     at run time: 6.2k -> 4.2k instructions a pair;
@@ -52,8 +53,8 @@
 // phase B's barrier, before it arms that phase's barriers again, and before it
 // adds a tile to y; it then issues no more copies, makes the step the last one,
 // waits (bounded) for the copies in flight, sets *err to MSTMG_ERR_CUDA and
-// leaves the tile out of y.  (500 spheres of order 9, 2 columns: 1172 -> 1198
-// us, 0 to 2 % of a pass at other orders; a vote of the CTA in its barriers
+// leaves the tile out of y.  (500 spheres of order 9, 2 columns: 1174 -> 1202
+// us, up to 2 % of a pass at other orders; a vote of the CTA in its barriers
 // took 5 %, waits by the copying warp alone 6 %.)
 //
 // Clusters of one order (3 .. 10) have instances with that order and the
@@ -116,12 +117,20 @@ __device__ __forceinline__ int scol(int n, int m, int col) { return col ^ (m & 3
 
 // barrier of the CTA, from the copying warp's code and the others'
 __device__ __forceinline__ void cta_sync() { asm volatile("bar.sync 0;" ::: "memory"); }
-// bounded wait of a whole warp
-__device__ __forceinline__ bool mb_wait_warp(uint64_t* bar, uint32_t parity)
+// bounded wait of a whole warp.  With the first poll before the loop the
+// compiler orders what follows it otherwise: passes of orders up to 6 and of
+// mixed orders are 1 to 5 % faster, those of orders 7 to 10 2 to 4 % slower.
+template <int LC> __device__ __forceinline__ bool mb_wait_warp(uint64_t* bar, uint32_t parity)
 {
-    for (int it = 0; it < WAIT_POLLS; ++it)
-        if (__all_sync(0xffffffffu, mb_try(bar, parity))) return true;
-    return false;
+    if constexpr (LC < 7) {
+        bool in = __all_sync(0xffffffffu, mb_try(bar, parity));
+        for (int it = 1; !in && it < WAIT_POLLS; ++it) in = __all_sync(0xffffffffu, mb_try(bar, parity));
+        return in;
+    } else {
+        for (int it = 0; it < WAIT_POLLS; ++it)
+            if (__all_sync(0xffffffffu, mb_try(bar, parity))) return true;
+        return false;
+    }
 }
 // y[] += shared values, `bytes` long, by one bulk reduction
 __device__ __forceinline__ void bulk_add(void* dst, const void* src, uint32_t bytes)
@@ -448,7 +457,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
             cta_sync();
         }
         const int par = !LC && a.recs == 2 ? (t >> 1) & 1 : t & 1;
-        if (!mb_wait_warp(&bar[rb], par) || (SRC && !mb_wait_warp(&bar[SRC], t & 1))) {
+        if (!mb_wait_warp<LC>(&bar[rb], par) || (SRC && !mb_wait_warp<LC>(&bar[SRC], t & 1))) {
             *gave_up = 1;
             return;
         }
@@ -523,7 +532,7 @@ template <int LC, int NW, int MINB> __global__ void __launch_bounds__((NW + 1) *
                 });
             }
             cta_sync();
-            if (!mb_wait_warp(&bar[1 + b], (t >> 1) & 1)) {
+            if (!mb_wait_warp<LC>(&bar[1 + b], (t >> 1) & 1)) {
                 *gave_up = 1;
                 return;
             }
@@ -955,9 +964,10 @@ template <int LC, int NW, int MINB> int launch_nw(MmaArgs& a, int nsm, cudaStrea
 }  // namespace
 
 // Warps a CTA and CTAs per SM by order, the fastest of 2 to 8 warps and the
-// CTAs that fit (us, 2 columns FP64; spheres x order: 1200 x 4 1831, 1000 x 5
-// 1700, 700 x 6 1160, 700 x 7 1353, 500 x 8 887, 500 x 9 1172, 300 x 10 659;
-// e.g. order 9 at 4 warps x 3 CTAs 1389, 8 x 2 2160; order 5 at 4 x 4 2030).
+// CTAs that fit (us, 2 columns FP64; spheres x order: 1200 x 4 1840, 1000 x 5
+// 1737, 700 x 6 1182, 700 x 7 1356, 500 x 8 889, 500 x 9 1202, 300 x 10 635;
+// when they were chosen order 9 took 1172, at 4 warps x 3 CTAs 1389, at 8 x 2
+// 2160; order 5 1700, at 4 x 4 2030).
 int launch_translate_mma(MmaArgs& a, int nsm, cudaStream_t st)
 {
     if (a.uniform) {
