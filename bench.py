@@ -46,7 +46,7 @@ sys.path.insert(0, ROOT)
 EPS = 1.0e-12          # squared-norm criterion: ||r||/||b|| < 1e-6
 # DRAM bytes per byte of records and vectors of the translation pass of 2
 # columns, from the ncu capture of the 200-sphere aggregate (343.5 MB of 338.8 MB)
-TRAFFIC_PER_ALG_BYTE = 343.5 / 338.8
+TRAFFIC_PER_ALG_BYTE = 343.7 / 338.8
 NITER = 10000
 WORKLOAD = "fractal500"
 METRIC = "solves/s at 1e-6 residual (fractal aggregate N=500, x=2, both polarisations)"
@@ -89,7 +89,7 @@ def bench_config(ws):
                         "L=9, +z incidence, both polarisations",
             "neqns": 99000, "pairs": 124750, "residual": "||r||/||b|| < 1e-6 (squared-norm eps 1e-12)",
             "parallelism": "replicas" if ws > 1 else "single GPU",
-            "l2": "operators (2 GB FP64 / 1 GB FP32) exceed the 126 MB L2; no flush needed"}
+            "l2": "operators (2.1 GB) exceed the 126 MB L2; no flush needed"}
 
 
 def oracle_fixture(name):
@@ -569,24 +569,21 @@ def report_line(args, ws, R, ne):
     plain = job_value(ws, args.steps, p["ms_total"])
     # dominant kernel: the FP32 translation pass of the tuned path
     ms32, n32 = m["k32"]
-    stored32, canon32 = m["bytes32"]   # record bytes the pass reads (FP64), and the reference layout's bytes at 4 B per real
-    folded32 = stored32
-    # algorithmic bytes per launch, as the canonical matvec bytes define them
-    # (the reference layout's stored operator at 4 B per real, read once, +
-    # x read + y written; one column per active polarisation: the tuned
-    # path's Arnoldi passes carry 2 columns while both polarisations are
-    # active, iterations count Arnoldi steps in pairs).  The kernel itself
-    # reads the operator folded by the Wigner and axial symmetries, in FP64
-    # records (stored32), which is its DRAM traffic; the same pass against
-    # those bytes is reported beside.
+    # what the pass reads and writes: the operator folded by the Wigner and
+    # axial symmetries, in FP64 records, and FP64 copies of its columns (one per
+    # active polarisation: the tuned path's Arnoldi passes carry 2 while both
+    # are active, iterations count Arnoldi steps in pairs).  Beside it the
+    # canonical matvec bytes: the reference layout's operator at 4 B per real
+    # and the FP32 columns, each once.
+    records, canon32 = m["bytes32"]
     it = m["stats"]["iterations"]
     n32p = max(1, m["stats"]["passes32"])
     avg_cols = min(2.0, 2.0 * sum(it) / n32p) if sum(it) > 0 else 2.0
-    vec_bytes = 2.0 * ne * 8 * avg_cols
-    alg = canon32 + vec_bytes
+    pass_bytes = records + 2.0 * ne * 16 * avg_cols
+    canonical = canon32 + 2.0 * ne * 8 * avg_cols
     dur = ms32 / max(1, n32)
-    achieved = alg / (dur * 1e-3) / 1e9 if n32 else None
-    folded_gbs = (folded32 + vec_bytes) / (dur * 1e-3) / 1e9 if n32 else None
+    achieved = pass_bytes / (dur * 1e-3) / 1e9 if n32 else None
+    canonical_gbs = canonical / (dur * 1e-3) / 1e9 if n32 else None
     ms64, n64 = p["k64"]
     stored64, _ = p["bytes64"]
     dur64 = ms64 / max(1, n64)
@@ -613,23 +610,23 @@ def report_line(args, ws, R, ne):
         "tuned": {"iterations": it, "outer": m["stats"]["outer"], "passes64": m["stats"]["passes64"],
                   "passes32": m["stats"]["passes32"], "qext": m["qtot"][0, 0], "qext_plain": p["qtot"][0, 0],
                   "qext_rel_diff": abs(m["qtot"][0, 0] / p["qtot"][0, 0] - 1)},
-        "roofline": {"kernel": "translate_mma_kernel<9, 3, 4> (pair translation pass of FP32 columns, FP64 tensor cores)", "bound": "hbm",
+        "roofline": {"kernel": "translate_mma_kernel<9, 3, 4> (pair translation pass of FP32 columns, FP64 tensor cores)",
+                     "bound": "latency of a pair's phases",
                      "achieved": round(achieved, 1) if achieved else None, "peak": hbm, "unit": "GB/s",
                      "frac": round(achieved / hbm, 4) if achieved else None,
-                     "traffic": round(TRAFFIC_PER_ALG_BYTE * (stored32 + vec_bytes)),
-                     "record_bytes": stored32,
+                     "traffic": round(TRAFFIC_PER_ALG_BYTE * pass_bytes),
+                     "record_bytes": records,
                      "traffic_source": "ncu dram__bytes_read+write of this kernel on the 200-sphere aggregate "
                                        "(profiles/translate_mma_aggregate200.md: 1.01x the FP64 records and vectors "
                                        "read and written), scaled to this workload's records",
                      "peak_source": peak_src,
-                     "algorithmic_bytes_per_launch": alg,
-                     "algorithmic_bytes_source": "canonical matvec bytes (reference operator layout at 4 B per real, "
-                                                 "read once, + x and y): the kernel reads the symmetry-folded operator, "
-                                                 "so its traffic is below this",
+                     "algorithmic_bytes_per_launch": pass_bytes,
+                     "algorithmic_bytes_source": "folded FP64 operator records and FP64 columns, each read or written once",
                      "launch_ms": round(dur, 4), "launches": n32,
-                     "folded_bytes_per_launch": folded32 + vec_bytes,
-                     "folded_gbs": round(folded_gbs, 1) if folded_gbs else None,
-                     "frac_of_folded_bytes": round(folded_gbs / hbm, 4) if folded_gbs else None},
+                     "canonical_bytes_per_launch": canonical,
+                     "canonical_bytes_source": "reference operator layout at 4 B per real, read once, + FP32 x and y",
+                     "canonical_gbs": round(canonical_gbs, 1) if canonical_gbs else None,
+                     "frac_of_canonical_bytes": round(canonical_gbs / hbm, 4) if canonical_gbs else None},
         "e2e": {"value": round(ws * 1000.0 * args.steps / e2e["ms"], 4), "unit": "solves/s",
                 "h2d_bytes_per_step": e2e["h2d"], "d2h_bytes_per_step": e2e["d2h"]},
         "gpu_launches": int(m["launches"]),
@@ -766,11 +763,11 @@ def run_translation_case(args):
         w = C.workload(args.workload)
     prec = "mixed" if args.precision == "tc" else args.precision
     g = api.SphereCluster(w["pos"], w["radius"], w["ref_index"], mie_epsilon=-w["order"], precision=prec,
-                          fp32_chunk=args.fp32_chunk, tile_ctas_per_sm=args.ctas_per_sm, tile_pairs=args.tile_pairs)
+                          tile_ctas_per_sm=args.ctas_per_sm)
     ms = g.time_translation(args.precision, args.nrhs, args.translation_passes)
     sb, cb = g.operator_bytes(prec)
-    print(json.dumps({"workload": args.workload, "precision": args.precision, "nrhs": args.nrhs, "fp32_chunk": args.fp32_chunk,
-                      "ctas_per_sm": args.ctas_per_sm, "tile_pairs": args.tile_pairs, "ms_per_pass": ms, "operator_bytes": sb, "operator_gbs": sb / ms / 1e6}))
+    print(json.dumps({"workload": args.workload, "precision": args.precision, "nrhs": args.nrhs,
+                      "ctas_per_sm": args.ctas_per_sm, "ms_per_pass": ms, "operator_bytes": sb, "operator_gbs": sb / ms / 1e6}))
     g.close()
 
 
@@ -809,9 +806,7 @@ def main():
                     help="profiling case: only run this many translation passes (no solve)")
     ap.add_argument("--workload", default=WORKLOAD)
     ap.add_argument("--precision", default="mixed", choices=["mixed", "fp64", "tc"])
-    ap.add_argument("--fp32-chunk", type=int, default=0, help="profiling case: FP32 column chunk (2 or 4; 0 default)")
     ap.add_argument("--ctas-per-sm", type=int, default=0, help="profiling case: most CTAs per SM of the pair kernel (0: as many as fit)")
-    ap.add_argument("--tile-pairs", type=int, default=0, help="accepted without effect")
     ap.add_argument("--nrhs", type=int, default=4)
     ap.add_argument("--tmatrix-case", type=int, default=0, help="profiling case: one T matrix of this many spheres")
     ap.add_argument("--tensor-core", type=int, default=0, help="profiling case: 0 tensor-core passes where they apply, -1 never")
