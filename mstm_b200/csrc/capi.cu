@@ -1041,9 +1041,6 @@ extern "C" int mstmg_kernel_time_tc(mstmg_ctx* c, double* ms, int* n)
 
 extern "C" long long mstmg_kernel_launches(void) { return launch_counter().load(); }
 
-// One translation pass over nrhs columns laid out as BiCG packs them
-// ([p, A^T conj w] pairs, odd columns conjugate-transpose products), timed with
-// CUDA events on the context's stream (mean of reps after one warm-up).
 extern "C" int mstmg_selftest_bounded_wait(int device, int limit, int* status)
 {
     if (!status || limit < 1 || limit > (1 << 22)) {

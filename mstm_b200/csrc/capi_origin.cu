@@ -359,7 +359,7 @@ extern "C" int mstmg_tmatrix(mstmg_ctx* c, int t_matrix_order, double solution_e
     if ((rc = w64.init(Smax, ne, c->nsm, !mixed))) return rc;
     GmresWork& gw = c->tm_gm;
     if (mixed && c->opts.mixed_solver == 2 && !(gw.hh && gw.ne == ne && gw.S >= Smax) &&
-        (rc = gw.setup(Smax, ne, c->opts.gmres_restart, "mstmg_tmatrix")))
+        (rc = gw.setup(Smax, ne, c->opts.gmres_restart, "mstmg_tmatrix", [] { return false; })))   // what is kept is in use
         return rc;
     if (mixed) {
         CK(X64.alloc((size_t)ne * Smax));

@@ -57,8 +57,12 @@ int ensure_ops_both(mstmg_ctx* c, bool want64, bool want32, bool force)
     if (c->npairs == 0 || !(want64 || want32) || (c->rot_ready && !force)) return MSTMG_OK;
     {
         const void* was = c->op64.p;
-        if (c->op64.n < (size_t)c->op_units) c->make_room(sizeof(double) * (size_t)c->op_units);
-        CK(c->op64.alloc(c->op_units));
+        cudaError_t e = c->op64.alloc(c->op_units);
+        if (e != cudaSuccess && c->give_back()) {
+            cudaGetLastError();
+            e = c->op64.alloc(c->op_units);
+        }
+        CK(e);
         if (was != c->op64.p) c->layout_gen++;
     }
     NvtxRange nvtx_("pair operator generation");
@@ -335,9 +339,9 @@ int ensure_tc(mstmg_ctx* c)
     }
     rstart[c->n] = (int)rsrc.size();
     const size_t need = ent.size() * tc_himg_floats(g) * sizeof(float);
-    c->make_room(3 * need);
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
+    if (need > fr / 3 && c->give_back()) CK(cudaMemGetInfo(&fr, &tot));
     if (need > fr / 3) {
         c->tc_state = -1;
         set_err("tensor-core operator images (" + std::to_string(need >> 20) + " MiB) exceed a third of the free device memory");

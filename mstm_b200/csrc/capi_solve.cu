@@ -450,8 +450,8 @@ static int fixed_orientation_impl(mstmg_ctx* c, double alpha, double sinc, int d
         } else if (c->opts.mixed_solver == 2) {
             // both polarisations as two systems of the restarted GMRES
             if (!c->fo_gm_ready) {
-                c->make_room(GmresWork::room(2, ne, c->opts.gmres_restart));
-                if ((rc = c->fo64.init(2, ne, c->nsm, false)) || (rc = c->fo_gm.setup(2, ne, c->opts.gmres_restart, "mstmg_fixed_orientation")))
+                if ((rc = c->fo64.init(2, ne, c->nsm, false)) ||
+                    (rc = c->fo_gm.setup(2, ne, c->opts.gmres_restart, "mstmg_fixed_orientation", [&] { return c->give_back(); })))
                     return rc;
                 c->fo_gm_ready = true;
             }
@@ -549,8 +549,8 @@ extern "C" int mstmg_ensemble_fixed_orientation(mstmg_ctx* c, double alpha, doub
         mie_all(c, 1, 0, c->pmnp.p + (size_t)p * ne, bvec + (size_t)p * ne);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(c->amnp.p, bvec, sizeof(zd) * 2 * (size_t)ne, cudaMemcpyDeviceToDevice, c->st));
-    if (!c->ens_gm.hh) c->make_room(GmresWork::room(S, c->ens_ldv, c->opts.gmres_restart));
-    if (!c->ens_gm.hh && (rc = c->ens_gm.setup(S, c->ens_ldv, c->opts.gmres_restart, "mstmg_ensemble_fixed_orientation"))) return rc;
+    if (!c->ens_gm.hh && (rc = c->ens_gm.setup(S, c->ens_ldv, c->opts.gmres_restart, "mstmg_ensemble_fixed_orientation", [&] { return c->give_back(); })))
+        return rc;
     const EnsSeg seg{c->ens_off.p, c->ens_len.p, c->ens_ldv};
     std::vector<int> its, sts;
     std::vector<double> ers;

@@ -82,8 +82,8 @@ template <typename T> struct DevBuf {
 // buffers: 3.3 ms of a 5.4 ms scattering call, 11.6 ms of a 111 ms T matrix.
 // One call at a time has the blocks; one that finds them taken by another
 // thread works in blocks of its own.  Where device memory is short the idle
-// ones go: before an allocation here fails, and before the context judges what
-// room there is for operators, images or a basis (mstmg_ctx::make_room).
+// ones go: before an allocation here or of the operators fails, and before
+// images or a basis turn out smaller for want of room (mstmg_ctx::give_back).
 #define CALL_POOL_MAX ((size_t)1 << 30)
 #define CALL_POOL_BLOCK ((size_t)32 << 20)
 struct CallPool {
@@ -342,7 +342,6 @@ struct GmresWork {
     // basis length from the free device memory: at most `cap` vectors a
     // system (200 when cap is 0), the basis within a quarter of the free memory
     static int max_m(int cap) { return cap > 0 ? cap : 200; }
-    static size_t room(int S, int ne, int cap) { return 4 * sizeof(zf) * (size_t)S * ne * (max_m(cap) + 1); }   // for the longest
     static int pick_m(int S, int ne, int cap)
     {
         const int mmax = max_m(cap);
@@ -353,11 +352,13 @@ struct GmresWork {
         return (int)std::min<size_t>(mmax, fit > 1 ? fit - 1 : 0);
     }
     // allocate for S systems of ne elements with the basis length pick_m
-    // allows (an error when it is below 8 steps, or below the cap when smaller)
-    int setup(int S_, int ne_, int cap, const char* who)
+    // allows (an error when it is below 8 steps, or below the cap when smaller);
+    // more(): whether there is more memory now, asked when the length is not the longest
+    template <typename F> int setup(int S_, int ne_, int cap, const char* who, F&& more)
     {
         V.release();   // the old basis does not count against the new one's memory
-        const int m_ = pick_m(S_, ne_, cap);
+        int m_ = pick_m(S_, ne_, cap);
+        if (m_ < max_m(cap) && more()) m_ = pick_m(S_, ne_, cap);
         if (m_ < (cap > 0 ? std::min(cap, 8) : 8)) {
             set_err(std::string(who) + ": no device memory for the GMRES basis");
             return MSTMG_ERR_CUDA;
@@ -498,15 +499,15 @@ struct mstmg_ctx {
     GmresWork tm_gm;   // mixed_solver 2, T-matrix columns: kept across calls (sized for the largest order)
     CallPool pool;
     MultiWork<double> tm64;   // FP64 work of the T-matrix columns, kept likewise while below CALL_POOL_MAX; the call that has the pool has it
-    // Free what is kept between calls, where the device has not `need` bytes
-    // to spare and no call is using it
-    void make_room(size_t need)
+    // Free what is kept between calls, unless a call is using it: whether there was any
+    bool give_back()
     {
-        size_t fr = 0, tot = 0;
-        if (cudaMemGetInfo(&fr, &tot) != cudaSuccess || fr >= need || pool.taken.exchange(true)) return;
+        if (pool.taken.exchange(true)) return false;
+        const bool any = !pool.blocks.empty() || tm64.bytes() > 0;
         pool.clear();
         tm64.release();
         pool.taken = false;
+        return any;
     }
     // the reference's constant tables on the device: bcof, square roots, bcof(n, n)
     std::mutex big_mu;
