@@ -23,7 +23,7 @@ Arms:
                      criterion).
 
 Timing: CUDA events on the stream the library launches on, W untimed warm-up
-solves, K timed solves; operators (2 GB FP64 + 1 GB FP32) exceed the 126 MB L2,
+solves, K timed solves; operators (2.1 GB) exceed the 126 MB L2,
 so every pass streams from HBM.  Under torchrun each rank solves its own
 configuration (replicas, no data-path collective) and rank 0 reports the
 maximum time over ranks.
@@ -45,7 +45,7 @@ sys.path.insert(0, ROOT)
 
 EPS = 1.0e-12          # squared-norm criterion: ||r||/||b|| < 1e-6
 # DRAM bytes per byte of records and vectors of the translation pass of 2
-# columns, from the ncu capture of the 200-sphere aggregate (343.5 MB of 338.8 MB)
+# columns, from the ncu capture of the 200-sphere aggregate (343.7 MB of 338.8 MB)
 TRAFFIC_PER_ALG_BYTE = 343.7 / 338.8
 NITER = 10000
 WORKLOAD = "fractal500"
